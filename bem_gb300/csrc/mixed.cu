@@ -41,7 +41,10 @@ constexpr int FIRST_SLICES = 2;  // slices of the complex64 path's first iterate
 constexpr int TRACE_SLICES = 4;  // slices of X in the full trace products H1 X, H2 X^H (10 products):
                                  // ~2^-33 of |H||X| per entry; the trace of a product of two
                                  // absorption (semi-definite) operators does not cancel, so S keeps
-                                 // ~1e-9 (measured 4e-10 against 5 slices at N = 7680)
+                                 // ~1e-9 (measured 4e-10 against 5 slices at N = 7680).  The FP64-class
+                                 // solve, whose W is ill-conditioned and whose X is large where H is
+                                 // small, takes MIXED_SLICES: a tip 40 nm over a plate at N = 5688 is
+                                 // 1e-8 from the FP64 path with them and 1e-6 with four
 
 __global__ void c128_to_c64_kernel(const double *__restrict__ S, int64_t lds, float *__restrict__ D, int64_t ldd, int m,
                                    int n) {
@@ -224,13 +227,13 @@ float ev_ms(cudaEvent_t a, cudaEvent_t b) {
   return ms;
 }
 
-// S from B1 = H1 X and C = H2 X^H.  incremental: X moved by the correction
-// dY of the last step, so B1 += H1 dX and C += H2 dX^H (3-slice products of
-// the small correction) instead of the full 5-slice products.
+// S from B1 = H1 X and C = H2 X^H, X in `slices` slices.  incremental: X moved
+// by the correction dY of the last step, so B1 += H1 dX and C += H2 dX^H
+// (3-slice products of the small correction) instead of the full products.
 int spectral_trace(bemgpu_ctx_s *ctx, MixedBufs &b, int n, int ns2, int nt2, cudaStream_t st, double S[2],
-                   bool incremental) {
+                   bool incremental, int slices) {
   const double *X = incremental ? b.dY : b.Y;  // rows [0, ns2), leading dimension n
-  const int sl = incremental ? DELTA_SLICES : TRACE_SLICES;
+  const int sl = incremental ? DELTA_SLICES : slices;
   const int acc = incremental ? 1 : 0;
   ExactOperand opX, opXH;
   int rc = bem_exact_prep(ctx, "X", false, X, n, nt2, ns2, 1.0, sl, opX, st);
@@ -306,7 +309,7 @@ int fp64lu_solve(bemgpu_ctx_s *ctx, double *W, int n, int ns2, MixedBufs &b, cud
   rc = bem_zgetrs_exact(ctx, W, n, n, b.ipiv, b.Y, n, nt2, st);
   if (rc) return rc;
   double Sprev[2] = {0, 0};
-  rc = spectral_trace(ctx, b, n, ns2, nt2, st, S, false);
+  rc = spectral_trace(ctx, b, n, ns2, nt2, st, S, false, MIXED_SLICES);
   if (rc) return rc;
   err = 1.0;
   double err_prev = 1.0;
@@ -337,7 +340,7 @@ int fp64lu_solve(bemgpu_ctx_s *ctx, double *W, int n, int ns2, MixedBufs &b, cud
     const bool small = correction_is_small(ctx, opDY, eb_y, st);
     Sprev[0] = S[0];
     Sprev[1] = S[1];
-    rc = spectral_trace(ctx, b, n, ns2, nt2, st, S, small);
+    rc = spectral_trace(ctx, b, n, ns2, nt2, st, S, small, MIXED_SLICES);
     if (rc) return rc;
     if (bem_tc_error(ctx, true))
       return bem_fail(ctx, BEMGPU_ERR_TIMEOUT, "FP64-class solve: a tensor-core pipeline wait ran out");
@@ -498,7 +501,7 @@ int bem_mixed_solve(bemgpu_ctx_s *ctx, double *W, int n, int ns2, const double *
     iters++;
     Sprev[0] = S[0];
     Sprev[1] = S[1];
-    rc = spectral_trace(ctx, b, n, ns2, nt2, st, S, iters > 1 && small);
+    rc = spectral_trace(ctx, b, n, ns2, nt2, st, S, iters > 1 && small, TRACE_SLICES);
     if (rc) return rc;
     if (bem_tc_error(ctx, true))
       return bem_fail(ctx, BEMGPU_ERR_TIMEOUT, "mixed solve: a tensor-core pipeline wait ran out");
