@@ -42,7 +42,7 @@ struct TriRec {
   int nh;             // number of half-RWGs on this triangle in this tree (1..3)
   int hrwg[3];        // RWG index (row/column pair of the matrix)
   int hneg[3];        // 0 for the positive half, 1 for the negative half
-  int pad;
+  int hvert;          // bits 2h, 2h+1: the frame vertex (0, 1, 2) that is half h's free vertex
 };
 
 // A (test, source) near pair: shares at least one vertex, or is the same triangle.
@@ -63,6 +63,10 @@ struct bemgpu_tree_s {
   std::vector<int> tri_gid;     // local triangle -> geometry triangle id
   std::vector<TriRec> host_rec;
   TriRec *d_rec = nullptr;
+  double emax = 0.0;            // longest triangle edge
+  void set_emax() {
+    for (const TriRec &r : host_rec) emax = emax < r.emax ? r.emax : emax;
+  }
 };
 
 struct NearList {

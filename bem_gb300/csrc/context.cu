@@ -501,7 +501,7 @@ int bemgpu_tree_create(bemgpu_geom_t g, const int *rwg, int nrwg, bemgpu_tree_t 
   t->geom = g;
   t->nrwg = nrwg;
   t->rwg.assign(rwg, rwg + 4 * (size_t)nrwg);
-  std::vector<int> local(g->nt, -1);
+  std::vector<int> local(g->nt, -1), rot0;  // rot0: the frame's first vertex, per local triangle
   // TriangleRWGMap construction order (src/Impedance.cpp:397-406)
   for (int i = 0; i < nrwg; i++) {
     int tp = rwg[4 * i], tn = rwg[4 * i + 1], e1 = rwg[4 * i + 2], e2 = rwg[4 * i + 3];
@@ -537,6 +537,8 @@ int bemgpu_tree_create(bemgpu_geom_t g, const int *rwg, int nrwg, bemgpu_tree_t 
       int rot = (tv[0] != e1 && tv[0] != e2) ? 0 : ((tv[1] != e1 && tv[1] != e2) ? 1 : 2);
       V3 p0 = vtx(g, tv[rot]), p1 = vtx(g, tv[(rot + 1) % 3]), p2 = vtx(g, tv[(rot + 2) % 3]);
       int h = r.nh++;
+      if (h == 0) rot0.push_back(rot);
+      r.hvert |= ((rot - rot0[local[tr]] + 3) % 3) << (2 * h);
       put(r.hp0[h], p0);
       r.helen[h] = std::sqrt(norm2(sub(vtx(g, e2), vtx(g, e1))));  // Edge::length
       r.hrwg[h] = i;
@@ -571,6 +573,7 @@ int bemgpu_tree_create(bemgpu_geom_t g, const int *rwg, int nrwg, bemgpu_tree_t 
       delete t;
       return bem_fail(ctx, BEMGPU_ERR_MESH, "tree_create: degenerate triangle %d", r.gid);
     }
+  t->set_emax();
   cudaSetDevice(ctx->device);
   if (cudaMalloc(&t->d_rec, sizeof(TriRec) * t->ntri) != cudaSuccess) {
     cudaGetLastError();

@@ -7,8 +7,15 @@
 //     transformations;
 //   * the "sloppy" df addition of Dekker / Bailey's double-double libraries
 //     (error ~2^-47 of |a| + |b|) and the FMA-based df product;
-//   * square root and reciprocal by one Newton step from the FP32 value
+//   * square root and reciprocal from the FP32 approximation: one Newton step
+//     in FP32 to a value accurate to its last bit, one more for the low part
 //     (Karp-Markstein form);
+//   * sums of products in unnormalized accumulators (the compensated dot
+//     product of Ogita, Rump and Oishi): 12 FP32 operations a term against 18
+//     of a df product and a df addition, the same rounding behaviour over the
+//     ~100 terms of a quadrature rule;
+//   * polynomials by a Horner step that knows |c| >= |p s|: 9 operations
+//     against 18;
 //   * sin, cos on [-pi/4, pi/4] and exp on [-ln2/2, ln2/2] by their Taylor
 //     series (argument reduction by Cody-Waite in FP64 by the caller), the
 //     high-order terms in FP32 where they are below 2^-25 of the result.
@@ -74,20 +81,90 @@ __device__ __forceinline__ df df_sqr(df a) {
 // a * 2^k for a float power of two p2 (exact)
 __device__ __forceinline__ df df_scale2(df a, float p2) { return {a.hi * p2, a.lo * p2}; }
 
-// sqrt(a), a > 0: s = a.hi * r (r ~ 1/sqrt(a.hi)), then s + (a - s^2) r / 2.
+// sqrt(a), a > 0: s = a.hi * r (r ~ 1/sqrt(a.hi)) refined to FP32 accuracy,
+// then the low part from a - s^2.
 __device__ __forceinline__ df df_sqrt(df a) {
-  const float r = rsqrtf(a.hi);
+  const float r = rsqrtf(a.hi), h = 0.5f * r;
   const float s = a.hi * r;
-  const df s2 = df_sqr({s, 0.f});
-  const df d = df_sub(a, s2);  // small: a - s^2
-  return fast_two_sum(s, 0.5f * d.hi * r);
+  const float s1 = fmaf(h, fmaf(-s, s, a.hi), s);
+  const float e = fmaf(-s1, s1, a.hi) + a.lo;
+  return fast_two_sum(s1, h * e);
 }
 // 1 / a: r = 1/a.hi, then r + r (1 - a r).
 __device__ __forceinline__ df df_rcp(df a) {
   const float r = __frcp_rn(a.hi);
-  const df ar = df_mul_f(a, r);
-  const df e = df_add_f(df_neg(ar), 1.f);  // 1 - a r, small
-  return fast_two_sum(r, r * e.hi);
+  const float e = fmaf(-a.lo, r, fmaf(-a.hi, r, 1.f));
+  return fast_two_sum(r, r * e);
+}
+// R = sqrt(a) and 1/R at once, from one FP32 reciprocal square root.
+__device__ __forceinline__ void df_sqrt_rcp(df a, df &R, df &Ri) {
+  const float r = rsqrtf(a.hi), h = 0.5f * r;
+  const float s = a.hi * r;
+  const float s1 = fmaf(h, fmaf(-s, s, a.hi), s);
+  const float e = fmaf(-s1, s1, a.hi) + a.lo;
+  R = fast_two_sum(s1, h * e);
+  const float r1 = fmaf(r, fmaf(-R.hi, r, 1.f), r);
+  const float d = fmaf(-R.lo, r1, fmaf(-R.hi, r1, 1.f));
+  Ri = fast_two_sum(r1, r1 * d);
+}
+
+// a - b without the final normalization: the low part may exceed half an ulp
+// of a high part that cancelled, which products of the difference tolerate.
+__device__ __forceinline__ df df_diff(df a, df b) {
+  const float s = a.hi - b.hi, t = s - a.hi;
+  return {s, ((a.hi - (s - t)) - (b.hi + t)) + (a.lo - b.lo)};
+}
+// x^2 + y^2 + z^2 of unnormalized differences.
+__device__ __forceinline__ df df_sumsq(df x, df y, df z) {
+  const float px = x.hi * x.hi, py = y.hi * y.hi, pz = z.hi * z.hi;
+  const float ex = fmaf(x.hi + x.hi, x.lo, fmaf(x.hi, x.hi, -px));
+  const float ey = fmaf(y.hi + y.hi, y.lo, fmaf(y.hi, y.hi, -py));
+  const float ez = fmaf(z.hi + z.hi, z.lo, fmaf(z.hi, z.hi, -pz));
+  const df s = two_sum(px, py), t = two_sum(s.hi, pz);
+  return fast_two_sum(t.hi, (s.lo + t.lo) + (ex + (ey + ez)));
+}
+// acc += x y, acc unnormalized (df_fin normalizes it).
+__device__ __forceinline__ void df_mac(df &acc, df x, df y) {
+  const float p = x.hi * y.hi;
+  float e = fmaf(x.hi, y.hi, -p);
+  e = fmaf(x.hi, y.lo, e);
+  e = fmaf(x.lo, y.hi, e);
+  const df s = two_sum(acc.hi, p);
+  acc.hi = s.hi;
+  acc.lo += s.lo + e;
+}
+__device__ __forceinline__ df df_fin(df a) { return fast_two_sum(a.hi, a.lo); }
+// c + p s, |c.hi| >= |p s|: a Horner step; the result is unnormalized (its low
+// part within about an ulp of the high one).
+__device__ __forceinline__ df df_horner(df p, df s, df c) {
+  const float m = p.hi * s.hi;
+  float e = fmaf(p.hi, s.hi, -m);
+  e = fmaf(p.hi, s.lo, e);
+  e = fmaf(p.lo, s.hi, e);
+  const float h = c.hi + m;
+  return {h, (m - (h - c.hi)) + (e + c.lo)};
+}
+// The same with an FP32 p (the first step after an FP32 tail).
+__device__ __forceinline__ df df_horner_f(float p, df s, df c) {
+  const float m = p * s.hi;
+  const float e = fmaf(p, s.lo, fmaf(p, s.hi, -m));
+  const float h = c.hi + m;
+  return {h, (m - (h - c.hi)) + (e + c.lo)};
+}
+// a b + c d.
+__device__ __forceinline__ df df_dot2(df a, df b, df c, df d) {
+  const float p = a.hi * b.hi, q = c.hi * d.hi;
+  const float e = fmaf(a.lo, b.hi, fmaf(a.hi, b.lo, fmaf(a.hi, b.hi, -p)));
+  const float f = fmaf(c.lo, d.hi, fmaf(c.hi, d.lo, fmaf(c.hi, d.hi, -q)));
+  const df s = two_sum(p, q);
+  return fast_two_sum(s.hi, s.lo + (e + f));
+}
+// a b + c.
+__device__ __forceinline__ df df_muladd(df a, df b, df c) {
+  const float p = a.hi * b.hi;
+  const float e = fmaf(a.lo, b.hi, fmaf(a.hi, b.lo, fmaf(a.hi, b.hi, -p)));
+  const df s = two_sum(p, c.hi);
+  return fast_two_sum(s.hi, s.lo + (e + c.lo));
 }
 
 // Taylor coefficient 1/n! as df (exact values from df_constants.h).
@@ -108,23 +185,19 @@ __device__ __forceinline__ void df_sincos_reduced(df r, df &sn, df &cs) {
   tc = fmaf(tc, sf, inv_fact(14).hi);
   tc = fmaf(tc, sf, -inv_fact(12).hi);
   // df Horner for the leading terms
-  df ps = {ts, 0.f};
-  ps = df_add(df_mul(ps, s), df_neg(inv_fact(9)));
-  ps = df_add(df_mul(ps, s), inv_fact(7));
-  ps = df_add(df_mul(ps, s), df_neg(inv_fact(5)));
-  ps = df_add(df_mul(ps, s), inv_fact(3));
-  // sin = r - r s (1/3! - s (1/5! - ...)) : ps now holds -(coefficient series of r^3 term)/...
-  // ps = -1/3! + s/5! - ... is the series of (sin r - r)/(r^3) with the sign folded:
-  ps = df_neg(ps);
-  sn = df_add(r, df_mul(df_mul(ps, s), r));
-  df pc = {tc, 0.f};
-  pc = df_add(df_mul(pc, s), inv_fact(10));
-  pc = df_add(df_mul(pc, s), df_neg(inv_fact(8)));
-  pc = df_add(df_mul(pc, s), inv_fact(6));
-  pc = df_add(df_mul(pc, s), df_neg(inv_fact(4)));
-  pc = df_add(df_mul(pc, s), inv_fact(2));
+  df ps = df_horner_f(ts, s, df_neg(inv_fact(9)));
+  ps = df_horner(ps, s, inv_fact(7));
+  ps = df_horner(ps, s, df_neg(inv_fact(5)));
+  ps = df_horner(ps, s, inv_fact(3));
+  // ps = 1/3! - s/5! + ...: sin = r - r s ps
+  sn = df_fin(df_horner(df_neg(ps), df_mul(r, s), r));
+  df pc = df_horner_f(tc, s, inv_fact(10));
+  pc = df_horner(pc, s, df_neg(inv_fact(8)));
+  pc = df_horner(pc, s, inv_fact(6));
+  pc = df_horner(pc, s, df_neg(inv_fact(4)));
+  pc = df_horner(pc, s, inv_fact(2));
   // cos = 1 - s (1/2! - s/4! + ...)
-  cs = df_add_f(df_neg(df_mul(pc, s)), 1.f);
+  cs = df_fin(df_horner(df_neg(pc), s, {1.f, 0.f}));
 }
 
 // e^r - 1 for |r| <= 0.35 (df): Taylor series up to r^13, tail in FP32.
@@ -136,14 +209,13 @@ __device__ __forceinline__ df df_expm1_reduced(df r) {
   t = fmaf(t, rf, inv_fact(10).hi);
   t = fmaf(t, rf, inv_fact(9).hi);
   t = fmaf(t, rf, inv_fact(8).hi);
-  df p = {t, 0.f};
-  p = df_add(df_mul(p, r), inv_fact(7));
-  p = df_add(df_mul(p, r), inv_fact(6));
-  p = df_add(df_mul(p, r), inv_fact(5));
-  p = df_add(df_mul(p, r), inv_fact(4));
-  p = df_add(df_mul(p, r), inv_fact(3));
-  p = df_add(df_mul(p, r), inv_fact(2));
-  p = df_add_f(df_mul(p, r), 1.f);
+  df p = df_horner_f(t, r, inv_fact(7));
+  p = df_horner(p, r, inv_fact(6));
+  p = df_horner(p, r, inv_fact(5));
+  p = df_horner(p, r, inv_fact(4));
+  p = df_horner(p, r, inv_fact(3));
+  p = df_horner(p, r, inv_fact(2));
+  p = df_horner(p, r, {1.f, 0.f});
   return df_mul(p, r);  // r (1 + r/2 + r^2/6 + ...)
 }
 
@@ -171,23 +243,20 @@ __device__ __forceinline__ df df_exp(double x) {
   return df_scale2(e, p2);
 }
 
-// x - n (c0 + c1 + c2 + c3) for an integer n, |n| < 2^8, with FP32 parts c0..c2
-// of 16 bits (exact products) and a 24-bit c3.  When x.hi - n c0 cancels
-// (Sterbenz) the first step is exact, so the reduced argument keeps ~2^-48 of
-// its own size.
-__device__ __forceinline__ df df_reduce(df x, float n, float c0, float c1, float c2, float c3) {
-  df r = df_add_f(x, -n * c0);
-  r = df_add_f(r, -n * c1);
-  r = df_add_f(r, -n * c2);
-  r.lo = fmaf(-n, c3, r.lo);
-  return fast_two_sum(r.hi, r.lo);
+// x - n (c0 + c1 + c2) for an integer n, |n| < 2^8, with FP32 parts of 16
+// bits (exact products; the rest of the constant is below 2^-56 of it).  The
+// first difference is exact: x.hi and n c0 are multiples of 2^-24 for the
+// smallest reduced x and their difference stays below one.
+__device__ __forceinline__ df df_reduce(df x, float n, float c0, float c1, float c2) {
+  const df r = two_sum(fmaf(-n, c0, x.hi), -n * c1);
+  return fast_two_sum(r.hi, r.lo + fmaf(-n, c2, x.lo));
 }
 
 // (sin x, cos x) for a df argument, |x| < 200 (quadrant count below 2^8),
 // everything on the FP32 pipes.
 __device__ __forceinline__ void df_sincos_df(df x, df &sn, df &cs) {
   const float n = rintf(x.hi * DF_TWO_OVER_PI_F);
-  const df r = df_reduce(x, n, DF_PIO2_F0, DF_PIO2_F1, DF_PIO2_F2, DF_PIO2_F3);
+  const df r = df_reduce(x, n, DF_PIO2_F0, DF_PIO2_F1, DF_PIO2_F2);
   df s, c;
   df_sincos_reduced(r, s, c);
   const int q = ((int)n) & 3;
@@ -200,7 +269,7 @@ __device__ __forceinline__ void df_sincos_df(df x, df &sn, df &cs) {
 // e^x for a df argument, -85 < x < 85, on the FP32 pipes.
 __device__ __forceinline__ df df_exp_df(df x) {
   const float n = rintf(x.hi * DF_LOG2E_F);
-  const df r = df_reduce(x, n, DF_LN2_F0, DF_LN2_F1, DF_LN2_F2, DF_LN2_F3);
+  const df r = df_reduce(x, n, DF_LN2_F0, DF_LN2_F1, DF_LN2_F2);
   const df e = df_add_f(df_expm1_reduced(r), 1.f);
   return df_scale2(e, __int_as_float((127 + (int)n) << 23));
 }

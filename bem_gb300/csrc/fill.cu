@@ -1,14 +1,16 @@
 // PMCHWT RWG impedance fill on the GPU: Zts (src/Impedance.cpp:276-413).
 //
 // Work decomposition
-//   * far pairs (no shared vertex): one thread per (test, source) triangle
-//     pair over a 2-D grid, FP64 (plain path).  The reference contracts the
-//     inner integrals per half-RWG (Gphi[j], DGxphi[j], src/Impedance.cpp:126-167);
-//     here the inner loop accumulates four j-independent moments
-//        I0 = sum w g,  A = sum w g (r_s - P_s),  Q0 = sum w q,  Q1 = sum w q (r_s - P_s)
-//     (g, q of GreensFunction::scalar_gradient, gradient = q (r_t - r_s)), and the
-//     outer loop eight moments U0..U3, V0..V3, from which all nine (i, j)
-//     products L_ij, K_ij follow in closed form (derivation beside far_pair()).
+//   * far pairs (no shared vertex): the reference contracts the inner integrals
+//     per half-RWG (Gphi[j], DGxphi[j], src/Impedance.cpp:126-167); here a pair
+//     is reduced to the 3 x 3 moments over {1, eta1, eta2} x {1, xi1, xi2} (the
+//     two triangles' barycentric coordinates) of g and of q (g, q of
+//     GreensFunction::scalar_gradient, gradient = q (r_t - r_s)), from which all
+//     nine (i, j) products L_ij, K_ij follow in closed form (far_contract()).
+//     One thread per pair with the 6-point rule, one warp per pair with a larger
+//     one.  Both triangles of a far pair take the same rule, so L and K are
+//     symmetric in the pair: a fill of a tree against itself integrates each
+//     unordered pair once and writes both its places.
 //   * near pairs (same triangle or a shared vertex): one warp per pair, lanes over
 //     the 105 outer nodes, each lane runs the 91-node smooth inner rule, the
 //     analytic singular terms (EHNonSmoothIntegral, src/Source.cpp:16-86) and the
@@ -22,9 +24,11 @@
 //     coalesced stores (src/Impedance.cpp:365-384).
 #include "bemgpu_internal.h"
 #include "quadrature_tables.h"
-#include "df64.cuh"
+#include "fill_num.cuh"
 
 #include <cmath>
+#include <cstring>
+#include <type_traits>
 #include <vector>
 
 namespace {
@@ -45,6 +49,21 @@ struct FarOpts {
 // or double-float for every quadrature node pair.
 enum { FILL_FP64 = 0, FILL_FP32_FAR = 1, FILL_DF = 2 };
 
+// A node of a triangle rule: barycentric coordinates, weight, weight times each.
+template <typename T>
+struct RuleNode {
+  T x1, x2, w, w1, w2;
+};
+// The far rules' nodes one after the other, in both number types.
+enum { NODES6 = 0, NODES10 = 6, NODES15 = 16, NODES21 = 31, NODES36 = 52, NODES_FAR = 88 };
+__constant__ RuleNode<double> c_far_d[NODES_FAR];
+__constant__ RuleNode<df> c_far_f[NODES_FAR];
+template <typename T>
+__device__ __forceinline__ RuleNode<T> far_node(int k);
+template <>
+__device__ __forceinline__ RuleNode<double> far_node<double>(int k) { return c_far_d[k]; }
+template <>
+__device__ __forceinline__ RuleNode<df> far_node<df>(int k) { return c_far_f[k]; }
 __constant__ double c_rule6[6][3];
 __constant__ double c_rule10[10][3];
 __constant__ double c_rule15[15][3];
@@ -53,13 +72,6 @@ __constant__ double c_rule36[36][3];
 __constant__ double c_rule91[91][3];
 __constant__ double c_rule105[105][3];
 __constant__ double c_line15[15][2];
-// The triangle rules as double-float (xi1, xi2, w) -> (hi, lo) x 3, for the df fill.
-__constant__ float c_rdf6[6][6];
-__constant__ float c_rdf10[10][6];
-__constant__ float c_rdf15[15][6];
-__constant__ float c_rdf21[21][6];
-__constant__ float c_rdf36[36][6];
-__constant__ float c_rdf91[91][6];
 
 // ---------------- small FP64 vector / complex helpers ----------------
 struct d3 {
@@ -154,95 +166,6 @@ __device__ __forceinline__ double scatter_coef(const TriRec &T, int i, const Tri
   return (T.hneg[i] != S.hneg[j]) ? -c : c;
 }
 
-// The nine (c L_ij, c K_ij) of a far pair from its outer moments (closed form
-// beside far_pair()).
-__device__ __forceinline__ void far_contract(const TriRec &T, const TriRec &S, const GreenDev &g, z1 U0, z1 U1, z3 U2,
-                                             z3 U3, z1 V0, z3 V1, z3 V2, z3 V3, HalfPairBlock *H, int ntr) {
-  const d3 Pt = ld3(T.p0), Ps = ld3(S.p0);
-  const z1 ksq = {g.ksqr, g.ksqi};
-  for (int i = 0; i < T.nh; i++) {
-    const d3 p0i = ld3(T.hp0[i]);
-    const d3 ei = p0i - Pt;
-    for (int j = 0; j < S.nh; j++) {
-      const d3 p0j = ld3(S.hp0[j]);
-      const d3 dj = p0j - Ps;
-      const d3 D = p0i - p0j;
-      // L_ij
-      z1 bracket = zsub(zsub(U1, rdot(dj, U2)), rdot(ei, U3));
-      zacc(bracket, zscale(dot(ei, dj), U0));
-      const z1 L = zsub(zscale(0.25, zmul(ksq, bracket)), U0);
-      // K_ij
-      z3 X = z3sub(z3sub(V1, zcross(V2, ei)), rcross(dj, V3));
-      X = z3add(X, zs_v(V0, cross(dj, ei)));
-      const z1 K = zscale(-0.25, rdot(D, X));
-      const double c = scatter_coef(T, i, S, j);
-      store_block(H, ntr, T.hrwg[i], T.hneg[i], S.hrwg[j], S.hneg[j], zscale(c, L), zscale(c, K));
-    }
-  }
-}
-
-// ---------------- far pairs ----------------
-//
-// Closed form of the nine products.  With P_t, P_s the frame origins (p0 of
-// t[0], s[0]), rho = r_t - P_t, l = r_s - P_s, e_i = p0_i - P_t, d_j = p0_j - P_s,
-// D_ij = p0_i - p0_j (test half i, source half j):
-//   Gphi_j(r_t)   = 1/2 (A - d_j I0)
-//   DGxphi_j(r_t) = 1/2 (r_t - p0_j) x (Q1 - d_j Q0)     [(r_t-r_s)x(r_s-p0_j) = (r_t-p0_j)x(r_s-p0_j)]
-//   phi_i . DGxphi_j = 1/4 D_ij . ((Q1 - d_j Q0) x (rho - e_i))   [a.(a x X) = 0]
-// and, with the outer moments U0 = sum w I0, U1 = sum w rho.A, U2 = sum w I0 rho,
-// U3 = sum w A, V0 = sum w Q0, V1 = sum w Q1 x rho, V2 = sum w Q1, V3 = sum w Q0 rho:
-//   L_ij = k^2/4 [U1 - d_j.U2 - e_i.U3 + (e_i.d_j) U0] - U0
-//   K_ij = -1/4 D_ij . [V1 - V2 x e_i - d_j x V3 + V0 (d_j x e_i)]
-// which is LKFarOuterIntegrand (src/Impedance.cpp:154-168) summed over the outer rule.
-__device__ __noinline__ void far_pair(const TriRec &T, const TriRec &S, const GreenDev &g,
-                                      const double (*rule)[3], int nr, HalfPairBlock *H, int ntr) {
-  const d3 Pt = ld3(T.p0), Ps = ld3(S.p0);
-  const d3 v01t = ld3(T.v01), v02t = ld3(T.v02), v01s = ld3(S.v01), v02s = ld3(S.v02);
-  z1 U0 = {0, 0}, U1 = {0, 0}, V0 = {0, 0};
-  z3 U2 = z3zero(), U3 = z3zero(), V1 = z3zero(), V2 = z3zero(), V3 = z3zero();
-  for (int q = 0; q < nr; q++) {
-    const double a = rule[q][0], b = rule[q][1], w = rule[q][2];
-    const d3 rho = a * v01t + b * v02t;
-    const d3 rt = Pt + rho;
-    z1 I0 = {0, 0}, Q0 = {0, 0};
-    z3 A = z3zero(), Q1 = z3zero();
-    for (int u = 0; u < nr; u++) {
-      const double as = rule[u][0], bs = rule[u][1], ws = rule[u][2];
-      const d3 l = as * v01s + bs * v02s;
-      const d3 x = rt - (Ps + l);
-      const double R2 = dot(x, x);
-      const double Ri = rsqrt(R2);
-      const double R = R2 * Ri;
-      const z1 e = zexp_ikR(g, R);
-      // scalar_gradient, src/GreensFunction.cpp:41-52
-      const z1 gs = zscale(Ri, e);
-      const z1 one_m_ikR = {1.0 - g.ikr * R, -g.iki * R};
-      const z1 qq = zscale(Ri * Ri, zmul(gs, one_m_ikR));
-      const z1 gw = zscale(ws, gs), qw = zscale(ws, qq);
-      zacc(I0, gw);
-      A = z3add(A, zs_v(gw, l));
-      zacc(Q0, qw);
-      Q1 = z3add(Q1, zs_v(qw, l));
-    }
-    zacc(U0, zscale(w, I0));
-    zacc(U1, zscale(w, rdot(rho, A)));
-    U2 = z3add(U2, zs_v(zscale(w, I0), rho));
-    U3 = z3add(U3, z3scale(w, A));
-    zacc(V0, zscale(w, Q0));
-    V1 = z3add(V1, z3scale(w, zcross(Q1, rho)));
-    V2 = z3add(V2, z3scale(w, Q1));
-    V3 = z3add(V3, zs_v(zscale(w, Q0), rho));
-  }
-  far_contract(T, S, g, U0, U1, U2, U3, V0, V1, V2, V3, H, ntr);
-}
-
-// ---------------- far pairs in double-float (FP64-class on the FP32 pipes) ----------------
-//
-// far_pair() with the inner rule (the nr x nr node pairs, where the time goes)
-// in double-float: pair-centred coordinates x = (D0 + rho) - l with D0 = P_t -
-// P_s, e^{ikR} from df sincos / exp (quadrant and ln2 reductions in FP64), the
-// four inner moments summed in df and widened to FP64 for the outer moments
-// and the closed-form contraction, which stay as in far_pair().
 struct df3 {
   df x, y, z;
 };
@@ -273,40 +196,40 @@ __device__ __forceinline__ void df_exp_ikR(const GreenDev &g, df ikr, df iki, df
   ei = df_mul(m, sn);
 }
 
-// ---------------- far pairs entirely in double-float ----------------
-//
-// Per triangle a double-float record (edge vectors, half-RWG free vertices
-// relative to p0, scaled edge lengths) is built once per fill; the far pair
-// then runs both rules, the outer moments and the closed-form contraction in
-// df, and only widens the nine (c L, c K) products to FP64 for the store.
+// What a far pair reads of a triangle in double-float, built once per fill.
 struct TriDF {
   float p0[3][2];              // df frame origin (first half-RWG's free vertex)
   float v01[3][2], v02[3][2];  // df edge vectors of the first half-RWG's frame
-  float e[3][3][2];            // df hp0[i] - p0
   float hs[3][2];              // df helen[i] / sqrt(4 pi)
 };
 
-__global__ void tri_df_kernel(const TriRec *__restrict__ R, int n, TriDF *__restrict__ D) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const TriRec &T = R[i];
-  TriDF o;
-  const double sc = sqrt(BEM_ONEOVER4PI);
-  for (int c = 0; c < 3; c++) {
-    const df a = df_make(T.v01[c]), b = df_make(T.v02[c]), p = df_make(T.p0[c]);
-    o.p0[c][0] = p.hi; o.p0[c][1] = p.lo;
-    o.v01[c][0] = a.hi; o.v01[c][1] = a.lo;
-    o.v02[c][0] = b.hi; o.v02[c][1] = b.lo;
-  }
-  for (int h = 0; h < 3; h++) {
+// The records of every tree of a group of fills in one launch: task i's test
+// triangles at TD, its source triangles at SD (the same records when both
+// trees are one).
+struct TriDFJob {
+  const TriRec *R;
+  TriDF *D;
+  int n;
+};
+
+__global__ void tri_df_kernel(const TriDFJob *__restrict__ jobs) {
+  const TriDFJob jb = jobs[blockIdx.y];
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < jb.n; i += gridDim.x * blockDim.x) {
+    const TriRec &T = jb.R[i];
+    TriDF o;
+    const double sc = sqrt(BEM_ONEOVER4PI);
     for (int c = 0; c < 3; c++) {
-      const df e = df_make(h < T.nh ? T.hp0[h][c] - T.p0[c] : 0.0);
-      o.e[h][c][0] = e.hi; o.e[h][c][1] = e.lo;
+      const df a = df_make(T.v01[c]), b = df_make(T.v02[c]), p = df_make(T.p0[c]);
+      o.p0[c][0] = p.hi; o.p0[c][1] = p.lo;
+      o.v01[c][0] = a.hi; o.v01[c][1] = a.lo;
+      o.v02[c][0] = b.hi; o.v02[c][1] = b.lo;
     }
-    const df l = df_make(h < T.nh ? T.helen[h] * sc : 0.0);
-    o.hs[h][0] = l.hi; o.hs[h][1] = l.lo;
+    for (int h = 0; h < 3; h++) {
+      const df l = df_make(h < T.nh ? T.helen[h] * sc : 0.0);
+      o.hs[h][0] = l.hi; o.hs[h][1] = l.lo;
+    }
+    jb.D[i] = o;
   }
-  D[i] = o;
 }
 
 struct cdf {
@@ -315,7 +238,6 @@ struct cdf {
 struct cdf3 {
   cdf x, y, z;
 };
-__device__ __forceinline__ df3 ld_df3(const float (*v)[2]) { return {{v[0][0], v[0][1]}, {v[1][0], v[1][1]}, {v[2][0], v[2][1]}}; }
 __device__ __forceinline__ df3 df3_add(df3 a, df3 b) { return {df_add(a.x, b.x), df_add(a.y, b.y), df_add(a.z, b.z)}; }
 __device__ __forceinline__ df3 df3_sub(df3 a, df3 b) { return {df_sub(a.x, b.x), df_sub(a.y, b.y), df_sub(a.z, b.z)}; }
 __device__ __forceinline__ df3 df3_scale(df s, df3 a) { return {df_mul(s, a.x), df_mul(s, a.y), df_mul(s, a.z)}; }
@@ -349,93 +271,344 @@ __device__ __forceinline__ cdf3 cdf_rcross(df3 a, cdf3 b) {
   return {cdf_sub(cdf_scale(a.y, b.z), cdf_scale(a.z, b.y)), cdf_sub(cdf_scale(a.z, b.x), cdf_scale(a.x, b.z)),
           cdf_sub(cdf_scale(a.x, b.y), cdf_scale(a.y, b.x))};
 }
-__device__ __forceinline__ cdf3 cdf3_zero() {
-  const df z = {0.f, 0.f};
-  return {{z, z}, {z, z}, {z, z}};
+
+// Green's function constants in the fill's number type.
+template <typename T>
+struct GreenT {
+  T ikr, iki, k2r, k2i, ksqr, ksqi;
+};
+template <typename T>
+__device__ __forceinline__ GreenT<T> green_of(const GreenDev &g);
+template <>
+__device__ __forceinline__ GreenT<double> green_of<double>(const GreenDev &g) {
+  return {g.ikr, g.iki, g.k2r, g.k2i, g.ksqr, g.ksqi};
+}
+template <>
+__device__ __forceinline__ GreenT<df> green_of<df>(const GreenDev &g) {
+  return {{g.ikr_f[0], g.ikr_f[1]}, {g.iki_f[0], g.iki_f[1]}, {g.k2r_f[0], g.k2r_f[1]},
+          {g.k2i_f[0], g.k2i_f[1]}, {g.ksqr_f[0], g.ksqr_f[1]}, {g.ksqi_f[0], g.ksqi_f[1]}};
 }
 
-__device__ __noinline__ void far_pair_df2(const TriRec &T, const TriRec &S, const TriDF &TD, const TriDF &SD,
-                                          const GreenDev &g, const float (*rdf)[6], int nr, HalfPairBlock *H,
-                                          int ntr) {
-  const df3 D0 = df3_sub(ld_df3(TD.p0), ld_df3(SD.p0));  // P_t - P_s
-  const df3 v01t = ld_df3(TD.v01), v02t = ld_df3(TD.v02), v01s = ld_df3(SD.v01), v02s = ld_df3(SD.v02);
-  const df ikr = {g.ikr_f[0], g.ikr_f[1]}, iki = {g.iki_f[0], g.iki_f[1]};
-  const df z0 = {0.f, 0.f};
-  cdf U0 = {z0, z0}, U1 = {z0, z0}, V0 = {z0, z0};
-  cdf3 U2 = cdf3_zero(), U3 = cdf3_zero(), V1 = cdf3_zero(), V2 = cdf3_zero(), V3 = cdf3_zero();
-  for (int q = 0; q < nr; q++) {
-    const df a = {rdf[q][0], rdf[q][1]}, b = {rdf[q][2], rdf[q][3]}, w = {rdf[q][4], rdf[q][5]};
-    const df3 rho = df3_add(df3_scale(a, v01t), df3_scale(b, v02t));
-    const df3 rts = df3_add(D0, rho);  // r_t - P_s
-    df I0r = z0, I0i = z0, Q0r = z0, Q0i = z0;
-    df Ar[3] = {z0, z0, z0}, Ai[3] = {z0, z0, z0}, Qr[3] = {z0, z0, z0}, Qi[3] = {z0, z0, z0};
-    for (int u = 0; u < nr; u++) {
-      const df as = {rdf[u][0], rdf[u][1]}, bs = {rdf[u][2], rdf[u][3]}, ws = {rdf[u][4], rdf[u][5]};
-      const df l[3] = {df_add(df_mul(as, v01s.x), df_mul(bs, v02s.x)), df_add(df_mul(as, v01s.y), df_mul(bs, v02s.y)),
-                       df_add(df_mul(as, v01s.z), df_mul(bs, v02s.z))};
-      const df xx = df_sub(rts.x, l[0]), xy = df_sub(rts.y, l[1]), xz = df_sub(rts.z, l[2]);
-      const df R2 = df_add(df_add(df_sqr(xx), df_sqr(xy)), df_sqr(xz));
-      const df R = df_sqrt(R2);
-      const df Ri = df_rcp(R);
-      df er, ei;
-      df_exp_ikR(g, ikr, iki, R, er, ei);
-      const df gr = df_mul(er, Ri), gi = df_mul(ei, Ri);
-      const df zr = df_mul(ikr, R), zi = df_mul(iki, R);
-      const df mr = df_add_f(df_neg(zr), 1.f), mi = df_neg(zi);
-      const df Ri2 = df_sqr(Ri);
-      const df qr = df_mul(df_sub(df_mul(gr, mr), df_mul(gi, mi)), Ri2);
-      const df qi = df_mul(df_add(df_mul(gr, mi), df_mul(gi, mr)), Ri2);
-      const df gwr = df_mul(ws, gr), gwi = df_mul(ws, gi), qwr = df_mul(ws, qr), qwi = df_mul(ws, qi);
-      I0r = df_add(I0r, gwr);
-      I0i = df_add(I0i, gwi);
-      Q0r = df_add(Q0r, qwr);
-      Q0i = df_add(Q0i, qwi);
+// (er, ei) = e^{ikR} and (ur, ui) = e^{ikR} (1 - ikR).  REALK: a lossless
+// medium (ik imaginary), whose e^{ikR} has modulus one.
+template <typename T, bool REALK>
+__device__ __forceinline__ void wave_at(const GreenT<T> &g, T R, T &er, T &ei, T &ur, T &ui) {
+  typedef Num<T> N;
+  const T th = g.iki * R;
+  N::sincos_(th, ei, er);
+  if (REALK) {
+    ur = N::muladd(ei, th, er);
+    ui = N::muladd(-er, th, ei);
+    return;
+  }
+  const T a = g.ikr * R;
+  if (N::head(a) < -85) {  // below FP32's range: e^-85 of the neighbouring nodes' size
+    const T z = N::of(0.0);
+    er = ei = ur = ui = z;
+    return;
+  }
+  const T m = N::exp_(a);
+  er = m * er;
+  ei = m * ei;
+  const T om = N::of(1.0) - a;
+  ur = N::dot2(er, om, ei, th);
+  ui = N::dot2(ei, om, -er, th);
+}
+
+// scalar_gradient, src/GreensFunction.cpp:41-52, at the (unnormalized)
+// difference x: f = {Re g, Im g, Re q, Im q}.
+template <typename T, bool REALK>
+__device__ __forceinline__ void far_values(const GreenT<T> &g, V3<T> x, T (&f)[4]) {
+  typedef Num<T> N;
+  T R, Ri, er, ei, ur, ui;
+  N::sqrt_rcp(N::sumsq(x.x, x.y, x.z), R, Ri);
+  wave_at<T, REALK>(g, R, er, ei, ur, ui);
+  f[0] = er * Ri;
+  f[1] = ei * Ri;
+  const T Ri3 = Ri * (Ri * Ri);
+  f[2] = ur * Ri3;
+  f[3] = ui * Ri3;
+}
+
+// A far pair's triangles: origins' difference and edge vectors.
+template <typename T>
+struct FarGeom {
+  V3<T> D0;      // P_t - P_s
+  V3<T> a1, a2;  // test edges v01, v02
+  V3<T> c1, c2;  // source edges v01, v02
+};
+template <typename T>
+__device__ __forceinline__ FarGeom<T> far_geom(const TriRec &T_, const TriRec &S, const TriDF *TD, const TriDF *SD);
+template <>
+__device__ __forceinline__ FarGeom<double> far_geom<double>(const TriRec &T_, const TriRec &S, const TriDF *,
+                                                            const TriDF *) {
+  auto v = [](const double *p) { return V3<double>{p[0], p[1], p[2]}; };
+  return {v(T_.p0) - v(S.p0), v(T_.v01), v(T_.v02), v(S.v01), v(S.v02)};
+}
+template <>
+__device__ __forceinline__ FarGeom<df> far_geom<df>(const TriRec &, const TriRec &, const TriDF *TD, const TriDF *SD) {
+  auto v = [](const float (*p)[2]) { return V3<df>{{p[0][0], p[0][1]}, {p[1][0], p[1][1]}, {p[2][0], p[2][1]}}; };
+  return {v(TD->p0) - v(SD->p0), v(TD->v01), v(TD->v02), v(SD->v01), v(SD->v02)};
+}
+
+// Moments of a far pair with the 6-point rule, by one thread:
+// M[(c * 3 + a) * 3 + b] = sum_qu w_q w_u eta^a xi^b f_c.  rho: the outer
+// nodes relative to P_t (shared memory: the warp has one test triangle).
+template <typename T, bool REALK>
+__device__ __forceinline__ void far_moments6(const FarGeom<T> &ge, const GreenT<T> &g, const V3<T> *rho, T (&M)[36]) {
+  typedef Num<T> N;
 #pragma unroll
-      for (int c = 0; c < 3; c++) {
-        Ar[c] = df_add(Ar[c], df_mul(gwr, l[c]));
-        Ai[c] = df_add(Ai[c], df_mul(gwi, l[c]));
-        Qr[c] = df_add(Qr[c], df_mul(qwr, l[c]));
-        Qi[c] = df_add(Qi[c], df_mul(qwi, l[c]));
+  for (int k = 0; k < 36; k++) M[k] = N::of(0.0);
+#pragma unroll 1
+  for (int u = 0; u < 6; u++) {
+    const RuleNode<T> nu = far_node<T>(NODES6 + u);
+    const V3<T> base = ge.D0 - (nu.x1 * ge.c1 + nu.x2 * ge.c2);
+    T S[12];
+#pragma unroll
+    for (int k = 0; k < 12; k++) S[k] = N::of(0.0);
+#pragma unroll 1
+    for (int q = 0; q < 6; q++) {
+      const V3<T> r = rho[q];
+      const V3<T> x = {N::diff(base.x, -r.x), N::diff(base.y, -r.y), N::diff(base.z, -r.z)};
+      T f[4];
+      far_values<T, REALK>(g, x, f);
+      const RuleNode<T> nq = far_node<T>(NODES6 + q);
+#pragma unroll
+      for (int c = 0; c < 4; c++) {
+        N::mac(S[c * 3 + 0], f[c], nq.w);
+        N::mac(S[c * 3 + 1], f[c], nq.w1);
+        N::mac(S[c * 3 + 2], f[c], nq.w2);
       }
     }
-    const cdf I0 = {I0r, I0i}, Q0 = {Q0r, Q0i};
-    const cdf3 A = {{Ar[0], Ai[0]}, {Ar[1], Ai[1]}, {Ar[2], Ai[2]}};
-    const cdf3 Q1 = {{Qr[0], Qi[0]}, {Qr[1], Qi[1]}, {Qr[2], Qi[2]}};
-    const cdf wI0 = cdf_scale(w, I0), wQ0 = cdf_scale(w, Q0);
-    U0 = cdf_add(U0, wI0);
-    U1 = cdf_add(U1, cdf_scale(w, cdf_rdot(rho, A)));
-    U2 = cdf3_add(U2, cdf_v(wI0, rho));
-    U3 = cdf3_add(U3, cdf3_scale(w, A));
-    V0 = cdf_add(V0, wQ0);
-    V1 = cdf3_add(V1, cdf3_scale(w, cdf_zcross(Q1, rho)));
-    V2 = cdf3_add(V2, cdf3_scale(w, Q1));
-    V3 = cdf3_add(V3, cdf_v(wQ0, rho));
-  }
-  // the closed form of far_pair(), in df
-  const cdf ksq = {{g.ksqr_f[0], g.ksqr_f[1]}, {g.ksqi_f[0], g.ksqi_f[1]}};
-  const df quarter = {0.25f, 0.f};
-  for (int i = 0; i < T.nh; i++) {
-    const df3 ei = ld_df3(TD.e[i]);
-    for (int j = 0; j < S.nh; j++) {
-      const df3 dj = ld_df3(SD.e[j]);
-      const df3 D = df3_sub(df3_add(D0, ei), dj);  // p0_i - p0_j
-      cdf br = cdf_sub(cdf_sub(U1, cdf_rdot(dj, U2)), cdf_rdot(ei, U3));
-      br = cdf_add(br, cdf_scale(df3_dot(ei, dj), U0));
-      const cdf L = cdf_sub(cdf_scale(quarter, cdf_mul(ksq, br)), U0);
-      cdf3 X = cdf3_sub(cdf3_sub(V1, cdf_zcross(V2, ei)), cdf_rcross(dj, V3));
-      X = cdf3_add(X, cdf_v(V0, df3_cross(dj, ei)));
-      const cdf K = cdf_scale(df_neg(quarter), cdf_rdot(D, X));
-      df c = df_mul({TD.hs[i][0], TD.hs[i][1]}, {SD.hs[j][0], SD.hs[j][1]});
-      if (T.hneg[i] != S.hneg[j]) c = df_neg(c);
-      const cdf cL = cdf_scale(c, L), cK = cdf_scale(c, K);
-      store_block_df(H, ntr, T.hrwg[i], T.hneg[i], S.hrwg[j], S.hneg[j], cL.r, cL.i, cK.r, cK.i);
+#pragma unroll
+    for (int k = 0; k < 12; k++) {
+      const T v = N::fin(S[k]);
+      N::mac(M[k * 3 + 0], v, nu.w);
+      N::mac(M[k * 3 + 1], v, nu.w1);
+      N::mac(M[k * 3 + 2], v, nu.w2);
     }
   }
+#pragma unroll
+  for (int k = 0; k < 36; k++) M[k] = N::fin(M[k]);
+}
+
+// The same with an nr-point rule (first node off), by one warp: the lanes take
+// (outer node, run of inner nodes) pieces.  rt, rs: the warp's staging of the
+// pair's outer nodes (relative to P_s) and inner nodes.  The sums land in out[36].
+template <typename T>
+struct FarStage {
+  V3<T> p[36];
+  T w[36][3];
+};
+template <typename T, bool REALK>
+__device__ __forceinline__ void far_moments_warp(const FarGeom<T> &ge, const GreenT<T> &g, int off, int nr,
+                                                 FarStage<T> *st, FarStage<T> *ss, T *out, int lane) {
+  typedef Num<T> N;
+  for (int k = lane; k < nr; k += 32) {
+    const RuleNode<T> n = far_node<T>(off + k);
+    st->p[k] = ge.D0 + (n.x1 * ge.a1 + n.x2 * ge.a2);
+    ss->p[k] = n.x1 * ge.c1 + n.x2 * ge.c2;
+    st->w[k][0] = ss->w[k][0] = n.w;
+    st->w[k][1] = ss->w[k][1] = n.w1;
+    st->w[k][2] = ss->w[k][2] = n.w2;
+  }
+  __syncwarp();
+  T M[40];
+#pragma unroll
+  for (int k = 0; k < 40; k++) M[k] = N::of(0.0);
+  const int pieces = (nr + 8) / 9, run = (nr + pieces - 1) / pieces;
+#pragma unroll 1
+  for (int it = lane; it < nr * pieces; it += 32) {
+    const int q = it / pieces, u0 = (it - q * pieces) * run, u1 = min(nr, u0 + run);
+    const V3<T> r = st->p[q];
+    T S[12];
+#pragma unroll
+    for (int k = 0; k < 12; k++) S[k] = N::of(0.0);
+#pragma unroll 1
+    for (int u = u0; u < u1; u++) {
+      const V3<T> l = ss->p[u];
+      const V3<T> x = {N::diff(r.x, l.x), N::diff(r.y, l.y), N::diff(r.z, l.z)};
+      T f[4];
+      far_values<T, REALK>(g, x, f);
+#pragma unroll
+      for (int c = 0; c < 4; c++)
+#pragma unroll
+        for (int b = 0; b < 3; b++) N::mac(S[c * 3 + b], f[c], ss->w[u][b]);
+    }
+#pragma unroll
+    for (int c = 0; c < 4; c++)
+#pragma unroll
+      for (int b = 0; b < 3; b++) {
+        const T v = N::fin(S[c * 3 + b]);
+#pragma unroll
+        for (int a = 0; a < 3; a++) N::mac(M[(c * 3 + a) * 3 + b], v, st->w[q][a]);
+      }
+  }
+  const int at = reduce8_index(lane);
+#pragma unroll
+  for (int k = 0; k < 5; k++) {
+    T v[8];
+#pragma unroll
+    for (int j = 0; j < 8; j++) v[j] = N::fin(M[k * 8 + j]);
+    const T r = reduce8<T>(v, lane);
+    if ((lane & 3) == 0 && k * 8 + at < 36) out[k * 8 + at] = r;
+  }
+  __syncwarp();
+}
+
+// Scatter coefficient of src/Impedance.cpp:372-375 in the fill's number type.
+template <typename T>
+__device__ __forceinline__ T scatter_coef_t(const TriRec &T_, const TriDF *TD, int i, const TriRec &S, const TriDF *SD,
+                                            int j);
+template <>
+__device__ __forceinline__ double scatter_coef_t<double>(const TriRec &T_, const TriDF *, int i, const TriRec &S,
+                                                         const TriDF *, int j) {
+  return scatter_coef(T_, i, S, j);
+}
+template <>
+__device__ __forceinline__ df scatter_coef_t<df>(const TriRec &T_, const TriDF *TD, int i, const TriRec &S,
+                                                 const TriDF *SD, int j) {
+  const df c = df_mul({TD->hs[i][0], TD->hs[i][1]}, {SD->hs[j][0], SD->hs[j][1]});
+  return T_.hneg[i] != S.hneg[j] ? df_neg(c) : c;
+}
+__device__ __forceinline__ void store_pair(HalfPairBlock *H, int ntr, int i, int a, int j, int b, C1<double> L,
+                                           C1<double> K) {
+  store_block(H, ntr, i, a, j, b, {L.r, L.i}, {K.r, K.i});
+}
+__device__ __forceinline__ void store_pair(HalfPairBlock *H, int ntr, int i, int a, int j, int b, C1<df> L, C1<df> K) {
+  store_block_df(H, ntr, i, a, j, b, L.r, L.i, K.r, K.i);
+}
+
+// The nine (c L_ij, c K_ij) of a far pair from its moments.
+//
+// The half-RWGs' free vertices are the triangles' vertices P_v, S_w, so with
+// the edges a_1, a_2 of the test and c_1, c_2 of the source triangle from P_0
+// and S_0, phi_i = (rho - e_i)/2 and e_i in {0, a_1, a_2}:
+//   L_vw = k^2/4 sum_{ab} (a_a . c_b) [G_ab - [b=w] G_a0 - [a=v] G_0b + [a=v][b=w] G_00] - G_00
+// (a, b = 1, 2), G the moments of g.  In barycentric moments B of q,
+// phi_i . ((r_t - r_s) x phi_j) expands to the six-fold volumes of the
+// tetrahedra on an edge of each triangle:
+//   K_vw = -1/4 sum_{v' != v, w' != w} B_v'w' (P_v - S_w) . ((S_w' - S_w) x (P_v' - P_v)),
+// nine volumes for the nine edge pairs (src/Impedance.cpp:154-168 summed over
+// the outer rule).  mirror: the pair's transposed place too.
+template <typename T, bool REALK>
+__device__ __noinline__ void far_contract(const TriRec &T_, const TriRec &S, const TriDF *TD, const TriDF *SD,
+                                          const GreenT<T> &g, const T *M, HalfPairBlock *H, int ntr, bool mirror) {
+  typedef Num<T> N;
+  const FarGeom<T> ge = far_geom<T>(T_, S, TD, SD);
+  const V3<T> a[2] = {ge.a1, ge.a2}, cs[2] = {ge.c1, ge.c2};
+  // L's brackets
+  C1<T> G[3][3];
+#pragma unroll
+  for (int x = 0; x < 3; x++)
+#pragma unroll
+    for (int y = 0; y < 3; y++) G[x][y] = {M[x * 3 + y], M[9 + x * 3 + y]};
+  C1<T> br[3][3];
+  {
+    C1<T> U1 = {N::of(0.0), N::of(0.0)}, dU2[2] = {U1, U1}, eU3[2] = {U1, U1}, ed[2][2];
+#pragma unroll
+    for (int x = 0; x < 2; x++)
+#pragma unroll
+      for (int y = 0; y < 2; y++) {
+        const T d = vdot(a[x], cs[y]);
+        U1 = U1 + d * G[x + 1][y + 1];
+        dU2[y] = dU2[y] + d * G[x + 1][0];
+        eU3[x] = eU3[x] + d * G[0][y + 1];
+        ed[x][y] = d * G[0][0];
+      }
+    br[0][0] = U1;
+#pragma unroll
+    for (int x = 0; x < 2; x++) {
+      br[0][x + 1] = U1 - dU2[x];
+      br[x + 1][0] = U1 - eU3[x];
+    }
+#pragma unroll
+    for (int x = 0; x < 2; x++)
+#pragma unroll
+      for (int y = 0; y < 2; y++) br[x + 1][y + 1] = (br[0][y + 1] - eU3[x]) + ed[x][y];
+  }
+  // barycentric moments of q
+  C1<T> B[3][3];
+#pragma unroll
+  for (int x = 0; x < 3; x++)
+#pragma unroll
+    for (int y = 0; y < 3; y++) B[x][y] = {M[18 + x * 3 + y], M[27 + x * 3 + y]};
+#pragma unroll
+  for (int y = 0; y < 3; y++) B[0][y] = (B[0][y] - B[1][y]) - B[2][y];
+#pragma unroll
+  for (int x = 0; x < 3; x++) B[x][0] = (B[x][0] - B[x][1]) - B[x][2];
+  // volumes of the edge pairs (edges 01, 02, 12 of each triangle)
+  T V[3][3];
+  {
+    const V3<T> C00 = vcross(cs[0], a[0]), C01 = vcross(cs[0], a[1]), C10 = vcross(cs[1], a[0]),
+                C11 = vcross(cs[1], a[1]);  // C_xy = c_x x a_y
+    V[0][0] = vdot(ge.D0, C00);
+    V[0][1] = vdot(ge.D0, C10);
+    V[1][0] = vdot(ge.D0, C01);
+    V[1][1] = vdot(ge.D0, C11);
+    const T a01 = vdot(a[0], C01), a11 = vdot(a[0], C11);    // a_1 . (c_x x a_2)
+    const T c10 = vdot(cs[0], C10), c11 = vdot(cs[0], C11);  // c_1 . (c_2 x a_y)
+    V[2][0] = (V[1][0] - V[0][0]) + a01;
+    V[2][1] = (V[1][1] - V[0][1]) + a11;
+    V[0][2] = (V[0][1] - V[0][0]) - c10;
+    V[1][2] = (V[1][1] - V[1][0]) - c11;
+    V[2][2] = ((V[1][1] - V[0][1]) - (V[1][0] - V[0][0])) + ((a11 - a01) - (c11 - c10));
+  }
+  const T ksr = N::pow2(g.ksqr, 0.25f), ksi = N::pow2(g.ksqi, 0.25f);
+  int at[3], as[3];  // the halves (bits) whose free vertex is v
+#pragma unroll
+  for (int v = 0; v < 3; v++) {
+    at[v] = as[v] = 0;
+#pragma unroll
+    for (int h = 0; h < 3; h++) {
+      at[v] |= (h < T_.nh && ((T_.hvert >> (2 * h)) & 3) == v) ? 1 << h : 0;
+      as[v] |= (h < S.nh && ((S.hvert >> (2 * h)) & 3) == v) ? 1 << h : 0;
+    }
+  }
+#pragma unroll
+  for (int v = 0; v < 3; v++)
+#pragma unroll
+    for (int w = 0; w < 3; w++) {
+      C1<T> K = {N::of(0.0), N::of(0.0)};
+#pragma unroll
+      for (int x = 0; x < 3; x++)
+#pragma unroll
+        for (int y = 0; y < 3; y++) {
+          if (x == v || y == w) continue;
+          const T vol = V[v + x - 1][w + y - 1];  // edge {v, x} -> 01: 0, 02: 1, 12: 2
+          const bool minus = (v > x) != (w > y);
+          N::mac(K.r, B[x][y].r, minus ? vol : -vol);
+          N::mac(K.i, B[x][y].i, minus ? vol : -vol);
+        }
+      K = {N::pow2(N::fin(K.r), 0.25f), N::pow2(N::fin(K.i), 0.25f)};
+      C1<T> L;
+      if (REALK)
+        L = {N::muladd(ksr, br[v][w].r, -G[0][0].r), N::muladd(ksr, br[v][w].i, -G[0][0].i)};
+      else
+        L = cmul(C1<T>{ksr, ksi}, br[v][w]) - G[0][0];
+      for (int hi = at[v]; hi; hi &= hi - 1)
+        for (int hj = as[w]; hj; hj &= hj - 1) {
+          const int i = __ffs(hi) - 1, j = __ffs(hj) - 1;
+          const T c = scatter_coef_t<T>(T_, TD, i, S, SD, j);
+          const C1<T> cL = c * L, cK = c * K;
+          store_pair(H, ntr, T_.hrwg[i], T_.hneg[i], S.hrwg[j], S.hneg[j], cL, cK);
+          if (mirror) store_pair(H, ntr, S.hrwg[j], S.hneg[j], T_.hrwg[i], T_.hneg[i], cL, cK);
+        }
+    }
 }
 
 // ---------------- far pairs in FP32 (mixed precision) ----------------
 //
-// Same closed form as far_pair(), evaluated in FP32 with a pair-centred
+// Closed form of the nine products from outer moments.  With P_t, P_s the frame
+// origins (p0 of t[0], s[0]), rho = r_t - P_t, l = r_s - P_s, e_i = p0_i - P_t,
+// d_j = p0_j - P_s, D_ij = p0_i - p0_j, the inner moments I0 = sum w g,
+// A = sum w g l, Q0 = sum w q, Q1 = sum w q l and the outer ones U0 = sum w I0,
+// U1 = sum w rho.A, U2 = sum w I0 rho, U3 = sum w A, V0 = sum w Q0,
+// V1 = sum w Q1 x rho, V2 = sum w Q1, V3 = sum w Q0 rho:
+//   L_ij = k^2/4 [U1 - d_j.U2 - e_i.U3 + (e_i.d_j) U0] - U0
+//   K_ij = -1/4 D_ij . [V1 - V2 x e_i - d_j x V3 + V0 (d_j x e_i)]
+// which is LKFarOuterIntegrand (src/Impedance.cpp:154-168) summed over the
+// outer rule, here in FP32 with a pair-centred
 // distance: r_t - r_s = D0 + u, D0 = P_t - P_s (FP64 once per pair), u = rho - l
 // (small, FP32).  R = R0 + dR with R0 = |D0| in FP64 and
 // dR = (2 D0.u + u.u) / (R0 + R) in FP32, so the phase k R is k R0 reduced
@@ -563,6 +736,7 @@ struct FillTask {
   int64_t near0;             // first near work unit of the group that is this task's
   int64_t far0;              // first far tile of the group that is this task's
   int ntT, ntS, ntr, far_tx; // triangles of t and s, RWGs of t, far tiles along s
+  int sym;                   // t is s: each unordered far pair is integrated once
   GreenDev g;
 };
 
@@ -578,72 +752,160 @@ __device__ __forceinline__ int task_of_near(const FillTask *tk, int n, int64_t u
   return i;
 }
 
-// mixed != 0: pairs whose centroid distance exceeds 3 edge lengths (the longer
-// of the two triangles' longest edges) are integrated in FP32.
-__device__ __forceinline__ void far_pair_at(const TriRec *__restrict__ Tr, int ntT, const TriRec *__restrict__ Sr,
-                                            int ntS, const GreenDev &g, const FarOpts &o,
-                                            HalfPairBlock *__restrict__ H, int ntr, int mode,
-                                            const TriDF *__restrict__ TDr, const TriDF *__restrict__ SDr, int sb,
-                                            int ta) {
-  if (sb >= ntS || ta >= ntT) return;
-  const TriRec &T = Tr[ta];
-  const TriRec &S = Sr[sb];
-  if (T.gid == S.gid || shares_vertex(T.vid, S.vid)) return;  // near kernel
-  // far-rule choice, src/Impedance.cpp:329-360
-  const double d = dist2_rn(T.c, S.c);
-  const double e = fmax(T.emax, S.emax);
-  const double emax2 = __dmul_rn(e, e);
-  if (mode == FILL_DF) {
-    const TriDF &TD = TDr[ta], &SD = SDr[sb];
-    if (__dmul_rn(d, o.th6) > emax2) far_pair_df2(T, S, TD, SD, g, c_rdf6, 6, H, ntr);
-    else if (__dmul_rn(d, o.th10) > emax2) far_pair_df2(T, S, TD, SD, g, c_rdf10, 10, H, ntr);
-    else if (__dmul_rn(d, o.th15) > emax2) far_pair_df2(T, S, TD, SD, g, c_rdf15, 15, H, ntr);
-    else if (__dmul_rn(d, o.th21) > emax2) far_pair_df2(T, S, TD, SD, g, c_rdf21, 21, H, ntr);
-    else far_pair_df2(T, S, TD, SD, g, c_rdf36, 36, H, ntr);
-    return;
-  }
-  if (mode == FILL_FP32_FAR && d > 9.0 * emax2) {
-    // beyond 3 edge lengths every default threshold selects the 6-point rule;
-    // the cascade is kept for non-default Options
-    if (__dmul_rn(d, o.th6) > emax2) far_pair_fp32(T, S, g, c_rule6, 6, H, ntr);
-    else if (__dmul_rn(d, o.th10) > emax2) far_pair_fp32(T, S, g, c_rule10, 10, H, ntr);
-    else if (__dmul_rn(d, o.th15) > emax2) far_pair_fp32(T, S, g, c_rule15, 15, H, ntr);
-    else if (__dmul_rn(d, o.th21) > emax2) far_pair_fp32(T, S, g, c_rule21, 21, H, ntr);
-    else far_pair_fp32(T, S, g, c_rule36, 36, H, ntr);
-    return;
-  }
-  if (__dmul_rn(d, o.th6) > emax2) far_pair(T, S, g, c_rule6, 6, H, ntr);
-  else if (__dmul_rn(d, o.th10) > emax2) far_pair(T, S, g, c_rule10, 10, H, ntr);
-  else if (__dmul_rn(d, o.th15) > emax2) far_pair(T, S, g, c_rule15, 15, H, ntr);
-  else if (__dmul_rn(d, o.th21) > emax2) far_pair(T, S, g, c_rule21, 21, H, ntr);
-  else far_pair(T, S, g, c_rule36, 36, H, ntr);
+// Far tiles of one fill: 32 source x rows test triangles each; a symmetric
+// fill has those of the lower-triangular 32 x 32 blocks only.
+int64_t far_tiles_of(bool sym, int ntT, int ntS, int rows) {
+  if (!sym) return (int64_t)((ntS + 31) / 32) * ((ntT + rows - 1) / rows);
+  const int64_t nb = (ntT + 31) / 32;
+  return nb * (nb + 1) / 2 * (32 / rows);
 }
 
-// One fill (t, s, g) -> H: thread (x, y) of the 2-D grid takes the source
-// triangle blockIdx.x * 32 + x and the test triangle blockIdx.y * blockDim.y + y.
-__global__ void __launch_bounds__(256) far_pairs_kernel(const TriRec *__restrict__ Tr, int ntT,
-                                                        const TriRec *__restrict__ Sr, int ntS, GreenDev g,
-                                                        FarOpts o, HalfPairBlock *__restrict__ H, int ntr, int mode,
-                                                        const TriDF *__restrict__ TDr, const TriDF *__restrict__ SDr) {
-  far_pair_at(Tr, ntT, Sr, ntS, g, o, H, ntr, mode, TDr, SDr, blockIdx.x * blockDim.x + threadIdx.x,
-              blockIdx.y * blockDim.y + threadIdx.y);
+// The first test triangle and the first source triangle of a far tile.
+__device__ __forceinline__ void far_tile_at(const FillTask &tk, int64_t local, int rows, int &ta0, int &sb0) {
+  if (!tk.sym) {
+    sb0 = (int)(local % tk.far_tx) * 32;
+    ta0 = (int)(local / tk.far_tx) * rows;
+    return;
+  }
+  const int sub = 32 / rows;
+  const int64_t m = local / sub;  // block number: row r holds blocks r (r + 1) / 2 ...
+  int64_t r = (int64_t)((sqrt(8.0 * (double)m + 1.0) - 1.0) * 0.5);
+  while (r * (r + 1) / 2 > m) r--;
+  while ((r + 1) * (r + 2) / 2 <= m) r++;
+  ta0 = (int)r * 32 + (int)(local - m * sub) * rows;
+  sb0 = (int)(m - r * (r + 1) / 2) * 32;
 }
 
 // A group of fills in one launch (the three Zts of a solve, or of several
-// requests): CTA b takes far tile b of the task whose range holds it, a tile
-// being 32 source x blockDim.y test triangles.  The task's Green's function
-// is staged in shared memory (one task per CTA).
-__global__ void __launch_bounds__(256) far_pairs_group_kernel(const FillTask *__restrict__ tasks, int ntask,
-                                                              FarOpts o, int mode) {
+// requests): CTA b takes far tile b of the task whose range holds it, lane =
+// source triangle, warp = test triangle.  MODE FILL_FP32_FAR: pairs whose
+// centroid distance exceeds 3 edge lengths (the longer of the two triangles'
+// longest edges) in FP32, every ordered pair by itself; the others, and every
+// pair of the other modes, in FP64 (FILL_FP64, FILL_FP32_FAR) or double-float.
+//
+// A pair with the 6-point rule is one thread's; the others (triangles that
+// face each other across a gap narrower than their edges: 1296 node pairs
+// against 36) are listed in shared memory and taken by whole warps, so that
+// one such pair does not hold its warp's other 31 lanes.
+//
+// Bound by FP32 issue (double-float) or by the FP64 pipe.  The chains of one
+// node pair are long, so resident warps count: 168 registers (12 warps an SM)
+// against the 206 the compiler takes by itself (8) gave 6.1 -> 4.6 ms; two or
+// three nodes in flight per thread, or 128 registers with spills, were slower.
+// The three fills of a solve, before (every ordered pair, Cartesian moments,
+// normalized sums, one thread for every rule) and now: icospheres at N = 7680
+// 16.9 -> 4.6 ms, slabs 50 nm apart at N = 11520 43.7 -> 10.9 ms, cubes at
+// N = 288 1.08 -> 0.11 ms; in FP64 cubes at N = 1152 6.3 -> 0.87 ms.
+constexpr int FAR_BATCH = 32;  // listed pairs whose moments are held at once
+
+template <int MODE>
+__global__ void __maxnreg__(168) far_pairs_group_kernel(const FillTask *__restrict__ tasks, int ntask, FarOpts o) {
+  typedef typename std::conditional<MODE == FILL_DF, df, double>::type T;
   __shared__ GreenDev s_g;
-  const int i = task_of_far(tasks, ntask, blockIdx.x);
-  const FillTask &tk = tasks[i];
-  if (threadIdx.x == 0 && threadIdx.y == 0) s_g = tk.g;
+  __shared__ V3<T> s_rho[8][6];
+  __shared__ FarStage<T> s_st[8], s_ss[8];
+  __shared__ T s_mom[FAR_BATCH][36];
+  __shared__ int2 s_list[256];
+  __shared__ int s_rule[256], s_n;
+  const int lane = threadIdx.x, wid = threadIdx.y, rows = blockDim.y;
+  const int ti = task_of_far(tasks, ntask, blockIdx.x);
+  const FillTask &tk = tasks[ti];
+  if (lane == 0 && wid == 0) {
+    s_g = tk.g;
+    s_n = 0;
+  }
+  int ta0, sb0;
+  far_tile_at(tk, (int64_t)blockIdx.x - tk.far0, rows, ta0, sb0);
+  const int ta = ta0 + wid, sb = sb0 + lane;
+  const bool sym = MODE != FILL_FP32_FAR && tk.sym;
+  if (lane < 6 && ta < tk.ntT) {
+    const TriDF *TD = tk.TD ? tk.TD + ta : nullptr;
+    const FarGeom<T> ge = far_geom<T>(tk.T[ta], tk.T[ta], TD, TD);
+    const RuleNode<T> n = far_node<T>(NODES6 + lane);
+    s_rho[wid][lane] = n.x1 * ge.a1 + n.x2 * ge.a2;
+  }
   __syncthreads();
-  const int64_t local = (int64_t)blockIdx.x - tk.far0;
-  const int bx = (int)(local % tk.far_tx), by = (int)(local / tk.far_tx);
-  far_pair_at(tk.T, tk.ntT, tk.S, tk.ntS, s_g, o, tk.H, tk.ntr, mode, tk.TD, tk.SD, bx * 32 + threadIdx.x,
-              by * blockDim.y + threadIdx.y);
+  const GreenT<T> g = green_of<T>(s_g);
+  const bool realk = s_g.ikr == 0.0 && s_g.ksqi == 0.0;
+  if (ta < tk.ntT && sb < tk.ntS && (!sym || ta > sb)) {
+    const TriRec &Tr = tk.T[ta];
+    const TriRec &Sr = tk.S[sb];
+    if (Tr.gid != Sr.gid && !shares_vertex(Tr.vid, Sr.vid)) {  // else the near kernel's
+      // far-rule choice, src/Impedance.cpp:329-360
+      const double d = dist2_rn(Tr.c, Sr.c);
+      const double e = fmax(Tr.emax, Sr.emax);
+      const double emax2 = __dmul_rn(e, e);
+      const int rule = __dmul_rn(d, o.th6) > emax2    ? 6
+                       : __dmul_rn(d, o.th10) > emax2 ? 10
+                       : __dmul_rn(d, o.th15) > emax2 ? 15
+                       : __dmul_rn(d, o.th21) > emax2 ? 21
+                                                      : 36;
+      if (MODE == FILL_FP32_FAR && d > 9.0 * emax2) {
+        // beyond 3 edge lengths every default threshold selects the 6-point
+        // rule; the others serve non-default Options
+        const double(*nodes)[3] = rule == 6 ? c_rule6 : rule == 10 ? c_rule10 : rule == 15 ? c_rule15
+                                  : rule == 21 ? c_rule21 : c_rule36;
+        far_pair_fp32(Tr, Sr, s_g, nodes, rule, tk.H, tk.ntr);
+      } else if (rule == 6) {
+        const TriDF *TD = tk.TD ? tk.TD + ta : nullptr, *SD = tk.SD ? tk.SD + sb : nullptr;
+        T M[36];
+        const FarGeom<T> ge = far_geom<T>(Tr, Sr, TD, SD);
+        if (realk) {
+          far_moments6<T, true>(ge, g, s_rho[wid], M);
+          T Mc[36];
+#pragma unroll
+          for (int k = 0; k < 36; k++) Mc[k] = M[k];
+          far_contract<T, true>(Tr, Sr, TD, SD, g, Mc, tk.H, tk.ntr, sym);
+        } else {
+          far_moments6<T, false>(ge, g, s_rho[wid], M);
+          T Mc[36];
+#pragma unroll
+          for (int k = 0; k < 36; k++) Mc[k] = M[k];
+          far_contract<T, false>(Tr, Sr, TD, SD, g, Mc, tk.H, tk.ntr, sym);
+        }
+      } else {
+        const int at = atomicAdd(&s_n, 1);
+        s_list[at] = make_int2(ta, sb);
+        s_rule[at] = rule;
+      }
+    }
+  }
+  __syncthreads();
+  const int n = s_n;
+  for (int b = 0; b < n; b += FAR_BATCH) {
+    const int m = min(FAR_BATCH, n - b);
+    for (int k = wid; k < m; k += rows) {
+      const int2 pr = s_list[b + k];
+      const int nr = s_rule[b + k];
+      const int off = nr == 10 ? NODES10 : nr == 15 ? NODES15 : nr == 21 ? NODES21 : NODES36;
+      const FarGeom<T> ge = far_geom<T>(tk.T[pr.x], tk.S[pr.y], tk.TD ? tk.TD + pr.x : nullptr,
+                                        tk.SD ? tk.SD + pr.y : nullptr);
+      if (realk)
+        far_moments_warp<T, true>(ge, g, off, nr, &s_st[wid], &s_ss[wid], s_mom[k], lane);
+      else
+        far_moments_warp<T, false>(ge, g, off, nr, &s_st[wid], &s_ss[wid], s_mom[k], lane);
+    }
+    __syncthreads();
+    if (wid == 0 && lane < m) {
+      const int2 pr = s_list[b + lane];
+      const TriDF *TD = tk.TD ? tk.TD + pr.x : nullptr, *SD = tk.SD ? tk.SD + pr.y : nullptr;
+      if (realk)
+        far_contract<T, true>(tk.T[pr.x], tk.S[pr.y], TD, SD, g, s_mom[lane], tk.H, tk.ntr, sym);
+      else
+        far_contract<T, false>(tk.T[pr.x], tk.S[pr.y], TD, SD, g, s_mom[lane], tk.H, tk.ntr, sym);
+    }
+    __syncthreads();
+  }
+}
+
+void launch_far(int mode, unsigned tiles, int rows, cudaStream_t st, const FillTask *tasks, int ntask, FarOpts fo) {
+  const dim3 blk(32, rows);
+  if (mode == FILL_DF)
+    far_pairs_group_kernel<FILL_DF><<<tiles, blk, 0, st>>>(tasks, ntask, fo);
+  else if (mode == FILL_FP32_FAR)
+    far_pairs_group_kernel<FILL_FP32_FAR><<<tiles, blk, 0, st>>>(tasks, ntask, fo);
+  else
+    far_pairs_group_kernel<FILL_FP64><<<tiles, blk, 0, st>>>(tasks, ntask, fo);
 }
 
 // ---------------- near pairs ----------------
@@ -1500,6 +1762,11 @@ void split_df(double x, float out[2]) {
   out[1] = (float)(x - (double)out[0]);
 }
 
+df host_df(double x) {
+  const float h = (float)x;
+  return {h, (float)(x - (double)h)};
+}
+
 GreenDev to_dev(const bemgpu_green_t *g) {
   GreenDev d;
   d.ikr = g->ik[0]; d.iki = g->ik[1];
@@ -1532,28 +1799,21 @@ int load_tables(bemgpu_ctx_s *ctx) {
   BEM_CUDA_TRY(ctx, cudaMemcpyToSymbol(c_rule105, bemgpu_tri_rule105, sizeof(bemgpu_tri_rule105)));
   BEM_CUDA_TRY(ctx, cudaMemcpyToSymbol(c_line15, bemgpu_line_rule15, sizeof(bemgpu_line_rule15)));
   {
-    auto split = [](const double (*rule)[3], int n, std::vector<float> &out) {
-      out.resize(6 * (size_t)n);
-      for (int i = 0; i < n; i++)
-        for (int c = 0; c < 3; c++) {
-          const float h = (float)rule[i][c];
-          out[6 * i + 2 * c] = h;
-          out[6 * i + 2 * c + 1] = (float)(rule[i][c] - (double)h);
-        }
-    };
-    std::vector<float> v;
-    split(bemgpu_tri_rule6, 6, v);
-    BEM_CUDA_TRY(ctx, cudaMemcpyToSymbol(c_rdf6, v.data(), sizeof(float) * v.size()));
-    split(bemgpu_tri_rule10, 10, v);
-    BEM_CUDA_TRY(ctx, cudaMemcpyToSymbol(c_rdf10, v.data(), sizeof(float) * v.size()));
-    split(bemgpu_tri_rule15, 15, v);
-    BEM_CUDA_TRY(ctx, cudaMemcpyToSymbol(c_rdf15, v.data(), sizeof(float) * v.size()));
-    split(bemgpu_tri_rule21, 21, v);
-    BEM_CUDA_TRY(ctx, cudaMemcpyToSymbol(c_rdf21, v.data(), sizeof(float) * v.size()));
-    split(bemgpu_tri_rule36, 36, v);
-    BEM_CUDA_TRY(ctx, cudaMemcpyToSymbol(c_rdf36, v.data(), sizeof(float) * v.size()));
-    split(bemgpu_tri_rule91, 91, v);
-    BEM_CUDA_TRY(ctx, cudaMemcpyToSymbol(c_rdf91, v.data(), sizeof(float) * v.size()));
+    const struct {
+      const double (*rule)[3];
+      int off, n;
+    } far[5] = {{bemgpu_tri_rule6, NODES6, 6}, {bemgpu_tri_rule10, NODES10, 10}, {bemgpu_tri_rule15, NODES15, 15},
+                {bemgpu_tri_rule21, NODES21, 21}, {bemgpu_tri_rule36, NODES36, 36}};
+    std::vector<RuleNode<double>> nd(NODES_FAR);
+    std::vector<RuleNode<df>> nf(NODES_FAR);
+    for (const auto &r : far)
+      for (int k = 0; k < r.n; k++) {
+        const double x1 = r.rule[k][0], x2 = r.rule[k][1], w = r.rule[k][2];
+        nd[r.off + k] = {x1, x2, w, w * x1, w * x2};
+        nf[r.off + k] = {host_df(x1), host_df(x2), host_df(w), host_df(w * x1), host_df(w * x2)};
+      }
+    BEM_CUDA_TRY(ctx, cudaMemcpyToSymbol(c_far_d, nd.data(), sizeof(RuleNode<double>) * nd.size()));
+    BEM_CUDA_TRY(ctx, cudaMemcpyToSymbol(c_far_f, nf.data(), sizeof(RuleNode<df>) * nf.size()));
   }
   // the copies from host memory may return before they land: every stream
   // of the device reads the tables from now on
@@ -1574,35 +1834,45 @@ int bem_fill_group(bemgpu_ctx_s *ctx, FillJob *jobs, int njobs, const bemgpu_opt
   const int fr = ctx->tune.far_rows;
   std::vector<FillTask> tasks(njobs);
   std::vector<const NearList *> lists(njobs);
+  // double-float records: one set per tree of the group
+  std::vector<const bemgpu_tree_s *> trees;
+  std::vector<size_t> tree_off;
   size_t ndf = 0;
+  auto records_of = [&](const bemgpu_tree_s *x) {
+    for (size_t k = 0; k < trees.size(); k++)
+      if (trees[k] == x) return tree_off[k];
+    trees.push_back(x);
+    tree_off.push_back(ndf);
+    ndf += x->ntri;
+    return tree_off.back();
+  };
   for (int i = 0; i < njobs; i++) {
     lists[i] = bem_near_list(ctx, jobs[i].t, jobs[i].s);
     if (!lists[i]) return bem_fail(ctx, BEMGPU_ERR_OOM, "near list allocation failed");
-    ndf += (size_t)jobs[i].t->ntri + jobs[i].s->ntri;
+    records_of(jobs[i].t);
+    records_of(jobs[i].s);
   }
-  TriDF *df = nullptr;
+  TriDF *df_rec = nullptr;
   if (mode == FILL_DF) {
-    df = (TriDF *)bem_workspace(ctx, "fill_tdf", sizeof(TriDF) * ndf);
-    if (!df) return bem_fail(ctx, BEMGPU_ERR_OOM, "fill: double-float records");
+    df_rec = (TriDF *)bem_workspace(ctx, "fill_tdf", sizeof(TriDF) * ndf);
+    if (!df_rec) return bem_fail(ctx, BEMGPU_ERR_OOM, "fill: double-float records");
   }
-  FillTask *dtasks = (FillTask *)bem_workspace(ctx, "fill_tasks", sizeof(FillTask) * (size_t)njobs);
+  // one upload: the tasks, then the records' jobs
+  const size_t tasks_bytes = sizeof(FillTask) * (size_t)njobs, tdf_bytes = sizeof(TriDFJob) * trees.size();
+  unsigned char *dtable = (unsigned char *)bem_workspace(ctx, "fill_tasks", tasks_bytes + tdf_bytes);
+  FillTask *dtasks = (FillTask *)dtable;
   if (!dtasks) return bem_fail(ctx, BEMGPU_ERR_OOM, "fill: task table");
   double far_flops = 0, far_bytes = 0, near_flops = 0, near_bytes = 0;
   int64_t far_tiles = 0, near_units = 0;
-  size_t dfo = 0;
   for (int i = 0; i < njobs; i++) {
     const bemgpu_tree_s *t = jobs[i].t, *s = jobs[i].s;
     FillTask &tk = tasks[i];
     tk.T = t->d_rec;
     tk.S = s->d_rec;
     tk.TD = tk.SD = nullptr;
-    if (df) {
-      tk.TD = df + dfo;
-      tk.SD = df + dfo + t->ntri;
-      tri_df_kernel<<<(t->ntri + 127) / 128, 128, 0, stream>>>(t->d_rec, t->ntri, df + dfo);
-      tri_df_kernel<<<(s->ntri + 127) / 128, 128, 0, stream>>>(s->d_rec, s->ntri, df + dfo + t->ntri);
-      ctx->launches += 2;
-      dfo += (size_t)t->ntri + s->ntri;
+    if (df_rec) {
+      tk.TD = df_rec + records_of(t);
+      tk.SD = df_rec + records_of(s);
     }
     tk.near = lists[i]->d;
     tk.nnear = lists[i]->n;
@@ -1612,7 +1882,8 @@ int bem_fill_group(bemgpu_ctx_s *ctx, FillJob *jobs, int njobs, const bemgpu_opt
     tk.ntr = t->nrwg;
     tk.far_tx = (s->ntri + 31) / 32;
     tk.far0 = far_tiles;
-    far_tiles += (int64_t)tk.far_tx * ((t->ntri + fr - 1) / fr);
+    tk.sym = t == s && mode != FILL_FP32_FAR;
+    far_tiles += far_tiles_of(tk.sym, t->ntri, s->ntri, fr);
     tk.near0 = near_units;
     near_units += mode == FILL_DF ? (tk.nnear + 1) / 2 : tk.nnear;  // the df kernel works pair couples
     tk.g = to_dev(&jobs[i].g);
@@ -1629,13 +1900,25 @@ int bem_fill_group(bemgpu_ctx_s *ctx, FillJob *jobs, int njobs, const bemgpu_opt
       near_bytes += (double)tk.nnear * 9.0 * BEM_HALFPAIR_BYTES_FP64;
     }
   }
-  // the table is copied from this call's host vector before the call returns
-  BEM_CUDA_TRY(ctx, cudaMemcpyAsync(dtasks, tasks.data(), sizeof(FillTask) * (size_t)njobs, cudaMemcpyHostToDevice,
-                                    stream));
+  // the tables are copied from this call's host vector before the call returns
+  std::vector<unsigned char> table(tasks_bytes + tdf_bytes);
+  memcpy(table.data(), tasks.data(), tasks_bytes);
+  int most = 0;
+  for (size_t k = 0; k < trees.size(); k++) {
+    const TriDFJob jb = {trees[k]->d_rec, df_rec ? df_rec + tree_off[k] : nullptr, trees[k]->ntri};
+    memcpy(table.data() + tasks_bytes + k * sizeof(TriDFJob), &jb, sizeof jb);
+    most = std::max(most, jb.n);
+  }
+  BEM_CUDA_TRY(ctx, cudaMemcpyAsync(dtable, table.data(), table.size(), cudaMemcpyHostToDevice, stream));
+  if (df_rec) {
+    tri_df_kernel<<<dim3((most + 127) / 128, (unsigned)trees.size()), 128, 0, stream>>>(
+        (const TriDFJob *)(dtable + tasks_bytes));
+    ctx->launches++;
+  }
   if (far_tiles > 0) {
     if (far_tiles > 0x7fffffffll) return bem_fail(ctx, BEMGPU_ERR_ARG, "fill: %lld far tiles", (long long)far_tiles);
     ProfScope ps(ctx, BEMGPU_K_FILL_FAR, stream, far_flops, far_bytes);
-    far_pairs_group_kernel<<<(unsigned)far_tiles, dim3(32, fr), 0, stream>>>(dtasks, njobs, fo, mode);
+    launch_far(mode, (unsigned)far_tiles, fr, stream, dtasks, njobs, fo);
     ctx->launches++;
   }
   BEM_CUDA_TRY(ctx, cudaGetLastError());
@@ -1766,10 +2049,12 @@ namespace {
 constexpr size_t NOALLOC_SCRATCH_BYTES = 32u << 20;   // 32 MiB
 constexpr size_t NOALLOC_NEAR_BYTES = 2u << 20;       // first 2 MiB: the near-pair list
 static __device__ __align__(256) unsigned char g_noalloc_scratch[NOALLOC_SCRATCH_BYTES];
+static __device__ __align__(256) unsigned char g_noalloc_task[sizeof(FillTask)];
 
 std::mutex g_noalloc_mu;
 std::mutex g_noalloc_run_mu;  // one call at a time uses the shared scratch
 void *g_noalloc_addr[BEM_MAX_DEVICES] = {nullptr};
+void *g_noalloc_task_addr[BEM_MAX_DEVICES] = {nullptr};
 
 }  // namespace
 
@@ -1802,6 +2087,7 @@ extern "C" int bemgpu_zts_noalloc(bemgpu_ctx_t ctx, bemgpu_tree_t t, bemgpu_tree
   // Set-up, once per device with that device current: the host-side name of
   // the array is not a device address; ask the runtime for the address.
   unsigned char *base = nullptr;
+  FillTask *dtask = nullptr;
   {
     std::lock_guard<std::mutex> lk2(g_noalloc_mu);
     if (!g_noalloc_addr[ctx->device]) {
@@ -1809,9 +2095,15 @@ extern "C" int bemgpu_zts_noalloc(bemgpu_ctx_t ctx, bemgpu_tree_t t, bemgpu_tree
       cudaError_t e = cudaGetSymbolAddress(&p, g_noalloc_scratch);
       if (e != cudaSuccess || !p)
         return bem_fail(ctx, BEMGPU_ERR_CUDA, "zts_noalloc: cudaGetSymbolAddress failed: %s", cudaGetErrorString(e));
+      void *q = nullptr;
+      e = cudaGetSymbolAddress(&q, g_noalloc_task);
+      if (e != cudaSuccess || !q)
+        return bem_fail(ctx, BEMGPU_ERR_CUDA, "zts_noalloc: cudaGetSymbolAddress failed: %s", cudaGetErrorString(e));
       g_noalloc_addr[ctx->device] = p;
+      g_noalloc_task_addr[ctx->device] = q;
     }
     base = (unsigned char *)g_noalloc_addr[ctx->device];
+    dtask = (FillTask *)g_noalloc_task_addr[ctx->device];
   }
   int rc = load_tables(ctx);
   if (rc) return rc;
@@ -1824,10 +2116,20 @@ extern "C" int bemgpu_zts_noalloc(bemgpu_ctx_t ctx, bemgpu_tree_t t, bemgpu_tree
   // so nothing left by an earlier call needs clearing.
   const GreenDev gd = to_dev(g);
   const FarOpts fo = {o.farThresh6, o.farThresh10, o.farThresh15, o.farThresh21};
-  dim3 blk(32, 4);
-  dim3 grd((s->ntri + 31) / 32, (t->ntri + 3) / 4);
-  far_pairs_kernel<<<grd, blk, 0, st>>>(t->d_rec, t->ntri, s->d_rec, s->ntri, gd, fo, H, t->nrwg, FILL_FP64, nullptr,
-                                        nullptr);
+  FillTask task = {};
+  task.T = t->d_rec;
+  task.S = s->d_rec;
+  task.near = dnear;
+  task.H = H;
+  task.nnear = (int64_t)pairs.size();
+  task.ntT = t->ntri;
+  task.ntS = s->ntri;
+  task.ntr = t->nrwg;
+  task.far_tx = (s->ntri + 31) / 32;
+  task.sym = t == s;
+  task.g = gd;
+  BEM_CUDA_TRY(ctx, cudaMemcpyAsync(dtask, &task, sizeof task, cudaMemcpyHostToDevice, st));
+  launch_far(FILL_FP64, (unsigned)far_tiles_of(task.sym, t->ntri, s->ntri, 4), 4, st, dtask, 1, fo);
   ctx->launches++;
   if (!pairs.empty()) {
     const int64_t np = (int64_t)pairs.size();

@@ -236,11 +236,14 @@ __global__ void tri_records_kernel(const double *__restrict__ xyz, const int *__
       }
   r.gid = tri0 + t;
   r.nh = 3;
+  int rot0 = 0;
   for (int h = 0; h < 3; h++) {
     const int i = hr[h];
     const int e1 = rwg[4 * i + 2], e2 = rwg[4 * i + 3];
     const int rot = (tv[0] != e1 && tv[0] != e2) ? 0 : ((tv[1] != e1 && tv[1] != e2) ? 1 : 2);
     const D3 p0 = dvtx(xyz, tv[rot]), p1 = dvtx(xyz, tv[(rot + 1) % 3]), p2 = dvtx(xyz, tv[(rot + 2) % 3]);
+    if (h == 0) rot0 = rot;
+    r.hvert |= ((rot - rot0 + 3) % 3) << (2 * h);
     dput(r.hp0[h], p0);
     r.helen[h] = __dsqrt_rn(dnorm2(dsub(dvtx(xyz, e2), dvtx(xyz, e1))));
     r.hrwg[h] = i;
@@ -398,6 +401,7 @@ extern "C" int bemgpu_tree_create_body_device(bemgpu_geom_t g, int tri0, int ntr
   }
   t->tri_gid.resize(ntri);
   for (int k = 0; k < ntri; k++) t->tri_gid[k] = t->host_rec[k].gid;
+  t->set_emax();
   // the records stay on the device: the tree takes the buffer over
   for (auto it = B.p.begin(); it != B.p.end(); ++it)
     if (*it == (void *)recs) {
@@ -430,6 +434,7 @@ extern "C" int bemgpu_tree_concat(bemgpu_tree_t a, bemgpu_tree_t b, bemgpu_tree_
     for (int h = 0; h < r.nh; h++) r.hrwg[h] += a->nrwg;
     t->host_rec.push_back(r);
   }
+  t->set_emax();
   cudaSetDevice(ctx->device);
   if (cudaMalloc(&t->d_rec, sizeof(TriRec) * t->ntri) != cudaSuccess) {
     cudaGetLastError();
