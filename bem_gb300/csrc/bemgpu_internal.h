@@ -111,7 +111,7 @@ struct bemgpu_ctx_s {
   // launch shapes chosen by the autotuner (bemgpu_ctx_set_tuning); the
   // defaults are the measured best on the N = 7680 icosphere workload
   struct Tuning {
-    int near_minb = 2;   // CTAs per SM of the double-float near-pair kernel's register budget (2, 3, 4)
+    int near_minb = 3;   // CTAs per SM of the double-float near-pair kernel's register budget (2, 3, 4)
     int far_rows = 4;    // warps per CTA of the far-pair kernel (1, 2, 4, 8)
     int raster = 8;      // M-tiles per rasterization band of the tensor-core products (1..64)
     int panel_ctas = 0;  // CTAs of a cooperative LU panel at most (0: one per SM)

@@ -172,7 +172,8 @@ __device__ __forceinline__ df inv_fact(int n) { return {DF_FACT_HI[n], DF_FACT_L
 
 // sin r, cos r for |r| <= pi/4 + a little (df): Taylor series in s = r^2,
 // sin up to r^17, cos up to r^18; terms below 2^-25 of the result in FP32.
-__device__ __forceinline__ void df_sincos_reduced(df r, df &sn, df &cs) {
+// sm: sin r - r, accurate relative to itself.
+__device__ __forceinline__ void df_sincos_reduced(df r, df &sn, df &cs, df &sm) {
   const df s = df_sqr(r);
   const float sf = s.hi;
   // FP32 tails: sin coefficients of r^17 .. r^11, cos of r^18 .. r^12 (signs alternate)
@@ -190,7 +191,9 @@ __device__ __forceinline__ void df_sincos_reduced(df r, df &sn, df &cs) {
   ps = df_horner(ps, s, df_neg(inv_fact(5)));
   ps = df_horner(ps, s, inv_fact(3));
   // ps = 1/3! - s/5! + ...: sin = r - r s ps
-  sn = df_fin(df_horner(df_neg(ps), df_mul(r, s), r));
+  sm = df_mul(df_neg(ps), df_mul(r, s));
+  sn = {r.hi + sm.hi, 0.f};
+  sn = fast_two_sum(sn.hi, (sm.hi - (sn.hi - r.hi)) + (r.lo + sm.lo));
   df pc = df_horner_f(tc, s, inv_fact(10));
   pc = df_horner(pc, s, df_neg(inv_fact(8)));
   pc = df_horner(pc, s, inv_fact(6));
@@ -224,8 +227,8 @@ __device__ __forceinline__ df df_expm1_reduced(df r) {
 __device__ __forceinline__ void df_sincos(double x, df &sn, df &cs) {
   const double n = rint(x * DF_TWO_OVER_PI);
   const double r = fma(-n, DF_PIO2_LO, fma(-n, DF_PIO2_HI, x));
-  df s, c;
-  df_sincos_reduced(df_make(r), s, c);
+  df s, c, m;
+  df_sincos_reduced(df_make(r), s, c, m);
   const int q = ((int)n) & 3;
   if (q == 0) { sn = s; cs = c; }
   else if (q == 1) { sn = c; cs = df_neg(s); }
@@ -253,25 +256,40 @@ __device__ __forceinline__ df df_reduce(df x, float n, float c0, float c1, float
 }
 
 // (sin x, cos x) for a df argument, |x| < 200 (quadrant count below 2^8),
-// everything on the FP32 pipes.
-__device__ __forceinline__ void df_sincos_df(df x, df &sn, df &cs) {
+// everything on the FP32 pipes; sm: sin x - x, accurate relative to itself
+// where x needs no reduction.
+__device__ __forceinline__ void df_sincos_df(df x, df &sn, df &cs, df &sm) {
   const float n = rintf(x.hi * DF_TWO_OVER_PI_F);
   const df r = df_reduce(x, n, DF_PIO2_F0, DF_PIO2_F1, DF_PIO2_F2);
-  df s, c;
-  df_sincos_reduced(r, s, c);
+  df s, c, m;
+  df_sincos_reduced(r, s, c, m);
   const int q = ((int)n) & 3;
   if (q == 0) { sn = s; cs = c; }
   else if (q == 1) { sn = c; cs = df_neg(s); }
   else if (q == 2) { sn = df_neg(s); cs = df_neg(c); }
   else { sn = df_neg(c); cs = s; }
+  const df d = df_sub(sn, x);
+  sm = n == 0.f ? m : d;
+}
+__device__ __forceinline__ void df_sincos_df(df x, df &sn, df &cs) {
+  df sm;
+  df_sincos_df(x, sn, cs, sm);
 }
 
-// e^x for a df argument, -85 < x < 85, on the FP32 pipes.
-__device__ __forceinline__ df df_exp_df(df x) {
+// e^x for a df argument, -85 < x < 85, on the FP32 pipes; m1: e^x - 1,
+// accurate relative to itself where x needs no reduction.
+__device__ __forceinline__ df df_exp_df(df x, df &m1) {
   const float n = rintf(x.hi * DF_LOG2E_F);
   const df r = df_reduce(x, n, DF_LN2_F0, DF_LN2_F1, DF_LN2_F2);
-  const df e = df_add_f(df_expm1_reduced(r), 1.f);
-  return df_scale2(e, __int_as_float((127 + (int)n) << 23));
+  const df em1 = df_expm1_reduced(r);
+  const df e = df_scale2(df_add_f(em1, 1.f), __int_as_float((127 + (int)n) << 23));
+  const df d = df_add_f(e, -1.f);
+  m1 = n == 0.f ? em1 : d;
+  return e;
+}
+__device__ __forceinline__ df df_exp_df(df x) {
+  df m1;
+  return df_exp_df(x, m1);
 }
 
 __device__ __forceinline__ df df_abs(df a) { return a.hi < 0.f ? df_neg(a) : a; }

@@ -11,11 +11,10 @@
 //     one.  Both triangles of a far pair take the same rule, so L and K are
 //     symmetric in the pair: a fill of a tree against itself integrates each
 //     unordered pair once and writes both its places.
-//   * near pairs (same triangle or a shared vertex): one warp per pair, lanes over
-//     the 105 outer nodes, each lane runs the 91-node smooth inner rule, the
-//     analytic singular terms (EHNonSmoothIntegral, src/Source.cpp:16-86) and the
-//     close-pair contraction of src/Impedance.cpp:194-250 in FP64; the
-//     neighbour-edge K correction (src/Impedance.cpp:301-324) runs on the same warp.
+//   * near pairs (same triangle or a shared vertex): one warp per pair, which
+//     reduces the smooth inner rule and the closed-form singular terms to real
+//     moments (powers of R: no frequency in them) and serves the exterior and
+//     the interior Green's function of a body in one pass; see near_pairs_kernel.
 //   * every pair writes its nine (c L_ij, c K_ij) half-pair products into a
 //     half-pair block array H (one 128-byte block per RWG pair (i, j), four
 //     slots for (pos/neg test half) x (pos/neg source half)); each slot has
@@ -24,8 +23,10 @@
 //     coalesced stores (src/Impedance.cpp:365-384).
 #include "bemgpu_internal.h"
 #include "quadrature_tables.h"
+#include "even_rules.h"
 #include "fill_num.cuh"
 
+#include <algorithm>
 #include <cmath>
 #include <cstring>
 #include <type_traits>
@@ -58,6 +59,12 @@ struct RuleNode {
 enum { NODES6 = 0, NODES10 = 6, NODES15 = 16, NODES21 = 31, NODES36 = 52, NODES_FAR = 88 };
 __constant__ RuleNode<double> c_far_d[NODES_FAR];
 __constant__ RuleNode<df> c_far_f[NODES_FAR];
+// Sums of {w, w x1, w x2} per rule, and the square of the weights' sum less one.
+enum { SUM6, SUM10, SUM15, SUM21, SUM36, SUM91, SUM105, NSUMS };
+struct RuleSum {
+  double w[3], ww1;
+};
+__constant__ RuleSum c_sums[NSUMS];
 template <typename T>
 __device__ __forceinline__ RuleNode<T> far_node(int k);
 template <>
@@ -69,8 +76,6 @@ __constant__ double c_rule10[10][3];
 __constant__ double c_rule15[15][3];
 __constant__ double c_rule21[21][3];
 __constant__ double c_rule36[36][3];
-__constant__ double c_rule91[91][3];
-__constant__ double c_rule105[105][3];
 __constant__ double c_line15[15][2];
 
 // ---------------- small FP64 vector / complex helpers ----------------
@@ -80,56 +85,12 @@ struct d3 {
 struct z1 {
   double r, i;
 };
-struct z3 {
-  z1 x, y, z;
-};
 
 __device__ __forceinline__ d3 ld3(const double *p) { return {p[0], p[1], p[2]}; }
-__device__ __forceinline__ d3 operator+(d3 a, d3 b) { return {a.x + b.x, a.y + b.y, a.z + b.z}; }
 __device__ __forceinline__ d3 operator-(d3 a, d3 b) { return {a.x - b.x, a.y - b.y, a.z - b.z}; }
-__device__ __forceinline__ d3 operator*(double c, d3 a) { return {c * a.x, c * a.y, c * a.z}; }
 __device__ __forceinline__ double dot(d3 a, d3 b) { return a.x * b.x + a.y * b.y + a.z * b.z; }
-__device__ __forceinline__ d3 cross(d3 a, d3 b) {
-  return {a.y * b.z - a.z * b.y, a.z * b.x - a.x * b.z, a.x * b.y - a.y * b.x};
-}
 __device__ __forceinline__ z1 zmul(z1 a, z1 b) { return {a.r * b.r - a.i * b.i, a.r * b.i + a.i * b.r}; }
 __device__ __forceinline__ z1 zadd(z1 a, z1 b) { return {a.r + b.r, a.i + b.i}; }
-__device__ __forceinline__ z1 zsub(z1 a, z1 b) { return {a.r - b.r, a.i - b.i}; }
-__device__ __forceinline__ z1 zscale(double c, z1 a) { return {c * a.r, c * a.i}; }
-__device__ __forceinline__ z3 z3zero() { return {{0, 0}, {0, 0}, {0, 0}}; }
-// complex scalar times real vector
-__device__ __forceinline__ z3 zs_v(z1 c, d3 v) { return {{c.r * v.x, c.i * v.x}, {c.r * v.y, c.i * v.y}, {c.r * v.z, c.i * v.z}}; }
-__device__ __forceinline__ z3 z3add(z3 a, z3 b) { return {zadd(a.x, b.x), zadd(a.y, b.y), zadd(a.z, b.z)}; }
-__device__ __forceinline__ z3 z3sub(z3 a, z3 b) { return {zsub(a.x, b.x), zsub(a.y, b.y), zsub(a.z, b.z)}; }
-__device__ __forceinline__ z3 z3add_r(z3 a, d3 b) { return {{a.x.r + b.x, a.x.i}, {a.y.r + b.y, a.y.i}, {a.z.r + b.z, a.z.i}}; }
-__device__ __forceinline__ z3 z3scale(double c, z3 a) { return {zscale(c, a.x), zscale(c, a.y), zscale(c, a.z)}; }
-// dot(real, complex) — no conjugation (ComplexVector3.h:124-126)
-__device__ __forceinline__ z1 rdot(d3 a, z3 b) {
-  return {a.x * b.x.r + a.y * b.y.r + a.z * b.z.r, a.x * b.x.i + a.y * b.y.i + a.z * b.z.i};
-}
-// complex x real cross product
-__device__ __forceinline__ z3 zcross(z3 a, d3 b) {
-  return {{a.y.r * b.z - a.z.r * b.y, a.y.i * b.z - a.z.i * b.y},
-          {a.z.r * b.x - a.x.r * b.z, a.z.i * b.x - a.x.i * b.z},
-          {a.x.r * b.y - a.y.r * b.x, a.x.i * b.y - a.y.i * b.x}};
-}
-// real x complex cross product
-__device__ __forceinline__ z3 rcross(d3 a, z3 b) {
-  return {{a.y * b.z.r - a.z * b.y.r, a.y * b.z.i - a.z * b.y.i},
-          {a.z * b.x.r - a.x * b.z.r, a.z * b.x.i - a.x * b.z.i},
-          {a.x * b.y.r - a.y * b.x.r, a.x * b.y.i - a.y * b.x.i}};
-}
-__device__ __forceinline__ void zacc(z1 &a, z1 b) { a.r += b.r; a.i += b.i; }
-
-// exp(ikR) for real R: exp(Re(ik) R) * (cos(Im(ik) R), sin(Im(ik) R)).  A
-// lossless medium (real k: the exterior fill) skips the exp, whose value is 1.
-__device__ __forceinline__ z1 zexp_ikR(const GreenDev &g, double R) {
-  double s, c;
-  sincos(g.iki * R, &s, &c);
-  if (g.ikr == 0.0) return {c, s};
-  const double m = exp(g.ikr * R);
-  return {m * c, m * s};
-}
 
 __device__ __forceinline__ int shares_vertex(const int *a, const int *b) {
   int c = 0;
@@ -164,36 +125,6 @@ __device__ __forceinline__ void store_block_df(HalfPairBlock *H, int ntr, int i,
 __device__ __forceinline__ double scatter_coef(const TriRec &T, int i, const TriRec &S, int j) {
   double c = BEM_ONEOVER4PI * T.helen[i] * S.helen[j];
   return (T.hneg[i] != S.hneg[j]) ? -c : c;
-}
-
-struct df3 {
-  df x, y, z;
-};
-__device__ __forceinline__ df3 df3_make(d3 a) { return {df_make(a.x), df_make(a.y), df_make(a.z)}; }
-
-// e^{ikR} for the df distance R: (cos, sin)(Im(ik) R) e^{Re(ik) R}, all in df on
-// the FP32 pipes (FP64 reductions for phases of 200 rad and more).
-__device__ __forceinline__ void df_exp_ikR(const GreenDev &g, df ikr, df iki, df R, df &er, df &ei) {
-  df sn, cs;
-  const df th = df_mul(iki, R);
-  if (fabsf(th.hi) < 200.f)
-    df_sincos_df(th, sn, cs);
-  else
-    df_sincos(df_to_double(th), sn, cs);
-  if (ikr.hi == 0.f) {  // real k (df_make keeps zero exactly): no FP64 compare per node
-    er = cs;
-    ei = sn;
-    return;
-  }
-  const df a = df_mul(ikr, R);
-  if (a.hi < -85.f) {  // below FP32's range: e^-85 of the neighbouring nodes' size
-    er = {0.f, 0.f};
-    ei = {0.f, 0.f};
-    return;
-  }
-  const df m = df_exp_df(a);
-  er = df_mul(m, cs);
-  ei = df_mul(m, sn);
 }
 
 // What a far pair reads of a triangle in double-float, built once per fill.
@@ -232,46 +163,6 @@ __global__ void tri_df_kernel(const TriDFJob *__restrict__ jobs) {
   }
 }
 
-struct cdf {
-  df r, i;
-};
-struct cdf3 {
-  cdf x, y, z;
-};
-__device__ __forceinline__ df3 df3_add(df3 a, df3 b) { return {df_add(a.x, b.x), df_add(a.y, b.y), df_add(a.z, b.z)}; }
-__device__ __forceinline__ df3 df3_sub(df3 a, df3 b) { return {df_sub(a.x, b.x), df_sub(a.y, b.y), df_sub(a.z, b.z)}; }
-__device__ __forceinline__ df3 df3_scale(df s, df3 a) { return {df_mul(s, a.x), df_mul(s, a.y), df_mul(s, a.z)}; }
-__device__ __forceinline__ df df3_dot(df3 a, df3 b) {
-  return df_add(df_add(df_mul(a.x, b.x), df_mul(a.y, b.y)), df_mul(a.z, b.z));
-}
-__device__ __forceinline__ df3 df3_cross(df3 a, df3 b) {
-  return {df_sub(df_mul(a.y, b.z), df_mul(a.z, b.y)), df_sub(df_mul(a.z, b.x), df_mul(a.x, b.z)),
-          df_sub(df_mul(a.x, b.y), df_mul(a.y, b.x))};
-}
-__device__ __forceinline__ cdf cdf_add(cdf a, cdf b) { return {df_add(a.r, b.r), df_add(a.i, b.i)}; }
-__device__ __forceinline__ cdf cdf_sub(cdf a, cdf b) { return {df_sub(a.r, b.r), df_sub(a.i, b.i)}; }
-__device__ __forceinline__ cdf cdf_scale(df s, cdf a) { return {df_mul(s, a.r), df_mul(s, a.i)}; }
-__device__ __forceinline__ cdf cdf_mul(cdf a, cdf b) {
-  return {df_sub(df_mul(a.r, b.r), df_mul(a.i, b.i)), df_add(df_mul(a.r, b.i), df_mul(a.i, b.r))};
-}
-__device__ __forceinline__ cdf3 cdf3_add(cdf3 a, cdf3 b) { return {cdf_add(a.x, b.x), cdf_add(a.y, b.y), cdf_add(a.z, b.z)}; }
-__device__ __forceinline__ cdf3 cdf3_sub(cdf3 a, cdf3 b) { return {cdf_sub(a.x, b.x), cdf_sub(a.y, b.y), cdf_sub(a.z, b.z)}; }
-__device__ __forceinline__ cdf3 cdf_v(cdf c, df3 v) { return {cdf_scale(v.x, c), cdf_scale(v.y, c), cdf_scale(v.z, c)}; }
-__device__ __forceinline__ cdf3 cdf3_scale(df s, cdf3 a) { return {cdf_scale(s, a.x), cdf_scale(s, a.y), cdf_scale(s, a.z)}; }
-__device__ __forceinline__ cdf cdf_rdot(df3 a, cdf3 b) {
-  return cdf_add(cdf_add(cdf_scale(a.x, b.x), cdf_scale(a.y, b.y)), cdf_scale(a.z, b.z));
-}
-// (complex vector) x (real vector)
-__device__ __forceinline__ cdf3 cdf_zcross(cdf3 a, df3 b) {
-  return {cdf_sub(cdf_scale(b.z, a.y), cdf_scale(b.y, a.z)), cdf_sub(cdf_scale(b.x, a.z), cdf_scale(b.z, a.x)),
-          cdf_sub(cdf_scale(b.y, a.x), cdf_scale(b.x, a.y))};
-}
-// (real vector) x (complex vector)
-__device__ __forceinline__ cdf3 cdf_rcross(df3 a, cdf3 b) {
-  return {cdf_sub(cdf_scale(a.y, b.z), cdf_scale(a.z, b.y)), cdf_sub(cdf_scale(a.z, b.x), cdf_scale(a.x, b.z)),
-          cdf_sub(cdf_scale(a.x, b.y), cdf_scale(a.y, b.x))};
-}
-
 // Green's function constants in the fill's number type.
 template <typename T>
 struct GreenT {
@@ -290,12 +181,20 @@ __device__ __forceinline__ GreenT<df> green_of<df>(const GreenDev &g) {
 }
 
 // (er, ei) = e^{ikR} and (ur, ui) = e^{ikR} (1 - ikR).  REALK: a lossless
-// medium (ik imaginary), whose e^{ikR} has modulus one.
+// medium (ik imaginary), whose e^{ikR} has modulus one.  em: Im e^{ikR}, in
+// double-float less Im(ik) R.
+//
+// The double-float fill keeps Im g = Im e^{ikR}/R less its constant Im(ik).  An
+// RWG pair is the signed sum of four half-pair terms in which that constant's
+// share of -U0 cancels exactly, while what is left is only ~(kR)^2/6 of it: the
+// sum keeps as many more digits.  These decide the (small) dissipation that an
+// ill-conditioned solve rests on.  What each rule's weights leave of the
+// constant (their sum is 1 to ~1e-13) stays.
 template <typename T, bool REALK>
-__device__ __forceinline__ void wave_at(const GreenT<T> &g, T R, T &er, T &ei, T &ur, T &ui) {
+__device__ __forceinline__ void wave_at(const GreenT<T> &g, T R, T &er, T &ei, T &em, T &ur, T &ui) {
   typedef Num<T> N;
   const T th = g.iki * R;
-  N::sincos_(th, ei, er);
+  N::sincos_(th, ei, er, em);
   if (REALK) {
     ur = N::muladd(ei, th, er);
     ui = N::muladd(-er, th, ei);
@@ -305,26 +204,29 @@ __device__ __forceinline__ void wave_at(const GreenT<T> &g, T R, T &er, T &ei, T
   if (N::head(a) < -85) {  // below FP32's range: e^-85 of the neighbouring nodes' size
     const T z = N::of(0.0);
     er = ei = ur = ui = z;
+    em = N::LESS ? -th : z;
     return;
   }
-  const T m = N::exp_(a);
+  T m1;
+  const T m = N::exp_(a, m1);
   er = m * er;
   ei = m * ei;
+  em = N::LESS ? N::dot2(m, em, th, m1) : ei;
   const T om = N::of(1.0) - a;
   ur = N::dot2(er, om, ei, th);
   ui = N::dot2(ei, om, -er, th);
 }
 
 // scalar_gradient, src/GreensFunction.cpp:41-52, at the (unnormalized)
-// difference x: f = {Re g, Im g, Re q, Im q}.
+// difference x: f = {Re g, Im g (less Im(ik), see wave_at), Re q, Im q}.
 template <typename T, bool REALK>
 __device__ __forceinline__ void far_values(const GreenT<T> &g, V3<T> x, T (&f)[4]) {
   typedef Num<T> N;
-  T R, Ri, er, ei, ur, ui;
+  T R, Ri, er, ei, em, ur, ui;
   N::sqrt_rcp(N::sumsq(x.x, x.y, x.z), R, Ri);
-  wave_at<T, REALK>(g, R, er, ei, ur, ui);
+  wave_at<T, REALK>(g, R, er, ei, em, ur, ui);
   f[0] = er * Ri;
-  f[1] = ei * Ri;
+  f[1] = em * Ri;
   const T Ri3 = Ri * (Ri * Ri);
   f[2] = ur * Ri3;
   f[3] = ui * Ri3;
@@ -490,10 +392,11 @@ __device__ __forceinline__ void store_pair(HalfPairBlock *H, int ntr, int i, int
 // tetrahedra on an edge of each triangle:
 //   K_vw = -1/4 sum_{v' != v, w' != w} B_v'w' (P_v - S_w) . ((S_w' - S_w) x (P_v' - P_v)),
 // nine volumes for the nine edge pairs (src/Impedance.cpp:154-168 summed over
-// the outer rule).  mirror: the pair's transposed place too.
+// the outer rule).  sum: the rule's, for the constant of Im g (wave_at).
+// mirror: the pair's transposed place too.
 template <typename T, bool REALK>
 __device__ __noinline__ void far_contract(const TriRec &T_, const TriRec &S, const TriDF *TD, const TriDF *SD,
-                                          const GreenT<T> &g, const T *M, HalfPairBlock *H, int ntr, bool mirror) {
+                                          const GreenT<T> &g, const T *M, int sum, HalfPairBlock *H, int ntr, bool mirror) {
   typedef Num<T> N;
   const FarGeom<T> ge = far_geom<T>(T_, S, TD, SD);
   const V3<T> a[2] = {ge.a1, ge.a2}, cs[2] = {ge.c1, ge.c2};
@@ -503,6 +406,16 @@ __device__ __noinline__ void far_contract(const TriRec &T_, const TriRec &S, con
   for (int x = 0; x < 3; x++)
 #pragma unroll
     for (int y = 0; y < 3; y++) G[x][y] = {M[x * 3 + y], M[9 + x * 3 + y]};
+  C1<T> U0 = G[0][0];
+  if (N::LESS) {
+    U0.i = U0.i + g.iki * N::of(c_sums[sum].ww1);
+#pragma unroll
+    for (int x = 0; x < 3; x++) {
+      const T kw = g.iki * N::of(c_sums[sum].w[x]);
+#pragma unroll
+      for (int y = 0; y < 3; y++) G[x][y].i = N::muladd(kw, N::of(c_sums[sum].w[y]), G[x][y].i);
+    }
+  }
   C1<T> br[3][3];
   {
     C1<T> U1 = {N::of(0.0), N::of(0.0)}, dU2[2] = {U1, U1}, eU3[2] = {U1, U1}, ed[2][2];
@@ -583,9 +496,9 @@ __device__ __noinline__ void far_contract(const TriRec &T_, const TriRec &S, con
       K = {N::pow2(N::fin(K.r), 0.25f), N::pow2(N::fin(K.i), 0.25f)};
       C1<T> L;
       if (REALK)
-        L = {N::muladd(ksr, br[v][w].r, -G[0][0].r), N::muladd(ksr, br[v][w].i, -G[0][0].i)};
+        L = {N::muladd(ksr, br[v][w].r, -U0.r), N::muladd(ksr, br[v][w].i, -U0.i)};
       else
-        L = cmul(C1<T>{ksr, ksi}, br[v][w]) - G[0][0];
+        L = cmul(C1<T>{ksr, ksi}, br[v][w]) - U0;
       for (int hi = at[v]; hi; hi &= hi - 1)
         for (int hj = as[w]; hj; hj &= hj - 1) {
           const int i = __ffs(hi) - 1, j = __ffs(hj) - 1;
@@ -725,15 +638,12 @@ __device__ __noinline__ void far_pair_fp32(const TriRec &T, const TriRec &S, con
   }
 }
 
-// One fill of a group launch: Zts(t, s, g) into the half-pair blocks H, with
-// its share of the group's far tiles and near work units (prefix offsets).
+// The far pairs of one fill of a group launch: Zts(t, s, g) into the half-pair
+// blocks H, with its share of the group's far tiles (prefix offset).
 struct FillTask {
   const TriRec *T, *S;       // test and source trees' records
   const TriDF *TD, *SD;      // their double-float records (double-float mode), else null
-  const NearPair *near;      // the near-pair list of (t, s)
   HalfPairBlock *H;          // this fill's half-pair blocks
-  int64_t nnear;             // near pairs
-  int64_t near0;             // first near work unit of the group that is this task's
   int64_t far0;              // first far tile of the group that is this task's
   int ntT, ntS, ntr, far_tx; // triangles of t and s, RWGs of t, far tiles along s
   int sym;                   // t is s: each unordered far pair is integrated once
@@ -743,12 +653,6 @@ struct FillTask {
 __device__ __forceinline__ int task_of_far(const FillTask *tk, int n, int64_t u) {
   int i = n - 1;
   while (i > 0 && u < tk[i].far0) i--;
-  return i;
-}
-
-__device__ __forceinline__ int task_of_near(const FillTask *tk, int n, int64_t u) {
-  int i = n - 1;
-  while (i > 0 && u < tk[i].near0) i--;
   return i;
 }
 
@@ -799,7 +703,8 @@ __device__ __forceinline__ void far_tile_at(const FillTask &tk, int64_t local, i
 constexpr int FAR_BATCH = 32;  // listed pairs whose moments are held at once
 
 template <int MODE>
-__global__ void __maxnreg__(168) far_pairs_group_kernel(const FillTask *__restrict__ tasks, int ntask, FarOpts o) {
+__global__ void __maxnreg__(168) far_pairs_group_kernel(const FillTask *__restrict__ tasks, int ntask,
+                                                              FarOpts o) {
   typedef typename std::conditional<MODE == FILL_DF, df, double>::type T;
   __shared__ GreenDev s_g;
   __shared__ V3<T> s_rho[8][6];
@@ -855,13 +760,13 @@ __global__ void __maxnreg__(168) far_pairs_group_kernel(const FillTask *__restri
           T Mc[36];
 #pragma unroll
           for (int k = 0; k < 36; k++) Mc[k] = M[k];
-          far_contract<T, true>(Tr, Sr, TD, SD, g, Mc, tk.H, tk.ntr, sym);
+          far_contract<T, true>(Tr, Sr, TD, SD, g, Mc, SUM6, tk.H, tk.ntr, sym);
         } else {
           far_moments6<T, false>(ge, g, s_rho[wid], M);
           T Mc[36];
 #pragma unroll
           for (int k = 0; k < 36; k++) Mc[k] = M[k];
-          far_contract<T, false>(Tr, Sr, TD, SD, g, Mc, tk.H, tk.ntr, sym);
+          far_contract<T, false>(Tr, Sr, TD, SD, g, Mc, SUM6, tk.H, tk.ntr, sym);
         }
       } else {
         const int at = atomicAdd(&s_n, 1);
@@ -889,10 +794,12 @@ __global__ void __maxnreg__(168) far_pairs_group_kernel(const FillTask *__restri
     if (wid == 0 && lane < m) {
       const int2 pr = s_list[b + lane];
       const TriDF *TD = tk.TD ? tk.TD + pr.x : nullptr, *SD = tk.SD ? tk.SD + pr.y : nullptr;
+      const int nr = s_rule[b + lane];
+      const int sum = nr == 10 ? SUM10 : nr == 15 ? SUM15 : nr == 21 ? SUM21 : SUM36;
       if (realk)
-        far_contract<T, true>(tk.T[pr.x], tk.S[pr.y], TD, SD, g, s_mom[lane], tk.H, tk.ntr, sym);
+        far_contract<T, true>(tk.T[pr.x], tk.S[pr.y], TD, SD, g, s_mom[lane], sum, tk.H, tk.ntr, sym);
       else
-        far_contract<T, false>(tk.T[pr.x], tk.S[pr.y], TD, SD, g, s_mom[lane], tk.H, tk.ntr, sym);
+        far_contract<T, false>(tk.T[pr.x], tk.S[pr.y], TD, SD, g, s_mom[lane], sum, tk.H, tk.ntr, sym);
     }
     __syncthreads();
   }
@@ -909,765 +816,667 @@ void launch_far(int mode, unsigned tiles, int rows, cudaStream_t st, const FillT
 }
 
 // ---------------- near pairs ----------------
+//
+// A near pair (same triangle, or a shared vertex) is the smooth inner rule (91
+// source nodes at each of the 105 test nodes, LKSmoothInnerIntegrand,
+// src/Impedance.cpp:93-105, with scalar_gradient_smooth,
+// src/GreensFunction.cpp:54-69), the closed-form singular terms
+// (EHNonSmoothIntegral, src/Source.cpp:16-86) at the test nodes, the close-pair
+// contraction (src/Impedance.cpp:194-250) and, for neighbours, the edge
+// correction of K (src/Impedance.cpp:301-324).  One warp takes one pair and
+// reduces it to moments; the nine (i, j) products follow in closed form.
+//
+// Smooth part.  g~ = (e^{ikR} - 1)/R - k2 R and q~ = (e^{ikR}(1 - ikR) + k2 R^2
+// - 1)/R^3 are power series in R without the terms that the singular part
+// takes:
+//   g~ = sum_{n>=1, n!=2} (ik)^n R^{n-1}/n!,   q~ = sum_{n>=3} (1-n)(ik)^n R^{n-3}/n!.
+// Their moments over {1, eta1, eta2} x {1, xi1, xi2} (as a far pair's) are
+// therefore sums over the moments of the powers of R alone, which are real and
+// know no frequency and no medium:
+//   odd powers R^{2j+1}: 91 x 105 node pairs;
+//   even powers (R^2)^j: polynomials, which the rules integrate exactly up to
+//   their degree, so that 36 x 36 nodes give the same sums (even_rules.h: their
+//   weights carry the large rules' own moments).
+// So there is no sincos, exp or division per node pair, the cancellation in the
+// closed forms of g~ and q~ is gone, and one pass over a pair serves the
+// exterior and its body's interior Green's function at once.  The terms fall
+// like x^n/n!, x = |k| R: the first powers are carried in full, those below
+// 2^-24 of the singular part in FP32 (double-float fill).  Coordinates are
+// scaled by a power of two so that R <= 1.
+// Above x = 1.1 (coarse meshes at an interior resonance) g~ and q~ are evaluated
+// directly per node pair (NEAR_DIRECT).
+//
+// Singular part: with X = IL1 + ISn1 rho' (rho' the test node's foot on the
+// source plane) and its k2 counterpart, 23 real moments over the test nodes.
+enum { NEAR_DIRECT = 0, NEAR_SERIES1 = 1, NEAR_SERIES2 = 2, NEAR_KINDS = 3 };
+constexpr double NEAR_X1 = 0.47, NEAR_X2 = 1.1;  // largest |k| R of the two series kinds
 
-// EHNonSmoothIntegral, src/Source.cpp:16-86 (frame of the source triangle's s[0]).
-__device__ void eh_nonsmooth(const TriRec &S, d3 rt, double &ISn3h, double &ISn1, double &IS1, d3 &IL1,
-                             d3 &IL3) {
-  const double tol = 1e-6 * S.elen0;
-  const d3 p0 = rt - ld3(S.p0), p1 = rt - ld3(S.p1), p2 = rt - ld3(S.p2);
-  const double R02 = dot(p0, p0), R0 = sqrt(R02);
-  const double R12 = dot(p1, p1), R1 = sqrt(R12);
-  const double R22 = dot(p2, p2), R2 = sqrt(R22);
-  const d3 a0 = (1. / R0) * p0, a1 = (1. / R1) * p1, a2 = (1. / R2) * p2;
-  const d3 n = ld3(S.n);
-  const double x = 1.0 + dot(a0, a1 + a2) + dot(a1, a2);
-  const double y = fabs(dot(a0, cross(a1, a2)));
-  const double h = dot(p0, n);
-  ISn3h = (h < 0. ? -2. : 2.) * atan2(y, x);
-  const d3 v01 = ld3(S.v01), v12 = ld3(S.v12), v20 = ld3(S.v20);
-  double num, den;
-  const double s010 = S.nv01i * dot(v01, p0), s011 = S.nv01i * dot(v01, p1);
-  num = R1 - s011; den = R0 - s010;
-  const double ILn1_01 = (fabs(num) < tol || fabs(den) < tol) ? 0. : log(num / den);
-  const double s121 = S.nv12i * dot(v12, p1), s122 = S.nv12i * dot(v12, p2);
-  num = R2 - s122; den = R1 - s121;
-  const double ILn1_12 = (fabs(num) < tol || fabs(den) < tol) ? 0. : log(num / den);
-  const double s202 = S.nv20i * dot(v20, p2), s200 = S.nv20i * dot(v20, p0);
-  num = R0 - s200; den = R2 - s202;
-  const double ILn1_20 = (fabs(num) < tol || fabs(den) < tol) ? 0. : log(num / den);
-  const d3 m01 = ld3(S.m01), m12 = ld3(S.m12), m20 = ld3(S.m20);
-  const double t01 = dot(m01, p0), t12 = dot(m12, p1), t20 = dot(m20, p2);
-  ISn1 = -h * ISn3h - (t01 * ILn1_01 + t12 * ILn1_12 + t20 * ILn1_20);
-  const double R02_01 = R02 - s010 * s010;
-  const double IL1_01 = 0.5 * (R02_01 * ILn1_01 - (R1 * s011 - R0 * s010));
-  const double R02_12 = R12 - s121 * s121;
-  const double IL1_12 = 0.5 * (R02_12 * ILn1_12 - (R2 * s122 - R1 * s121));
-  const double R02_20 = R22 - s202 * s202;
-  const double IL1_20 = 0.5 * (R02_20 * ILn1_20 - (R0 * s200 - R2 * s202));
-  const double IL3_01 = 0.75 * R02_01 * IL1_01 - 0.25 * (R12 * R1 * s011 - R02 * R0 * s010);
-  const double IL3_12 = 0.75 * R02_12 * IL1_12 - 0.25 * (R22 * R2 * s122 - R12 * R1 * s121);
-  const double IL3_20 = 0.75 * R02_20 * IL1_20 - 0.25 * (R02 * R0 * s200 - R22 * R2 * s202);
-  IS1 = BEM_ONETHIRD * (h * h * ISn1 - (t01 * IL1_01 + t12 * IL1_12 + t20 * IL1_20));
-  IL1 = IL1_01 * m01 + IL1_12 * m12 + IL1_20 * m20;
-  IL3 = IL3_01 * m01 + IL3_12 * m12 + IL3_20 * m20;
-}
+// Powers carried: JF in full, JT in all (even powers 1..JT beside the constant).
+// Double-float: at x = 0.47 the first FP32 term is x^8/8! = 6e-8 and the first
+// dropped x^14/14! = 3e-16 of the singular part; at x = 1.1 6e-9 and 9e-16.
+template <typename T, int KIND>
+struct NearCfg;
+template <>
+struct NearCfg<df, NEAR_SERIES1> { static constexpr int JF = 3, JT = 6; };
+template <>
+struct NearCfg<df, NEAR_SERIES2> { static constexpr int JF = 5, JT = 8; };
+template <>
+struct NearCfg<double, NEAR_SERIES1> { static constexpr int JF = 7, JT = 7; };
+template <>
+struct NearCfg<double, NEAR_SERIES2> { static constexpr int JF = 9, JT = 9; };
+template <typename T>
+struct NearCfg<T, NEAR_DIRECT> { static constexpr int JF = 4, JT = 4; };  // the four values of g~ and q~
+constexpr int NEAR_NJ = 10;  // coefficients kept per series
 
-// LKEdgeIntegral, src/Impedance.cpp:13-73 (frame of the test triangle's t[0]).
-__device__ void lk_edge_integral(const TriRec &T, d3 rs, double &ISn1, d3 &IL1) {
-  const d3 p0 = rs - ld3(T.p0), p1 = rs - ld3(T.p1), p2 = rs - ld3(T.p2);
-  const double R02 = dot(p0, p0), R0 = sqrt(R02);
-  const double R12 = dot(p1, p1), R1 = sqrt(R12);
-  const double R22 = dot(p2, p2), R2 = sqrt(R22);
-  const double tol = 1e-8 * T.elen0;
-  const d3 a0 = (1. / R0) * p0, a1 = (1. / R1) * p1, a2 = (1. / R2) * p2;
-  const double h = dot(p0, ld3(T.n));
-  const double x = 1.0 + dot(a0, a1 + a2) + dot(a1, a2);
-  const double y = fabs(dot(a0, cross(a1, a2)));
-  const double ISn3h = (h < 0 ? -2. : 2.) * atan2(y, x);
-  const d3 m01 = ld3(T.m01), m12 = ld3(T.m12), m20 = ld3(T.m20);
-  const double t01 = dot(m01, p0), t12 = dot(m12, p1), t20 = dot(m20, p2);
-  const d3 v01 = ld3(T.v01), v12 = ld3(T.v12), v20 = ld3(T.v20);
-  double num, den;
-  const double s010 = T.nv01i * dot(v01, p0), s011 = T.nv01i * dot(v01, p1);
-  num = R1 - s011; den = R0 - s010;
-  const double ILn1_01 = (fabs(num) < tol || fabs(den) < tol) ? 0. : log(num / den);
-  const double s121 = T.nv12i * dot(v12, p1), s122 = T.nv12i * dot(v12, p2);
-  num = R2 - s122; den = R1 - s121;
-  const double ILn1_12 = (fabs(num) < tol || fabs(den) < tol) ? 0. : log(num / den);
-  const double s202 = T.nv20i * dot(v20, p2), s200 = T.nv20i * dot(v20, p0);
-  num = R0 - s200; den = R2 - s202;
-  const double ILn1_20 = (fabs(num) < tol || fabs(den) < tol) ? 0. : log(num / den);
-  ISn1 = -h * ISn3h - (t01 * ILn1_01 + t12 * ILn1_12 + t20 * ILn1_20);
-  const double IL1_01 = 0.5 * ((R02 - s010 * s010) * ILn1_01 - (R1 * s011 - R0 * s010));
-  const double IL1_12 = 0.5 * ((R12 - s121 * s121) * ILn1_12 - (R2 * s122 - R1 * s121));
-  const double IL1_20 = 0.5 * ((R22 - s202 * s202) * ILn1_20 - (R0 * s200 - R2 * s202));
-  IL1 = IL1_01 * m01 + IL1_12 * m12 + IL1_20 * m20;
-}
+// One Green's function of a near task: where its products go, the source and
+// test triangles it covers (all of the task's, or one body's of a two-body
+// tree), and its series coefficients (complex, in the fill's number type).
+struct NearGreen {
+  HalfPairBlock *H;
+  int ntr, rwg0;    // RWGs of its test tree; index of its first RWG in the task's tree
+  int tri0, tri1;   // its triangles of the task's tree
+  int realk;
+  GreenDev g;
+  // read 16 bytes at a time
+  alignas(16) double ge[NEAR_NJ][2];
+  alignas(16) double go[NEAR_NJ][2];
+  alignas(16) double qe[NEAR_NJ][2];
+  alignas(16) double qo[NEAR_NJ][2];
+};
+struct alignas(16) NearTask {
+  const TriRec *T, *S;
+  const NearPair *near;
+  int64_t nnear, unit0;  // pairs; the task's first unit of the launch
+  double scale;          // power of two: R scale <= 1
+  int ngreen;            // the first covers every pair, the others one body's
+  NearGreen g[3];
+};
+static_assert(sizeof(NearTask) % 16 == 0 && sizeof(NearGreen) % 16 == 0, "an array of tasks keeps their alignment");
 
-__device__ __forceinline__ double warp_sum(double v) {
+// The rules of the near kernels, in both number types: 105 test nodes, 91
+// source nodes, 36 + 36 even-power nodes.
+enum { NN105 = 0, NN91 = 105, NNE105 = 196, NNE91 = 232, NN_ALL = 268 };
+__constant__ RuleNode<double> c_near_d[NN_ALL];
+__constant__ RuleNode<df> c_near_f[NN_ALL];
+__constant__ double c_near_ww1;  // product of the 105- and 91-point weights' sums, less one
+template <typename T>
+__device__ __forceinline__ const RuleNode<T> *near_nodes();
+template <>
+__device__ __forceinline__ const RuleNode<double> *near_nodes<double>() { return c_near_d; }
+template <>
+__device__ __forceinline__ const RuleNode<df> *near_nodes<df>() { return c_near_f; }
+
+// A triangle relative to the test triangle's p0: vertices, normal, edges 01,
+// 12, 20, their outward in-plane normals, and inverse edge lengths.
+template <typename T>
+struct NearFrame {
+  V3<T> p[3], n, e[3], m[3];
+  T ei[3];
+};
+
+// The closed-form potential integrals of a triangle F seen from the point r:
+// the analytic part of EHNonSmoothIntegral (src/Source.cpp:16-86) and, with
+// full false, of LKEdgeIntegral (src/Impedance.cpp:13-73: ISn1, IL1, h only).
+// h = (r - p0) . n.  tol is the edge-line cut-off of the logarithms.
+template <typename T>
+struct NearPot {
+  T ISn3h, ISn1, IS1, h;
+  V3<T> IL1, IL3;
+};
+template <typename T>
+__device__ __noinline__ void near_potentials(const NearFrame<T> &F, V3<T> r, typename Num<T>::Tail tol, bool full,
+                                             NearPot<T> &o) {
+  typedef Num<T> N;
+  const T zero = N::of(0.0);
+  V3<T> p[3], a[3];
+  T R2[3], R[3];
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-  return v;
+  for (int k = 0; k < 3; k++) {
+    p[k] = r - F.p[k];
+    R2[k] = vdot(p[k], p[k]);
+    R[k] = N::sqrt_(R2[k]);
+    a[k] = N::rcp(R[k]) * p[k];
+  }
+  const T x = (vdot(a[0], a[1] + a[2]) + vdot(a[1], a[2])) + N::of(1.0);
+  const T y = N::abs_(vdot(a[0], vcross(a[1], a[2])));
+  o.h = vdot(p[0], F.n);
+  o.ISn3h = N::pow2(N::atan2_(y, x), N::head(o.h) < 0 ? -2.f : 2.f);
+  T tl = zero, tI = zero;
+  o.IL1 = vzero<T>();
+  o.IL3 = vzero<T>();
+#pragma unroll
+  for (int k = 0; k < 3; k++) {
+    const int k1 = (k + 1) % 3;
+    const T s0 = F.ei[k] * vdot(F.e[k], p[k]), s1 = F.ei[k] * vdot(F.e[k], p[k1]);
+    const T num = R[k1] - s1, den = R[k] - s0;
+    T ln = zero;
+    if (!(fabs(N::head(num)) < tol || fabs(N::head(den)) < tol)) ln = N::log_(num * N::rcp(den));
+    const T t = vdot(F.m[k], p[k]);
+    tl = N::muladd(t, ln, tl);
+    const T d2 = R2[k] - s0 * s0;
+    const T Rs0 = R[k] * s0, Rs1 = R[k1] * s1;
+    const T l1 = N::pow2(N::muladd(d2, ln, Rs0 - Rs1), 0.5f);
+    o.IL1 = o.IL1 + l1 * F.m[k];
+    if (full) {
+      const T l3 = N::muladd(N::of(0.75) * d2, l1, N::pow2(N::dot2(R2[k], Rs0, -R2[k1], Rs1), 0.25f));
+      tI = N::muladd(t, l1, tI);
+      o.IL3 = o.IL3 + l3 * F.m[k];
+    }
+  }
+  o.ISn1 = -N::muladd(o.h, o.ISn3h, tl);
+  if (full) o.IS1 = N::of(BEM_ONETHIRD) * N::muladd(o.h * o.h, o.ISn1, -tI);
+}
+
+// scalar_gradient_smooth, src/GreensFunction.cpp:54-69, directly.
+template <typename T, bool REALK>
+__device__ __forceinline__ void near_values(const GreenT<T> &g, V3<T> x, T (&f)[4]) {
+  typedef Num<T> N;
+  const T R2 = N::sumsq(x.x, x.y, x.z);
+  T R, Ri, er, ei, em, ur, ui;
+  N::sqrt_rcp(R2, R, Ri);
+  wave_at<T, REALK>(g, R, er, ei, em, ur, ui);
+  const T one = N::of(1.0), Ri3 = Ri * (Ri * Ri);
+  f[0] = N::dot2(er - one, Ri, -g.k2r, R);
+  f[2] = (N::muladd(R2, g.k2r, ur) - one) * Ri3;
+  if (REALK) {
+    f[1] = em * Ri;
+    f[3] = ui * Ri3;
+  } else {
+    f[1] = N::dot2(em, Ri, -g.k2i, R);
+    f[3] = N::muladd(R2, g.k2i, ui) * Ri3;
+  }
 }
 
 constexpr int NEAR_WARPS = 4;
 
-// Moments of the smooth inner rule at one outer node (complex df):
-// I0 = sum w g~, A = sum w g~ l, Q0 = sum w q~, Q1 = sum w q~ l.
-struct InnerMomDF {
-  cdf I0, Q0;
-  cdf3 A, Q1;
+// A test node as the loops over source nodes read it: position relative to the
+// source triangle's p0, weight, weight times each barycentric coordinate.
+template <typename T>
+struct __align__(16) NearNode {
+  V3<T> p;
+  T w, w1, w2;
 };
 
-// Smooth inner rule of a near pair at NP outer nodes at once, double-float
-// version: the same moments as the FP64 loop in near_pairs_kernel
-// (LKSmoothInnerIntegrand, src/Impedance.cpp:93-105, with
-// scalar_gradient_smooth, src/GreensFunction.cpp:54-69), summed in df from df
-// nodes (l, w).  The NP points are independent dependency chains over the same
-// inner nodes, which the scheduler interleaves.
-template <int NP>
-__device__ __noinline__ void near_inner_df(const float (*nd)[8], const df3 *rp, const GreenDev &g, InnerMomDF *out) {
-  const df ikr = {g.ikr_f[0], g.ikr_f[1]}, iki = {g.iki_f[0], g.iki_f[1]};
-  const df k2r = {g.k2r_f[0], g.k2r_f[1]}, k2i = {g.k2i_f[0], g.k2i_f[1]};
-  df3 r[NP];
-  df I0r[NP], I0i[NP], Q0r[NP], Q0i[NP], Ar[NP][3], Ai[NP][3], Qr[NP][3], Qi[NP][3];
-  const df z = {0.f, 0.f};
+// A warp's staging of its pair.
+template <typename T>
+struct NearStage {
+  NearNode<T> q[105];
+  // odd and even moments [j][a][b], or the four values' moments (NEAR_DIRECT)
+  T odd[9 * 9], even[9 * 10];
+  T sing[24];
+  T edge_sum[3][4];
+  // per Green's function: Re and Im of the moments of g~, Re and Im of the
+  // barycentric moments of q~, and Im of -U0 (its first entry)
+  T mom[2][5][9];
+  T qraw[2][2][9];
+  NearFrame<T> Sf, Tf;
+  // the 45 edge nodes' terms take the test nodes' place
+  __device__ __forceinline__ T *edge(int k) { return reinterpret_cast<T *>(q) + 4 * k; }
+};
+
+// Adds the warp's sums of NV values per lane, eight at a time, to out[0..NV).
+template <typename T, int NV, typename F>
+__device__ __forceinline__ void near_reduce(T *out, int lane, F value) {
+  const int at = reduce8_index(lane);
 #pragma unroll
-  for (int p = 0; p < NP; p++) {
-    r[p] = rp[p];
-    I0r[p] = z; I0i[p] = z; Q0r[p] = z; Q0i[p] = z;
+  for (int c = 0; c < (NV + 7) / 8; c++) {
+    T v[8];
 #pragma unroll
-    for (int c = 0; c < 3; c++) { Ar[p][c] = z; Ai[p][c] = z; Qr[p][c] = z; Qi[p][c] = z; }
+    for (int k = 0; k < 8; k++) v[k] = c * 8 + k < NV ? value(c * 8 + k) : Num<T>::of(0.0);
+    const T r = reduce8<T>(v, lane);
+    if ((lane & 3) == 0 && c * 8 + at < NV) out[c * 8 + at] = out[c * 8 + at] + r;
   }
-  for (int u = 0; u < BEMGPU_TRI_RULE91_N; u++) {
-    const float4 n0 = *reinterpret_cast<const float4 *>(&nd[u][0]);
-    const float4 n1 = *reinterpret_cast<const float4 *>(&nd[u][4]);
-    const df l[3] = {{n0.x, n0.y}, {n0.z, n0.w}, {n1.x, n1.y}};
-    const df ws = {n1.z, n1.w};
+}
+
+// Sums over the staged test nodes q0, q0 + step, ... < nq, seen from the lane's
+// source node (l relative to P_s): ODD the powers R^{2j+1}, else (R^2)^{j+1},
+// j < JT, times {w, w eta1, w eta2}.
+template <typename T, int JF, int JT, bool ODD>
+__device__ __forceinline__ void near_power_sums(const NearNode<T> *qn, int q0, int nq, int step, V3<T> l,
+                                                T (&S)[JF][3], typename Num<T>::Tail (&St)[JT - JF + 1][3]) {
+  typedef Num<T> N;
 #pragma unroll
-    for (int p = 0; p < NP; p++) {
-      const df xx = df_sub(r[p].x, l[0]), xy = df_sub(r[p].y, l[1]), xz = df_sub(r[p].z, l[2]);
-      const df R2 = df_add(df_add(df_sqr(xx), df_sqr(xy)), df_sqr(xz));
-      const df R = df_sqrt(R2);
-      const df Ri = df_rcp(R);
-      df er, ei;
-      df_exp_ikR(g, ikr, iki, R, er, ei);
-      // g~ = (e - 1)/R - k2 R
-      const df gr = df_sub(df_mul(df_add_f(er, -1.f), Ri), df_mul(k2r, R));
-      const df gi = df_sub(df_mul(ei, Ri), df_mul(k2i, R));
-      // q~ = (e (1 - ikR) + R^2 k2 - 1) / R^3
-      const df zr = df_mul(ikr, R), zi = df_mul(iki, R);
-      const df mr = df_add_f(df_neg(zr), 1.f), mi = df_neg(zi);
-      df nr = df_sub(df_mul(er, mr), df_mul(ei, mi));
-      df ni = df_add(df_mul(er, mi), df_mul(ei, mr));
-      nr = df_add_f(df_add(nr, df_mul(R2, k2r)), -1.f);
-      ni = df_add(ni, df_mul(R2, k2i));
-      const df Ri3 = df_mul(df_sqr(Ri), Ri);
-      const df qr = df_mul(Ri3, nr), qi = df_mul(Ri3, ni);
-      const df gwr = df_mul(ws, gr), gwi = df_mul(ws, gi), qwr = df_mul(ws, qr), qwi = df_mul(ws, qi);
-      I0r[p] = df_add(I0r[p], gwr);
-      I0i[p] = df_add(I0i[p], gwi);
-      Q0r[p] = df_add(Q0r[p], qwr);
-      Q0i[p] = df_add(Q0i[p], qwi);
+  for (int j = 0; j < JF; j++) S[j][0] = S[j][1] = S[j][2] = N::of(0.0);
 #pragma unroll
-      for (int c = 0; c < 3; c++) {
-        Ar[p][c] = df_add(Ar[p][c], df_mul(gwr, l[c]));
-        Ai[p][c] = df_add(Ai[p][c], df_mul(gwi, l[c]));
-        Qr[p][c] = df_add(Qr[p][c], df_mul(qwr, l[c]));
-        Qi[p][c] = df_add(Qi[p][c], df_mul(qwi, l[c]));
-      }
+  for (int j = 0; j < JT - JF; j++) St[j][0] = St[j][1] = St[j][2] = 0;
+#pragma unroll 1
+  for (int q = q0; q < nq; q += step) {
+    const NearNode<T> nd = qn[q];
+    const T s = N::sumsq(N::diff(nd.p.x, l.x), N::diff(nd.p.y, l.y), N::diff(nd.p.z, l.z));
+    T p = ODD ? N::sqrt_(s) : s;
+#pragma unroll
+    for (int j = 0; j < JF; j++) {
+      N::mac(S[j][0], p, nd.w);
+      N::mac(S[j][1], p, nd.w1);
+      N::mac(S[j][2], p, nd.w2);
+      if (j + 1 < JF) p = p * s;
+    }
+    typename N::Tail pt = N::head(p);
+#pragma unroll
+    for (int j = 0; j < JT - JF; j++) {
+      pt *= N::head(s);
+      St[j][0] += pt * N::head(nd.w);
+      St[j][1] += pt * N::head(nd.w1);
+      St[j][2] += pt * N::head(nd.w2);
     }
   }
 #pragma unroll
-  for (int p = 0; p < NP; p++) {
-    out[p].I0 = {I0r[p], I0i[p]};
-    out[p].Q0 = {Q0r[p], Q0i[p]};
-    out[p].A = {{Ar[p][0], Ai[p][0]}, {Ar[p][1], Ai[p][1]}, {Ar[p][2], Ai[p][2]}};
-    out[p].Q1 = {{Qr[p][0], Qi[p][0]}, {Qr[p][1], Qi[p][1]}, {Qr[p][2], Qi[p][2]}};
-  }
-}
-
-// A triangle in double-float, vertices relative to a chosen origin O (the
-// test triangle's p0): what the closed-form integrals below read.
-struct TriFrameDF {
-  df3 p0, p1, p2, n, v01, v12, v20, m01, m12, m20;
-  df nv01i, nv12i, nv20i;
-};
-
-__device__ void tri_frame_df(const TriRec &T, d3 O, TriFrameDF &F) {
-  F.p0 = df3_make(ld3(T.p0) - O);
-  F.p1 = df3_make(ld3(T.p1) - O);
-  F.p2 = df3_make(ld3(T.p2) - O);
-  F.n = df3_make(ld3(T.n));
-  F.v01 = df3_make(ld3(T.v01));
-  F.v12 = df3_make(ld3(T.v12));
-  F.v20 = df3_make(ld3(T.v20));
-  F.m01 = df3_make(ld3(T.m01));
-  F.m12 = df3_make(ld3(T.m12));
-  F.m20 = df3_make(ld3(T.m20));
-  F.nv01i = df_make(T.nv01i);
-  F.nv12i = df_make(T.nv12i);
-  F.nv20i = df_make(T.nv20i);
-}
-
-__device__ __forceinline__ df log_ratio_df(df num, df den, float tol) {
-  if (fabsf(num.hi) < tol || fabsf(den.hi) < tol) return {0.f, 0.f};
-  return df_log(df_mul(num, df_rcp(den)));
-}
-
-// The closed-form potential integrals of a triangle F seen from the point r
-// (both relative to the same origin), in double-float: the analytic part of
-// EHNonSmoothIntegral (src/Source.cpp:16-86, with full = true: ISn3h, ISn1,
-// IS1, IL1, IL3) and LKEdgeIntegral (src/Impedance.cpp:13-73, full = false:
-// ISn3h, ISn1, IL1), step for step as eh_nonsmooth / lk_edge_integral do them
-// in FP64; h = (r - p0) . n.  tol is the edge-line cut-off of the logarithms.
-__device__ __noinline__ void tri_potentials_df(const TriFrameDF &F, df3 r, float tol, bool full, df &ISn3h,
-                                               df &ISn1, df &IS1, df3 &IL1, df3 &IL3, df &h) {
-  const df3 p0 = df3_sub(r, F.p0), p1 = df3_sub(r, F.p1), p2 = df3_sub(r, F.p2);
-  const df R02 = df3_dot(p0, p0), R12 = df3_dot(p1, p1), R22 = df3_dot(p2, p2);
-  const df R0 = df_sqrt(R02), R1 = df_sqrt(R12), R2 = df_sqrt(R22);
-  const df3 a0 = df3_scale(df_rcp(R0), p0), a1 = df3_scale(df_rcp(R1), p1), a2 = df3_scale(df_rcp(R2), p2);
-  const df x = df_add_f(df_add(df3_dot(a0, df3_add(a1, a2)), df3_dot(a1, a2)), 1.f);
-  const df y = df_abs(df3_dot(a0, df3_cross(a1, a2)));
-  h = df3_dot(p0, F.n);
-  const df at = df_atan2(y, x);
-  ISn3h = df_scale2(at, h.hi < 0.f ? -2.f : 2.f);
-  const df s010 = df_mul(F.nv01i, df3_dot(F.v01, p0)), s011 = df_mul(F.nv01i, df3_dot(F.v01, p1));
-  const df s121 = df_mul(F.nv12i, df3_dot(F.v12, p1)), s122 = df_mul(F.nv12i, df3_dot(F.v12, p2));
-  const df s202 = df_mul(F.nv20i, df3_dot(F.v20, p2)), s200 = df_mul(F.nv20i, df3_dot(F.v20, p0));
-  const df ILn1_01 = log_ratio_df(df_sub(R1, s011), df_sub(R0, s010), tol);
-  const df ILn1_12 = log_ratio_df(df_sub(R2, s122), df_sub(R1, s121), tol);
-  const df ILn1_20 = log_ratio_df(df_sub(R0, s200), df_sub(R2, s202), tol);
-  const df t01 = df3_dot(F.m01, p0), t12 = df3_dot(F.m12, p1), t20 = df3_dot(F.m20, p2);
-  const df tl = df_add(df_add(df_mul(t01, ILn1_01), df_mul(t12, ILn1_12)), df_mul(t20, ILn1_20));
-  ISn1 = df_neg(df_add(df_mul(h, ISn3h), tl));
-  const df R02_01 = df_sub(R02, df_sqr(s010));
-  const df R02_12 = df_sub(R12, df_sqr(s121));
-  const df R02_20 = df_sub(R22, df_sqr(s202));
-  const df half = {0.5f, 0.f};
-  const df IL1_01 = df_mul(half, df_sub(df_mul(R02_01, ILn1_01), df_sub(df_mul(R1, s011), df_mul(R0, s010))));
-  const df IL1_12 = df_mul(half, df_sub(df_mul(R02_12, ILn1_12), df_sub(df_mul(R2, s122), df_mul(R1, s121))));
-  const df IL1_20 = df_mul(half, df_sub(df_mul(R02_20, ILn1_20), df_sub(df_mul(R0, s200), df_mul(R2, s202))));
-  IL1 = df3_add(df3_add(df3_scale(IL1_01, F.m01), df3_scale(IL1_12, F.m12)), df3_scale(IL1_20, F.m20));
-  if (!full) return;
-  const df q3 = {0.75f, 0.f}, q1 = {0.25f, 0.f};
-  const df IL3_01 = df_sub(df_mul(q3, df_mul(R02_01, IL1_01)),
-                           df_mul(q1, df_sub(df_mul(df_mul(R12, R1), s011), df_mul(df_mul(R02, R0), s010))));
-  const df IL3_12 = df_sub(df_mul(q3, df_mul(R02_12, IL1_12)),
-                           df_mul(q1, df_sub(df_mul(df_mul(R22, R2), s122), df_mul(df_mul(R12, R1), s121))));
-  const df IL3_20 = df_sub(df_mul(q3, df_mul(R02_20, IL1_20)),
-                           df_mul(q1, df_sub(df_mul(df_mul(R02, R0), s200), df_mul(df_mul(R22, R2), s202))));
-  const df third = {0x1.555556p-2f, -0x1.555556p-27f};
-  const df tI = df_add(df_add(df_mul(t01, IL1_01), df_mul(t12, IL1_12)), df_mul(t20, IL1_20));
-  IS1 = df_mul(third, df_sub(df_mul(df_sqr(h), ISn1), tI));
-  IL3 = df3_add(df3_add(df3_scale(IL3_01, F.m01), df3_scale(IL3_12, F.m12)), df3_scale(IL3_20, F.m20));
-}
-
-// Per-pair double-float constants of the close-pair contraction, relative to
-// the test triangle's frame origin P_t: e_i = p0_i - P_t, f_j = p0_j - P_t,
-// d_j = p0_j - P_s.  One per warp, in shared memory (every lane reads the same
-// words).
-struct NearPairDF {
-  TriFrameDF Sf, Tf;        // source and test triangles
-  df3 e[3], f[3], d[3];
-  df3 sPs, v01t, v02t;      // P_s - P_t and the test triangle's edge vectors
-  df Ai2;
-  cdf ksq, k2, k2_3;
-  float tol_eh, tol_plane, tol_edge;
-};
-// The nine L and K sums of a near pair (complex df).
-struct NearAccDF {
-  cdf L[9], K[9];
-};
-
-__device__ void near_pair_df_setup(const TriRec &T, const TriRec &S, const GreenDev &g, NearPairDF &pc) {
-  const d3 Pt = ld3(T.p0), Ps = ld3(S.p0);
-  tri_frame_df(S, Pt, pc.Sf);
-  tri_frame_df(T, Pt, pc.Tf);
-  for (int i = 0; i < 3; i++) {
-    pc.e[i] = df3_make(i < T.nh ? ld3(T.hp0[i]) - Pt : d3{0, 0, 0});
-    pc.f[i] = df3_make(i < S.nh ? ld3(S.hp0[i]) - Pt : d3{0, 0, 0});
-    pc.d[i] = df3_make(i < S.nh ? ld3(S.hp0[i]) - Ps : d3{0, 0, 0});
-  }
-  pc.sPs = df3_make(Ps - Pt);
-  pc.v01t = df3_make(ld3(T.v01));
-  pc.v02t = df3_make(ld3(T.v02));
-  pc.Ai2 = df_make(0.5 * S.Ai);
-  pc.ksq = {{g.ksqr_f[0], g.ksqr_f[1]}, {g.ksqi_f[0], g.ksqi_f[1]}};
-  pc.k2 = {{g.k2r_f[0], g.k2r_f[1]}, {g.k2i_f[0], g.k2i_f[1]}};
-  pc.k2_3 = {df_make(BEM_ONETHIRD * g.k2r), df_make(BEM_ONETHIRD * g.k2i)};
-  pc.tol_eh = (float)(1e-6 * S.elen0);
-  pc.tol_plane = (float)(1e-8 * S.elen0);
-  pc.tol_edge = (float)(1e-8 * T.elen0);
-}
-
-// One outer node of a near pair in double-float: given the node's smooth
-// inner moments (near_inner_df), the analytic singular terms
-// (tri_potentials_df) and the close-pair contraction of
-// src/Impedance.cpp:194-250, added to acc.  rt1 is the node relative to P_t.
-__device__ __noinline__ void near_outer_df(const InnerMomDF &m, const NearPairDF &pc, int nht, int nhs, df3 rt1,
-                                           df wd, NearAccDF &acc) {
-  const cdf I0 = m.I0, Q0 = m.Q0;
-  const cdf3 A = m.A, Q1 = m.Q1;
-  df ISn3h, ISn1, IS1, h;
-  df3 IL1, IL3;
-  tri_potentials_df(pc.Sf, rt1, pc.tol_eh, true, ISn3h, ISn1, IS1, IL1, IL3, h);
-  // IL13 = Ai2 (k2/3 IL3 + IL1), ISn11 = Ai2 (ISn1 + k2 IS1), L2 = 2 ISn11 + I0
-  cdf3 IL13 = cdf_v(pc.k2_3, IL3);
-  IL13.x.r = df_add(IL13.x.r, IL1.x);
-  IL13.y.r = df_add(IL13.y.r, IL1.y);
-  IL13.z.r = df_add(IL13.z.r, IL1.z);
-  IL13 = cdf3_scale(pc.Ai2, IL13);
-  const cdf ISn11 = cdf_scale(pc.Ai2, cdf{df_add(ISn1, df_mul(pc.k2.r, IS1)), df_mul(pc.k2.i, IS1)});
-  const cdf L2 = cdf_add(cdf_add(ISn11, ISn11), I0);
-  const df half = {0.5f, 0.f};
-  if (fabsf(h.hi) < pc.tol_plane) {
-    for (int j = 0; j < nhs; j++) {
-      const cdf3 Gphij = cdf3_scale(half, cdf3_sub(A, cdf_v(I0, pc.d[j])));
-      const cdf3 K21 = cdf3_add(IL13, cdf_v(ISn11, df3_sub(rt1, pc.f[j])));
-      const cdf3 GK = cdf3_add(Gphij, K21);
-      for (int i = 0; i < nht; i++) {
-        const df3 phi = df3_scale(half, df3_sub(rt1, pc.e[i]));
-        const cdf t = cdf_sub(cdf_mul(pc.ksq, cdf_rdot(phi, GK)), L2);
-        acc.L[i * 3 + j] = cdf_add(acc.L[i * 3 + j], cdf_scale(wd, t));
-      }
-    }
-  } else {
-    const df3 nS = pc.Sf.n;
-    const df3 ISn3hn = df3_scale(df_mul(pc.Ai2, ISn3h), nS);
-    const df3 rho1 = df3_sub(rt1, df3_scale(h, nS));
-    const cdf Ai2k2 = cdf_scale(pc.Ai2, pc.k2);
-    const cdf3 K31 = cdf_v(Ai2k2, df3_sub(IL1, df3_scale(df_mul(h, ISn1), nS)));
-    for (int j = 0; j < nhs; j++) {
-      const df3 rf = df3_sub(rt1, pc.f[j]);  // r_t - p0_j
-      const cdf3 Gphij = cdf3_scale(half, cdf3_sub(A, cdf_v(I0, pc.d[j])));
-      const cdf3 DGxphij = cdf3_scale(half, cdf_rcross(rf, cdf3_sub(Q1, cdf_v(Q0, pc.d[j]))));
-      const cdf3 K21 = cdf3_add(IL13, cdf_v(ISn11, df3_sub(rho1, pc.f[j])));
-      const cdf3 K41 = cdf_zcross(K31, rf);
-      const cdf3 GK = cdf3_add(Gphij, K21);
-      for (int i = 0; i < nht; i++) {
-        const df3 phi = df3_scale(half, df3_sub(rt1, pc.e[i]));
-        const cdf t = cdf_sub(cdf_mul(pc.ksq, cdf_rdot(phi, GK)), L2);
-        acc.L[i * 3 + j] = cdf_add(acc.L[i * 3 + j], cdf_scale(wd, t));
-        const df3 vx = df3_cross(df3_sub(pc.f[j], pc.e[i]), ISn3hn);  // (p0_j - p0_i) x ISn3hn
-        cdf3 KK = cdf3_add(DGxphij, K41);
-        KK.x.r = df_add(KK.x.r, vx.x);
-        KK.y.r = df_add(KK.y.r, vx.y);
-        KK.z.r = df_add(KK.z.r, vx.z);
-        const cdf kk = cdf_rdot(phi, KK);
-        acc.K[i * 3 + j] = cdf_sub(acc.K[i * 3 + j], cdf_scale(wd, kk));
-      }
-    }
-  }
-}
-
-// The neighbour-edge K correction of src/Impedance.cpp:301-324 at one source
-// edge node v (relative to P_t) in double-float: LKEdgeIntegral over the test
-// triangle, then Ke[i] += w (IL1 + ISn1 (rho - p0_i)).
-__device__ __noinline__ void near_edge_df(const NearPairDF &pc, int nht, df3 v, df w, df3 *Ke) {
-  df ISn3h, ISn1, IS1, h;
-  df3 IL1, IL3;
-  tri_potentials_df(pc.Tf, v, pc.tol_edge, false, ISn3h, ISn1, IS1, IL1, IL3, h);
-  const df3 rho = df3_sub(v, df3_scale(h, pc.Tf.n));
-  for (int i = 0; i < nht; i++) {
-    const df3 c = df3_add(IL1, df3_scale(ISn1, df3_sub(rho, pc.e[i])));
-    Ke[i] = df3_add(Ke[i], df3_scale(w, c));
-  }
-}
-
-__device__ __forceinline__ df warp_sum_df(df v) {
+  for (int j = 0; j < JF; j++)
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    const df u = {__shfl_xor_sync(0xffffffffu, v.hi, o), __shfl_xor_sync(0xffffffffu, v.lo, o)};
-    v = df_add(v, u);
-  }
-  return v;
+    for (int a = 0; a < 3; a++) S[j][a] = N::fin(S[j][a]);
 }
 
-// DF: the smooth inner rule in double-float (near_inner_df), else FP64.
-// The rest of one near pair in double-float once its nine L and K sums are in
-// acc (spread over the warp's lanes): the warp sums, the neighbour-edge K
-// correction of src/Impedance.cpp:301-324 (near_edge_df), and the scatter of
-// the nine (c L, c K) into the half-pair blocks as float pairs.
-__device__ __noinline__ void near_finish_df(const TriRec &T, const TriRec &S, int same, const NearPairDF &pc,
-                                            const NearAccDF &acc, HalfPairBlock *H, int ntr) {
-  const int lane = threadIdx.x & 31;
-  const int nht = T.nh, nhs = S.nh;
-  z1 L[9], K[9];
+// Green's function coefficients are stored as pairs of the number type.
+template <typename T>
+__device__ __forceinline__ C1<T> near_coef(const double (*c)[2], int j);
+template <>
+__device__ __forceinline__ C1<double> near_coef<double>(const double (*c)[2], int j) { return {c[j][0], c[j][1]}; }
+template <>
+__device__ __forceinline__ C1<df> near_coef<df>(const double (*c)[2], int j) {
+  const float4 v = *reinterpret_cast<const float4 *>(c[j]);
+  return {{v.x, v.y}, {v.z, v.w}};
+}
+
+// The pair's product (i, j) from its moments, by one lane.
+//   L_ij = k^2/4 sum_{ab} (a_a . c_b) [...] - G_00   (as far_contract's)
+//          + k^2 (A0_ij + k2 A1_ij) - 2 (B0 + k2 B1)
+//   A_ij = Ai/4 [s - e_i . S_X - p_j . S_1rho + (e_i . p_j) S_1],  B = Ai/2 S_1
+//   K_ij = -1/4 sum B_vw (volumes) - Ai/4 [(p_j - p_i) x n . T + k2 (p_i - p_j) . (Z - e_i x S_Y)] + edges
+// (positions relative to P_t; S_.., T, Z, S_Y the singular moments).
+template <typename T>
+__device__ __noinline__ void near_product(const NearStage<T> &st, const T (*mom)[9], const GreenDev &gd,
+                                             const TriRec &Tr, const TriRec &Sr, int vi, int vj, bool same,
+                                             C1<T> &L, C1<T> &K) {
+  typedef Num<T> N;
+  const GreenT<T> g = green_of<T>(gd);
+  const V3<T> pi = st.Tf.p[vi], pj = st.Sf.p[vj], P0 = st.Sf.p[0];
+  const V3<T> D = pi - pj;
+  // smooth L
+  C1<T> br = {N::of(0.0), N::of(0.0)};
+  auto G = [&](int a, int b) {
+    C1<T> v = {mom[0][a * 3 + b], mom[1][a * 3 + b]};
+    return v;
+  };
 #pragma unroll
-  for (int k = 0; k < 9; k++) {
-    L[k] = {df_to_double(warp_sum_df(acc.L[k].r)), df_to_double(warp_sum_df(acc.L[k].i))};
-    K[k] = {df_to_double(warp_sum_df(acc.K[k].r)), df_to_double(warp_sum_df(acc.K[k].i))};
+  for (int a = 1; a < 3; a++)
+#pragma unroll
+    for (int b = 1; b < 3; b++) {
+      const T d = vdot(st.Tf.p[a], st.Sf.p[b] - P0);
+      C1<T> m = G(a, b);
+      if (b == vj) m = m - G(a, 0);
+      if (a == vi) m = m - G(0, b);
+      if (a == vi && b == vj) m = m + G(0, 0);
+      br = br + d * m;
+    }
+  const C1<T> ksq = {g.ksqr, g.ksqi}, k2 = {g.k2r, g.k2i};
+  // singular L
+  const T Ai2 = N::of(0.5 * Sr.Ai);
+  const T *s0 = st.sing, *s1 = st.sing + 7;
+  const V3<T> a1 = st.Tf.p[1], a2 = st.Tf.p[2];
+  auto A_of = [&](const T *s) {
+    const V3<T> SX = {s[1], s[2], s[3]};
+    const V3<T> Sr1 = s[5] * a1 + s[6] * a2;
+    const T v = ((s[0] - vdot(pi, SX)) - vdot(pj, Sr1)) + vdot(pi, pj) * s[4];
+    return N::pow2(Ai2 * v, 0.5f);
+  };
+  const T A0 = A_of(s0), A1 = A_of(s1);
+  const T B0 = Ai2 * s0[4], B1 = Ai2 * s1[4];
+  const C1<T> inner = {N::muladd(g.k2r, A1, N::muladd(N::of(0.25), br.r, A0)), N::muladd(g.k2i, A1, N::pow2(br.i, 0.25f))};
+  C1<T> g00 = G(0, 0);
+  if (N::LESS) {
+    // Im g~'s constant Im(ik) is left out of -G_00 but for what the rules'
+    // weights leave of it (wave_at); the moments above hold it in full
+    g00.i = mom[4][0];
   }
+  L = cmul(ksq, inner) - g00;
+  L.r = L.r - N::pow2(N::muladd(k2.r, B1, B0), 2.f);
+  L.i = L.i - N::pow2(k2.i * B1, 2.f);
+  // smooth K
+  K = {N::of(0.0), N::of(0.0)};
+#pragma unroll
+  for (int v = 1; v < 3; v++)
+#pragma unroll
+    for (int w = 1; w < 3; w++) {
+      const int x = (vi + v) % 3, y = (vj + w) % 3;
+      const T vol = vdot(D, vcross(st.Sf.p[y] - pj, st.Tf.p[x] - pi));
+      N::mac(K.r, mom[2][x * 3 + y], vol);
+      N::mac(K.i, mom[3][x * 3 + y], vol);
+    }
+  const T q = N::of(-0.25);
+  K = {q * N::fin(K.r), q * N::fin(K.i)};
+  // singular K
+  const T *t = st.sing + 14;
+  const V3<T> n = st.Sf.n;
+  const V3<T> Tv = (t[1] * a1 + t[2] * a2) - t[0] * pi;
+  const T kt = vdot(vcross(-N::of(1.0) * D, n), Tv);
+  const V3<T> SY = {t[3], t[4], t[5]}, Z = {t[6], t[7], t[8]};
+  const T kz = vdot(D, Z - vcross(pi, SY));
+  const T h = N::pow2(Ai2, 0.5f);
+  K.r = K.r - h * N::muladd(k2.r, kz, kt);
+  K.i = K.i - h * (k2.i * kz);
   if (!same) {
-    df3 Kd[3][3];
-    const df z = {0.f, 0.f};
+    T ke = N::of(0.0);
 #pragma unroll
-    for (int e = 0; e < 3; e++)
-#pragma unroll
-      for (int i = 0; i < 3; i++) Kd[e][i] = {z, z, z};
-    for (int idx = lane; idx < 45; idx += 32) {
-      const int e = idx / 15, q = idx - e * 15;
-      const df3 v0 = e == 0 ? pc.Sf.p0 : (e == 1 ? pc.Sf.p1 : pc.Sf.p2);
-      const df3 v1 = e == 0 ? pc.Sf.v01 : (e == 1 ? pc.Sf.v12 : pc.Sf.v20);
-      const df3 v = df3_add(v0, df3_scale(df_make(c_line15[q][0]), v1));
-      near_edge_df(pc, nht, v, df_make(c_line15[q][1]), Kd[e]);
+    for (int e = 0; e < 3; e++) {
+      const T *x = st.edge_sum[e];
+      const V3<T> Ke = V3<T>{x[0], x[1], x[2]} - x[3] * pi;
+      ke = N::muladd(vdot(vcross(D, st.Sf.m[e]), Ke), N::rcp(st.Sf.ei[e]), ke);
     }
-    d3 Ke[3][3];
-#pragma unroll
-    for (int e = 0; e < 3; e++)
-#pragma unroll
-      for (int i = 0; i < 3; i++)
-        Ke[e][i] = {df_to_double(warp_sum_df(Kd[e][i].x)), df_to_double(warp_sum_df(Kd[e][i].y)),
-                    df_to_double(warp_sum_df(Kd[e][i].z))};
-    const double c = 0.125 * T.Ai * S.Ai;
-    const d3 m01 = ld3(S.m01), m12 = ld3(S.m12), m20 = ld3(S.m20);
-#pragma unroll
-    for (int i = 0; i < 3; i++)
-#pragma unroll
-      for (int j = 0; j < 3; j++) {
-        if (i >= nht || j >= nhs) continue;
-        const d3 v = ld3(T.hp0[i]) - ld3(S.hp0[j]);
-        K[i * 3 + j].r += c * (dot(cross(v, m01), Ke[0][i]) / S.nv01i + dot(cross(v, m12), Ke[1][i]) / S.nv12i +
-                               dot(cross(v, m20), Ke[2][i]) / S.nv20i);
-      }
-  }
-  if (lane < nht * nhs) {
-    const int i = lane / nhs, j = lane - (lane / nhs) * nhs;
-    z1 Lv = {0, 0}, Kv = {0, 0};
-#pragma unroll
-    for (int k = 0; k < 9; k++)
-      if (k == i * 3 + j) { Lv = L[k]; Kv = K[k]; }
-    const double c = scatter_coef(T, i, S, j);
-    const z1 cL = zscale(c, Lv), cK = zscale(c, Kv);
-    store_block_df(H, ntr, T.hrwg[i], T.hneg[i], S.hrwg[j], S.hneg[j], df_make(cL.r), df_make(cL.i), df_make(cK.r),
-                   df_make(cK.i));
+    K.r = N::muladd(N::of(0.125 * Tr.Ai * Sr.Ai), ke, K.r);
   }
 }
 
-// Near pairs in double-float, two pairs per warp: the 2 x 105 outer nodes of
-// the pair couple are spread over the lanes in 7 rounds of 32 (94 % of the
-// lanes busy, against 82 % for 105 nodes in 4 rounds); each lane adds to the
-// sums of the pair its node belongs to, and the warp finishes the pairs one
-// after the other.
-// The pair couple (p0, p0 + 1) of `list` (one pair when p0 + 1 == npairs),
-// worked by one warp in two parts: near_couple_df_sums runs the 2 x 105 outer
-// nodes (inner rule, closed forms, contraction) into acc, near_couple_df_finish
-// the warp sums, the neighbour-edge correction and the scatter.  nodes, pc:
-// the warp's shared staging, outer: the outer rule in double-float.
-struct NearCouple {
-  NearPair npr[2];
-  int np2;
-  NearAccDF acc[2];
-};
-
-__device__ __forceinline__ void near_couple_df_sums(const TriRec *__restrict__ Tr, const TriRec *__restrict__ Sr,
-                                                    const NearPair *__restrict__ list, int64_t npairs, int64_t p0,
-                                                    const GreenDev &g, float (*nodes)[BEMGPU_TRI_RULE91_N][8],
-                                                    const float (*outer)[6], NearPairDF *pcs, int lane,
-                                                    NearCouple &cp) {
-  const int np2 = p0 + 1 < npairs ? 2 : 1;
-  cp.np2 = np2;
-  NearPair *npr = cp.npr;
-  npr[0] = list[p0];
-  npr[1] = list[np2 == 2 ? p0 + 1 : p0];
-  // inner nodes l = r_s - P_s and weights of both pairs, then their records
-  for (int it = lane; it < np2 * BEMGPU_TRI_RULE91_N; it += 32) {
-    const int k = it >= BEMGPU_TRI_RULE91_N ? 1 : 0, u = it - k * BEMGPU_TRI_RULE91_N;
-    const TriRec &S = Sr[npr[k].s];
-    const d3 l = c_rule91[u][0] * ld3(S.v01) + c_rule91[u][1] * ld3(S.v02);
-    const double vals[4] = {l.x, l.y, l.z, c_rule91[u][2]};
-#pragma unroll
-    for (int c = 0; c < 4; c++) {
-      const df v = df_make(vals[c]);
-      nodes[k][u][2 * c] = v.hi;
-      nodes[k][u][2 * c + 1] = v.lo;
-    }
-  }
-  if (lane < np2) near_pair_df_setup(Tr[npr[lane].t], Sr[npr[lane].s], g, pcs[lane]);
-  __syncwarp();
-  NearAccDF *acc = cp.acc;
-  const df z = {0.f, 0.f};
-#pragma unroll
-  for (int k = 0; k < 9; k++) {
-    acc[0].L[k] = {z, z}; acc[0].K[k] = {z, z};
-    acc[1].L[k] = {z, z}; acc[1].K[k] = {z, z};
-  }
-  for (int it = lane; it < np2 * BEMGPU_TRI_RULE105_N; it += 32) {
-    const int k = it >= BEMGPU_TRI_RULE105_N ? 1 : 0, q = it - k * BEMGPU_TRI_RULE105_N;
-    const NearPairDF &pc = pcs[k];
-    const float *o = outer[q];
-    const df xi1 = {o[0], o[1]}, xi2 = {o[2], o[3]}, wq = {o[4], o[5]};
-    const df3 rt1 = df3_add(df3_scale(xi1, pc.v01t), df3_scale(xi2, pc.v02t));
-    const df3 rs = df3_sub(rt1, pc.sPs);
-    InnerMomDF mom;
-    near_inner_df<1>(nodes[k], &rs, g, &mom);
-    near_outer_df(mom, pc, Tr[npr[k].t].nh, Sr[npr[k].s].nh, rt1, wq, acc[k]);
-  }
+// Scatter coefficient of src/Impedance.cpp:372-375.
+template <typename T>
+__device__ __forceinline__ T near_scatter(const TriRec &T_, int i, const TriRec &S, int j) {
+  return Num<T>::of(scatter_coef(T_, i, S, j));
 }
 
-__device__ __forceinline__ void near_couple_df_finish(const TriRec *__restrict__ Tr, const TriRec *__restrict__ Sr,
-                                                      HalfPairBlock *__restrict__ H, int ntr, const NearPairDF *pcs,
-                                                      const NearCouple &cp) {
-  for (int k = 0; k < cp.np2; k++)
-    near_finish_df(Tr[cp.npr[k].t], Sr[cp.npr[k].s], cp.npr[k].same, pcs[k], cp.acc[k], H, ntr);
-  __syncwarp();
-}
-
-__device__ __forceinline__ void stage_outer_df(float (*outer)[6]) {
-  for (int u = threadIdx.x; u < BEMGPU_TRI_RULE105_N; u += blockDim.x)
-    for (int c = 0; c < 3; c++) {
-      const df v = df_make(c_rule105[u][c]);
-      outer[u][2 * c] = v.hi;
-      outer[u][2 * c + 1] = v.lo;
-    }
+// A launch's near pairs: warp w of CTA b takes units b * NEAR_WARPS + w + k *
+// (grid warps).  MINB: CTAs per SM that the register allocation must allow (the
+// context's tuning).  sync: the CTA's warps meet at a barrier after each pair,
+// which keeps them in the same code region.
+//
+// Bound by FP32 issue (double-float) or the FP64 pipe.  A warp's lanes take the
+// 91 source nodes (three rounds of 32, 95 % busy) and each loops over the 105
+// test nodes, which are the same for the whole warp (shared-memory broadcasts);
+// lanes over test nodes would need four rounds of 82 %.  Double-float, both
+// Green's functions of a body's pair at once: about 200 FP32 instructions a
+// node pair at |k| R <= 0.47, against about 900 for each of the two with sincos,
+// 1/R and Cartesian moments.  The near pairs of a solve's three fills, before
+// (two pairs per warp over the test nodes) and now: icospheres N = 7680 31.8 ->
+// 4.2 ms, slabs N = 11520 (interiors direct) 47.1 -> 21.0 ms, cubes N = 1152
+// 4.9 -> 2.1 ms; in FP64 cubes N = 1152 (interiors direct) 23.7 -> 14.6 ms, the
+// exterior fill of icospheres N = 1920 18.1 -> 8.1 ms.  168 registers (12 warps
+// an SM) against 226 (8): 4.7 -> 4.2 ms; 128 with spills the same; without the
+// barrier 4.4 ms.
+template <typename T, int KIND, int MINB>
+__global__ void __launch_bounds__(32 * NEAR_WARPS, MINB) near_pairs_kernel(const NearTask *__restrict__ tasks, int ntask,
+                                                                           int64_t units, int sync) {
+  typedef Num<T> N;
+  typedef NearCfg<T, KIND> Cfg;
+  constexpr int JF = Cfg::JF, JT = Cfg::JT;
+  __shared__ RuleNode<T> rule[NN_ALL];
+  __shared__ NearStage<T> stages[NEAR_WARPS];
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  NearStage<T> &st = stages[wid];
+  for (int k = threadIdx.x; k < NN_ALL; k += blockDim.x) rule[k] = near_nodes<T>()[k];
   __syncthreads();
-}
-
-// A group of fills: the warps walk the group's pair couples (a task's couples
-// are units [near0, near0 + ceil(nnear / 2)) of the group), each staging its
-// task's Green's function in shared memory.  MINB: CTAs per SM that the
-// register allocation must allow (2: ~250 registers; 3: 168; 4: 128 with
-// spills), chosen by the context's tuning.
-// Warp w of CTA b takes units b * NEAR_WARPS + w + k * (grid warps), k = 0, 1, ...
-// SYNC: the CTA's warps meet at a barrier after the outer nodes of each unit
-// and after its finish.  A pair couple runs several large code regions (the
-// inner rule, the closed-form potentials, the edge correction); with two warps
-// per scheduler, warps that have drifted into different regions stall on
-// instruction fetch, which the barriers prevent.
-// The units and their order per warp are the same either way.
-template <int MINB, bool SYNC>
-__global__ void __launch_bounds__(32 * NEAR_WARPS, MINB) near_pairs_df_group_kernel(const FillTask *__restrict__ tasks,
-                                                                                    int ntask, int64_t units) {
-  __shared__ __align__(16) float s_nodes[NEAR_WARPS][2][BEMGPU_TRI_RULE91_N][8];
-  __shared__ float s_outer[BEMGPU_TRI_RULE105_N][6];
-  __shared__ NearPairDF s_pc[NEAR_WARPS][2];
-  __shared__ GreenDev s_g[NEAR_WARPS];
-  const int lane = threadIdx.x & 31;
-  const int wid = threadIdx.x >> 5;
-  stage_outer_df(s_outer);
   const int64_t nw = (int64_t)gridDim.x * NEAR_WARPS;
-  int cur = -1;
   for (int64_t base = (int64_t)blockIdx.x * NEAR_WARPS; base < units; base += nw) {
     const int64_t u = base + wid;
-    const bool active = u < units;
-    NearCouple cp;
-    const FillTask *tk = nullptr;
-    if (active) {
-      const int i = task_of_near(tasks, ntask, u);
-      tk = &tasks[i];
-      if (i != cur) {
-        if (lane == 0) s_g[wid] = tk->g;
-        __syncwarp();
-        cur = i;
-      }
-      near_couple_df_sums(tk->T, tk->S, tk->near, tk->nnear, 2 * (u - tk->near0), s_g[wid], s_nodes[wid], s_outer,
-                          s_pc[wid], lane, cp);
-    }
-    // base is the same for the whole CTA: every warp meets both barriers
-    if (SYNC) __syncthreads();
-    if (active) near_couple_df_finish(tk->T, tk->S, tk->H, tk->ntr, s_pc[wid], cp);
-    if (SYNC) __syncthreads();
-  }
-}
-
-template <int MINB>
-void launch_near_df(bool sync, int nb, cudaStream_t stream, const FillTask *tasks, int ntask, int64_t units) {
-  if (sync)
-    near_pairs_df_group_kernel<MINB, true><<<nb, 32 * NEAR_WARPS, 0, stream>>>(tasks, ntask, units);
-  else
-    near_pairs_df_group_kernel<MINB, false><<<nb, 32 * NEAR_WARPS, 0, stream>>>(tasks, ntask, units);
-}
-
-// Near pairs in FP64 (the plain path), one pair per warp: lanes take the
-// outer nodes, each runs the 91-node smooth inner rule, the analytic singular
-// terms and the close-pair contraction; the warp sums, adds the neighbour-edge
-// K correction and scatters.
-// Near pair p of `list` in FP64, worked by one warp (nodes: the warp's
-// shared staging of the inner rule).
-__device__ __forceinline__ void near_pair_fp64(const TriRec *__restrict__ Tr, const TriRec *__restrict__ Sr,
-                                               const NearPair *__restrict__ list, int64_t p, const GreenDev &g,
-                                               HalfPairBlock *__restrict__ H, int ntr, double (*nodes)[4], int lane) {
-  const z1 ksq = {g.ksqr, g.ksqi};
-  const z1 k2 = {g.k2r, g.k2i};
-  const NearPair np = list[p];
-  const TriRec &T = Tr[np.t];
-  const TriRec &S = Sr[np.s];
-  const d3 Pt = ld3(T.p0), Ps = ld3(S.p0);
-  const d3 v01t = ld3(T.v01), v02t = ld3(T.v02);
-  {
-    const d3 v01s = ld3(S.v01), v02s = ld3(S.v02);
-    for (int u = lane; u < BEMGPU_TRI_RULE91_N; u += 32) {
-      const d3 l = c_rule91[u][0] * v01s + c_rule91[u][1] * v02s;
-      nodes[u][0] = l.x; nodes[u][1] = l.y; nodes[u][2] = l.z;
-      nodes[u][3] = c_rule91[u][2];
-    }
-  }
-  __syncwarp();
-  const int nht = T.nh, nhs = S.nh;
-  d3 dj[3];
-  for (int j = 0; j < 3; j++) dj[j] = (j < nhs) ? ld3(S.hp0[j]) - Ps : d3{0, 0, 0};
-  z1 L[9], K[9];
-#pragma unroll
-  for (int k = 0; k < 9; k++) { L[k] = {0, 0}; K[k] = {0, 0}; }
-  const d3 nS = ld3(S.n);
-  const double Ai2 = 0.5 * S.Ai;
-  for (int q = lane; q < BEMGPU_TRI_RULE105_N; q += 32) {
-    const double w = c_rule105[q][2];
-    const d3 rt = (Pt + c_rule105[q][0] * v01t) + c_rule105[q][1] * v02t;
-    const d3 rts = rt - Ps;
-    // LKSmoothInnerIntegrand over s[0] (src/Impedance.cpp:93-105) as moments
-    z1 I0 = {0, 0}, Q0 = {0, 0};
-    z3 A = z3zero(), Q1 = z3zero();
-    for (int u = 0; u < BEMGPU_TRI_RULE91_N; u++) {
-      const d3 l = {nodes[u][0], nodes[u][1], nodes[u][2]};
-      const double ws = nodes[u][3];
-      const d3 x = rts - l;
-      const double R2 = dot(x, x);
-      const double R = sqrt(R2);
-      const z1 e = zexp_ikR(g, R);
-      // scalar_gradient_smooth, src/GreensFunction.cpp:54-69
-      const double Ri = 1.0 / R;
-      const z1 gs = zsub(zscale(Ri, z1{e.r - 1.0, e.i}), zscale(R, k2));
-      const z1 ikR = {g.ikr * R, g.iki * R};
-      z1 num = zmul(e, z1{1.0 - ikR.r, -ikR.i});
-      num = zadd(num, zscale(R2, k2));
-      num.r -= 1.0;
-      const z1 qq = zscale(Ri * Ri * Ri, num);
-      const z1 gw = zscale(ws, gs), qw = zscale(ws, qq);
-      zacc(I0, gw);
-      A = z3add(A, zs_v(gw, l));
-      zacc(Q0, qw);
-      Q1 = z3add(Q1, zs_v(qw, l));
-    }
-    // LKCloseOuterIntegrand::weighPoint, src/Impedance.cpp:194-250
-    double ISn3h, ISn1, IS1;
-    d3 IL1, IL3;
-    eh_nonsmooth(S, rt, ISn3h, ISn1, IS1, IL1, IL3);
-    const z3 IL13 = z3scale(Ai2, z3add_r(zs_v(zscale(BEM_ONETHIRD, k2), IL3), IL1));
-    z1 ISn11 = zscale(Ai2, z1{ISn1 + k2.r * IS1, k2.i * IS1});
-    const double h = dot(rt - Ps, nS);
-    const z1 L2 = zadd(zscale(2.0, ISn11), I0);
-    if (fabs(h) < 1e-8 * S.elen0) {
-#pragma unroll
-      for (int j = 0; j < 3; j++) {
-        if (j >= nhs) break;
-        const z3 Gphij = z3scale(0.5, z3sub(A, zs_v(I0, dj[j])));
-        const z3 K21 = z3add(IL13, zs_v(ISn11, rt - ld3(S.hp0[j])));
-        const z3 GK = z3add(Gphij, K21);
-#pragma unroll
-        for (int i = 0; i < 3; i++) {
-          if (i >= nht) break;
-          const d3 phi = 0.5 * (rt - ld3(T.hp0[i]));
-          const z1 t = zsub(zmul(ksq, rdot(phi, GK)), L2);
-          zacc(L[i * 3 + j], zscale(w, t));
+    if (u < units) {
+      int ti = ntask - 1;
+      while (ti > 0 && u < tasks[ti].unit0) ti--;
+      const NearTask &tk = tasks[ti];
+      const NearPair np = tk.near[u - tk.unit0];
+      const TriRec &Tr = tk.T[np.t];
+      const TriRec &Sr = tk.S[np.s];
+      const bool same = np.same != 0;
+      // the Green's functions of this pair
+      int second = 0;
+      for (int k = 1; k < tk.ngreen; k++)
+        if (np.t >= tk.g[k].tri0 && np.t < tk.g[k].tri1 && np.s >= tk.g[k].tri0 && np.s < tk.g[k].tri1) second = k;
+      // both triangles relative to P_t, the test nodes relative to P_s (scaled)
+      {
+        const double *O = Tr.p0;
+        T *Fs = reinterpret_cast<T *>(&st.Sf), *Ft = reinterpret_cast<T *>(&st.Tf);
+        for (int k = lane; k < 66; k += 32) {
+          const int f = k < 33 ? k : k - 33;
+          // NearFrame's order within a TriRec: p0 p1 p2 | n | v01 v12 v20 | m01 m12 m20 | 1/|v|
+          const int src = f < 9 ? f : f < 12 ? f + 12 : f < 21 ? f - 3 : f + 3;
+          const double *rec = reinterpret_cast<const double *>(k < 33 ? &Sr : &Tr);
+          const T v = N::of(f < 9 ? rec[src] - O[f % 3] : rec[src]);
+          if (k < 33) Fs[f] = v;
+          else Ft[f] = v;
         }
       }
-    } else {
-      const d3 ISn3hn = (Ai2 * ISn3h) * nS;
-      const d3 rho = rt - h * nS;
-      const z1 Ai2k2 = zscale(Ai2, k2);
-      const z3 K31 = zs_v(Ai2k2, IL1 - (h * ISn1) * nS);
-#pragma unroll
-      for (int j = 0; j < 3; j++) {
-        if (j >= nhs) break;
-        const d3 p0j = ld3(S.hp0[j]);
-        const z3 Gphij = z3scale(0.5, z3sub(A, zs_v(I0, dj[j])));
-        const z3 DGxphij = z3scale(0.5, rcross(rt - p0j, z3sub(Q1, zs_v(Q0, dj[j]))));
-        const z3 K21 = z3add(IL13, zs_v(ISn11, rho - p0j));
-        const z3 K41 = zcross(K31, rt - p0j);
-        const z3 GK = z3add(Gphij, K21);
-#pragma unroll
-        for (int i = 0; i < 3; i++) {
-          if (i >= nht) break;
-          const d3 p0i = ld3(T.hp0[i]);
-          const d3 phi = 0.5 * (rt - p0i);
-          const z1 t = zsub(zmul(ksq, rdot(phi, GK)), L2);
-          zacc(L[i * 3 + j], zscale(w, t));
-          const d3 vts = p0j - p0i;
-          const z3 KK = z3add(z3add_r(DGxphij, cross(vts, ISn3hn)), K41);
-          const z1 kk = rdot(phi, KK);
-          K[i * 3 + j].r -= w * kk.r;
-          K[i * 3 + j].i -= w * kk.i;
-        }
+      const float sc = (float)tk.scale;
+      V3<T> d0, a1, a2, c1, c2;
+      {
+        auto v = [](const double *p) { return V3<T>{N::of(p[0]), N::of(p[1]), N::of(p[2])}; };
+        d0 = vscale2(V3<T>{N::of(Tr.p0[0] - Sr.p0[0]), N::of(Tr.p0[1] - Sr.p0[1]), N::of(Tr.p0[2] - Sr.p0[2])}, sc);
+        a1 = vscale2(v(Tr.v01), sc);
+        a2 = vscale2(v(Tr.v02), sc);
+        c1 = vscale2(v(Sr.v01), sc);
+        c2 = vscale2(v(Sr.v02), sc);
       }
-    }
-  }
-#pragma unroll
-  for (int k = 0; k < 9; k++) {
-    L[k].r = warp_sum(L[k].r); L[k].i = warp_sum(L[k].i);
-    K[k].r = warp_sum(K[k].r); K[k].i = warp_sum(K[k].i);
-  }
-  if (!np.same) {
-    // neighbour-edge K correction, src/Impedance.cpp:301-324: three source
-    // edges x QuadratureGauss15, LKNeighborEdgeIntegrand over t[0].
-    d3 Ke[3][3];
-#pragma unroll
-    for (int e = 0; e < 3; e++)
-#pragma unroll
-      for (int i = 0; i < 3; i++) Ke[e][i] = {0, 0, 0};
-    const d3 nT = ld3(T.n);
-    for (int idx = lane; idx < 45; idx += 32) {
-      const int e = idx / 15, q = idx - e * 15;
-      const d3 v0 = e == 0 ? ld3(S.p0) : (e == 1 ? ld3(S.p1) : ld3(S.p2));
-      const d3 v1 = e == 0 ? ld3(S.v01) : (e == 1 ? ld3(S.v12) : ld3(S.v20));
-      const d3 v = v0 + c_line15[q][0] * v1;
-      const double w = c_line15[q][1];
-      double ISn1;
-      d3 IL1;
-      lk_edge_integral(T, v, ISn1, IL1);
-      const double h = dot(v - Pt, nT);
-      const d3 rho = v - h * nT;
-#pragma unroll
-      for (int i = 0; i < 3; i++) {
-        if (i >= nht) break;
-        const d3 c = IL1 + ISn1 * (rho - ld3(T.hp0[i]));
-        if (e == 0) Ke[0][i] = Ke[0][i] + w * c;
-        else if (e == 1) Ke[1][i] = Ke[1][i] + w * c;
-        else Ke[2][i] = Ke[2][i] + w * c;
+      for (int k = lane; k < 105; k += 32) {
+        const RuleNode<T> n = rule[NN105 + k];
+        st.q[k] = {d0 + (n.x1 * a1 + n.x2 * a2), n.w, n.w1, n.w2};
       }
-    }
-#pragma unroll
-    for (int e = 0; e < 3; e++)
-#pragma unroll
-      for (int i = 0; i < 3; i++) {
-        Ke[e][i].x = warp_sum(Ke[e][i].x);
-        Ke[e][i].y = warp_sum(Ke[e][i].y);
-        Ke[e][i].z = warp_sum(Ke[e][i].z);
-      }
-    const double c = 0.125 * T.Ai * S.Ai;
-    const d3 m01 = ld3(S.m01), m12 = ld3(S.m12), m20 = ld3(S.m20);
-#pragma unroll
-    for (int i = 0; i < 3; i++)
-#pragma unroll
-      for (int j = 0; j < 3; j++) {
-        if (i >= nht || j >= nhs) continue;
-        const d3 v = ld3(T.hp0[i]) - ld3(S.hp0[j]);
-        K[i * 3 + j].r += c * (dot(cross(v, m01), Ke[0][i]) / S.nv01i + dot(cross(v, m12), Ke[1][i]) / S.nv12i +
-                               dot(cross(v, m20), Ke[2][i]) / S.nv20i);
-      }
-  }
-  if (lane < nht * nhs) {
-    const int i = lane / nhs, j = lane - (lane / nhs) * nhs;
-    z1 Lv = {0, 0}, Kv = {0, 0};
-#pragma unroll
-    for (int k = 0; k < 9; k++)
-      if (k == i * 3 + j) { Lv = L[k]; Kv = K[k]; }
-    const double c = scatter_coef(T, i, S, j);
-    store_block(H, ntr, T.hrwg[i], T.hneg[i], S.hrwg[j], S.hneg[j], zscale(c, Lv), zscale(c, Kv));
-  }
-  __syncwarp();
-}
-
-__global__ void __launch_bounds__(32 * NEAR_WARPS) near_pairs_kernel(
-    const TriRec *__restrict__ Tr, const TriRec *__restrict__ Sr, const NearPair *__restrict__ list, int64_t npairs,
-    GreenDev g, HalfPairBlock *__restrict__ H, int ntr) {
-  __shared__ double s_nodes[NEAR_WARPS][BEMGPU_TRI_RULE91_N][4];  // l = r_s - P_s (xyz), weight
-  const int lane = threadIdx.x & 31;
-  const int wid = threadIdx.x >> 5;
-  for (int64_t p = (int64_t)blockIdx.x * NEAR_WARPS + wid; p < npairs; p += (int64_t)gridDim.x * NEAR_WARPS)
-    near_pair_fp64(Tr, Sr, list, p, g, H, ntr, s_nodes[wid], lane);
-}
-
-// A group of fills in FP64: the warps walk the group's near pairs (a task's
-// pairs are units [near0, near0 + nnear) of the group).
-__global__ void __launch_bounds__(32 * NEAR_WARPS) near_pairs_group_kernel(const FillTask *__restrict__ tasks,
-                                                                           int ntask, int64_t units) {
-  __shared__ double s_nodes[NEAR_WARPS][BEMGPU_TRI_RULE91_N][4];
-  __shared__ GreenDev s_g[NEAR_WARPS];
-  const int lane = threadIdx.x & 31;
-  const int wid = threadIdx.x >> 5;
-  int cur = -1;
-  for (int64_t u = (int64_t)blockIdx.x * NEAR_WARPS + wid; u < units; u += (int64_t)gridDim.x * NEAR_WARPS) {
-    const int i = task_of_near(tasks, ntask, u);
-    const FillTask &tk = tasks[i];
-    if (i != cur) {
-      if (lane == 0) s_g[wid] = tk.g;
+      for (int k = lane; k < 81; k += 32) st.odd[k] = N::of(0.0);
+      for (int k = lane; k < 90; k += 32) st.even[k] = N::of(0.0);
+      if (lane < 24) st.sing[lane] = N::of(0.0);
       __syncwarp();
-      cur = i;
+      // ---- smooth part: moments of the powers of R, or of g~ and q~
+#pragma unroll 1
+      for (int r = 0; r < 3; r++) {
+        const int k = lane + 32 * r;
+        RuleNode<T> n = rule[NN91 + (k < 91 ? k : 0)];
+        if (k >= 91) n.w = n.w1 = n.w2 = N::of(0.0);
+        const V3<T> l = n.x1 * c1 + n.x2 * c2;
+        if constexpr (KIND == NEAR_DIRECT) {
+          const GreenT<T> g = green_of<T>(tk.g[0].g);
+          // unscaled coordinates: scale is 1 in this kind
+          T S[4][3];
+#pragma unroll
+          for (int c = 0; c < 4; c++) S[c][0] = S[c][1] = S[c][2] = N::of(0.0);
+          auto loop = [&](auto real) {
+#pragma unroll 1
+            for (int q = 0; q < 105; q++) {
+              const NearNode<T> nd = st.q[q];
+              T f[4];
+              near_values<T, decltype(real)::value>(
+                  g, {N::diff(nd.p.x, l.x), N::diff(nd.p.y, l.y), N::diff(nd.p.z, l.z)}, f);
+#pragma unroll
+              for (int c = 0; c < 4; c++) {
+                N::mac(S[c][0], f[c], nd.w);
+                N::mac(S[c][1], f[c], nd.w1);
+                N::mac(S[c][2], f[c], nd.w2);
+              }
+            }
+          };
+          if (tk.g[0].realk) loop(std::true_type{});
+          else loop(std::false_type{});
+#pragma unroll
+          for (int c = 0; c < 4; c++)
+#pragma unroll
+            for (int a = 0; a < 3; a++) S[c][a] = N::fin(S[c][a]);
+          near_reduce<T, 36>(st.odd, lane, [&](int v) {
+            const int b = v % 3;
+            return (b == 0 ? n.w : b == 1 ? n.w1 : n.w2) * S[v / 9][v / 3 % 3];
+          });
+        } else {
+          T S[JF][3];
+          typename N::Tail St[JT - JF + 1][3];
+          near_power_sums<T, JF, JT, true>(st.q, 0, 105, 1, l, S, St);
+          near_reduce<T, JF * 9>(st.odd, lane, [&](int v) {
+            const int b = v % 3;
+            return (b == 0 ? n.w : b == 1 ? n.w1 : n.w2) * S[v / 9][v / 3 % 3];
+          });
+          if constexpr (JT > JF)
+            near_reduce<T, (JT - JF) * 9>(st.odd + JF * 9, lane, [&](int v) {
+              const int b = v % 3;
+              return N::tail(N::head(b == 0 ? n.w : b == 1 ? n.w1 : n.w2) * St[v / 9][v / 3 % 3]);
+            });
+        }
+      }
+      if constexpr (KIND != NEAR_DIRECT) {
+        // even powers over 36 x 36 nodes: 32 source nodes by the lanes, then the
+        // last four by eight lanes each
+        __syncwarp();
+        for (int k = lane; k < 36; k += 32) {
+          const RuleNode<T> n = rule[NNE105 + k];
+          st.q[k] = {d0 + (n.x1 * a1 + n.x2 * a2), n.w, n.w1, n.w2};
+        }
+        __syncwarp();
+#pragma unroll 1
+        for (int r = 0; r < 2; r++) {
+          const RuleNode<T> n = rule[NNE91 + (r == 0 ? lane : 32 + (lane & 3))];
+          const V3<T> l = n.x1 * c1 + n.x2 * c2;
+          T S[JF][3];
+          typename N::Tail St[JT - JF + 1][3];
+          near_power_sums<T, JF, JT, false>(st.q, r == 0 ? 0 : lane >> 2, 36, r == 0 ? 1 : 8, l, S, St);
+          near_reduce<T, JF * 9>(st.even + 9, lane, [&](int v) {
+            const int b = v % 3;
+            return (b == 0 ? n.w : b == 1 ? n.w1 : n.w2) * S[v / 9][v / 3 % 3];
+          });
+          if constexpr (JT > JF)
+            near_reduce<T, (JT - JF) * 9>(st.even + 9 + JF * 9, lane, [&](int v) {
+              const int b = v % 3;
+              return N::tail(N::head(b == 0 ? n.w : b == 1 ? n.w1 : n.w2) * St[v / 9][v / 3 % 3]);
+            });
+        }
+        // the constant's moments: products of the rules' sums
+        if (lane < 9) st.even[lane] = N::of(c_sums[SUM105].w[lane / 3]) * N::of(c_sums[SUM91].w[lane % 3]);
+      }
+      // ---- singular part: the 105 test nodes, then the neighbours' 45 edge nodes
+      {
+        T s[23];
+#pragma unroll
+        for (int k = 0; k < 23; k++) s[k] = N::of(0.0);
+        const V3<T> e1 = st.Tf.p[1], e2 = st.Tf.p[2];
+        const typename N::Tail tol = (typename N::Tail)(1e-6 * Sr.elen0),
+                               tol_plane = (typename N::Tail)(1e-8 * Sr.elen0),
+                               tol_edge = (typename N::Tail)(1e-8 * Tr.elen0);
+#pragma unroll 1
+        for (int it = lane; it < (same ? 105 : 150); it += 32) {
+          const bool node = it < 105;
+          RuleNode<T> n = rule[NN105 + (node ? it : 0)];
+          V3<T> r;
+          T wl = N::of(0.0);
+          if (node) {
+            r = n.x1 * e1 + n.x2 * e2;
+          } else {
+            const int e = (it - 105) / 15, k = (it - 105) - e * 15;
+            r = st.Sf.p[e] + N::of(c_line15[k][0]) * st.Sf.e[e];
+            wl = N::of(c_line15[k][1]);
+          }
+          NearPot<T> o;
+          near_potentials<T>(node ? st.Sf : st.Tf, r, node ? tol : tol_edge, node, o);
+          if (node) {
+            const bool flat = fabs(N::head(o.h)) < tol_plane;
+            const V3<T> rp = flat ? r : r - o.h * st.Sf.n;
+            const V3<T> X0 = o.IL1 + o.ISn1 * rp, X1 = N::of(BEM_ONETHIRD) * o.IL3 + o.IS1 * rp;
+            N::mac(s[0], n.w, vdot(r, X0));
+            N::mac(s[1], n.w, X0.x); N::mac(s[2], n.w, X0.y); N::mac(s[3], n.w, X0.z);
+            N::mac(s[4], n.w, o.ISn1); N::mac(s[5], n.w1, o.ISn1); N::mac(s[6], n.w2, o.ISn1);
+            N::mac(s[7], n.w, vdot(r, X1));
+            N::mac(s[8], n.w, X1.x); N::mac(s[9], n.w, X1.y); N::mac(s[10], n.w, X1.z);
+            N::mac(s[11], n.w, o.IS1); N::mac(s[12], n.w1, o.IS1); N::mac(s[13], n.w2, o.IS1);
+            if (!flat) {
+              N::mac(s[14], n.w, o.ISn3h); N::mac(s[15], n.w1, o.ISn3h); N::mac(s[16], n.w2, o.ISn3h);
+              const V3<T> Y = o.IL1 - (o.h * o.ISn1) * st.Sf.n;
+              const V3<T> rY = vcross(r, Y);
+              N::mac(s[17], n.w, Y.x); N::mac(s[18], n.w, Y.y); N::mac(s[19], n.w, Y.z);
+              N::mac(s[20], n.w, rY.x); N::mac(s[21], n.w, rY.y); N::mac(s[22], n.w, rY.z);
+            }
+          } else {
+            const V3<T> X = wl * (o.IL1 + o.ISn1 * (r - o.h * st.Tf.n));
+            T *e = st.edge(it - 105);
+            e[0] = X.x; e[1] = X.y; e[2] = X.z;
+            e[3] = wl * o.ISn1;
+          }
+        }
+        __syncwarp();
+        near_reduce<T, 23>(st.sing, lane, [&](int v) { return N::fin(s[v]); });
+        if (!same && lane < 12) {
+          T a = N::of(0.0);
+          for (int k = 0; k < 15; k++) a = a + st.edge((lane >> 2) * 15 + k)[lane & 3];
+          st.edge_sum[lane >> 2][lane & 3] = a;
+        }
+      }
+      __syncwarp();
+      // ---- moments of g~ and q~ of the pair's Green's functions
+      const int ng = second ? 2 : 1;
+      for (int k = lane; k < 18 * ng; k += 32) {
+        const int gi = k / 18, c = (k - gi * 18) / 9, ab = k % 9;
+        const NearGreen &G = tk.g[gi ? second : 0];
+        C1<T> v;
+        if constexpr (KIND == NEAR_DIRECT) {
+          v = {st.odd[c * 18 + ab], st.odd[c * 18 + 9 + ab]};
+          // the constant that near_values leaves out of Im g~ (wave_at)
+          if (N::LESS && c == 0) {
+            const T kk = green_of<T>(G.g).iki;
+            if (ab == 0) st.mom[gi][4][0] = v.i + kk * N::of(c_near_ww1);
+            v.i = N::muladd(kk * N::of(c_sums[SUM105].w[ab / 3]), N::of(c_sums[SUM91].w[ab % 3]), v.i);
+          }
+        } else {
+          const double(*ce)[2] = c ? G.qe : G.ge, (*co)[2] = c ? G.qo : G.go;
+          T vr = N::of(0.0), vi = vr;
+#pragma unroll 1
+          for (int j = JT; j >= 1; j--) {
+            const C1<T> e = near_coef<T>(ce, j), o = near_coef<T>(co, j - 1);
+            N::mac(vr, e.r, st.even[j * 9 + ab]);
+            N::mac(vi, e.i, st.even[j * 9 + ab]);
+            N::mac(vr, o.r, st.odd[(j - 1) * 9 + ab]);
+            N::mac(vi, o.i, st.odd[(j - 1) * 9 + ab]);
+          }
+          const C1<T> e = near_coef<T>(ce, 0);
+          vr = N::fin(vr);
+          vi = N::fin(vi);
+          // -G_00 without the constant Im(ik) (wave_at)
+          if (N::LESS && c == 0 && ab == 0) st.mom[gi][4][0] = vi + e.i * N::of(c_near_ww1);
+          v = {N::muladd(e.r, st.even[ab], vr), N::muladd(e.i, st.even[ab], vi)};
+        }
+        if (c == 0) {
+          st.mom[gi][0][ab] = v.r;
+          st.mom[gi][1][ab] = v.i;
+        } else {
+          st.qraw[gi][0][ab] = v.r;
+          st.qraw[gi][1][ab] = v.i;
+        }
+      }
+      __syncwarp();
+      for (int k = lane; k < 18 * ng; k += 32) {  // barycentric: B_v = sum over {1, x1, x2} with 1 - x1 - x2 for v = 0
+        const int gi = k / 18, ri = (k - gi * 18) / 9, ab = k % 9, x = ab / 3, y = ab % 3;
+        const T *Q = st.qraw[gi][ri];
+        auto along = [&](int row) { return y ? Q[row * 3 + y] : (Q[row * 3] - Q[row * 3 + 1]) - Q[row * 3 + 2]; };
+        st.mom[gi][2 + ri][ab] = x ? along(x) : (along(0) - along(1)) - along(2);
+      }
+      __syncwarp();
+      // ---- the nine products: lanes 0..8 the first Green's function, 16..24 the second
+      {
+        const int gi = lane >> 4, ij = lane & 15;
+        if (gi < ng && ij < 9 && ij / 3 < Tr.nh && ij % 3 < Sr.nh) {
+          const int i = ij / 3, j = ij % 3;
+          const NearGreen &G = tk.g[gi ? second : 0];
+          C1<T> L, K;
+          near_product<T>(st, st.mom[gi], G.g, Tr, Sr, (Tr.hvert >> (2 * i)) & 3,
+                          (Sr.hvert >> (2 * j)) & 3, same, L, K);
+          const T c = near_scatter<T>(Tr, i, Sr, j);
+          store_pair(G.H, G.ntr, Tr.hrwg[i] - G.rwg0, Tr.hneg[i], Sr.hrwg[j] - G.rwg0, Sr.hneg[j], c * L, c * K);
+        }
+      }
+      __syncwarp();
     }
-    near_pair_fp64(tk.T, tk.S, tk.near, u - tk.near0, s_g[wid], tk.H, tk.ntr, s_nodes[wid], lane);
+    // base is the same for the whole CTA: every warp meets the barrier
+    if (sync) __syncthreads();
   }
+}
+
+template <typename T, int MINB>
+void launch_near_kind(int kind, int nb, cudaStream_t st, const NearTask *tasks, int ntask, int64_t units, int sync) {
+  if (kind == NEAR_SERIES1)
+    near_pairs_kernel<T, NEAR_SERIES1, MINB><<<nb, 32 * NEAR_WARPS, 0, st>>>(tasks, ntask, units, sync);
+  else if (kind == NEAR_SERIES2)
+    near_pairs_kernel<T, NEAR_SERIES2, MINB><<<nb, 32 * NEAR_WARPS, 0, st>>>(tasks, ntask, units, sync);
+  else
+    near_pairs_kernel<T, NEAR_DIRECT, MINB><<<nb, 32 * NEAR_WARPS, 0, st>>>(tasks, ntask, units, sync);
+}
+
+// The near pairs of `ntask` tasks of one kind.
+void launch_near(bool dfl, int minb, int kind, int nb, cudaStream_t st, const NearTask *tasks, int ntask, int64_t units,
+                 int sync) {
+  if (!dfl)
+    launch_near_kind<double, 2>(kind, nb, st, tasks, ntask, units, sync);
+  else if (minb == 3)
+    launch_near_kind<df, 3>(kind, nb, st, tasks, ntask, units, sync);
+  else if (minb == 4)
+    launch_near_kind<df, 4>(kind, nb, st, tasks, ntask, units, sync);
+  else
+    launch_near_kind<df, 2>(kind, nb, st, tasks, ntask, units, sync);
 }
 
 // ---------------- gather: half-pair blocks -> Z ----------------
@@ -1780,6 +1589,75 @@ GreenDev to_dev(const bemgpu_green_t *g) {
 
 ZDev to_zdev(const bemgpu_green_t *g) { return {g->Zeps[0], g->Zeps[1], g->Zmu[0], g->Zmu[1]}; }
 
+// The kind of a near task whose Green's functions have wavenumbers of at most
+// kabs and whose triangles' edges are at most emax long: two triangles that
+// share a vertex have no points farther apart than two edges.
+int near_kind(double kabs, double emax) {
+  const double x = kabs * 2.0 * emax;
+  return x <= NEAR_X1 ? NEAR_SERIES1 : x <= NEAR_X2 ? NEAR_SERIES2 : NEAR_DIRECT;
+}
+
+double green_kabs(const bemgpu_green_t *g) { return std::hypot(g->ik[0], g->ik[1]); }
+
+// The power of two that brings distances of up to 2 emax below one.
+double near_scale(double emax) {
+  int e = 0;
+  std::frexp(2.0 * emax, &e);
+  return std::ldexp(1.0, -e);
+}
+
+// One Green's function of a near task: (ik)^n / n! (times 1 - n for q~) in
+// powers of the scaled distance.
+NearGreen near_green(const bemgpu_green_t *g, double scale, bool dfl, HalfPairBlock *H, int ntr, int rwg0, int tri0,
+                     int tri1) {
+  NearGreen G;
+  memset(&G, 0, sizeof G);
+  G.H = H;
+  G.ntr = ntr;
+  G.rwg0 = rwg0;
+  G.tri0 = tri0;
+  G.tri1 = tri1;
+  G.realk = g->ik[0] == 0.0 && g->ksquared[1] == 0.0;
+  G.g = to_dev(g);
+  const long double kr = (long double)g->ik[0] / scale, ki = (long double)g->ik[1] / scale;
+  long double pr = 1.0L, pi = 0.0L;  // (ik / scale)^n / n!
+  auto put = [&](double (*c)[2], int j, long double f) {
+    if (j < 0 || j >= NEAR_NJ) return;
+    const double re = (double)(f * pr), im = (double)(f * pi);
+    if (dfl) {
+      const df a = host_df(re), b = host_df(im);
+      const float v[4] = {a.hi, a.lo, b.hi, b.lo};
+      memcpy(c[j], v, sizeof v);
+    } else {
+      c[j][0] = re;
+      c[j][1] = im;
+    }
+  };
+  const long double s1 = scale, s3 = (long double)scale * scale * scale;
+  for (int n = 1; n <= 2 * NEAR_NJ + 2; n++) {
+    const long double r = (pr * kr - pi * ki) / n, i = (pr * ki + pi * kr) / n;
+    pr = r;
+    pi = i;
+    if (n % 2) {
+      put(G.ge, (n - 1) / 2, s1);
+      if (n >= 3) put(G.qe, (n - 3) / 2, s3 * (1 - n));
+    } else if (n >= 4) {
+      put(G.go, (n - 2) / 2, s1);
+      put(G.qo, (n - 4) / 2, s3 * (1 - n));
+    }
+  }
+  return G;
+}
+
+// Whether top is the tree of a's RWGs followed by b's, on separate triangles:
+// its triangles are then a's followed by b's, with the same frames.
+bool is_two_body(const bemgpu_tree_s *top, const bemgpu_tree_s *a, const bemgpu_tree_s *b) {
+  return top->geom == a->geom && top->geom == b->geom && top->nrwg == a->nrwg + b->nrwg &&
+         top->ntri == a->ntri + b->ntri && top->rwg.size() == a->rwg.size() + b->rwg.size() &&
+         std::equal(a->rwg.begin(), a->rwg.end(), top->rwg.begin()) &&
+         std::equal(b->rwg.begin(), b->rwg.end(), top->rwg.begin() + (std::ptrdiff_t)a->rwg.size());
+}
+
 bool g_tables_loaded[BEM_MAX_DEVICES] = {false};
 
 std::mutex g_tables_mu;
@@ -1795,8 +1673,6 @@ int load_tables(bemgpu_ctx_s *ctx) {
   BEM_CUDA_TRY(ctx, cudaMemcpyToSymbol(c_rule15, bemgpu_tri_rule15, sizeof(bemgpu_tri_rule15)));
   BEM_CUDA_TRY(ctx, cudaMemcpyToSymbol(c_rule21, bemgpu_tri_rule21, sizeof(bemgpu_tri_rule21)));
   BEM_CUDA_TRY(ctx, cudaMemcpyToSymbol(c_rule36, bemgpu_tri_rule36, sizeof(bemgpu_tri_rule36)));
-  BEM_CUDA_TRY(ctx, cudaMemcpyToSymbol(c_rule91, bemgpu_tri_rule91, sizeof(bemgpu_tri_rule91)));
-  BEM_CUDA_TRY(ctx, cudaMemcpyToSymbol(c_rule105, bemgpu_tri_rule105, sizeof(bemgpu_tri_rule105)));
   BEM_CUDA_TRY(ctx, cudaMemcpyToSymbol(c_line15, bemgpu_line_rule15, sizeof(bemgpu_line_rule15)));
   {
     const struct {
@@ -1812,6 +1688,44 @@ int load_tables(bemgpu_ctx_s *ctx) {
         nd[r.off + k] = {x1, x2, w, w * x1, w * x2};
         nf[r.off + k] = {host_df(x1), host_df(x2), host_df(w), host_df(w * x1), host_df(w * x2)};
       }
+    const struct {
+      const double (*rule)[3];
+      int n;
+    } all[NSUMS] = {{bemgpu_tri_rule6, 6},   {bemgpu_tri_rule10, 10}, {bemgpu_tri_rule15, 15},  {bemgpu_tri_rule21, 21},
+                    {bemgpu_tri_rule36, 36}, {bemgpu_tri_rule91, 91}, {bemgpu_tri_rule105, 105}};
+    RuleSum sums[NSUMS];
+    double less[NSUMS];
+    for (int i = 0; i < NSUMS; i++) {
+      long double a[3] = {-1.0L, 0.0L, 0.0L};  // the weights' sum less one
+      for (int k = 0; k < all[i].n; k++) {
+        const long double w = all[i].rule[k][2];
+        a[0] += w;
+        a[1] += w * all[i].rule[k][0];
+        a[2] += w * all[i].rule[k][1];
+      }
+      less[i] = (double)a[0];
+      sums[i] = {{(double)(1.0L + a[0]), (double)a[1], (double)a[2]}, (double)(2.0L * a[0] + a[0] * a[0])};
+    }
+    BEM_CUDA_TRY(ctx, cudaMemcpyToSymbol(c_sums, sums, sizeof sums));
+    {
+      std::vector<RuleNode<double>> qd(NN_ALL);
+      std::vector<RuleNode<df>> qf(NN_ALL);
+      auto put = [&](int at, const double *node, double w) {
+        const double x1 = node[0], x2 = node[1];
+        qd[at] = {x1, x2, w, w * x1, w * x2};
+        qf[at] = {host_df(x1), host_df(x2), host_df(w), host_df(w * x1), host_df(w * x2)};
+      };
+      for (int k = 0; k < 105; k++) put(NN105 + k, bemgpu_tri_rule105[k], bemgpu_tri_rule105[k][2]);
+      for (int k = 0; k < 91; k++) put(NN91 + k, bemgpu_tri_rule91[k], bemgpu_tri_rule91[k][2]);
+      for (int k = 0; k < 36; k++) {
+        put(NNE105 + k, bemgpu_tri_rule36[k], bemgpu_even_w105[k]);
+        put(NNE91 + k, bemgpu_tri_rule36[k], bemgpu_even_w91[k]);
+      }
+      BEM_CUDA_TRY(ctx, cudaMemcpyToSymbol(c_near_d, qd.data(), sizeof(RuleNode<double>) * NN_ALL));
+      BEM_CUDA_TRY(ctx, cudaMemcpyToSymbol(c_near_f, qf.data(), sizeof(RuleNode<df>) * NN_ALL));
+      const double ww1 = less[SUM105] + less[SUM91] + less[SUM105] * less[SUM91];
+      BEM_CUDA_TRY(ctx, cudaMemcpyToSymbol(c_near_ww1, &ww1, sizeof ww1));
+    }
     BEM_CUDA_TRY(ctx, cudaMemcpyToSymbol(c_far_d, nd.data(), sizeof(RuleNode<double>) * nd.size()));
     BEM_CUDA_TRY(ctx, cudaMemcpyToSymbol(c_far_f, nf.data(), sizeof(RuleNode<df>) * nf.size()));
   }
@@ -1857,13 +1771,56 @@ int bem_fill_group(bemgpu_ctx_s *ctx, FillJob *jobs, int njobs, const bemgpu_opt
     df_rec = (TriDF *)bem_workspace(ctx, "fill_tdf", sizeof(TriDF) * ndf);
     if (!df_rec) return bem_fail(ctx, BEMGPU_ERR_OOM, "fill: double-float records");
   }
-  // one upload: the tasks, then the records' jobs
-  const size_t tasks_bytes = sizeof(FillTask) * (size_t)njobs, tdf_bytes = sizeof(TriDFJob) * trees.size();
-  unsigned char *dtable = (unsigned char *)bem_workspace(ctx, "fill_tasks", tasks_bytes + tdf_bytes);
+  // the near pairs' tasks, by kind: a fill of a two-body tree takes the two
+  // bodies' own fills that follow it along (their near pairs are its own, with
+  // other Green's functions), unless one of them needs the direct kind
+  std::vector<NearTask> near[NEAR_KINDS];
+  int64_t near_units[NEAR_KINDS] = {};
+  {
+    std::vector<char> taken(njobs, 0);
+    const bool dfl = mode == FILL_DF;
+    for (int i = 0; i < njobs; i++) {
+      if (taken[i] || lists[i]->n == 0) continue;
+      const bemgpu_tree_s *t = jobs[i].t, *s = jobs[i].s;
+      const double emax = std::max(t->emax, s->emax);
+      int kind = near_kind(green_kabs(&jobs[i].g), emax);
+      const double scale = kind == NEAR_DIRECT ? 1.0 : near_scale(emax);
+      NearTask nt;
+      memset(&nt, 0, sizeof nt);
+      nt.T = t->d_rec;
+      nt.S = s->d_rec;
+      nt.near = lists[i]->d;
+      nt.nnear = lists[i]->n;
+      nt.scale = scale;
+      nt.ngreen = 1;
+      nt.g[0] = near_green(&jobs[i].g, scale, dfl, jobs[i].H, t->nrwg, 0, 0, t->ntri);
+      if (kind != NEAR_DIRECT && t == s && i + 2 < njobs && jobs[i + 1].t == jobs[i + 1].s &&
+          jobs[i + 2].t == jobs[i + 2].s && is_two_body(t, jobs[i + 1].t, jobs[i + 2].t)) {
+        for (int k = 1; k <= 2; k++) {
+          const bemgpu_tree_s *b = jobs[i + k].t;
+          const int kb = near_kind(green_kabs(&jobs[i + k].g), emax);
+          if (taken[i + k] || kb == NEAR_DIRECT) continue;
+          const int rwg0 = k == 1 ? 0 : jobs[i + 1].t->nrwg, tri0 = k == 1 ? 0 : jobs[i + 1].t->ntri;
+          nt.g[nt.ngreen++] = near_green(&jobs[i + k].g, scale, dfl, jobs[i + k].H, b->nrwg, rwg0, tri0, tri0 + b->ntri);
+          kind = std::max(kind, kb);  // SERIES2 carries more powers than SERIES1
+          taken[i + k] = 1;
+        }
+      }
+      nt.unit0 = near_units[kind];
+      near_units[kind] += nt.nnear;
+      near[kind].push_back(nt);
+    }
+  }
+  const size_t nnear = near[0].size() + near[1].size() + near[2].size();
+  // one upload: the far tasks, the near tasks, the records' jobs
+  const size_t tasks_bytes = (sizeof(FillTask) * (size_t)njobs + 15) / 16 * 16, near_bytes_ = sizeof(NearTask) * nnear,
+               tdf_bytes = sizeof(TriDFJob) * trees.size();
+  unsigned char *dtable = (unsigned char *)bem_workspace(ctx, "fill_tasks", tasks_bytes + near_bytes_ + tdf_bytes);
+  if (!dtable) return bem_fail(ctx, BEMGPU_ERR_OOM, "fill: task table");
   FillTask *dtasks = (FillTask *)dtable;
-  if (!dtasks) return bem_fail(ctx, BEMGPU_ERR_OOM, "fill: task table");
+  const NearTask *dnear = (const NearTask *)(dtable + tasks_bytes);
   double far_flops = 0, far_bytes = 0, near_flops = 0, near_bytes = 0;
-  int64_t far_tiles = 0, near_units = 0;
+  int64_t far_tiles = 0;
   for (int i = 0; i < njobs; i++) {
     const bemgpu_tree_s *t = jobs[i].t, *s = jobs[i].s;
     FillTask &tk = tasks[i];
@@ -1874,8 +1831,6 @@ int bem_fill_group(bemgpu_ctx_s *ctx, FillJob *jobs, int njobs, const bemgpu_opt
       tk.TD = df_rec + records_of(t);
       tk.SD = df_rec + records_of(s);
     }
-    tk.near = lists[i]->d;
-    tk.nnear = lists[i]->n;
     tk.H = jobs[i].H;
     tk.ntT = t->ntri;
     tk.ntS = s->ntri;
@@ -1884,11 +1839,9 @@ int bem_fill_group(bemgpu_ctx_s *ctx, FillJob *jobs, int njobs, const bemgpu_opt
     tk.far0 = far_tiles;
     tk.sym = t == s && mode != FILL_FP32_FAR;
     far_tiles += far_tiles_of(tk.sym, t->ntri, s->ntri, fr);
-    tk.near0 = near_units;
-    near_units += mode == FILL_DF ? (tk.nnear + 1) / 2 : tk.nnear;  // the df kernel works pair couples
     tk.g = to_dev(&jobs[i].g);
-    jobs[i].near = tk.nnear;
-    jobs[i].far = (int64_t)t->ntri * s->ntri - tk.nnear;
+    jobs[i].near = lists[i]->n;
+    jobs[i].far = (int64_t)t->ntri * s->ntri - lists[i]->n;
     if (ctx->prof) {
       const int64_t *fc = bem_far_rule_counts(ctx, t, s, opt);
       const int P[5] = {6, 10, 15, 21, 36};
@@ -1896,23 +1849,30 @@ int bem_fill_group(bemgpu_ctx_s *ctx, FillJob *jobs, int njobs, const bemgpu_opt
       for (int k = 0; k < 5; k++) { far_flops += fc[k] * bem_far_pair_flops(P[k]); nfar += fc[k]; }
       // half-pair products written: 9 per pair on average (nh_t * nh_s)
       far_bytes += (double)nfar * 9.0 * BEM_HALFPAIR_BYTES_FP64;
-      near_flops += (double)tk.nnear * bem_near_pair_flops(true);
-      near_bytes += (double)tk.nnear * 9.0 * BEM_HALFPAIR_BYTES_FP64;
+      near_flops += (double)lists[i]->n * bem_near_pair_flops(true);
+      near_bytes += (double)lists[i]->n * 9.0 * BEM_HALFPAIR_BYTES_FP64;
     }
   }
   // the tables are copied from this call's host vector before the call returns
-  std::vector<unsigned char> table(tasks_bytes + tdf_bytes);
-  memcpy(table.data(), tasks.data(), tasks_bytes);
+  std::vector<unsigned char> table(tasks_bytes + near_bytes_ + tdf_bytes);
+  memcpy(table.data(), tasks.data(), sizeof(FillTask) * (size_t)njobs);
+  {
+    size_t at = tasks_bytes;
+    for (int k = 0; k < NEAR_KINDS; k++) {
+      if (!near[k].empty()) memcpy(table.data() + at, near[k].data(), sizeof(NearTask) * near[k].size());
+      at += sizeof(NearTask) * near[k].size();
+    }
+  }
   int most = 0;
   for (size_t k = 0; k < trees.size(); k++) {
     const TriDFJob jb = {trees[k]->d_rec, df_rec ? df_rec + tree_off[k] : nullptr, trees[k]->ntri};
-    memcpy(table.data() + tasks_bytes + k * sizeof(TriDFJob), &jb, sizeof jb);
+    memcpy(table.data() + tasks_bytes + near_bytes_ + k * sizeof(TriDFJob), &jb, sizeof jb);
     most = std::max(most, jb.n);
   }
   BEM_CUDA_TRY(ctx, cudaMemcpyAsync(dtable, table.data(), table.size(), cudaMemcpyHostToDevice, stream));
   if (df_rec) {
     tri_df_kernel<<<dim3((most + 127) / 128, (unsigned)trees.size()), 128, 0, stream>>>(
-        (const TriDFJob *)(dtable + tasks_bytes));
+        (const TriDFJob *)(dtable + tasks_bytes + near_bytes_));
     ctx->launches++;
   }
   if (far_tiles > 0) {
@@ -1922,20 +1882,18 @@ int bem_fill_group(bemgpu_ctx_s *ctx, FillJob *jobs, int njobs, const bemgpu_opt
     ctx->launches++;
   }
   BEM_CUDA_TRY(ctx, cudaGetLastError());
-  if (near_units > 0) {
-    const int nb = (int)std::min<int64_t>((near_units + NEAR_WARPS - 1) / NEAR_WARPS,
-                                          (int64_t)ctx->num_sms * ctx->tune.near_grid);
+  if (nnear > 0) {
     ProfScope ps(ctx, BEMGPU_K_FILL_NEAR, stream, near_flops, near_bytes);
-    const bool sync = ctx->tune.near_sync != 0;
-    if (mode == FILL_DF && ctx->tune.near_minb == 3)
-      launch_near_df<3>(sync, nb, stream, dtasks, njobs, near_units);
-    else if (mode == FILL_DF && ctx->tune.near_minb == 4)
-      launch_near_df<4>(sync, nb, stream, dtasks, njobs, near_units);
-    else if (mode == FILL_DF)
-      launch_near_df<2>(sync, nb, stream, dtasks, njobs, near_units);
-    else
-      near_pairs_group_kernel<<<nb, 32 * NEAR_WARPS, 0, stream>>>(dtasks, njobs, near_units);
-    ctx->launches++;
+    size_t at = 0;
+    for (int k = 0; k < NEAR_KINDS; k++) {
+      if (near[k].empty()) continue;
+      const int nb = (int)std::min<int64_t>((near_units[k] + NEAR_WARPS - 1) / NEAR_WARPS,
+                                            (int64_t)ctx->num_sms * ctx->tune.near_grid);
+      launch_near(mode == FILL_DF, ctx->tune.near_minb, k, nb, stream, dnear + at, (int)near[k].size(), near_units[k],
+                  ctx->tune.near_sync);
+      ctx->launches++;
+      at += near[k].size();
+    }
   }
   BEM_CUDA_TRY(ctx, cudaGetLastError());
   return BEMGPU_OK;
@@ -2049,7 +2007,12 @@ namespace {
 constexpr size_t NOALLOC_SCRATCH_BYTES = 32u << 20;   // 32 MiB
 constexpr size_t NOALLOC_NEAR_BYTES = 2u << 20;       // first 2 MiB: the near-pair list
 static __device__ __align__(256) unsigned char g_noalloc_scratch[NOALLOC_SCRATCH_BYTES];
-static __device__ __align__(256) unsigned char g_noalloc_task[sizeof(FillTask)];
+// its task table: the far pairs' and the near pairs'
+struct NoallocTasks {
+  FillTask far;
+  NearTask near;
+};
+static __device__ __align__(256) unsigned char g_noalloc_task[sizeof(NoallocTasks)];
 
 std::mutex g_noalloc_mu;
 std::mutex g_noalloc_run_mu;  // one call at a time uses the shared scratch
@@ -2087,7 +2050,7 @@ extern "C" int bemgpu_zts_noalloc(bemgpu_ctx_t ctx, bemgpu_tree_t t, bemgpu_tree
   // Set-up, once per device with that device current: the host-side name of
   // the array is not a device address; ask the runtime for the address.
   unsigned char *base = nullptr;
-  FillTask *dtask = nullptr;
+  NoallocTasks *dtask = nullptr;
   {
     std::lock_guard<std::mutex> lk2(g_noalloc_mu);
     if (!g_noalloc_addr[ctx->device]) {
@@ -2103,7 +2066,7 @@ extern "C" int bemgpu_zts_noalloc(bemgpu_ctx_t ctx, bemgpu_tree_t t, bemgpu_tree
       g_noalloc_task_addr[ctx->device] = q;
     }
     base = (unsigned char *)g_noalloc_addr[ctx->device];
-    dtask = (FillTask *)g_noalloc_task_addr[ctx->device];
+    dtask = (NoallocTasks *)g_noalloc_task_addr[ctx->device];
   }
   int rc = load_tables(ctx);
   if (rc) return rc;
@@ -2114,27 +2077,36 @@ extern "C" int bemgpu_zts_noalloc(bemgpu_ctx_t ctx, bemgpu_tree_t t, bemgpu_tree
     BEM_CUDA_TRY(ctx, cudaMemcpyAsync(dnear, pairs.data(), pairs.size() * sizeof(NearPair), cudaMemcpyHostToDevice, st));
   // Every half-pair slot of H has exactly one writer (the pair kernels below),
   // so nothing left by an earlier call needs clearing.
-  const GreenDev gd = to_dev(g);
   const FarOpts fo = {o.farThresh6, o.farThresh10, o.farThresh15, o.farThresh21};
-  FillTask task = {};
+  NoallocTasks tasks;
+  memset(&tasks, 0, sizeof tasks);
+  FillTask &task = tasks.far;
   task.T = t->d_rec;
   task.S = s->d_rec;
-  task.near = dnear;
   task.H = H;
-  task.nnear = (int64_t)pairs.size();
   task.ntT = t->ntri;
   task.ntS = s->ntri;
   task.ntr = t->nrwg;
   task.far_tx = (s->ntri + 31) / 32;
   task.sym = t == s;
-  task.g = gd;
-  BEM_CUDA_TRY(ctx, cudaMemcpyAsync(dtask, &task, sizeof task, cudaMemcpyHostToDevice, st));
-  launch_far(FILL_FP64, (unsigned)far_tiles_of(task.sym, t->ntri, s->ntri, 4), 4, st, dtask, 1, fo);
+  task.g = to_dev(g);
+  const double emax = std::max(t->emax, s->emax);
+  const int kind = near_kind(green_kabs(g), emax);
+  const int64_t np = (int64_t)pairs.size();
+  NearTask &nt = tasks.near;
+  nt.T = t->d_rec;
+  nt.S = s->d_rec;
+  nt.near = dnear;
+  nt.nnear = np;
+  nt.scale = kind == NEAR_DIRECT ? 1.0 : near_scale(emax);
+  nt.ngreen = 1;
+  nt.g[0] = near_green(g, nt.scale, false, H, t->nrwg, 0, 0, t->ntri);
+  BEM_CUDA_TRY(ctx, cudaMemcpyAsync(dtask, &tasks, sizeof tasks, cudaMemcpyHostToDevice, st));
+  launch_far(FILL_FP64, (unsigned)far_tiles_of(task.sym, t->ntri, s->ntri, 4), 4, st, &dtask->far, 1, fo);
   ctx->launches++;
-  if (!pairs.empty()) {
-    const int64_t np = (int64_t)pairs.size();
+  if (np > 0) {
     const int nb = (int)std::min<int64_t>((np + NEAR_WARPS - 1) / NEAR_WARPS, (int64_t)ctx->num_sms * 16);
-    near_pairs_kernel<<<nb, 32 * NEAR_WARPS, 0, st>>>(t->d_rec, s->d_rec, dnear, np, gd, H, t->nrwg);
+    launch_near(false, 2, kind, nb, st, &dtask->near, 1, np, 0);
     ctx->launches++;
   }
   dim3 gblk(128);

@@ -12,13 +12,16 @@ __device__ __forceinline__ df operator-(df a) { return df_neg(a); }
 __device__ __forceinline__ df operator*(df a, df b) { return df_mul(a, b); }
 
 // Num<T>: what the two types do differently.  Tail is the type that carries
-// terms below 2^-24 of a sum.
+// terms below 2^-24 of a sum.  LESS: sincos_ and exp_ also give sin x - x and
+// e^x - 1, accurate relative to themselves where x needs no reduction (double:
+// the functions' values again).
 template <typename T>
 struct Num;
 
 template <>
 struct Num<double> {
   typedef double Tail;
+  static constexpr bool LESS = false;
   __device__ __forceinline__ static double of(double x) { return x; }
   __device__ __forceinline__ static double to_double(double x) { return x; }
   __device__ __forceinline__ static double head(double x) { return x; }
@@ -35,8 +38,11 @@ struct Num<double> {
     Ri = rsqrt(a);
     R = a * Ri;
   }
-  __device__ __forceinline__ static void sincos_(double x, double &s, double &c) { sincos(x, &s, &c); }
-  __device__ __forceinline__ static double exp_(double x) { return exp(x); }
+  __device__ __forceinline__ static void sincos_(double x, double &s, double &c, double &sm) {
+    sincos(x, &s, &c);
+    sm = s;
+  }
+  __device__ __forceinline__ static double exp_(double x, double &m1) { return m1 = exp(x); }
   __device__ __forceinline__ static double log_(double x) { return log(x); }
   __device__ __forceinline__ static double atan2_(double y, double x) { return atan2(y, x); }
   __device__ __forceinline__ static double abs_(double x) { return fabs(x); }
@@ -47,6 +53,7 @@ struct Num<double> {
 template <>
 struct Num<df> {
   typedef float Tail;
+  static constexpr bool LESS = true;
   __device__ __forceinline__ static df of(double x) { return df_make(x); }
   __device__ __forceinline__ static double to_double(df x) { return df_to_double(x); }
   __device__ __forceinline__ static float head(df x) { return x.hi; }
@@ -60,13 +67,16 @@ struct Num<df> {
   __device__ __forceinline__ static df sqrt_(df a) { return df_sqrt(a); }
   __device__ __forceinline__ static df rcp(df a) { return df_rcp(a); }
   __device__ __forceinline__ static void sqrt_rcp(df a, df &R, df &Ri) { df_sqrt_rcp(a, R, Ri); }
-  __device__ __forceinline__ static void sincos_(df x, df &s, df &c) {
-    if (fabsf(x.hi) < 200.f)
-      df_sincos_df(x, s, c);
-    else
+  // sm = sin x - x
+  __device__ __forceinline__ static void sincos_(df x, df &s, df &c, df &sm) {
+    if (fabsf(x.hi) < 200.f) {
+      df_sincos_df(x, s, c, sm);
+    } else {
       df_sincos(df_to_double(x), s, c);  // FP64 reduction for phases of 200 rad and more
+      sm = df_sub(s, x);
+    }
   }
-  __device__ __forceinline__ static df exp_(df x) { return df_exp_df(x); }
+  __device__ __forceinline__ static df exp_(df x, df &m1) { return df_exp_df(x, m1); }  // m1 = e^x - 1
   __device__ __forceinline__ static df log_(df x) { return df_log(x); }
   __device__ __forceinline__ static df atan2_(df y, df x) { return df_atan2(y, x); }
   __device__ __forceinline__ static df abs_(df x) { return df_abs(x); }

@@ -29,7 +29,7 @@ KNOBS = {
     "far_rows": (_lib.TUNE_FAR_ROWS, (1, 2, 4, 8), ("fill_far",)),
     "raster": (_lib.TUNE_RASTER, (4, 8, 16), ("lu_gemm", "trsm", "solve_gemm", "trace", "refine_gemm")),
 }
-DEFAULTS = {"near_minb": 2, "far_rows": 4, "raster": 8}
+DEFAULTS = {"near_minb": 3, "far_rows": 4, "raster": 8}
 
 _lock = threading.Lock()
 

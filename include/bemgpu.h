@@ -130,7 +130,7 @@ int bemgpu_ctx_set_fp64_fallback_tol(bemgpu_ctx_t ctx, double tol);
  * project's autotuner (bem_gb300/tuning.py: it times each candidate on the
  * caller's workload and caches the best per GPU and size class).
  *   BEMGPU_TUNE_NEAR_MINB  CTAs per SM that the double-float near-pair kernel's
- *                          register budget allows: 2 (default), 3 (168
+ *                          register budget allows: 2, 3 (default, 168
  *                          registers) or 4 (128, some spilled);
  *   BEMGPU_TUNE_FAR_ROWS   warps per CTA of the far-pair kernel: 1, 2, 4 (default), 8;
  *   BEMGPU_TUNE_RASTER     M-tiles per rasterization band of the tensor-core
