@@ -15,6 +15,8 @@
 #include "bemgpu_internal.h"
 
 #include <algorithm>
+#include <mutex>
+#include <type_traits>
 
 namespace {
 
@@ -603,6 +605,459 @@ __global__ void __launch_bounds__(COOP_THREADS)
   }
 }
 
+// ---------------- panel factorization by one thread-block cluster ----------------
+//
+// A sub-panel of SW columns, rows [k0, n), by a cluster of up to 16 CTAs: each
+// thread holds RPT rows in registers, so a column costs no pass over shared
+// memory, and the pivot exchange is one hop through distributed shared memory
+// instead of a barrier over the whole grid.  Per column j:
+//   1. every CTA finds its candidate (largest |re| + |im|, the first position
+//      among equals, as izamax): a reduction per warp, one CTA barrier;
+//   2. the candidate's warp writes the row into the CTA's rows in shared memory
+//      and sends it (header: key, position, 1/pivot) to every CTA of the
+//      cluster with asynchronous stores that count into the receiver's mbarrier;
+//   3. every warp waits for the G messages, picks the same winner, and updates
+//      its rows.
+// Rows never move: a row knows its position (LAPACK's interchanges applied to
+// the position only), and goes to its place when the sub-panel is written back.
+// The registers rotate: column j is always a[0], the update writes column c to
+// a[c - 1], so that the loop over j needs no register indexing; it runs in four
+// phases of SW/4 columns whose width shrinks with the columns left.
+// Messages are double-buffered by column parity: a CTA sends for column j + 1
+// only after every CTA's message for column j, which each sends after all its
+// warps are done with column j - 1.
+// Afterwards the cluster applies the interchanges to the rest of the panel
+// [p0, p1) and solves the columns right of the sub-panel with its unit-lower
+// triangle; what is left of the panel's update is one product
+// (panel_update_kernel).
+//
+// Bound by latency: a complex64 column is ~2060 cycles at up to 128 rows a CTA
+// (candidate 300, row out 150, reciprocal 190, sends 370, their flight 210,
+// choice 330, update 420) and ~2600 at 480, against ~8700 for a column of the
+// kernel above, whose exchange is a barrier over 152 CTAs.  The panels of a
+// factorization with what belongs to them (interchanges, updates inside the
+// panel): N = 7680 32.7 -> 18.1 ms, N = 1152 4.3 -> 2.3 ms; complex128 N = 1152
+// 10.8 -> 6.2 ms.
+constexpr int CP_MAX_THREADS = 512;
+constexpr int CP_MAX_CLUSTER = 16;
+constexpr unsigned CP_SPIN_LIMIT = 1u << 20;
+
+template <typename T>
+struct CpHeader;
+template <>
+struct CpHeader<float> {
+  unsigned key, pos;
+  float rr, ri;  // reciprocal of the pivot
+};
+template <>
+struct __align__(16) CpHeader<double> {
+  unsigned lo, pos;
+  unsigned key, pad;
+  double rr, ri;
+};
+
+__device__ __forceinline__ uint32_t cp_smem(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
+__device__ __forceinline__ uint32_t cp_map(uint32_t addr, int cta) {
+  uint32_t r;
+  asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(cta));
+  return r;
+}
+// 16 bytes to a CTA of the cluster, counted into its mbarrier.
+__device__ __forceinline__ void cp_send16(uint32_t dst, uint32_t bar, uint4 v) {
+  asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v4.b32 [%0], {%1, %2, %3, %4}, [%5];" ::"r"(dst),
+               "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w), "r"(bar)
+               : "memory");
+}
+__device__ __forceinline__ bool cp_try_wait(uint32_t bar, unsigned parity) {
+  unsigned ok;
+  asm volatile(
+      "{\n .reg .pred p;\n mbarrier.try_wait.parity.acquire.cta.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}\n"
+      : "=r"(ok)
+      : "r"(bar), "r"(parity)
+      : "memory");
+  return ok != 0;
+}
+__device__ __forceinline__ void cp_cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+// Pivot keys: magnitude bits (complex128: high word, then low word); 0 for
+// zero and NaN, which are no pivots.
+__device__ __forceinline__ void cp_key(float re, float im, unsigned &hi, unsigned &lo) {
+  const float v = fabsf(re) + fabsf(im);
+  hi = v > 0.f ? __float_as_uint(v) : 0u;
+  lo = 0u;
+}
+__device__ __forceinline__ void cp_key(double re, double im, unsigned &hi, unsigned &lo) {
+  const double v = fabs(re) + fabs(im);
+  const unsigned long long b = v > 0.0 ? (unsigned long long)__double_as_longlong(v) : 0ull;
+  hi = (unsigned)(b >> 32);
+  lo = (unsigned)b;
+}
+// The warp's largest (hi, lo), the smallest position among equals.
+template <typename T>
+__device__ __forceinline__ void cp_reduce(unsigned &hi, unsigned &lo, unsigned &pos) {
+  const unsigned m = __reduce_max_sync(0xffffffffu, hi);
+  bool in = hi == m;
+  hi = m;
+  if (sizeof(T) == 8) {
+    const unsigned ml = __reduce_max_sync(0xffffffffu, in ? lo : 0u);
+    in = in && lo == ml;
+    lo = ml;
+  }
+  pos = __reduce_min_sync(0xffffffffu, in ? pos : 0xffffffffu);
+}
+
+// 1/a by one division; the plain form where |a|^2 leaves the range in which its
+// reciprocal is a normal number.
+template <typename T>
+__device__ __forceinline__ cx<T> cp_recip(cx<T> a) {
+  const T d = a.r * a.r + a.i * a.i;
+  const T small = sizeof(T) == 8 ? T(1e-290) : T(1e-30);
+  if (!(d > small && d < T(1) / small)) return crecip(a);
+  const T q = T(1) / d;
+  return {a.r * q, -a.i * q};
+}
+
+template <typename T, int SW, int RPT>
+struct CpSmem {
+  static constexpr int ROW = SW + 16 / (int)(2 * sizeof(T));  // complex entries of a padded row: 16-byte aligned
+  static constexpr int MSG = SW * 2 * (int)sizeof(T) + (int)sizeof(CpHeader<T>);
+  static constexpr size_t bytes(int chunk) {
+    return (size_t)(2 * CP_MAX_CLUSTER + 1) * MSG + (size_t)SW * ROW * 2 * sizeof(T) + (size_t)chunk * ROW * 2 * sizeof(T);
+  }
+};
+
+template <typename T, int SW, int RPT>
+__global__ void __launch_bounds__(CP_MAX_THREADS, 1)
+    panel_cluster_kernel(T *A, int64_t lda, int n, int k0, int w, int p0, int p1, int chunk, int *ipiv, int *info,
+                         int *err, int64_t strideA) {
+  typedef typename V2<T>::type T2;
+  typedef CpSmem<T, SW, RPT> S;
+  constexpr int ROW = S::ROW, MSG = S::MSG, HP = (int)sizeof(CpHeader<T>) / 16;
+  extern __shared__ __align__(16) unsigned char cp_smem_raw[];
+  unsigned char *msg = cp_smem_raw;                                        // [2][CP_MAX_CLUSTER][MSG]
+  T2 *out = reinterpret_cast<T2 *>(msg + 2 * CP_MAX_CLUSTER * MSG);        // the candidate's row, as sent
+  T2 *LU = reinterpret_cast<T2 *>(msg + (2 * CP_MAX_CLUSTER + 1) * MSG);   // [SW][ROW] the factored diagonal block
+  T2 *P = LU + SW * ROW;                                                   // [chunk][ROW] the CTA's rows, final values
+  __shared__ __align__(8) unsigned long long bars[2];
+  __shared__ unsigned s_hi[CP_MAX_THREADS / 32], s_lo[CP_MAX_THREADS / 32], s_pos[CP_MAX_THREADS / 32];
+  __shared__ int s_piv[SW];
+  __shared__ volatile int s_abort;
+  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5, nt = blockDim.x, nwarps = nt >> 5;
+  const int G = gridDim.x, g = blockIdx.x;
+  {
+    const int64_t bb = blockIdx.y;  // a batch of equal-size matrices: one cluster each
+    A += bb * strideA;
+    ipiv += bb * n;
+    info += bb;
+  }
+  T2 *A2 = reinterpret_cast<T2 *>(A);
+  const T2 zero2 = V2<T>::make(0, 0);
+  if (tid == 0) {
+    s_abort = 0;
+    for (int k = 0; k < 2; k++)
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(cp_smem(&bars[k])) : "memory");
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  // rows into registers
+  T2 a[RPT][SW];
+  unsigned pos[RPT];
+  bool act[RPT];
+#pragma unroll
+  for (int r = 0; r < RPT; r++) {
+    const int i = tid + r * nt, row = k0 + g * chunk + i;
+    act[r] = i < chunk && row < n;
+    pos[r] = (unsigned)row;
+#pragma unroll
+    for (int c = 0; c < SW; c++) a[r][c] = act[r] && c < w ? A2[row + lda * (int64_t)(k0 + c)] : zero2;
+  }
+  cp_cluster_sync();
+
+  int j = 0;
+  auto step = [&](auto width) {
+    constexpr int W = decltype(width)::value;  // registers in use: columns j .. j + W - 1
+    const int par = j & 1;
+    const unsigned dr = (unsigned)(k0 + j);
+    const uint32_t bar = cp_smem(&bars[par]);
+    if (tid == 0)
+      asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(G * (W * 2 * (int)sizeof(T) + (int)sizeof(CpHeader<T>))) : "memory");
+    // 1. the CTA's candidate
+    unsigned hi = 0, lo = 0, cp = 0xffffffffu;
+#pragma unroll
+    for (int r = 0; r < RPT; r++) {
+      unsigned h, l;
+      cp_key(a[r][0].x, a[r][0].y, h, l);
+      if (!act[r]) h = l = 0;
+      const unsigned q = act[r] ? pos[r] : 0xffffffffu;
+      const bool better = r == 0 || h > hi || (h == hi && (l > lo || (l == lo && q < cp)));
+      hi = better ? h : hi;
+      lo = better ? l : lo;
+      cp = better ? q : cp;
+    }
+    cp_reduce<T>(hi, lo, cp);
+    if (lane == 0) {
+      s_hi[wid] = hi;
+      s_lo[wid] = lo;
+      s_pos[wid] = cp;
+    }
+    __syncthreads();
+    hi = lane < nwarps ? s_hi[lane] : 0u;
+    lo = lane < nwarps ? s_lo[lane] : 0u;
+    cp = lane < nwarps ? s_pos[lane] : 0xffffffffu;
+    cp_reduce<T>(hi, lo, cp);
+    // 2. its warp sends the row (warp 0 an empty message when there is none)
+    int own = -1;
+#pragma unroll
+    for (int r = 0; r < RPT; r++)
+      if (act[r] && pos[r] == cp) own = tid + r * nt;
+    const unsigned who = __ballot_sync(0xffffffffu, own >= 0);
+    if (who || (cp == 0xffffffffu && wid == 0)) {
+      const int from = who ? __ffs(who) - 1 : 0;
+      T2 pv = a[0][0];
+#pragma unroll
+      for (int r = 0; r < RPT; r++)
+        if (own == tid + r * nt) {
+          pv = a[r][0];
+#pragma unroll
+          for (int c = 0; c < W; c++) out[c] = a[r][c];
+        }
+      pv.x = __shfl_sync(0xffffffffu, pv.x, from);
+      pv.y = __shfl_sync(0xffffffffu, pv.y, from);
+      CpHeader<T> h;
+      if (sizeof(T) == 8) reinterpret_cast<unsigned *>(&h)[0] = lo;
+      h.key = who ? hi : 0u;
+      h.pos = cp;
+      const cx<T> rp = who && (hi | lo) ? cp_recip(cx<T>{pv.x, pv.y}) : cx<T>{0, 0};
+      h.rr = rp.r;
+      h.ri = rp.i;
+      __syncwarp();
+      const uint32_t to = cp_smem(msg + (par * CP_MAX_CLUSTER + g) * MSG);
+      constexpr int PIECES = W * 2 * (int)sizeof(T) / 16, PER = 32 / PIECES;  // 16-byte pieces, CTAs per round
+      if (lane < PER * PIECES) {
+        const int q = lane % PIECES;
+        const uint4 v = reinterpret_cast<const uint4 *>(out)[q];
+        const uint32_t at = to + (int)sizeof(CpHeader<T>) + 16 * q;
+        for (int cta = lane / PIECES; cta < G; cta += PER) cp_send16(cp_map(at, cta), cp_map(bar, cta), v);
+      }
+      for (int cta = lane / HP; cta < G; cta += 32 / HP) {
+        const int q = lane % HP;
+        const uint4 v = reinterpret_cast<const uint4 *>(&h)[HP == 1 || q == 0 ? 0 : HP - 1];
+        cp_send16(cp_map(to + 16 * q, cta), cp_map(bar, cta), v);
+      }
+    }
+    // 3. the G messages
+    {
+      const unsigned ph = (unsigned)(j >> 1) & 1u;
+      unsigned it = 0;
+      while (!s_abort && !cp_try_wait(bar, ph))
+        if (++it > CP_SPIN_LIMIT) {
+          atomicExch(err, 1);
+          s_abort = 1;
+        }
+    }
+    const unsigned char *in = msg + par * CP_MAX_CLUSTER * MSG;
+    unsigned wh = 0, wl = 0;
+    if (lane < G) {
+      const CpHeader<T> *hd = reinterpret_cast<const CpHeader<T> *>(in + lane * MSG);
+      wh = hd->key;
+      if (sizeof(T) == 8) wl = reinterpret_cast<const unsigned *>(hd)[0];
+    }
+    const unsigned top = __reduce_max_sync(0xffffffffu, wh);
+    bool best = lane < G && wh == top;
+    unsigned topl = 0;
+    if (sizeof(T) == 8) {
+      topl = __reduce_max_sync(0xffffffffu, best ? wl : 0u);
+      best = best && wl == topl;
+    }
+    unsigned win = __ballot_sync(0xffffffffu, best);
+    if (__popc(win) > 1) {  // equal magnitudes: the first position
+      const unsigned q = best ? reinterpret_cast<const CpHeader<T> *>(in + lane * MSG)->pos : 0xffffffffu;
+      const unsigned first = __reduce_min_sync(0xffffffffu, q);
+      win = __ballot_sync(0xffffffffu, best && q == first);
+    }
+    const bool none = top == 0u && topl == 0u;  // no pivot in this column: the row at its place stays
+    const int wc = win ? __ffs(win) - 1 : 0;
+    const CpHeader<T> *hd = reinterpret_cast<const CpHeader<T> *>(in + wc * MSG);
+    const T2 *u = reinterpret_cast<const T2 *>(in + wc * MSG + sizeof(CpHeader<T>));  // columns j, j + 1, ...
+    const unsigned pv = none ? dr : hd->pos;
+    if (tid == 0) {
+      s_piv[j] = s_abort ? (int)dr : (int)pv;
+      if (g == 0) {
+        ipiv[dr] = s_abort ? (int)dr : (int)pv;
+        if (none && *info == 0) *info = (int)dr + 1;
+      }
+    }
+    const cx<T> rp = {hd->rr, hd->ri};
+#pragma unroll
+    for (int r = 0; r < RPT; r++) {
+      const int i = tid + r * nt;
+      if (act[r]) {
+        if (pos[r] == pv) {  // the pivot row: its U part is final
+          act[r] = false;
+          pos[r] = dr;
+#pragma unroll
+          for (int c = 0; c < W; c++)
+            if (j + c < SW) P[i * ROW + j + c] = a[r][c];
+        } else {
+          if (pos[r] == dr) pos[r] = pv;
+          // without a pivot the column stays and nothing is updated
+          const cx<T> m = cmul(cx<T>{a[r][0].x, a[r][0].y}, rp);
+          const cx<T> l = none ? cx<T>{a[r][0].x, a[r][0].y} : m;
+          P[i * ROW + j] = V2<T>::make(l.r, l.i);
+          const T fr = none ? T(0) : m.r, fi = none ? T(0) : m.i;
+#pragma unroll
+          for (int c = 1; c < W; c++) {
+            const T2 uc = u[c];
+            a[r][c - 1].x = fma(fi, uc.y, fma(-fr, uc.x, a[r][c].x));
+            a[r][c - 1].y = fma(-fi, uc.x, fma(-fr, uc.y, a[r][c].y));
+          }
+        }
+      }
+    }
+    j++;
+  };
+  constexpr int Q = SW / 4;
+#pragma unroll 1
+  while (j < min(w, Q)) step(std::integral_constant<int, SW>{});
+#pragma unroll 1
+  while (j < min(w, 2 * Q)) step(std::integral_constant<int, SW - Q>{});
+#pragma unroll 1
+  while (j < min(w, 3 * Q)) step(std::integral_constant<int, SW - 2 * Q>{});
+#pragma unroll 1
+  while (j < w) step(std::integral_constant<int, SW - 3 * Q>{});
+  __syncthreads();
+  // the rows to their places
+#pragma unroll
+  for (int r = 0; r < RPT; r++) {
+    const int i = tid + r * nt;
+    if (i < chunk && k0 + g * chunk + i < n && !s_abort)
+      for (int c = 0; c < w; c++) A2[pos[r] + lda * (int64_t)(k0 + c)] = P[i * ROW + c];
+  }
+  cp_cluster_sync();  // release and acquire: the rows are in L2 for the whole cluster
+  // the rest of the panel: interchanges, and U12 = L11^-1 A12 on the right.
+  // Entry d of a column comes from where d leads back through the interchanges.
+  const int nc = (k0 - p0) + (p1 - k0 - w);
+  if (nc > 0) {
+    for (int k = tid; k < w * w; k += nt) {
+      const int r = k % w, c = k / w;
+      LU[r * ROW + c] = __ldcg(A2 + k0 + r + lda * (int64_t)(k0 + c));
+    }
+    __syncthreads();
+    const int d1 = k0 + lane, d2 = lane < w ? s_piv[lane] : 0;
+    const bool on1 = lane < w, on2 = lane < w && d2 >= k0 + w;
+    int s1 = d1, s2 = d2;
+    for (int q = w - 1; q >= 0; q--) {
+      const int p = s_piv[q], t = k0 + q;
+      s1 = s1 == t ? p : s1 == p ? t : s1;
+      s2 = s2 == t ? p : s2 == p ? t : s2;
+    }
+    constexpr int NC = 4;  // columns in flight per warp
+    for (int q0 = (g * nwarps + wid) * NC; q0 < nc; q0 += G * nwarps * NC) {
+      T2 x1[NC], x2[NC];
+      T2 *b[NC];
+#pragma unroll
+      for (int e = 0; e < NC; e++) {
+        const int q = min(q0 + e, nc - 1);  // the last column again where there are fewer
+        b[e] = A2 + lda * (int64_t)(q < k0 - p0 ? p0 + q : k0 + w + (q - (k0 - p0)));
+        x1[e] = on1 ? b[e][s1] : zero2;
+        x2[e] = on2 ? b[e][s2] : zero2;
+      }
+      __syncwarp();
+      if (q0 + NC > k0 - p0)
+        for (int i = 0; i + 1 < w; i++) {
+          const T2 l = lane > i && on1 ? LU[lane * ROW + i] : zero2;
+#pragma unroll
+          for (int e = 0; e < NC; e++) {
+            const T xr = __shfl_sync(0xffffffffu, x1[e].x, i), xi = __shfl_sync(0xffffffffu, x1[e].y, i);
+            if (q0 + e >= k0 - p0) {
+              x1[e].x -= l.x * xr - l.y * xi;
+              x1[e].y -= l.x * xi + l.y * xr;
+            }
+          }
+        }
+#pragma unroll
+      for (int e = 0; e < NC; e++)
+        if (q0 + e < nc) {
+          if (on1) b[e][d1] = x1[e];
+          if (on2) b[e][d2] = x2[e];
+        }
+    }
+  }
+  cp_cluster_sync();  // no CTA leaves while another's message to it may be under way
+}
+
+// C (m x n) -= A (m x K) B (K x n), K = 8..32: what a sub-panel leaves to the rest
+// of its panel.  One CTA per TM x TN tile with the whole K in shared memory: a
+// single load round and barrier, and small tiles so that the few columns still
+// spread over the GPU (a 128 x 64 tile took 30 us where this takes ~5).
+template <typename T, int K>
+struct PuCfg;
+template <>
+struct PuCfg<float, 32> { static constexpr int TM = 64, TN = 32, PR = 4, PC = 2; };
+template <>
+struct PuCfg<float, 16> { static constexpr int TM = 64, TN = 32, PR = 4, PC = 2; };
+template <>
+struct PuCfg<double, 8> { static constexpr int TM = 32, TN = 8, PR = 1, PC = 1; };
+template <>
+struct PuCfg<double, 4> { static constexpr int TM = 32, TN = 8, PR = 1, PC = 1; };
+template <typename T, int K>
+__global__ void __launch_bounds__(256) panel_update_kernel(int m, int n, int k, const T *__restrict__ A, const T *__restrict__ B,
+                                                           T *__restrict__ C, int64_t ld, int64_t strideA) {
+  typedef typename V2<T>::type T2;
+  typedef PuCfg<T, K> Cfg;
+  constexpr int TM = Cfg::TM, TN = Cfg::TN, PR = Cfg::PR, PC = Cfg::PC, TX = TM / PR;
+  static_assert(TX * (TN / PC) == 256, "256 threads");
+  __shared__ T2 As[K][TM], Bs[K][TN];
+  const int64_t off = strideA * blockIdx.z;
+  const T2 *A2 = reinterpret_cast<const T2 *>(A + off), *B2 = reinterpret_cast<const T2 *>(B + off);
+  T2 *C2 = reinterpret_cast<T2 *>(C + off);
+  const int m0 = blockIdx.x * TM, n0 = blockIdx.y * TN, tid = threadIdx.x;
+  const T2 zero = V2<T>::make(0, 0);
+#pragma unroll
+  for (int q = tid; q < TM * K; q += 256) {
+    const int r = q % TM, c = q / TM;
+    As[c][r] = m0 + r < m && c < k ? A2[m0 + r + ld * (int64_t)c] : zero;
+  }
+#pragma unroll
+  for (int q = tid; q < TN * K; q += 256) {
+    const int r = q % K, c = q / K;
+    Bs[r][c] = n0 + c < n && r < k ? B2[r + ld * (int64_t)(n0 + c)] : zero;
+  }
+  const int tx = tid % TX, ty = tid / TX;
+  T2 acc[PR][PC];
+#pragma unroll
+  for (int r = 0; r < PR; r++)
+#pragma unroll
+    for (int c = 0; c < PC; c++) {
+      const int row = m0 + tx + TX * r, col = n0 + ty * PC + c;
+      acc[r][c] = row < m && col < n ? C2[row + ld * (int64_t)col] : zero;
+    }
+  __syncthreads();
+#pragma unroll
+  for (int kk = 0; kk < K; kk++) {
+    T2 a[PR], b[PC];
+#pragma unroll
+    for (int r = 0; r < PR; r++) a[r] = As[kk][tx + TX * r];
+#pragma unroll
+    for (int c = 0; c < PC; c++) b[c] = Bs[kk][ty * PC + c];
+#pragma unroll
+    for (int r = 0; r < PR; r++)
+#pragma unroll
+      for (int c = 0; c < PC; c++) {
+        acc[r][c].x = fma(-a[r].x, b[c].x, fma(a[r].y, b[c].y, acc[r][c].x));
+        acc[r][c].y = fma(-a[r].x, b[c].y, fma(-a[r].y, b[c].x, acc[r][c].y));
+      }
+  }
+#pragma unroll
+  for (int r = 0; r < PR; r++)
+#pragma unroll
+    for (int c = 0; c < PC; c++) {
+      const int row = m0 + tx + TX * r, col = n0 + ty * PC + c;
+      if (row < m && col < n) C2[row + ld * (int64_t)col] = acc[r][c];
+    }
+}
+
 // B[0:w, :] <- L11^{-1} B (unit lower) or U11^{-1} B (upper) with the w x w
 // diagonal block (w <= 32 R) in shared memory; one warp per right-hand-side
 // column, lane holds rows lane + 32 r, r < R.
@@ -985,6 +1440,118 @@ bool panel_coop(bemgpu_ctx_s *ctx, T *A, int64_t lda, int n, int k0, int w, int 
   return true;
 }
 
+// The panel [k0, k0 + w) in sub-panels, each by one cluster (panel_cluster_kernel)
+// and one product for what is left of the panel.  False (nothing launched) when
+// the rows do not fit a cluster's registers or the device cannot place one.
+//
+// Sub-panel width: 32 columns of one row per thread are 64 registers; from 8192
+// rows on half as many columns of two rows.  Complex128: 8 columns, since a
+// warp's FP64 instruction holds its scheduler's pipe for 64 cycles and the
+// update of a wider sub-panel would be most of a column's time (the product that
+// follows has the whole GPU).  CTAs: 32 rows each, at most 16: a hop to another
+// CTA costs no more than one to the own (~200 cycles).
+template <typename T, int SW, int RPT>
+bool cluster_ready(bemgpu_ctx_s *ctx) {
+  static signed char state[BEM_MAX_DEVICES] = {};  // 0 unknown, 1 usable, -1 not: a property of the device
+  static std::mutex mu;
+  std::lock_guard<std::mutex> lk(mu);
+  signed char &st = state[ctx->device];
+  if (st == 0) {
+    auto kern = panel_cluster_kernel<T, SW, RPT>;
+    const size_t smem = CpSmem<T, SW, RPT>::bytes(CP_MAX_THREADS * RPT);
+    bool ok = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) == cudaSuccess &&
+              cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess;
+    if (ok) {
+      cudaLaunchConfig_t cfg = {};
+      cfg.gridDim = dim3(CP_MAX_CLUSTER);
+      cfg.blockDim = dim3(CP_MAX_THREADS);
+      cfg.dynamicSmemBytes = smem;
+      cudaLaunchAttribute at = {};
+      at.id = cudaLaunchAttributeClusterDimension;
+      at.val.clusterDim.x = CP_MAX_CLUSTER;
+      at.val.clusterDim.y = at.val.clusterDim.z = 1;
+      cfg.attrs = &at;
+      cfg.numAttrs = 1;
+      int clusters = 0;
+      ok = cudaOccupancyMaxActiveClusters(&clusters, kern, &cfg) == cudaSuccess && clusters > 0;
+    }
+    if (!ok) cudaGetLastError();
+    st = ok ? 1 : -1;
+  }
+  return st > 0;
+}
+
+template <typename T, int SW, int RPT>
+int panel_cluster_run(bemgpu_ctx_s *ctx, T *A, int64_t lda, int n, int k0, int w, int *d_ipiv, int *d_info, int *err,
+                      cudaStream_t stream, int nb, int64_t strideA) {
+  constexpr int PER = 32;
+  for (int p = k0; p < k0 + w; p += SW) {
+    const int sw = std::min(SW, k0 + w - p), rows = n - p;
+    int G = 1;
+    while (G < CP_MAX_CLUSTER && rows > G * PER) G *= 2;
+    // BEMGPU_TUNE_PANEL_CTAS: fewer CTAs as far as their threads hold the rows
+    while (ctx->tune.panel_ctas > 0 && G > ctx->tune.panel_ctas && rows <= G / 2 * CP_MAX_THREADS * RPT) G /= 2;
+    const int chunk = (rows + G - 1) / G;
+    // four warps at least: they share the panel's other columns
+    const int nt = std::max(128, std::min(CP_MAX_THREADS, ((chunk + RPT - 1) / RPT + 31) / 32 * 32));
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(G, nb);
+    cfg.blockDim = dim3(nt);
+    cfg.dynamicSmemBytes = CpSmem<T, SW, RPT>::bytes(chunk);
+    cfg.stream = stream;
+    cudaLaunchAttribute at = {};
+    at.id = cudaLaunchAttributeClusterDimension;
+    at.val.clusterDim.x = G;
+    at.val.clusterDim.y = at.val.clusterDim.z = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    {
+      const double cb = 2.0 * sizeof(T);
+      ProfScope ps(ctx, BEMGPU_K_LU_PANEL, stream, 4.0 * (double)rows * sw * sw * nb, cb * 2.0 * rows * sw * nb);
+      const cudaError_t e = cudaLaunchKernelEx(&cfg, panel_cluster_kernel<T, SW, RPT>, A, lda, n, p, sw, k0, k0 + w,
+                                               chunk, d_ipiv, d_info, err, strideA);
+      ctx->launches++;
+      if (e != cudaSuccess) {
+        cudaGetLastError();
+        return bem_fail(ctx, BEMGPU_ERR_CUDA, "getrf: cluster panel launch: %s", cudaGetErrorString(e));
+      }
+    }
+    const int nr = n - p - sw, nc = k0 + w - p - sw;
+    if (nr > 0 && nc > 0) {
+      typedef PuCfg<T, SW> Cfg;
+      ProfScope ps(ctx, BEMGPU_K_LU_PANEL, stream, 8.0 * nr * nc * sw * nb,
+                   2.0 * sizeof(T) * ((double)nr * sw + (double)sw * nc + 2.0 * nr * nc) * nb);
+      panel_update_kernel<T, SW><<<dim3((nr + Cfg::TM - 1) / Cfg::TM, (nc + Cfg::TN - 1) / Cfg::TN, nb), 256, 0, stream>>>(
+          nr, nc, sw, A + 2 * (p + sw + lda * (int64_t)p), A + 2 * (p + lda * (int64_t)(p + sw)),
+          A + 2 * (p + sw + lda * (int64_t)(p + sw)), lda, strideA);
+      ctx->launches++;
+      BEM_CUDA_TRY(ctx, cudaGetLastError());
+    }
+  }
+  return BEMGPU_OK;
+}
+
+template <typename T>
+bool panel_cluster(bemgpu_ctx_s *ctx, T *A, int64_t lda, int n, int k0, int w, int *d_ipiv, int *d_info,
+                   cudaStream_t stream, int &rc, int nb = 1, int64_t strideA = 0) {
+  constexpr int SW = sizeof(T) == 8 ? 8 : 32;
+  const int rows = n - k0, cap = CP_MAX_CLUSTER * CP_MAX_THREADS;
+  rc = BEMGPU_OK;
+  if (rows > 2 * cap || !(rows <= cap ? cluster_ready<T, SW, 1>(ctx) : cluster_ready<T, SW / 2, 2>(ctx))) return false;
+  int *err = (int *)bem_workspace(ctx, "tc_err", sizeof(int));
+  if (!err) {
+    rc = bem_fail(ctx, BEMGPU_ERR_OOM, "getrf: panel workspace");
+    return true;
+  }
+  if (!ctx->tc_err_ready) {
+    cudaMemsetAsync(err, 0, sizeof(int), stream);
+    ctx->tc_err_ready = true;
+  }
+  rc = rows <= cap ? panel_cluster_run<T, SW, 1>(ctx, A, lda, n, k0, w, d_ipiv, d_info, err, stream, nb, strideA)
+                   : panel_cluster_run<T, SW / 2, 2>(ctx, A, lda, n, k0, w, d_ipiv, d_info, err, stream, nb, strideA);
+  return true;
+}
+
 // LU with partial pivoting of nb equal-size matrices A + i strideA (pivots
 // d_ipiv + i n, info d_info + i): every panel of the batch in one cooperative
 // launch (each matrix with its own CTAs and barrier), the interchanges,
@@ -1016,7 +1583,9 @@ int getrf_impl(bemgpu_ctx_s *ctx, T *A0, int64_t lda, int n, int *d_ipiv0, int *
     const int K0 = second_half ? k0 - NBL : k0;              // the pair's first column
     const int blocks = std::max(1, std::min(ctx->num_sms * 2, (rows + PANEL_THREADS - 1) / PANEL_THREADS));
     int prc = BEMGPU_OK;
-    bool coop = ctx->coop_panel && panel_coop<T>(ctx, A0, lda, n, k0, w, d_ipiv0, d_info0, stream, prc, nb, strideA);
+    bool coop = ctx->coop_panel &&
+                (panel_cluster<T>(ctx, A0, lda, n, k0, w, d_ipiv0, d_info0, stream, prc, nb, strideA) ||
+                 panel_coop<T>(ctx, A0, lda, n, k0, w, d_ipiv0, d_info0, stream, prc, nb, strideA));
     if (prc) return prc;
     if (!coop && nb > 1 && ctx->coop_panel) {
       // the batch's panels do not fit at once: one cooperative panel per matrix
@@ -1233,7 +1802,8 @@ int bem_zgetrf_exact(bemgpu_ctx_s *ctx, double *A, int64_t lda, int n, int *d_ip
     for (int k0 = K0; k0 < K0 + WO && !rc; k0 += NB) {
       const int w = std::min(NB, K0 + WO - k0);
       int prc = BEMGPU_OK;
-      const bool coop = ctx->coop_panel && panel_coop<double>(ctx, A, lda, n, k0, w, d_ipiv, d_info, stream, prc);
+      const bool coop = ctx->coop_panel && (panel_cluster<double>(ctx, A, lda, n, k0, w, d_ipiv, d_info, stream, prc) ||
+                                            panel_coop<double>(ctx, A, lda, n, k0, w, d_ipiv, d_info, stream, prc));
       if (prc) return prc;
       if (!coop) {  // one launch per column when the panel does not fit the cooperative kernel
         PivCand *cand = (PivCand *)bem_workspace(ctx, "lu_cand", sizeof(PivCand) * 1024);
