@@ -253,11 +253,16 @@ int bem_cgetrs(bemgpu_ctx_s *ctx, const float *A, int64_t lda, int n, const int 
 // leading dimension ld), each stored dense (n x n, zeros in the other triangle).
 int bem_ctri_inverses(bemgpu_ctx_s *ctx, const float *LU, int64_t ld, int n, float *Linv, float *Uinv,
                       cudaStream_t st);
-// B <- U^{-1} L^{-1} P B with the explicit inverses (tmp: n x nrhs complex64).
-int bem_capply_inverse_identity(bemgpu_ctx_s *ctx, const float *Linv, const float *Uinv, int n, const int *d_ipiv,
+// The row permutation of the interchanges d_ipiv[0..n): perm[i] = the row whose
+// content ends in row i, then its inverse (2 n ints in the context's workspace,
+// valid until the next call); null on failure.
+int *bem_row_permutation(bemgpu_ctx_s *ctx, const int *d_ipiv, int n, cudaStream_t st);
+// B = U^{-1} L^{-1} P E for identity columns, and out = U^{-1} L^{-1} P B (B is
+// overwritten; out n x nrhs, leading dimension n), with the explicit inverses.
+int bem_capply_inverse_identity(bemgpu_ctx_s *ctx, const float *Linv, const float *Uinv, int n, const int *perm,
                                 int row0, float *B, int64_t ldb, int nrhs, float *tmp, cudaStream_t st);
-int bem_capply_inverse(bemgpu_ctx_s *ctx, const float *Linv, const float *Uinv, int n, const int *d_ipiv, float *B,
-                       int64_t ldb, int nrhs, float *tmp, cudaStream_t st);
+int bem_capply_inverse(bemgpu_ctx_s *ctx, const float *Linv, const float *Uinv, int n, const int *perm, float *B,
+                       int64_t ldb, int nrhs, float *out, cudaStream_t st);
 // complex64 GEMM: tensor cores where the shape allows (gemm_tc.cu), else FMA pipes.
 int bem_cgemm(bemgpu_ctx_s *ctx, int kind, char opA, int m, int n, int k, const float alpha[2], const float *A,
               int64_t lda, const float *B, int64_t ldb, const float beta[2], float *C, int64_t ldc,

@@ -184,46 +184,36 @@ __global__ void __launch_bounds__(PANEL_THREADS) panel_step_kernel(T *A, int64_t
   }
 }
 
-// Applies the interchanges ipiv[k1..k2) to columns [c0, c1) (zlaswp).
-template <typename T>
-__global__ void laswp_kernel(T *A, int64_t lda, int c0, int c1, int k1, int k2, const int *ipiv) {
-  const int c = c0 + blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= c1) return;
-  const int64_t col = (int64_t)c * lda;
-  for (int k = k1; k < k2; k++) {
-    const int p = ipiv[k];
-    if (p != k) {
-      const cx<T> a = cld(A, k + col), b = cld(A, p + col);
-      cst(A, k + col, b);
-      cst(A, p + col, a);
-    }
+// Where the content of position d comes from once the interchanges ipiv[k1..k2)
+// (in order, as laswp applies them) are done: d led back through them.  piv holds
+// ipiv[k1..k2) in shared memory.
+__device__ __forceinline__ int interchange_source(const int *piv, int k1, int k2, int d) {
+  int x = d;
+#pragma unroll 8
+  for (int k = k2 - 1; k >= k1; k--) {
+    const int p = piv[k - k1];
+    x = x == k ? p : x == p ? k : x;
   }
+  return x;
 }
 
-// The row interchanges ipiv[0..n) (applied in order, as laswp does) as one
-// permutation: perm[i] = the row whose content ends in row i.  One CTA: ipiv
-// and the row labels in shared memory, one thread replays the swaps.
-constexpr int PERM_MAX_N = 24576;  // 2 x 96 KB of shared memory
+// The row interchanges ipiv[0..n) as one permutation: perm[i] = the row whose
+// content ends in row i, and its inverse.  Every row leads itself back (n steps
+// of shared-memory broadcasts: ~20 us at n = 7680, where one thread's replay of
+// the swaps took 295).
+constexpr int PERM_MAX_N = 49152;  // 192 KB of shared memory; beyond, the pivots are read from global memory
 
-__global__ void perm_from_ipiv_kernel(const int *__restrict__ ipiv, int n, int *__restrict__ perm) {
+__global__ void __launch_bounds__(128) perm_from_ipiv_kernel(const int *__restrict__ ipiv, int n, int *__restrict__ perm,
+                                                             int *__restrict__ inverse, int staged) {
   extern __shared__ int perm_smem[];
-  int *pr = perm_smem, *pv = perm_smem + n;
-  for (int i = threadIdx.x; i < n; i += blockDim.x) {
-    pr[i] = i;
-    pv[i] = ipiv[i];
-  }
+  if (staged)
+    for (int i = threadIdx.x; i < n; i += blockDim.x) perm_smem[i] = ipiv[i];
   __syncthreads();
-  if (threadIdx.x == 0)
-    for (int k = 0; k < n; k++) {
-      const int p = pv[k];
-      if (p != k) {
-        const int t = pr[k];
-        pr[k] = pr[p];
-        pr[p] = t;
-      }
-    }
-  __syncthreads();
-  for (int i = threadIdx.x; i < n; i += blockDim.x) perm[i] = pr[i];
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  const int s = staged ? interchange_source(perm_smem, 0, n, i) : interchange_source(ipiv, 0, n, i);
+  perm[i] = s;
+  inverse[s] = i;
 }
 
 // out[i, c] = B[perm[i], c] for complex64 column-major B (n x ncols).
@@ -235,95 +225,35 @@ __global__ void gather_rows_c64_kernel(const float *__restrict__ B, int64_t ldb,
   reinterpret_cast<float2 *>(out)[i + ldo * c] = reinterpret_cast<const float2 *>(B)[perm[i] + ldb * c];
 }
 
-// The same interchanges for a panel of at most LASWP_MAXW rows, as one
-// permutation: warp 0 of each CTA replays the swaps on row labels in shared
-// memory (the panel's rows and the pivot rows below it), which gives for
-// every touched row the row its final content comes from; then one warp per
-// column gathers those entries into registers and writes them back (all
-// loads of a column before its stores).  Same result as the swaps in order;
-// each entry moves once instead of once per swap that touches it.
+// The interchanges of a panel of at most LASWP_MAXW rows on columns [c0, c1):
+// thread t of a CTA has one of the at most 2 w touched rows (the panel's own and
+// the pivot rows below it), knows its source (interchange_source), and moves that
+// entry of LASWP_COLS columns at a time, all loads before the stores.  Each entry
+// moves once.  (One warp's replay of the swaps took most of the 22 us of a launch
+// at n = 7680; this takes ~6.)
 constexpr int LASWP_MAXW = 128;
-constexpr int LASWP_WARPS = 8;
+constexpr int LASWP_COLS = 8;
 
 template <typename T>
-__global__ void __launch_bounds__(32 * LASWP_WARPS)
+__global__ void __launch_bounds__(2 * LASWP_MAXW)
     laswp_perm_kernel(T *A, int64_t lda, int c0, int c1, int k1, int k2, const int *ipiv) {
-  __shared__ int row[2 * LASWP_MAXW], from[2 * LASWP_MAXW];
-  __shared__ int nslot, nmove;
-  __shared__ int mdst[2 * LASWP_MAXW], msrc[2 * LASWP_MAXW];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, m = k2 - k1;
-  if (warp == 0) {
-    for (int s = lane; s < m; s += 32) {
-      row[s] = k1 + s;
-      from[s] = k1 + s;
-    }
-    if (lane == 0) nslot = m;
-    __syncwarp();
-    for (int k = k1; k < k2; k++) {
-      const int p = ipiv[k];
-      if (p == k) continue;
-      int sp;
-      if (p < k2) {
-        sp = p - k1;
-      } else {
-        // the slot of pivot row p among the rows below the panel (appended
-        // on first use)
-        const int ns = nslot;
-        int found = -1;
-        for (int s0 = m; s0 < ns; s0 += 32) {
-          const int s = s0 + lane;
-          const unsigned hit = __ballot_sync(0xffffffffu, s < ns && row[s] == p);
-          if (hit) {
-            found = s0 + __ffs(hit) - 1;
-            break;
-          }
-        }
-        if (found < 0) {
-          found = ns;
-          if (lane == 0) {
-            row[ns] = p;
-            from[ns] = p;
-            nslot = ns + 1;
-          }
-        }
-        __syncwarp();
-        sp = found;
-      }
-      if (lane == 0) {
-        const int t = from[k - k1];
-        from[k - k1] = from[sp];
-        from[sp] = t;
-      }
-      __syncwarp();
-    }
-    if (lane == 0) {
-      int c = 0;
-      for (int s = 0; s < nslot; s++)
-        if (from[s] != row[s]) {
-          mdst[c] = row[s];
-          msrc[c] = from[s];
-          c++;
-        }
-      nmove = c;
-    }
-  }
+  __shared__ int piv[LASWP_MAXW];
+  const int t = threadIdx.x, m = k2 - k1;
+  for (int k = t; k < m; k += blockDim.x) piv[k] = ipiv[k1 + k];
   __syncthreads();
-  const int nm = nmove;
-  constexpr int PER = 2 * LASWP_MAXW / 32;
-  for (int c = c0 + blockIdx.x * LASWP_WARPS + warp; c < c1; c += gridDim.x * LASWP_WARPS) {
-    const int64_t col = (int64_t)c * lda;
-    cx<T> v[PER];
+  const int d = t < m ? k1 + t : t < 2 * m ? piv[t - m] : -1;
+  const bool mine = t < m || (t < 2 * m && d >= k2);
+  const int src = mine ? interchange_source(piv, k1, k2, d) : d;
+  const bool on = mine && src != d;
+  for (int c = c0 + blockIdx.x * LASWP_COLS; c < c1; c += gridDim.x * LASWP_COLS) {
+    cx<T> v[LASWP_COLS];
 #pragma unroll
-    for (int j = 0; j < PER; j++) {
-      const int i = lane + 32 * j;
-      if (i < nm) v[j] = cld(A, msrc[i] + col);
-    }
-    __syncwarp();
+    for (int e = 0; e < LASWP_COLS; e++)
+      if (on && c + e < c1) v[e] = cld(A, src + (int64_t)(c + e) * lda);
+    __syncthreads();
 #pragma unroll
-    for (int j = 0; j < PER; j++) {
-      const int i = lane + 32 * j;
-      if (i < nm) cst(A, mdst[i] + col, v[j]);
-    }
+    for (int e = 0; e < LASWP_COLS; e++)
+      if (on && c + e < c1) cst(A, d + (int64_t)(c + e) * lda, v[e]);
   }
 }
 
@@ -1058,75 +988,118 @@ __global__ void __launch_bounds__(256) panel_update_kernel(int m, int n, int k, 
     }
 }
 
-// B[0:w, :] <- L11^{-1} B (unit lower) or U11^{-1} B (upper) with the w x w
-// diagonal block (w <= 32 R) in shared memory; one warp per right-hand-side
-// column, lane holds rows lane + 32 r, r < R.
-template <typename T, bool UPPER, int R>
-__global__ void __launch_bounds__(256) trsm_block_kernel(const T *Ad, int64_t lda, int w, T *B, int64_t ldb,
-                                                         int ncols) {
+// B[0:w, :] <- T^{-1} B for the w x w (w <= W) unit-lower or upper triangle T: NC
+// right-hand sides per CTA in shared memory, in blocks of 32 rows: the block's
+// own triangle by substitution (a warp has NC / warps columns, lane = row), then
+// its product with the rows that remain.
+//
+// Complex64 (NC = 32): the update is most of the work and runs from shared
+// memory at one load per 3.7 FMA; a warp that substituted all 128 rows of one
+// column by itself took 95 us at n = 7680 where this takes ~15.  Complex128
+// (NC = 4, a warp per scheduler): bound by the FP64 pipe, so the columns spread
+// over as many SMs as there are.
+template <typename T>
+struct TriCfg;
+template <>
+struct TriCfg<float> { static constexpr int NC = 32, THREADS = 256; };
+template <>
+struct TriCfg<double> { static constexpr int NC = 4, THREADS = 128; };
+
+template <typename T, int W, bool UPPER>
+__global__ void __launch_bounds__(TriCfg<T>::THREADS) tri_block_kernel(const T *Ad, int64_t lda, int w, T *B, int64_t ldb,
+                                                                       int ncols) {
   typedef typename V2<T>::type T2;
-  constexpr int LDS = 32 * R;
-  extern __shared__ __align__(16) unsigned char trsm_smem[];
-  T2 *Ls = reinterpret_cast<T2 *>(trsm_smem);  // LDS * LDS
-  for (int idx = threadIdx.x; idx < w * w; idx += blockDim.x) {
-    const int r = idx % w, c = idx / w;
-    Ls[r + LDS * c] = reinterpret_cast<const T2 *>(Ad)[r + lda * (int64_t)c];
+  constexpr int NC = TriCfg<T>::NC, THREADS = TriCfg<T>::THREADS, WARPS = THREADS / 32, CPW = NC / WARPS;
+  constexpr int RPP = THREADS / NC, PER = (W - 32) / RPP;  // rows per pass of the update, passes
+  extern __shared__ __align__(16) unsigned char tri_raw[];
+  T2 *X = reinterpret_cast<T2 *>(tri_raw);  // [W][NC]
+  T2 *Ts = X + W * NC;                      // [W][33] the triangle's columns of one block
+  T2 *rd = Ts + W * 33;                     // [W] reciprocals of the diagonal (upper)
+  const T2 *A2 = reinterpret_cast<const T2 *>(Ad);
+  T2 *B2 = reinterpret_cast<T2 *>(B);
+  const T2 zero = V2<T>::make(0, 0);
+  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5, n0 = blockIdx.x * NC;
+  for (int k = tid; k < W * NC; k += THREADS) {
+    const int r = k % W, c = k / W;
+    X[r * NC + c] = r < w && n0 + c < ncols ? B2[r + ldb * (int64_t)(n0 + c)] : zero;
+  }
+  if (UPPER)
+    for (int r = tid; r < W; r += THREADS) {
+      cx<T> d = {1, 0};
+      if (r < w) d = crecip(cld(Ad, r + lda * (int64_t)r));
+      rd[r] = V2<T>::make(d.r, d.i);
+    }
+  const int nblk = (w + 31) / 32;
+#pragma unroll 1
+  for (int q = 0; q < nblk; q++) {
+    const int b = UPPER ? nblk - 1 - q : q, o = b * 32;
+    const int r0 = UPPER ? 0 : o, r1 = UPPER ? min(w, o + 32) : w;  // the block column's rows
+    __syncthreads();  // the previous block's readers are done
+    for (int k = tid; k < (r1 - r0) * 32; k += THREADS) {
+      const int r = r0 + k % (r1 - r0), c = k / (r1 - r0);
+      Ts[r * 33 + c] = o + c < w ? A2[r + lda * (int64_t)(o + c)] : zero;
+    }
+    __syncthreads();
+    {
+      const int row = o + lane;
+      T2 x[CPW];
+#pragma unroll
+      for (int e = 0; e < CPW; e++) x[e] = row < W ? X[row * NC + wid * CPW + e] : zero;
+      const int m = min(32, w - o);
+      for (int i0 = 0; i0 < m; i0++) {
+        const int i = UPPER ? m - 1 - i0 : i0;
+        const T2 t = row < w && (UPPER ? lane < i : lane > i) ? Ts[row * 33 + i] : zero;
+        const T2 rdi = UPPER ? rd[o + i] : zero;
+#pragma unroll
+        for (int e = 0; e < CPW; e++) {
+          if (UPPER && lane == i) {
+            const cx<T> y = cmul(cx<T>{x[e].x, x[e].y}, cx<T>{rdi.x, rdi.y});
+            x[e] = V2<T>::make(y.r, y.i);
+          }
+          const T xr = __shfl_sync(0xffffffffu, x[e].x, i), xi = __shfl_sync(0xffffffffu, x[e].y, i);
+          x[e].x -= t.x * xr - t.y * xi;
+          x[e].y -= t.x * xi + t.y * xr;
+        }
+      }
+#pragma unroll
+      for (int e = 0; e < CPW; e++)
+        if (row < W) X[row * NC + wid * CPW + e] = x[e];
+    }
+    __syncthreads();
+    // the remaining rows: [o + 32, w) below, or [0, o) above
+    const int u0 = UPPER ? 0 : o + 32, u1 = UPPER ? o : w;
+    if (u1 > u0) {
+      const int c = tid % NC, ry = tid / NC;
+      T2 acc[PER];
+#pragma unroll
+      for (int e = 0; e < PER; e++) {
+        const int r = u0 + ry + RPP * e;
+        acc[e] = r < u1 ? X[r * NC + c] : zero;
+      }
+#pragma unroll 4
+      for (int k = 0; k < 32; k++) {
+        const T2 x = o + k < W ? X[(o + k) * NC + c] : zero;
+#pragma unroll
+        for (int e = 0; e < PER; e++) {
+          const int r = u0 + ry + RPP * e;
+          if (r < u1) {
+            const T2 t = Ts[r * 33 + k];
+            acc[e].x = fma(t.y, x.y, fma(-t.x, x.x, acc[e].x));
+            acc[e].y = fma(-t.y, x.x, fma(-t.x, x.y, acc[e].y));
+          }
+        }
+      }
+#pragma unroll
+      for (int e = 0; e < PER; e++) {
+        const int r = u0 + ry + RPP * e;
+        if (r < u1) X[r * NC + c] = acc[e];
+      }
+    }
   }
   __syncthreads();
-  const int lane = threadIdx.x & 31;
-  const int warp = threadIdx.x >> 5;
-  const int nwarps = blockDim.x >> 5;
-  for (int col = blockIdx.x * nwarps + warp; col < ncols; col += gridDim.x * nwarps) {
-    T2 *b = reinterpret_cast<T2 *>(B) + ldb * (int64_t)col;
-    cx<T> x[R];
-#pragma unroll
-    for (int r = 0; r < R; r++) {
-      x[r] = {0, 0};
-      if (lane + 32 * r < w) x[r] = {b[lane + 32 * r].x, b[lane + 32 * r].y};
-    }
-    if (!UPPER) {
-      for (int i = 0; i < w; i++) {
-        cx<T> own = {0, 0};
-#pragma unroll
-        for (int r = 0; r < R; r++)
-          if ((i >> 5) == r) own = x[r];
-        const cx<T> xi = {__shfl_sync(0xffffffffu, own.r, i & 31), __shfl_sync(0xffffffffu, own.i, i & 31)};
-#pragma unroll
-        for (int r = 0; r < R; r++) {
-          const int row = lane + 32 * r;
-          if (row > i && row < w) {
-            const T2 l = Ls[row + LDS * i];
-            x[r].r -= l.x * xi.r - l.y * xi.i;
-            x[r].i -= l.x * xi.i + l.y * xi.r;
-          }
-        }
-      }
-    } else {
-      for (int i = w - 1; i >= 0; i--) {
-        // x_i /= U_ii on the owning lane, then broadcast
-        const T2 d = Ls[i + LDS * i];
-        cx<T> own = {0, 0};
-#pragma unroll
-        for (int r = 0; r < R; r++)
-          if ((i >> 5) == r) {
-            if (lane == (i & 31)) x[r] = cmul(x[r], crecip(cx<T>{d.x, d.y}));
-            own = x[r];
-          }
-        const cx<T> xi = {__shfl_sync(0xffffffffu, own.r, i & 31), __shfl_sync(0xffffffffu, own.i, i & 31)};
-#pragma unroll
-        for (int r = 0; r < R; r++) {
-          const int row = lane + 32 * r;
-          if (row < i) {
-            const T2 u = Ls[row + LDS * i];
-            x[r].r -= u.x * xi.r - u.y * xi.i;
-            x[r].i -= u.x * xi.i + u.y * xi.r;
-          }
-        }
-      }
-    }
-#pragma unroll
-    for (int r = 0; r < R; r++)
-      if (lane + 32 * r < w) b[lane + 32 * r] = V2<T>::make(x[r].r, x[r].i);
+  for (int k = tid; k < W * NC; k += THREADS) {
+    const int r = k % W, c = k / W;
+    if (r < w && n0 + c < ncols) B2[r + ldb * (int64_t)(n0 + c)] = X[r * NC + c];
   }
 }
 
@@ -1267,22 +1240,44 @@ struct GemmCfg<float> {
   static constexpr int BM = 128, BN = 64, TM = 8, TN = 4, BK = 8;
 };
 
-template <typename T, int R = NB / 32>
-constexpr int trsm_smem_bytes() { return 32 * R * 32 * R * (int)sizeof(typename V2<T>::type); }
+template <typename T, int W>
+constexpr int tri_smem_bytes() { return (W * TriCfg<T>::NC + W * 33 + W) * (int)sizeof(typename V2<T>::type); }
 
 template <typename T>
-int set_trsm_attrs(bemgpu_ctx_s *ctx) {
-  static bool done[64] = {false};
+int set_tri_attrs(bemgpu_ctx_s *ctx) {
+  static bool done[BEM_MAX_DEVICES] = {false};
   if (done[ctx->device]) return BEMGPU_OK;
-  constexpr int RL = LuCfg<T>::NBL / 32;
-  BEM_CUDA_TRY(ctx, cudaFuncSetAttribute(trsm_block_kernel<T, false, NB / 32>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, trsm_smem_bytes<T>()));
-  BEM_CUDA_TRY(ctx, cudaFuncSetAttribute(trsm_block_kernel<T, true, NB / 32>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, trsm_smem_bytes<T>()));
-  BEM_CUDA_TRY(ctx, cudaFuncSetAttribute(trsm_block_kernel<T, false, RL>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         trsm_smem_bytes<T, RL>()));
+  constexpr int NBL = LuCfg<T>::NBL;
+  BEM_CUDA_TRY(ctx, cudaFuncSetAttribute(tri_block_kernel<T, NB, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         tri_smem_bytes<T, NB>()));
+  BEM_CUDA_TRY(ctx, cudaFuncSetAttribute(tri_block_kernel<T, NB, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         tri_smem_bytes<T, NB>()));
+  BEM_CUDA_TRY(ctx, cudaFuncSetAttribute(tri_block_kernel<T, NBL, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         tri_smem_bytes<T, NBL>()));
   done[ctx->device] = true;
   return BEMGPU_OK;
+}
+
+template <typename T, int W, bool UPPER>
+void launch_tri_block(bemgpu_ctx_s *ctx, const T *Ad, int64_t lda, int w, T *B, int64_t ldb, int ncols, cudaStream_t st) {
+  ProfScope ps(ctx, BEMGPU_K_TRSM, st, 4.0 * w * w * ncols, 4.0 * sizeof(T) * w * ncols);
+  constexpr int NC = TriCfg<T>::NC;
+  tri_block_kernel<T, W, UPPER>
+      <<<(ncols + NC - 1) / NC, TriCfg<T>::THREADS, tri_smem_bytes<T, W>(), st>>>(Ad, lda, w, B, ldb, ncols);
+  ctx->launches++;
+}
+
+// The interchanges ipiv[k1..k2) on columns [c0, c1), at most 128 rows a launch.
+template <typename T>
+void launch_laswp(bemgpu_ctx_s *ctx, T *A, int64_t lda, int c0, int c1, int k1, int k2, const int *ipiv,
+                  cudaStream_t st) {
+  if (c1 <= c0) return;
+  ProfScope ps(ctx, BEMGPU_K_LU_PANEL, st, 0.0, 8.0 * sizeof(T) * (k2 - k1) * (double)(c1 - c0));
+  const int g = std::min((c1 - c0 + LASWP_COLS - 1) / LASWP_COLS, 8 * ctx->num_sms);
+  for (int k = k1; k < k2; k += LASWP_MAXW) {
+    laswp_perm_kernel<T><<<g, 2 * LASWP_MAXW, 0, st>>>(A, lda, c0, c1, k, std::min(k2, k + LASWP_MAXW), ipiv);
+    ctx->launches++;
+  }
 }
 
 template <typename T>
@@ -1560,7 +1555,7 @@ bool panel_cluster(bemgpu_ctx_s *ctx, T *A, int64_t lda, int n, int k0, int w, i
 template <typename T>
 int getrf_impl(bemgpu_ctx_s *ctx, T *A0, int64_t lda, int n, int *d_ipiv0, int *d_info0, cudaStream_t stream,
                int nb = 1, int64_t strideA = 0) {
-  if (int rc0 = set_trsm_attrs<T>(ctx)) return rc0;
+  if (int rc0 = set_tri_attrs<T>(ctx)) return rc0;
   PivCand *cand = (PivCand *)bem_workspace(ctx, "lu_cand", sizeof(PivCand) * 1024);
   unsigned int *counter = (unsigned int *)bem_workspace(ctx, "lu_counter", sizeof(unsigned int));
   if (!cand || !counter) return bem_fail(ctx, BEMGPU_ERR_OOM, "getrf: workspace");
@@ -1610,25 +1605,12 @@ int getrf_impl(bemgpu_ctx_s *ctx, T *A0, int64_t lda, int n, int *d_ipiv0, int *
       BEM_CUDA_TRY(ctx, cudaGetLastError());
       // interchanges to the left and right of the panel
       static_assert(NBL <= LASWP_MAXW, "panel wider than the interchange kernel's permutation");
-      if (k0 > 0) {
-        ProfScope ps(ctx, BEMGPU_K_LU_PANEL, stream, 0.0, 4.0 * cb * w * k0);
-        const int g = std::min((k0 + LASWP_WARPS - 1) / LASWP_WARPS, 2 * ctx->num_sms);
-        laswp_perm_kernel<T><<<g, 32 * LASWP_WARPS, 0, stream>>>(A, lda, 0, k0, k0, k0 + w, d_ipiv);
-        ctx->launches++;
-      }
+      launch_laswp<T>(ctx, A, lda, 0, k0, k0, k0 + w, d_ipiv, stream);
       if (k0 + w < n) {
         const int nr = n - k0 - w;
         T *A11 = A + 2 * (k0 + lda * (int64_t)k0);
         T *A12 = A + 2 * (k0 + lda * (int64_t)(k0 + w));
-        // one CTA per SM at most: each CTA stages the w x w diagonal block in
-        // shared memory once and walks its share of the columns
-        const int tb = std::min((nr + 7) / 8, NBL > 64 ? ctx->num_sms : ctx->num_sms * 4);
-        {
-          ProfScope ps(ctx, BEMGPU_K_LU_PANEL, stream, 0.0, 4.0 * cb * w * nr);
-          const int g = std::min((nr + LASWP_WARPS - 1) / LASWP_WARPS, 2 * ctx->num_sms);
-          laswp_perm_kernel<T><<<g, 32 * LASWP_WARPS, 0, stream>>>(A, lda, k0 + w, n, k0, k0 + w, d_ipiv);
-          ctx->launches++;
-        }
+        launch_laswp<T>(ctx, A, lda, k0 + w, n, k0, k0 + w, d_ipiv, stream);
         if (second_half) {
           // panel A's update of B's rows beyond the pair:
           // A[k0:k0+w, k0+w:n] -= L[k0:k0+w, K0:k0] U[K0:k0, k0+w:n]
@@ -1636,12 +1618,7 @@ int getrf_impl(bemgpu_ctx_s *ctx, T *A0, int64_t lda, int n, int *d_ipiv0, int *
                                lda, A + 2 * (K0 + lda * (int64_t)(k0 + w)), lda, one, A12, lda, stream);
           if (rc) return rc;
         }
-        {
-          ProfScope ps(ctx, BEMGPU_K_TRSM, stream, 4.0 * w * w * nr, 2.0 * cb * w * nr);
-          trsm_block_kernel<T, false, NBL / 32>
-              <<<tb, 256, trsm_smem_bytes<T, NBL / 32>(), stream>>>(A11, lda, w, A12, lda, nr);
-          ctx->launches++;
-        }
+        launch_tri_block<T, NBL, false>(ctx, A11, lda, w, A12, lda, nr, stream);
         T *A22 = A + 2 * (k0 + w + lda * (int64_t)(k0 + w));
         int rc;
         if (first_half) {
@@ -1667,25 +1644,16 @@ int getrf_impl(bemgpu_ctx_s *ctx, T *A0, int64_t lda, int n, int *d_ipiv0, int *
 template <typename T>
 int getrs_impl(bemgpu_ctx_s *ctx, const T *A, int64_t lda, int n, const int *d_ipiv, T *B, int64_t ldb, int nrhs,
                cudaStream_t stream) {
-  if (int rc0 = set_trsm_attrs<T>(ctx)) return rc0;
+  if (int rc0 = set_tri_attrs<T>(ctx)) return rc0;
   const T mone[2] = {T(-1), T(0)}, one[2] = {T(1), T(0)};
   const double cb = 2.0 * sizeof(T);
-  {
-    ProfScope ps(ctx, BEMGPU_K_LU_PANEL, stream, 0.0, 4.0 * cb * n * nrhs);
-    laswp_kernel<T><<<(nrhs + 127) / 128, 128, 0, stream>>>(B, ldb, 0, nrhs, 0, n, d_ipiv);
-    ctx->launches++;
-  }
-  const int tb = std::min((nrhs + 7) / 8, ctx->num_sms * 4);
+  launch_laswp<T>(ctx, B, ldb, 0, nrhs, 0, n, d_ipiv, stream);
   // forward: L Y = P B
   for (int k0 = 0; k0 < n; k0 += NB) {
     const int w = std::min(NB, n - k0);
     const T *L11 = A + 2 * (k0 + lda * (int64_t)k0);
     T *Bk = B + 2 * (int64_t)k0;
-    {
-      ProfScope ps(ctx, BEMGPU_K_TRSM, stream, 4.0 * w * w * nrhs, 2.0 * cb * w * nrhs);
-      trsm_block_kernel<T, false, NB / 32><<<tb, 256, trsm_smem_bytes<T>(), stream>>>(L11, lda, w, Bk, ldb, nrhs);
-      ctx->launches++;
-    }
+    launch_tri_block<T, NB, false>(ctx, L11, lda, w, Bk, ldb, nrhs, stream);
     if (k0 + w < n) {
       const T *L21 = A + 2 * (k0 + w + lda * (int64_t)k0);
       int rc = gemm_any<T>(ctx, BEMGPU_K_SOLVE_GEMM, 'N', n - k0 - w, nrhs, w, mone, L21, lda, Bk, ldb, one,
@@ -1700,11 +1668,7 @@ int getrs_impl(bemgpu_ctx_s *ctx, const T *A, int64_t lda, int n, const int *d_i
     const int w = std::min(NB, n - k0);
     const T *U11 = A + 2 * (k0 + lda * (int64_t)k0);
     T *Bk = B + 2 * (int64_t)k0;
-    {
-      ProfScope ps(ctx, BEMGPU_K_TRSM, stream, 4.0 * w * w * nrhs, 2.0 * cb * w * nrhs);
-      trsm_block_kernel<T, true, NB / 32><<<tb, 256, trsm_smem_bytes<T>(), stream>>>(U11, lda, w, Bk, ldb, nrhs);
-      ctx->launches++;
-    }
+    launch_tri_block<T, NB, true>(ctx, U11, lda, w, Bk, ldb, nrhs, stream);
     if (k0 > 0) {
       const T *U01 = A + 2 * (lda * (int64_t)k0);
       int rc = gemm_any<T>(ctx, BEMGPU_K_SOLVE_GEMM, 'N', k0, nrhs, w, mone, U01, lda, Bk, ldb, one, B, ldb, stream);
@@ -1737,26 +1701,19 @@ __global__ void identity_block_kernel(double *X, int64_t ld, int w) {
 
 // X (w x ncols, ld ldx) <- T^{-1} X for the w x w triangle T at (A, lda):
 // unit lower (UPPER false) or upper; 64-row diagonal blocks in FP64
-// (trsm_block_kernel), off-diagonal updates as 5-slice exact products.
+// (tri_block_kernel), off-diagonal updates as 5-slice exact products.
 int tri_solve_exact(bemgpu_ctx_s *ctx, const double *A, int64_t lda, int w, bool upper, double *X, int64_t ldx,
                     int ncols, cudaStream_t st) {
-  const int tb = std::min((ncols + 7) / 8, ctx->num_sms * 4);
   const int nblk = (w + NB - 1) / NB;
   int rc = BEMGPU_OK;
   for (int q = 0; q < nblk && !rc; q++) {
     const int bi = upper ? nblk - 1 - q : q;
     const int j0 = bi * NB, jw = std::min(NB, w - j0);
     double *Xj = X + 2 * (int64_t)j0;
-    {
-      ProfScope ps(ctx, BEMGPU_K_TRSM, st, 4.0 * jw * jw * ncols, 32.0 * jw * ncols);
-      if (upper)
-        trsm_block_kernel<double, true, NB / 32><<<tb, 256, trsm_smem_bytes<double>(), st>>>(
-            A + 2 * (j0 + lda * (int64_t)j0), lda, jw, Xj, ldx, ncols);
-      else
-        trsm_block_kernel<double, false, NB / 32><<<tb, 256, trsm_smem_bytes<double>(), st>>>(
-            A + 2 * (j0 + lda * (int64_t)j0), lda, jw, Xj, ldx, ncols);
-      ctx->launches++;
-    }
+    if (upper)
+      launch_tri_block<double, NB, true>(ctx, A + 2 * (j0 + lda * (int64_t)j0), lda, jw, Xj, ldx, ncols, st);
+    else
+      launch_tri_block<double, NB, false>(ctx, A + 2 * (j0 + lda * (int64_t)j0), lda, jw, Xj, ldx, ncols, st);
     const int m = upper ? j0 : w - j0 - jw;  // rows still to update
     if (m > 0) {
       ExactOperand oa, ob;
@@ -1790,12 +1747,11 @@ int exact_mul(bemgpu_ctx_s *ctx, int kind, const double *Ablk, int64_t lda, int 
 // inverses of the diagonal super-blocks (L and U) are kept for
 // bem_zgetrs_exact ("lu_Lb", "lu_Ub": n x 512, block K at rows [K0, K0+512)).
 int bem_zgetrf_exact(bemgpu_ctx_s *ctx, double *A, int64_t lda, int n, int *d_ipiv, int *d_info, cudaStream_t stream) {
-  if (int rc0 = set_trsm_attrs<double>(ctx)) return rc0;
+  if (int rc0 = set_tri_attrs<double>(ctx)) return rc0;
   double *Lb = (double *)bem_workspace(ctx, "lu_Lb", 16 * (size_t)n * NBO);
   double *Ub = (double *)bem_workspace(ctx, "lu_Ub", 16 * (size_t)n * NBO);
   if (!Lb || !Ub) return bem_fail(ctx, BEMGPU_ERR_OOM, "getrf_exact: workspace");
   BEM_CUDA_TRY(ctx, cudaMemsetAsync(d_info, 0, sizeof(int), stream));
-  const double cb = 16.0;
   int rc = BEMGPU_OK;
   for (int K0 = 0; K0 < n && !rc; K0 += NBO) {
     const int WO = std::min(NBO, n - K0);
@@ -1819,27 +1775,12 @@ int bem_zgetrf_exact(bemgpu_ctx_s *ctx, double *A, int64_t lda, int n, int *d_ip
           ctx->launches++;
         }
       }
-      {
-        ProfScope ps(ctx, BEMGPU_K_LU_PANEL, stream, 0.0, 4.0 * cb * w * WO);
-        if (k0 > K0) {
-          laswp_kernel<double><<<(k0 - K0 + 127) / 128, 128, 0, stream>>>(A, lda, K0, k0, k0, k0 + w, d_ipiv);
-          ctx->launches++;
-        }
-        if (k0 + w < K0 + WO) {
-          laswp_kernel<double><<<(K0 + WO - k0 - w + 127) / 128, 128, 0, stream>>>(A, lda, k0 + w, K0 + WO, k0, k0 + w,
-                                                                                 d_ipiv);
-          ctx->launches++;
-        }
-      }
+      launch_laswp<double>(ctx, A, lda, K0, k0, k0, k0 + w, d_ipiv, stream);
+      launch_laswp<double>(ctx, A, lda, k0 + w, K0 + WO, k0, k0 + w, d_ipiv, stream);
       const int nc = K0 + WO - k0 - w;  // super-panel columns right of this panel
       if (nc > 0) {
-        const int tb = std::min((nc + 7) / 8, ctx->num_sms * 4);
-        {
-          ProfScope ps(ctx, BEMGPU_K_TRSM, stream, 4.0 * w * w * nc, 2.0 * cb * w * nc);
-          trsm_block_kernel<double, false, NB / 32><<<tb, 256, trsm_smem_bytes<double>(), stream>>>(
-              A + 2 * (k0 + lda * (int64_t)k0), lda, w, A + 2 * (k0 + lda * (int64_t)(k0 + w)), lda, nc);
-          ctx->launches++;
-        }
+        launch_tri_block<double, NB, false>(ctx, A + 2 * (k0 + lda * (int64_t)k0), lda, w,
+                                            A + 2 * (k0 + lda * (int64_t)(k0 + w)), lda, nc, stream);
         if (k0 + w < n)
           rc = exact_mul(ctx, BEMGPU_K_LU_GEMM, A + 2 * (k0 + w + lda * (int64_t)k0), lda, n - k0 - w, w, -1.0,
                          A + 2 * (k0 + lda * (int64_t)(k0 + w)), lda, nc, A + 2 * (k0 + w + lda * (int64_t)(k0 + w)),
@@ -1847,17 +1788,8 @@ int bem_zgetrf_exact(bemgpu_ctx_s *ctx, double *A, int64_t lda, int n, int *d_ip
       }
     }
     if (rc) break;
-    {
-      ProfScope ps(ctx, BEMGPU_K_LU_PANEL, stream, 0.0, 4.0 * cb * WO * (n - WO));
-      if (K0 > 0) {
-        laswp_kernel<double><<<(K0 + 127) / 128, 128, 0, stream>>>(A, lda, 0, K0, K0, K0 + WO, d_ipiv);
-        ctx->launches++;
-      }
-      if (K0 + WO < n) {
-        laswp_kernel<double><<<(n - K0 - WO + 127) / 128, 128, 0, stream>>>(A, lda, K0 + WO, n, K0, K0 + WO, d_ipiv);
-        ctx->launches++;
-      }
-    }
+    launch_laswp<double>(ctx, A, lda, 0, K0, K0, K0 + WO, d_ipiv, stream);
+    launch_laswp<double>(ctx, A, lda, K0 + WO, n, K0, K0 + WO, d_ipiv, stream);
     // inverses of the diagonal super-block's triangles
     const double *AKK = A + 2 * (K0 + lda * (int64_t)K0);
     double *LbK = Lb + 2 * (int64_t)K0, *UbK = Ub + 2 * (int64_t)K0;
@@ -1886,11 +1818,7 @@ int bem_zgetrs_exact(bemgpu_ctx_s *ctx, const double *A, int64_t lda, int n, con
   const double *Lb = (const double *)bem_workspace(ctx, "lu_Lb", 16 * (size_t)n * NBO);
   const double *Ub = (const double *)bem_workspace(ctx, "lu_Ub", 16 * (size_t)n * NBO);
   if (!Lb || !Ub) return bem_fail(ctx, BEMGPU_ERR_OOM, "getrs_exact: workspace");
-  {
-    ProfScope ps(ctx, BEMGPU_K_LU_PANEL, stream, 0.0, 64.0 * n * (double)nrhs);
-    laswp_kernel<double><<<(nrhs + 127) / 128, 128, 0, stream>>>(B, ldb, 0, nrhs, 0, n, d_ipiv);
-    ctx->launches++;
-  }
+  launch_laswp<double>(ctx, B, ldb, 0, nrhs, 0, n, d_ipiv, stream);
   int rc = BEMGPU_OK;
   for (int K0 = 0; K0 < n && !rc; K0 += NBO) {  // forward: L Y = P B
     const int WO = std::min(NBO, n - K0);
@@ -2096,89 +2024,72 @@ int bem_ctri_inverses(bemgpu_ctx_s *ctx, const float *LU, int64_t ld, int n, flo
 
 namespace {
 
-// T(:, c) = Linv(:, pos(row0 + c)): L^-1 applied to the interchanged identity
-// column row0 + c, where pos follows that column's 1 through the row
-// interchanges ipiv[0..n) (laswp order).
-__global__ void gather_linv_cols_kernel(const float *__restrict__ Linv, int n, const int *__restrict__ ipiv, int row0,
-                                        int ncols, float *__restrict__ T) {
-  __shared__ int s_pos;
+// T(:, c) = Linv(:, inverse[row0 + c]): L^-1 applied to the interchanged identity
+// column row0 + c, whose 1 the interchanges have taken to row inverse[row0 + c].
+__global__ void gather_linv_cols_kernel(const float *__restrict__ Linv, int n, const int *__restrict__ inverse, int row0,
+                                        float *__restrict__ T) {
   const int c = blockIdx.x;
-  if (c >= ncols) return;
-  if (threadIdx.x == 0) {
-    int pos = row0 + c;
-    for (int k = 0; k < n; k++) {
-      const int p = ipiv[k];
-      if (pos == k) pos = p;
-      else if (pos == p) pos = k;
-    }
-    s_pos = pos;
-  }
-  __syncthreads();
-  const float2 *src = reinterpret_cast<const float2 *>(Linv) + (int64_t)n * s_pos;
+  const float2 *src = reinterpret_cast<const float2 *>(Linv) + (int64_t)n * inverse[row0 + c];
   float2 *dst = reinterpret_cast<float2 *>(T) + (int64_t)n * c;
   for (int r = threadIdx.x; r < n; r += blockDim.x) dst[r] = src[r];
 }
 
 }  // namespace
 
+int *bem_row_permutation(bemgpu_ctx_s *ctx, const int *d_ipiv, int n, cudaStream_t st) {
+  int *perm = (int *)bem_workspace(ctx, "lu_perm", 2 * sizeof(int) * (size_t)n);
+  if (!perm) return nullptr;
+  if (!ctx->perm_ready) {
+    if (cudaFuncSetAttribute(perm_from_ipiv_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)(sizeof(int) * PERM_MAX_N)) != cudaSuccess) {
+      cudaGetLastError();
+      return nullptr;
+    }
+    ctx->perm_ready = true;
+  }
+  const bool staged = n <= PERM_MAX_N;
+  ProfScope ps(ctx, BEMGPU_K_LU_PANEL, st, 0.0, 12.0 * n);
+  perm_from_ipiv_kernel<<<(n + 127) / 128, 128, staged ? sizeof(int) * (size_t)n : 0, st>>>(d_ipiv, n, perm, perm + n,
+                                                                                            staged);
+  ctx->launches++;
+  return perm;
+}
+
+namespace {
+
+// D = T S for a triangle T (tri as bem_cgemm_tc's) of n rows.
+int tri_product(bemgpu_ctx_s *ctx, const float *T, int n, const float *S, int64_t lds, float *D, int64_t ldd, int nrhs,
+                int tri, cudaStream_t st) {
+  if (ctx->gemm_engine != 2 && n >= 64 && nrhs >= 64)  // tensor cores, the zero triangle skipped
+    return bem_cgemm_tc(ctx, BEMGPU_K_SOLVE_GEMM, n, nrhs, n, 1.f, T, n, S, lds, D, ldd, TC_OUT_F32, 0, st, tri);
+  const float one[2] = {1.f, 0.f}, zero[2] = {0.f, 0.f};
+  return bem_cgemm(ctx, BEMGPU_K_SOLVE_GEMM, 'N', n, nrhs, n, one, T, n, S, lds, zero, D, ldd, st);
+}
+
+}  // namespace
+
 // B = W32^-1 E_t for the identity columns row0 .. row0 + nrhs: the interchanges
 // and L^-1 reduce to gathering columns of L^-1, then one product with U^-1.
-int bem_capply_inverse_identity(bemgpu_ctx_s *ctx, const float *Linv, const float *Uinv, int n, const int *d_ipiv,
+int bem_capply_inverse_identity(bemgpu_ctx_s *ctx, const float *Linv, const float *Uinv, int n, const int *perm,
                                 int row0, float *B, int64_t ldb, int nrhs, float *tmp, cudaStream_t st) {
   {
     ProfScope ps(ctx, BEMGPU_K_SOLVE_GEMM, st, 0.0, 16.0 * (double)n * nrhs);
-    gather_linv_cols_kernel<<<nrhs, 256, 0, st>>>(Linv, n, d_ipiv, row0, nrhs, tmp);
+    gather_linv_cols_kernel<<<nrhs, 256, 0, st>>>(Linv, n, perm + n, row0, tmp);
     ctx->launches++;
   }
-  if (ctx->gemm_engine != 2 && n >= 64 && nrhs >= 64)
-    return bem_cgemm_tc(ctx, BEMGPU_K_SOLVE_GEMM, n, nrhs, n, 1.f, Uinv, n, tmp, n, B, ldb, TC_OUT_F32, 0, st, 2);
-  const float one[2] = {1.f, 0.f}, zero[2] = {0.f, 0.f};
-  return bem_cgemm(ctx, BEMGPU_K_SOLVE_GEMM, 'N', n, nrhs, n, one, Uinv, n, tmp, n, zero, B, ldb, st);
+  return tri_product(ctx, Uinv, n, tmp, n, B, ldb, nrhs, 2, st);
 }
 
-int bem_capply_inverse(bemgpu_ctx_s *ctx, const float *Linv, const float *Uinv, int n, const int *d_ipiv, float *B,
-                       int64_t ldb, int nrhs, float *tmp, cudaStream_t st) {
-  const bool gather = n <= PERM_MAX_N && ctx->gemm_engine != 2 && n >= 64 && nrhs >= 64;
-  if (gather) {
-    // the interchanges as one row permutation, gathered into tmp; the two
-    // products then alternate between tmp and B, and tmp goes back to B
-    int *perm = (int *)bem_workspace(ctx, "lu_perm", sizeof(int) * (size_t)n);
-    if (!perm) return bem_fail(ctx, BEMGPU_ERR_OOM, "apply inverse: permutation");
-    if (!ctx->perm_ready) {
-      BEM_CUDA_TRY(ctx, cudaFuncSetAttribute(perm_from_ipiv_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             (int)(2 * sizeof(int) * PERM_MAX_N)));
-      ctx->perm_ready = true;
-    }
-    {
-      ProfScope ps(ctx, BEMGPU_K_LU_PANEL, st, 0.0, 8.0 * n + 24.0 * (double)n * nrhs);
-      perm_from_ipiv_kernel<<<1, 256, 2 * sizeof(int) * (size_t)n, st>>>(d_ipiv, n, perm);
-      gather_rows_c64_kernel<<<dim3((unsigned)((n + 255) / 256), (unsigned)nrhs), 256, 0, st>>>(B, ldb, perm, n,
-                                                                                                tmp, n);
-      ctx->launches += 2;
-    }
-    BEM_CUDA_TRY(ctx, cudaGetLastError());
-    int rc = bem_cgemm_tc(ctx, BEMGPU_K_SOLVE_GEMM, n, nrhs, n, 1.f, Linv, n, tmp, n, B, ldb, TC_OUT_F32, 0, st, 1);
-    if (!rc) rc = bem_cgemm_tc(ctx, BEMGPU_K_SOLVE_GEMM, n, nrhs, n, 1.f, Uinv, n, B, ldb, tmp, n, TC_OUT_F32, 0, st, 2);
-    if (rc) return rc;
-    {
-      ProfScope ps(ctx, BEMGPU_K_LU_PANEL, st, 0.0, 16.0 * (double)n * nrhs);
-      BEM_CUDA_TRY(ctx, cudaMemcpy2DAsync(B, sizeof(float) * 2 * ldb, tmp, sizeof(float) * 2 * (size_t)n,
-                                          sizeof(float) * 2 * (size_t)n, nrhs, cudaMemcpyDeviceToDevice, st));
-    }
-    return BEMGPU_OK;
-  }
+// out = U^-1 L^-1 P B: the interchanged rows are gathered into out, the two
+// products go to B and back.
+int bem_capply_inverse(bemgpu_ctx_s *ctx, const float *Linv, const float *Uinv, int n, const int *perm, float *B,
+                       int64_t ldb, int nrhs, float *out, cudaStream_t st) {
   {
-    ProfScope ps(ctx, BEMGPU_K_LU_PANEL, st, 0.0, 32.0 * (double)n * nrhs);
-    laswp_kernel<float><<<(nrhs + 127) / 128, 128, 0, st>>>(B, ldb, 0, nrhs, 0, n, d_ipiv);
+    ProfScope ps(ctx, BEMGPU_K_LU_PANEL, st, 0.0, 16.0 * (double)n * nrhs);
+    gather_rows_c64_kernel<<<dim3((unsigned)((n + 255) / 256), (unsigned)nrhs), 256, 0, st>>>(B, ldb, perm, n, out, n);
     ctx->launches++;
   }
-  if (ctx->gemm_engine != 2 && n >= 64 && nrhs >= 64) {  // tensor cores, zero triangles skipped
-    int rc = bem_cgemm_tc(ctx, BEMGPU_K_SOLVE_GEMM, n, nrhs, n, 1.f, Linv, n, B, ldb, tmp, n, TC_OUT_F32, 0, st, 1);
-    if (!rc) rc = bem_cgemm_tc(ctx, BEMGPU_K_SOLVE_GEMM, n, nrhs, n, 1.f, Uinv, n, tmp, n, B, ldb, TC_OUT_F32, 0, st, 2);
-    return rc;
-  }
-  const float one[2] = {1.f, 0.f}, zero[2] = {0.f, 0.f};
-  int rc = bem_cgemm(ctx, BEMGPU_K_SOLVE_GEMM, 'N', n, nrhs, n, one, Linv, n, B, ldb, zero, tmp, n, st);
-  if (!rc) rc = bem_cgemm(ctx, BEMGPU_K_SOLVE_GEMM, 'N', n, nrhs, n, one, Uinv, n, tmp, n, zero, B, ldb, st);
-  return rc;
+  BEM_CUDA_TRY(ctx, cudaGetLastError());
+  const int rc = tri_product(ctx, Linv, n, out, n, B, ldb, nrhs, 1, st);
+  return rc ? rc : tri_product(ctx, Uinv, n, B, ldb, out, n, nrhs, 2, st);
 }

@@ -447,7 +447,9 @@ int bem_mixed_solve(bemgpu_ctx_s *ctx, double *W, int n, int ns2, const double *
   if (!rc) rc = bem_ctri_inverses(ctx, b.W32, n, n, b.Linv, b.Uinv, st);
   if (rc) return rc;
   cudaEventRecord(ev[2], st);
-  rc = bem_capply_inverse_identity(ctx, b.Linv, b.Uinv, n, b.ipiv, ns2, b.R32, n, nt2, b.T32, st);
+  const int *perm = bem_row_permutation(ctx, b.ipiv, n, st);
+  if (!perm) return bem_fail(ctx, BEMGPU_ERR_OOM, "mixed solve: row permutation");
+  rc = bem_capply_inverse_identity(ctx, b.Linv, b.Uinv, n, perm, ns2, b.R32, n, nt2, b.T32, st);
   if (rc) return rc;
   update_kernel<<<gm, 256, 0, st>>>(b.Y, b.R32, n, n, 0, nullptr);
   ctx->launches++;
@@ -485,13 +487,13 @@ int bem_mixed_solve(bemgpu_ctx_s *ctx, double *W, int n, int ns2, const double *
     if (rc) return rc;
     residual_finish_kernel<<<gm, 256, 0, st>>>(b.R64, b.R32, n, n, ns2);
     ctx->launches++;
-    rc = bem_capply_inverse(ctx, b.Linv, b.Uinv, n, b.ipiv, b.R32, n, nt2, b.T32, st);
+    rc = bem_capply_inverse(ctx, b.Linv, b.Uinv, n, perm, b.R32, n, nt2, b.T32, st);
     if (rc) return rc;
     // dY = widen(correction), quantized in place to the 3 slices the next
     // residual multiplies, then Y += dY: -W Y in R64 stays exact to the
     // product's 2^-40 however large the correction is (a slowly contracting
     // refinement's corrections are not small)
-    update_kernel<<<gm, 256, 0, st>>>(b.dY, b.R32, n, n, 0, nullptr);
+    update_kernel<<<gm, 256, 0, st>>>(b.dY, b.T32, n, n, 0, nullptr);
     ctx->launches++;
     rc = bem_exact_prep(ctx, "Y", false, b.dY, n, nt2, n, 1.0, DELTA_SLICES, opDY, st, b.dY);
     if (rc) return rc;
