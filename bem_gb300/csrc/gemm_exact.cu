@@ -159,7 +159,7 @@ __global__ void __launch_bounds__(EX_THREADS, 1)
   const uint32_t tmem = *tmem_slot;
 
   if (warp == 0) {
-    if (lane == 0) {
+    if (elect_one()) {
       int issued = 0;
       for (int kt = 0; kt < ktiles; kt++) {
         const int s = kt % EX_STAGES, round = kt / EX_STAGES;
@@ -178,7 +178,7 @@ __global__ void __launch_bounds__(EX_THREADS, 1)
         if (!mbar_wait(&full[kt % EX_STAGES], (kt / EX_STAGES) & 1, err)) break;
     }
   } else if (warp == 1) {
-    if (lane == 0) {
+    if (elect_one()) {
       constexpr uint32_t idesc = tc_idesc(EX_BM, EX_BN);
       for (int kt = 0; kt < ktiles; kt++) {
         // drain step dt = kt / EX_DRAIN covers EX_DRAIN stages (one exponent block)
@@ -372,7 +372,7 @@ __global__ void __launch_bounds__(EXW_THREADS, 1)
   const uint32_t tmem = *tmem_slot;
 
   if (warp == 0) {
-    if (lane == 0) {
+    if (elect_one()) {
       int issued = 0;
       for (int kt = 0; kt < ktiles; kt++) {
         const int s = kt % NST, round = kt / NST;
@@ -390,7 +390,7 @@ __global__ void __launch_bounds__(EXW_THREADS, 1)
         if (!mbar_wait(&full[kt % NST], (kt / NST) & 1, err)) break;
     }
   } else if (warp == 1) {
-    if (lane == 0) {
+    if (elect_one()) {
       constexpr uint32_t idesc = tc_idesc(EX_BM, EXW_BN);
       bool ok = true, zfirst = true;
       for (int kt = 0; kt < ktiles && ok; kt++) {

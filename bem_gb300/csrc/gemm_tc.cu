@@ -98,7 +98,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
   const int ke = tri == 1 ? min(ktiles, (m0 + TC_BM + TC_BK - 1) / TC_BK) : ktiles;
   const int nk = max(0, ke - kb);
   if (warp == 0) {
-    if (lane == 0) {
+    if (elect_one()) {
       int issued = 0;
       for (int j = 0; j < nk; j++) {
         const int kt = kb + j, s = j % TC_STAGES, round = j / TC_STAGES;
@@ -115,7 +115,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
       drain_copies(full, issued, err);
     }
   } else if (warp == 1) {
-    if (lane == 0) {
+    if (elect_one()) {
       constexpr uint32_t idesc = tc_idesc(TC_BM, TC_BN);
       bool ok = true;
       for (int j = 0; j < nk && ok; j++) {
@@ -240,7 +240,7 @@ __global__ void __launch_bounds__(TCC_THREADS, 1)
   const uint32_t tmem = *tmem_slot;
 
   if (warp == 0) {
-    if (lane == 0) {
+    if (elect_one()) {
       int issued = 0;
       for (int kt = 0; kt < ktiles; kt++) {
         const int s = kt % TCC_STAGES, round = kt / TCC_STAGES;
@@ -258,7 +258,7 @@ __global__ void __launch_bounds__(TCC_THREADS, 1)
         if (!mbar_wait(&full[kt % TCC_STAGES], (kt / TCC_STAGES) & 1, err)) break;
     }
   } else if (warp == 1) {
-    if (lane == 0) {
+    if (elect_one()) {
       constexpr uint32_t idesc = tc_idesc(TC_BM, TCC_BN);
       for (int kt = 0; kt < ktiles; kt++) {
         const int s = kt % TCC_STAGES, round = kt / TCC_STAGES, b = kt & 1, use = kt >> 1;
