@@ -20,15 +20,18 @@
 //     (double-buffered by step parity); levels 3..SL-1 (below 2^-24 of level 0)
 //     run in FP32 TMEM sums over the whole K.  Products of level >= SL are
 //     dropped (below 2^(-8 SL) of the block maxima's product).
-//   * eight epilogue warps drain each step while the next runs (three TMEM
-//     loads behind one wait per 8 columns): hi + lo += X0
-//     and += X1 (TwoSum each: exact), lo += X2 (rounding ~2^-40 of the sum);
+//   * eight epilogue warps drain each step while the next runs (six TMEM
+//     loads behind one wait per 16 columns), two columns an instruction: hi + lo
+//     += X0 and += X1 (TwoSum each: exact), lo += X2 (rounding ~2^-40 of the sum);
 //     at the end C = 2^-(sa+sb) (hi + lo + levels
 //     3..) [+ C] in FP64.
-//   * pipeline: warp 0 TMA (64-byte swizzle, 32-deep K steps, 3 stages),
-//     warp 1 tcgen05.mma (M=128, N=64, K=16, bf16 -> FP32) and TMEM
-//     allocation, warps 2..9 epilogue.  Every wait is bounded; a wait that
-//     runs out sets the error flag and the CTA finishes.
+//   * pipeline: warp 0 TMA, warp 1 tcgen05.mma (M=128, N=64, K=16, bf16 ->
+//     FP32) and TMEM allocation, warps 2..9 epilogue.  The MMA warp shares its
+//     scheduler with epilogue warps and issues one MMA every 48 cycles at best:
+//     descriptors in uniform registers and half as many epilogue instructions took
+//     n = 3840 from 6.63 to 5.49 ms (5 x 5), 4.54 to 3.74 (4 x 4) and 3.39 to
+//     2.48 (3 x 3).  Every wait is bounded; a wait that runs out sets the error
+//     flag and the CTA finishes.
 #include "bemgpu_internal.h"
 
 #include "tc_common.cuh"
@@ -131,7 +134,7 @@ __global__ void __launch_bounds__(EX_THREADS, 1)
   uint64_t *acce = accf + 2;           // step buffer b drained (epilogue -> MMA)
   uint64_t *fin = acce + 2;            // all MMAs of this CTA complete
   uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(fin + 1);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_uniform((int)(threadIdx.x >> 5)), lane = threadIdx.x & 31;
   int mt, nt;
   grouped_tile(raster, mt, nt);
   const int m0 = mt * EX_BM, n0 = nt * EX_BN;
@@ -156,7 +159,7 @@ __global__ void __launch_bounds__(EX_THREADS, 1)
   }
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;");
-  const uint32_t tmem = *tmem_slot;
+  const uint32_t tmem = warp_uniform(*tmem_slot);
 
   if (warp == 0) {
     if (elect_one()) {
@@ -178,19 +181,19 @@ __global__ void __launch_bounds__(EX_THREADS, 1)
         if (!mbar_wait(&full[kt % EX_STAGES], (kt / EX_STAGES) & 1, err)) break;
     }
   } else if (warp == 1) {
-    if (elect_one()) {
-      constexpr uint32_t idesc = tc_idesc(EX_BM, EX_BN);
-      for (int kt = 0; kt < ktiles; kt++) {
-        // drain step dt = kt / EX_DRAIN covers EX_DRAIN stages (one exponent block)
-        const int s = kt % EX_STAGES, round = kt / EX_STAGES, dt = kt / EX_DRAIN, b = dt & 1, use = dt >> 1;
-        const bool opening = kt % EX_DRAIN == 0, closing = kt % EX_DRAIN == EX_DRAIN - 1;
-        if (opening && dt >= 2 && !mbar_wait(&acce[b], (use - 1) & 1, err)) break;
-        if (!mbar_wait(&full[s], round & 1, err)) break;
-        asm volatile("tcgen05.fence::after_thread_sync;");
-        // descriptors: one per stage, the tiles and K steps as compile-time
-        // offsets added to its address field (which never carries: smem < 256 KB)
-        const uint64_t dbase =
-            EX_BK == 64 ? smem_desc_sw128(smem_u32(smem + s * STAGE)) : smem_desc_sw64(smem_u32(smem + s * STAGE));
+    constexpr uint32_t idesc = tc_idesc(EX_BM, EX_BN);
+    for (int kt = 0; kt < ktiles; kt++) {
+      // drain step dt = kt / EX_DRAIN covers EX_DRAIN stages (one exponent block)
+      const int s = kt % EX_STAGES, round = kt / EX_STAGES, dt = kt / EX_DRAIN, b = dt & 1, use = dt >> 1;
+      const bool opening = kt % EX_DRAIN == 0, closing = kt % EX_DRAIN == EX_DRAIN - 1;
+      if (opening && dt >= 2 && !mbar_wait_warp(&acce[b], (use - 1) & 1, err)) break;
+      if (!mbar_wait_warp(&full[s], round & 1, err)) break;
+      asm volatile("tcgen05.fence::after_thread_sync;");
+      // descriptors: one per stage, the tiles and K steps as compile-time
+      // offsets added to its address field (which never carries: smem < 256 KB)
+      const uint64_t dbase =
+          EX_BK == 64 ? smem_desc_sw128(smem_u32(smem + s * STAGE)) : smem_desc_sw64(smem_u32(smem + s * STAGE));
+      if (elect_one()) {
 #pragma unroll
         for (int ks = 0; ks < EX_BK / 16; ks++) {
 #pragma unroll
@@ -208,15 +211,17 @@ __global__ void __launch_bounds__(EX_THREADS, 1)
         tc_commit(&empty[s]);
         if (closing) tc_commit(&accf[b]);
       }
-      tc_commit(fin);
-      mbar_wait(fin, 0, err);
+      __syncwarp();
     }
+    if (elect_one()) tc_commit(fin);
+    __syncwarp();
+    mbar_wait_warp(fin, 0, err);
   } else {
     const int quarter = warp & 3, group = (warp - 2) >> 2;
     const uint32_t lane_base = tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(group * 32);
-    float hi[32], lo[32];
+    uint64_t hi[16], lo[16];  // column pairs
 #pragma unroll
-    for (int j = 0; j < 32; j++) hi[j] = lo[j] = 0.f;
+    for (int j = 0; j < 16; j++) hi[j] = lo[j] = 0;
     bool ok = true;
 #pragma unroll 1
     for (int dt = 0; dt < ktiles / EX_DRAIN; dt++) {
@@ -241,10 +246,11 @@ __global__ void __launch_bounds__(EX_THREADS, 1)
         }
         tc_wait_ld();
 #pragma unroll
-        for (int j = 0; j < 16; j++) {
-          two_sum_acc(hi[16 * h + j], lo[16 * h + j], __uint_as_float(x[j]));
-          two_sum_acc(hi[16 * h + j], lo[16 * h + j], __uint_as_float(y1[j]));
-          lo[16 * h + j] += __uint_as_float(y2[j]);
+        for (int j = 0; j < 16; j += 2) {
+          uint64_t &H = hi[8 * h + j / 2], &L = lo[8 * h + j / 2];
+          f2_two_sum_acc(H, L, f2_pack(x[j], x[j + 1]));
+          f2_two_sum_acc(H, L, f2_pack(y1[j], y1[j + 1]));
+          L = f2_add(L, f2_pack(y2[j], y2[j + 1]));
         }
       }
       asm volatile("tcgen05.fence::before_thread_sync;");
@@ -270,13 +276,17 @@ __global__ void __launch_bounds__(EX_THREADS, 1)
       }
       if (ok && rho < mvalid) {
 #pragma unroll
-        for (int j = 0; j < 8; j++) {
-          const int c = n0 + group * 32 + 8 * q + j;
-          if (c < nvalid) {
-            double *p = C + rho + ldcf * (int64_t)c;
-            const double v =
-                scale * (((double)hi[8 * q + j] + (double)lo[8 * q + j]) + ((double)z3[j] + (double)z4[j]));
-            *p = accumulate ? *p + v : v;
+        for (int j = 0; j < 8; j += 2) {
+          double v[2];
+          f2_sum(hi[4 * q + j / 2], lo[4 * q + j / 2], v[0], v[1]);
+#pragma unroll
+          for (int e = 0; e < 2; e++) {
+            const int c = n0 + group * 32 + 8 * q + j + e;
+            if (c < nvalid) {
+              double *p = C + rho + ldcf * (int64_t)c;
+              const double w = scale * (v[e] + ((double)z3[j + e] + (double)z4[j + e]));
+              *p = accumulate ? *p + w : w;
+            }
           }
         }
       }
@@ -290,74 +300,87 @@ __global__ void __launch_bounds__(EX_THREADS, 1)
   }
 }
 
-// ---------------- wide tiles: 128 x 128 of D' ----------------
+// ---------------- wide tiles: 128 x 128 or 128 x 96 of D' ----------------
 //
-// The same exact product with N = 128 MMAs (the tensor rate of M = 128, N =
-// 128 against two thirds of it for N = 64).  TMEM holds 4 x 128 columns: the
-// exact levels below ZLEV once each (not double-buffered: 768 columns would
-// not fit) and one FP32 buffer summing the levels from ZLEV up over the whole
-// K.  ZLEV = 3 keeps levels 0..2 exact as ex_gemm_kernel does (the quantized
-// 5 x 2 and 5 x 3 products, whose truncation is 2^-40); ZLEV = 2 for the
-// plain 4 x 4 and 3 x 3 products, whose truncation (2^-32, 2^-24 of the
-// block maxima products) is far above the 2^-40 an FP32 level 2 adds.  Per
-// 128-deep exponent block (4 TMA stages of 32-deep K steps, 64-byte rows)
-// the MMA thread issues each stage's FP32-summed products (levels ZLEV and up)
-// first; at a block's first stage it then waits, level by level, until the
-// epilogue has drained that exact level of the previous block (one mbarrier
-// per level), so the drain runs under the FP32-summed products and the MMAs
-// into levels already drained.  The host takes these tiles for grids of 4
-// waves or more (a smaller grid loses more in its last wave than it gains).
-// Sixteen epilogue warps (a TMEM lane quarter and 32 columns each) drain the
-// exact levels one after the other into their two-float (hi, lo) sums in the
-// same order per entry as ex_gemm_kernel (TwoSum X0, TwoSum X1, lo += X2).
-// Every wait is bounded.
-constexpr int EXW_BN = 128;
+// The same exact product with wider MMAs (N = 128 takes 64 cycles and N = 96 56;
+// N = 64, bound by the reads of A from shared memory, 48).  TMEM holds the exact
+// levels below ZLEV once each (double-buffered they would not fit) and FP32 sums of
+// the levels from ZLEV up over the whole K: one for all of them with 128 columns,
+// one a level with 96 (5 x 96 columns).  ZLEV = 3 keeps levels 0..2 exact as
+// ex_gemm_kernel does; ZLEV = 2 for the plain 4 x 4 product, whose truncation
+// (2^-32 of the block maxima products) is far above the 2^-40 an FP32 level 2
+// adds.  The plain 5 x 5 product has 96 columns: a common sum of levels 3 and 4 is
+// truncated at each product where the one of level 3 is mostly exact, which
+// doubled its error (rms 8.6e-13 -> 1.8e-12 of the largest entry at k = 3001).
+//
+// What bounds it beside the MMAs is that a level is not written again before the
+// epilogue has drained it (without the drain the products run at 0.8 of the
+// tensor peak, without the copies as with them).  A 128-deep exponent block is
+// four TMA stages of 32-deep K steps (64-byte rows).  Its last stage takes the
+// exact levels first, each handed over by itself, and then the FP32-summed
+// products; its first stage takes the FP32-summed products first, and each level
+// then waits until the epilogue has drained it (one mbarrier per level): the
+// drain runs under two stages' FP32-summed products and the MMAs into levels
+// already drained.  Sixteen epilogue warps (a TMEM lane quarter and 32 columns
+// each) drain the levels one after the other into their two-float (hi, lo) sums,
+// two columns an instruction, in the same order per entry as ex_gemm_kernel
+// (TwoSum X0, TwoSum X1, lo += X2); one of them polls for all, because every
+// polling warp slows the MMA warp's waits.  The level loop stays rolled: unrolled,
+// its registers spill.  Every wait is bounded.
+//
+// n = 3840 (8 n^3 flops a slice product): 5 x 5 4.39 ms (1.55 PF/s of slice products; 6.63
+// in 128 x 64 tiles before), 5 x 3 3.47 ms (1.57 PF/s; 4.13), 4 x 4 3.08 ms (1.47; 3.59).
+constexpr int EXW_BN = 128;  // the widest; B is padded to it
 constexpr int EXW_BK = 32;
 constexpr int EXW_DRAIN = 128 / EXW_BK;  // TMA stages per exponent block
 constexpr int EXW_EPI_WARPS = 16;
 constexpr int EXW_THREADS = 64 + 32 * EXW_EPI_WARPS;
-constexpr int EXW_TMEM_COLS = 512;  // three exact-level buffers and the FP32 sum, 128 columns each
-constexpr int EXW_ZCOL = 3 * EXW_BN;
+constexpr int EXW_TMEM_COLS = 512;
 
-template <int SA, int SB>
+template <int SA, int SB, int ZLEV, int BN>
 struct ExWCfg {
-  static constexpr int TILE = EX_BM * EXW_BK * 2;  // one slice tile, A or B (128 rows)
-  static constexpr int STAGE = (SA + SB) * TILE;
+  static constexpr int A_TILE = EX_BM * EXW_BK * 2, B_TILE = BN * EXW_BK * 2;  // one slice
+  static constexpr int STAGE = SA * A_TILE + SB * B_TILE;
   static constexpr int STAGES = (EX_SMEM_MAX - 1280) / STAGE < 4 ? (EX_SMEM_MAX - 1280) / STAGE : 4;
   static constexpr int SMEM = STAGES * STAGE + 1024 + 256;
-  static_assert(STAGES >= 3 && SMEM <= EX_SMEM_MAX, "exact gemm (wide tiles): shared memory");
+  static constexpr int SUMS = SB == 5 ? SA : ZLEV + 1;  // accumulators: one a level, or a common last one
+  static_assert(STAGES >= 3 && SMEM <= EX_SMEM_MAX && SUMS * BN <= EXW_TMEM_COLS && BN % 32 == 0,
+                "exact gemm (wide tiles): shared memory, TMEM");
 };
-template <int SA, int SB>
-__host__ __device__ constexpr int exw_smem_bytes() { return ExWCfg<SA, SB>::SMEM; }
+// Columns of the built (SA, SB) kernels, on the host.
+inline int exw_bn(int SA, int SB) { return SA == 5 && SB == 5 ? 96 : 128; }
 
-template <int SA, int SB, int ZLEV>
+template <int SA, int SB, int ZLEV, int BN>
 __global__ void __launch_bounds__(EXW_THREADS, 1)
     ex_gemm_wide_kernel(const __grid_constant__ ExMaps maps, int ktiles, double *__restrict__ C, int64_t ldcf,
                         int mvalid, int nvalid, int accumulate, const int *__restrict__ shifts, int raster, int *err) {
-  typedef ExWCfg<SA, SB> CF;
-  constexpr int STAGE = CF::STAGE, NST = CF::STAGES, TILE = CF::TILE;
+  typedef ExWCfg<SA, SB, ZLEV, BN> CF;
+  constexpr int STAGE = CF::STAGE, NST = CF::STAGES, A_TILE = CF::A_TILE, B_TILE = CF::B_TILE;
+  constexpr int SUMS = CF::SUMS, CW = BN / 4;  // accumulators, columns of an epilogue warp
   static_assert(ZLEV >= 2 && ZLEV <= 3 && SA > ZLEV, "wide tiles need FP32-summed levels to hide the drain under");
   extern __shared__ unsigned char ex_smem_raw[];
   unsigned char *smem = reinterpret_cast<unsigned char *>((reinterpret_cast<uintptr_t>(ex_smem_raw) + 1023) &
                                                           ~(uintptr_t)1023);
   uint64_t *full = reinterpret_cast<uint64_t *>(smem + NST * STAGE);
   uint64_t *empty = full + NST;
-  uint64_t *accf = empty + NST;  // a block's levels 0..2 written (MMA -> epilogue)
-  uint64_t *accx = accf + 1;     // level L of the last block drained (epilogue -> MMA), L = 0, 1, 2
+  uint64_t *accf = empty + NST;  // a block's level L written (MMA -> epilogue), L = 0, 1, 2
+  uint64_t *accx = accf + 3;     // level L of the last block drained (epilogue -> MMA), L = 0, 1, 2
   uint64_t *fin = accx + 3;      // all MMAs of this CTA complete
   uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(fin + 1);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_uniform((int)(threadIdx.x >> 5)), lane = threadIdx.x & 31;
   int mt, nt;
   grouped_tile(raster, mt, nt);
-  const int m0 = mt * EX_BM, n0 = nt * EXW_BN;
+  const int m0 = mt * EX_BM, n0 = nt * BN;
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < NST; s++) {
       mbar_init(&full[s], 1);
       mbar_init(&empty[s], 1);
     }
-    mbar_init(accf, 1);
-    for (int l = 0; l < 3; l++) mbar_init(&accx[l], EXW_EPI_WARPS);
+    for (int l = 0; l < 3; l++) {
+      mbar_init(&accf[l], 1);
+      mbar_init(&accx[l], EXW_EPI_WARPS);
+    }
     mbar_init(fin, 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
@@ -369,7 +392,7 @@ __global__ void __launch_bounds__(EXW_THREADS, 1)
   }
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;");
-  const uint32_t tmem = *tmem_slot;
+  const uint32_t tmem = warp_uniform(*tmem_slot);
 
   if (warp == 0) {
     if (elect_one()) {
@@ -380,9 +403,10 @@ __global__ void __launch_bounds__(EXW_THREADS, 1)
         mbar_expect_tx(&full[s], STAGE);
         unsigned char *st = smem + s * STAGE;
 #pragma unroll
-        for (int a = 0; a < SA; a++) tma_load_2d(st + a * TILE, &maps.a[a], kt * EXW_BK, m0, &full[s]);
+        for (int a = 0; a < SA; a++) tma_load_2d(st + a * A_TILE, &maps.a[a], kt * EXW_BK, m0, &full[s]);
 #pragma unroll
-        for (int b = 0; b < SB; b++) tma_load_2d(st + (SA + b) * TILE, &maps.b[b], kt * EXW_BK, n0, &full[s]);
+        for (int b = 0; b < SB; b++) 
+          tma_load_2d(st + SA * A_TILE + b * B_TILE, &maps.b[b], kt * EXW_BK, n0, &full[s]);
         issued = kt + 1;
       }
       // copies still in flight after an early stop land before the CTA exits
@@ -390,88 +414,115 @@ __global__ void __launch_bounds__(EXW_THREADS, 1)
         if (!mbar_wait(&full[kt % NST], (kt / NST) & 1, err)) break;
     }
   } else if (warp == 1) {
-    if (elect_one()) {
-      constexpr uint32_t idesc = tc_idesc(EX_BM, EXW_BN);
-      bool ok = true, zfirst = true;
-      for (int kt = 0; kt < ktiles && ok; kt++) {
-        const int s = kt % NST, round = kt / NST, dt = kt / EXW_DRAIN, q = kt % EXW_DRAIN;
-        if (!mbar_wait(&full[s], round & 1, err)) break;
-        asm volatile("tcgen05.fence::after_thread_sync;");
-        const uint64_t dbase = smem_desc_sw64(smem_u32(smem + s * STAGE));
-        // levels >= 3: one FP32 sum over the whole K
+    constexpr uint32_t idesc = tc_idesc(EX_BM, BN);
+    bool ok = true;
+    for (int kt = 0; kt < ktiles && ok; kt++) {
+      const int s = kt % NST, round = kt / NST, dt = kt / EXW_DRAIN, q = kt % EXW_DRAIN;
+      ok = mbar_wait_warp(&full[s], round & 1, err);
+      if (!ok) break;
+      asm volatile("tcgen05.fence::after_thread_sync;");
+      const uint64_t dbase = smem_desc_sw64(smem_u32(smem + s * STAGE));
+      // the products (a, b) of the levels [l0, l1) into one accumulator
+      auto products = [&](int l0, int l1, bool first) {
+        const uint32_t col = (uint32_t)(l0 * BN);
+        bool fresh = first;
 #pragma unroll
         for (int ks = 0; ks < EXW_BK / 16; ks++)
 #pragma unroll
           for (int a = 0; a < SA; a++)
 #pragma unroll
             for (int b = 0; b < SB; b++) {
-              if (a + b < ZLEV || a + b >= SA) continue;
-              const uint64_t da = dbase + (uint64_t)((a * TILE + ks * 32) >> 4);
-              const uint64_t db = dbase + (uint64_t)(((SA + b) * TILE + ks * 32) >> 4);
-              tc_mma(tmem + (uint32_t)EXW_ZCOL, da, db, idesc, zfirst ? 0u : 1u);
-              zfirst = false;
+              if (a + b < l0 || a + b >= l1) continue;
+              tc_mma(tmem + col, dbase + (uint64_t)((a * A_TILE + ks * 32) >> 4),
+                     dbase + (uint64_t)((SA * A_TILE + b * B_TILE + ks * 32) >> 4), idesc, fresh ? 0u : 1u);
+              fresh = false;
             }
-        // levels 0..2: exact per block; at its first stage a level waits until
-        // the epilogue has drained it
+      };
+      // the FP32-summed levels; with ZLEV = 2 their one sum is the accumulator of level 2
+      auto summed = [&](bool first) {
+        if (SUMS == SA) {
+#pragma unroll
+          for (int l = ZLEV; l < SA; l++) products(l, l + 1, first);
+        } else {
+          products(ZLEV, SA, first);
+        }
+      };
+      if (q == EXW_DRAIN - 1) {
+        // a block's last stage: each level complete as early as can be
+        if (elect_one()) {
+#pragma unroll
+          for (int l = 0; l < ZLEV; l++) {
+            products(l, l + 1, false);
+            tc_commit(&accf[l]);
+          }
+          summed(false);
+          tc_commit(&empty[s]);
+        }
+      } else if (q == 0) {
+        if (elect_one()) summed(kt == 0);
+        __syncwarp();
+        // at a block's first stage a level waits until the epilogue has drained it
 #pragma unroll
         for (int l = 0; l < ZLEV; l++) {
-          if (q == 0 && dt >= 1) {
-            if (!mbar_wait(&accx[l], (dt - 1) & 1, err)) {
-              ok = false;
-              break;
-            }
+          if (dt >= 1) {
+            ok = ok && mbar_wait_warp(&accx[l], (dt - 1) & 1, err);
+            if (!ok) break;
             asm volatile("tcgen05.fence::after_thread_sync;");
           }
-          const int amin = l - (SB - 1) > 0 ? l - (SB - 1) : 0;
-#pragma unroll
-          for (int ks = 0; ks < EXW_BK / 16; ks++)
-#pragma unroll
-            for (int a = 0; a < SA; a++) {
-              const int b = l - a;
-              if (a > l || b >= SB) continue;
-              const uint64_t da = dbase + (uint64_t)((a * TILE + ks * 32) >> 4);
-              const uint64_t db = dbase + (uint64_t)(((SA + b) * TILE + ks * 32) >> 4);
-              const bool first = q == 0 && ks == 0 && a == amin;
-              tc_mma(tmem + (uint32_t)(l * EXW_BN), da, db, idesc, first ? 0u : 1u);
-            }
+          if (elect_one()) products(l, l + 1, true);
+          __syncwarp();
         }
         if (!ok) break;
-        tc_commit(&empty[s]);
-        if (q == EXW_DRAIN - 1) tc_commit(accf);
-      }
-      tc_commit(fin);
-      mbar_wait(fin, 0, err);
-    }
-  } else {
-    const int quarter = warp & 3, group = (warp - 2) >> 2;  // TMEM lanes 32 quarter.., columns 32 group..
-    const uint32_t lane_base = tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(group * 32);
-    float hi[32], lo[32];
+        if (elect_one()) tc_commit(&empty[s]);
+      } else {
+        if (elect_one()) {
+          summed(false);
 #pragma unroll
-    for (int j = 0; j < 32; j++) hi[j] = lo[j] = 0.f;
+          for (int l = 0; l < ZLEV; l++) products(l, l + 1, false);
+          tc_commit(&empty[s]);
+        }
+      }
+      __syncwarp();
+    }
+    if (elect_one()) tc_commit(fin);
+    __syncwarp();
+    mbar_wait_warp(fin, 0, err);
+  } else {
+    // warp 2 polls for all sixteen
+    auto epi_wait = [&](uint64_t *bar, unsigned par) {
+      uint32_t got = 1;
+      if (warp == 2) got = warp_uniform(lane == 0 ? (uint32_t)mbar_wait(bar, par, err) : 0u);
+      asm volatile("{\n .reg .pred p, q;\n setp.ne.u32 q, %0, 0;\n bar.red.and.pred p, 1, %1, q;\n selp.u32 %0, 1, 0, p;\n}\n"
+                   : "+r"(got)
+                   : "n"(32 * EXW_EPI_WARPS)
+                   : "memory");
+      return got != 0;
+    };
+    const int quarter = warp & 3, group = (warp - 2) >> 2;  // TMEM lanes 32 quarter.., columns CW group..
+    const uint32_t lane_base = tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(group * CW);
+    uint64_t hi[CW / 2], lo[CW / 2];  // column pairs
+#pragma unroll
+    for (int j = 0; j < CW / 2; j++) hi[j] = lo[j] = 0;
     bool ok = true;
 #pragma unroll 1
-    for (int dt = 0; dt < ktiles / EXW_DRAIN; dt++) {
-      int got = 1;
-      if (lane == 0) got = mbar_wait(accf, dt & 1, err) ? 1 : 0;
-      got = __shfl_sync(0xffffffffu, got, 0);
-      if (!got) {
-        ok = false;
-        break;
-      }
-      asm volatile("tcgen05.fence::after_thread_sync;");
-#pragma unroll
+    for (int dt = 0; dt < ktiles / EXW_DRAIN && ok; dt++) {
+#pragma unroll(ZLEV == 3 ? 1 : 2)
       for (int l = 0; l < ZLEV; l++) {
+        ok = epi_wait(&accf[l], dt & 1);
+        if (!ok) break;
+        asm volatile("tcgen05.fence::after_thread_sync;");
 #pragma unroll
-        for (int c = 0; c < 4; c++) {  // 8 columns per load batch
+        for (int c = 0; c < CW / 8; c++) {  // 8 columns per load batch
           uint32_t v[8];
-          tc_ld8_nowait(lane_base + (uint32_t)(l * EXW_BN + 8 * c), v);
-          tc_wait_ld();
+          tc_ld8_nowait(lane_base + (uint32_t)(l * BN + 8 * c), v);
+          tc_wait_ld8(v);
 #pragma unroll
-          for (int j = 0; j < 8; j++) {
+          for (int j = 0; j < 4; j++) {
+            const uint64_t p = f2_pack(v[2 * j], v[2 * j + 1]);
             if (l < 2)
-              two_sum_acc(hi[8 * c + j], lo[8 * c + j], __uint_as_float(v[j]));
+              f2_two_sum_acc(hi[4 * c + j], lo[4 * c + j], p);
             else
-              lo[8 * c + j] += __uint_as_float(v[j]);
+              lo[4 * c + j] = f2_add(lo[4 * c + j], p);
           }
         }
         asm volatile("tcgen05.fence::before_thread_sync;");
@@ -479,28 +530,32 @@ __global__ void __launch_bounds__(EXW_THREADS, 1)
         if (lane == 0) mbar_arrive(&accx[l]);
       }
     }
-    if (ok) {
-      int got = 1;
-      if (lane == 0) got = mbar_wait(fin, 0, err) ? 1 : 0;
-      ok = __shfl_sync(0xffffffffu, got, 0) != 0;
-    }
+    if (ok) ok = epi_wait(fin, 0);
     const int rho = m0 + quarter * 32 + lane;
     const double scale = ldexp(1.0, -(shifts[0] + shifts[1]));
     if (ok) asm volatile("tcgen05.fence::after_thread_sync;");
 #pragma unroll
-    for (int c = 0; c < 4; c++) {
-      float z[8];
+    for (int c = 0; c < CW / 8; c++) {
+      float z[8], z4[8];
 #pragma unroll
-      for (int j = 0; j < 8; j++) z[j] = 0.f;
-      if (ok) tc_ld8(lane_base + (uint32_t)(EXW_ZCOL + 8 * c), z);
+      for (int j = 0; j < 8; j++) z[j] = z4[j] = 0.f;
+      if (ok) {
+        tc_ld8(lane_base + (uint32_t)(ZLEV * BN + 8 * c), z);
+        if (SUMS > ZLEV + 1) tc_ld8(lane_base + (uint32_t)((ZLEV + 1) * BN + 8 * c), z4);
+      }
       if (ok && rho < mvalid) {
 #pragma unroll
-        for (int j = 0; j < 8; j++) {
-          const int col = n0 + group * 32 + 8 * c + j;
-          if (col < nvalid) {
-            double *p = C + rho + ldcf * (int64_t)col;
-            const double v = scale * (((double)hi[8 * c + j] + (double)lo[8 * c + j]) + (double)z[j]);
-            *p = accumulate ? *p + v : v;
+        for (int j = 0; j < 8; j += 2) {
+          double v[2];
+          f2_sum(hi[4 * c + j / 2], lo[4 * c + j / 2], v[0], v[1]);
+#pragma unroll
+          for (int e = 0; e < 2; e++) {
+            const int col = n0 + group * CW + 8 * c + j + e;
+            if (col < nvalid) {
+              double *p = C + rho + ldcf * (int64_t)col;
+              const double w = scale * (v[e] + ((double)z[j + e] + (double)z4[j + e]));
+              *p = accumulate ? *p + w : w;
+            }
           }
         }
       }
@@ -755,15 +810,21 @@ int bem_exact_gemm(bemgpu_ctx_s *ctx, int kind, const ExactOperand &a, const Exa
   if (!((SA == SB && SA >= 3 && SA <= 5) || (SA == 5 && (SB == 3 || SB == 2))))
     return bem_fail(ctx, BEMGPU_ERR_ARG, "exact gemm: slices (%d, %d) not built", SA, SB);
   const int SL = SB;
-  // 128 x 128 tiles where level-3/4 products hide the single-buffered drain,
-  // for grids of at least 4 waves (a smaller grid leaves more of its last
-  // wave's SMs idle with half as many tiles; ex_gemm_wide_kernel<5, 2> at
-  // 240 tiles took 342 us against 312 for 450 narrow ones); BEMGPU_TUNE_EX_WIDE
-  // 2 takes them whatever the grid
-  const int64_t wtiles = (a.rows_p / EX_BM) * ((b.rows_p + EXW_BN - 1) / EXW_BN);
-  const bool wide = ((SA == 5 && (SB == 2 || SB == 3)) || (SA == SB && (SA == 4 || SA == 3))) &&
-                    (ctx->tune.ex_wide == 2 || (ctx->tune.ex_wide == 1 && wtiles >= 4 * (int64_t)ctx->num_sms));
-  const int bn = wide ? EXW_BN : EX_BN;
+  // Wide tiles.  Plain 5 x 5 (128 x 96, the same sums as 128 x 64): where they take less
+  // time by their waves, a wide tile taking 1.2 times a narrow one (n = 7680: 33.8 ms
+  // against 41.5; n = 1440, 3 waves against 4: 379 us against 410).  The others
+  // (128 x 128, a common FP32 sum of their upper levels, truncated at each product):
+  // on grids of 4 waves or more; smaller products are faster too (n = 1440: 272 us
+  // against 337) but keep their separate sums.  Not 3 x 3, whose few FP32-summed
+  // products do not hide the drain (n = 7680: 18.6 ms against 18.2).
+  // BEMGPU_TUNE_EX_WIDE 2 takes them whatever the grid.
+  const int wbn = exw_bn(SA, SB);
+  const int64_t mtiles = a.rows_p / EX_BM, wtiles = mtiles * ((b.rows + wbn - 1) / wbn);
+  auto waves = [&](int64_t tiles) { return (tiles + ctx->num_sms - 1) / ctx->num_sms; };
+  const bool faster = SB == 5 ? 6 * waves(wtiles) <= 5 * waves(mtiles * ((b.rows + EX_BN - 1) / EX_BN))
+                              : wtiles >= 4 * (int64_t)ctx->num_sms;
+  const bool wide = SA >= 4 && (ctx->tune.ex_wide == 2 || (ctx->tune.ex_wide == 1 && faster));
+  const int bn = wide ? wbn : EX_BN;
   ExMaps maps;
   const int bk = wide ? EXW_BK : ex_bk(SA, SB);
   if (!ex_maps(maps.a, (const __nv_bfloat16 *)a.S, SA, a.rows_p, a.kp, EX_BM, bk) ||
@@ -782,14 +843,14 @@ int bem_exact_gemm(bemgpu_ctx_s *ctx, int kind, const ExactOperand &a, const Exa
                                            ex_smem_bytes<5, 3>()));
     BEM_CUDA_TRY(ctx, cudaFuncSetAttribute(ex_gemm_kernel<5, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                            ex_smem_bytes<5, 2>()));
-    BEM_CUDA_TRY(ctx, cudaFuncSetAttribute(ex_gemm_wide_kernel<5, 2, 3>,
-                                           cudaFuncAttributeMaxDynamicSharedMemorySize, exw_smem_bytes<5, 2>()));
-    BEM_CUDA_TRY(ctx, cudaFuncSetAttribute(ex_gemm_wide_kernel<5, 3, 3>,
-                                           cudaFuncAttributeMaxDynamicSharedMemorySize, exw_smem_bytes<5, 3>()));
-    BEM_CUDA_TRY(ctx, cudaFuncSetAttribute(ex_gemm_wide_kernel<4, 4, 2>,
-                                           cudaFuncAttributeMaxDynamicSharedMemorySize, exw_smem_bytes<4, 4>()));
-    BEM_CUDA_TRY(ctx, cudaFuncSetAttribute(ex_gemm_wide_kernel<3, 3, 2>,
-                                           cudaFuncAttributeMaxDynamicSharedMemorySize, exw_smem_bytes<3, 3>()));
+    BEM_CUDA_TRY(ctx, cudaFuncSetAttribute(ex_gemm_wide_kernel<5, 2, 3, 128>,
+                                           cudaFuncAttributeMaxDynamicSharedMemorySize, ExWCfg<5, 2, 3, 128>::SMEM));
+    BEM_CUDA_TRY(ctx, cudaFuncSetAttribute(ex_gemm_wide_kernel<5, 3, 3, 128>,
+                                           cudaFuncAttributeMaxDynamicSharedMemorySize, ExWCfg<5, 3, 3, 128>::SMEM));
+    BEM_CUDA_TRY(ctx, cudaFuncSetAttribute(ex_gemm_wide_kernel<4, 4, 2, 128>,
+                                           cudaFuncAttributeMaxDynamicSharedMemorySize, ExWCfg<4, 4, 2, 128>::SMEM));
+    BEM_CUDA_TRY(ctx, cudaFuncSetAttribute(ex_gemm_wide_kernel<5, 5, 3, 96>,
+                                           cudaFuncAttributeMaxDynamicSharedMemorySize, ExWCfg<5, 5, 3, 96>::SMEM));
     ctx->ex_ready = true;
   }
   if (!ctx->tc_err_ready) {
@@ -802,7 +863,7 @@ int bem_exact_gemm(bemgpu_ctx_s *ctx, int kind, const ExactOperand &a, const Exa
   BEM_CUDA_TRY(ctx, cudaMemcpyAsync(shifts, a.aux, sizeof(int), cudaMemcpyDeviceToDevice, st));
   BEM_CUDA_TRY(ctx, cudaMemcpyAsync(shifts + 1, b.aux, sizeof(int), cudaMemcpyDeviceToDevice, st));
   ProfScope ps(ctx, kind, st, 8.0 * m * (double)n * a.k,
-               2.0 * SA * ((double)a.rows_p * a.kp * ((b.rows_p + bn - 1) / bn) / 8.0) +
+               2.0 * SA * ((double)a.rows_p * a.kp * ((b.rows + bn - 1) / bn) / 8.0) +
                    2.0 * SB * (double)b.rows_p * b.kp + 16.0 * m * (double)n * (accumulate ? 2 : 1));
   (void)SL;
   {
@@ -812,19 +873,19 @@ int bem_exact_gemm(bemgpu_ctx_s *ctx, int kind, const ExactOperand &a, const Exa
       for (int j = 0; j < SB; j++) products += (i + j < SA);
     ps.tensor = products * ps.flops;
   }
-  const dim3 grid((unsigned)(a.rows_p / EX_BM), (unsigned)(b.rows_p / bn));
+  const dim3 grid((unsigned)(a.rows_p / EX_BM), (unsigned)((b.rows + bn - 1) / bn));
   const int ktiles = (int)(a.kp / bk);
   if (wide && SA == 5 && SB == 2)
-    ex_gemm_wide_kernel<5, 2, 3><<<grid, EXW_THREADS, exw_smem_bytes<5, 2>(), st>>>(
+    ex_gemm_wide_kernel<5, 2, 3, 128><<<grid, EXW_THREADS, ExWCfg<5, 2, 3, 128>::SMEM, st>>>(
         maps, ktiles, C, 2 * ldc, 2 * m, n, accumulate, shifts, ctx->tune.raster, err);
   else if (wide && SA == 5 && SB == 3)
-    ex_gemm_wide_kernel<5, 3, 3><<<grid, EXW_THREADS, exw_smem_bytes<5, 3>(), st>>>(
+    ex_gemm_wide_kernel<5, 3, 3, 128><<<grid, EXW_THREADS, ExWCfg<5, 3, 3, 128>::SMEM, st>>>(
+        maps, ktiles, C, 2 * ldc, 2 * m, n, accumulate, shifts, ctx->tune.raster, err);
+  else if (wide && SA == 5)
+    ex_gemm_wide_kernel<5, 5, 3, 96><<<grid, EXW_THREADS, ExWCfg<5, 5, 3, 96>::SMEM, st>>>(
         maps, ktiles, C, 2 * ldc, 2 * m, n, accumulate, shifts, ctx->tune.raster, err);
   else if (wide && SA == 4)
-    ex_gemm_wide_kernel<4, 4, 2><<<grid, EXW_THREADS, exw_smem_bytes<4, 4>(), st>>>(
-        maps, ktiles, C, 2 * ldc, 2 * m, n, accumulate, shifts, ctx->tune.raster, err);
-  else if (wide)
-    ex_gemm_wide_kernel<3, 3, 2><<<grid, EXW_THREADS, exw_smem_bytes<3, 3>(), st>>>(
+    ex_gemm_wide_kernel<4, 4, 2, 128><<<grid, EXW_THREADS, ExWCfg<4, 4, 2, 128>::SMEM, st>>>(
         maps, ktiles, C, 2 * ldc, 2 * m, n, accumulate, shifts, ctx->tune.raster, err);
   else if (SA == 5 && SB == 2)
     ex_gemm_kernel<5, 2><<<grid, EX_THREADS, ex_smem_bytes<5, 2>(), st>>>(maps, ktiles, C, 2 * ldc, 2 * m, n,

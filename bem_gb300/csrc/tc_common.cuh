@@ -16,9 +16,12 @@ __device__ __forceinline__ uint32_t smem_u32(const void *p) {
   return static_cast<uint32_t>(__cvta_generic_to_shared(p));
 }
 
-// One lane of a converged warp.  The branches that issue tcgen05.mma and TMA
-// copies are entered through elect.sync: the compiler then knows that a single
-// lane runs them and keeps descriptors and addresses in uniform registers.
+// One lane of a converged warp, for the branches that issue tcgen05.mma and TMA copies:
+// the compiler knows that a single lane runs them and can keep descriptors and
+// addresses in uniform registers.  Issued from an "if (lane == 0)" branch an MMA took 70
+// cycles, whatever its width, and more than 100 beside a busy epilogue; N = 128
+// needs 64.  Where the epilogue is busy (gemm_exact.cu) the MMA warp runs its loop
+// as a whole, on warp-uniform values, and only the issue itself is entered here.
 __device__ __forceinline__ bool elect_one() {
   uint32_t p;
   asm volatile("{\n .reg .pred P;\n elect.sync _|P, 0xffffffff;\n selp.u32 %0, 1, 0, P;\n}\n" : "=r"(p));
@@ -47,6 +50,16 @@ __device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity, int *e
   }
   atomicExch(err, 1);
   return false;
+}
+
+// The whole warp waits; the result is uniform.
+__device__ __forceinline__ bool mbar_wait_warp(uint64_t *bar, uint32_t parity, int *err) {
+  return __all_sync(0xffffffffu, mbar_wait(bar, parity, err)) != 0;
+}
+
+template <typename T>
+__device__ __forceinline__ T warp_uniform(T v) {
+  return __shfl_sync(0xffffffffu, v, 0);
 }
 
 __device__ __forceinline__ void mbar_arrive(uint64_t *bar) {
@@ -116,6 +129,15 @@ __device__ __forceinline__ void tc_ld8_nowait(uint32_t taddr, uint32_t *r) {
 
 __device__ __forceinline__ void tc_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 
+// Waits for the warp's TMEM loads; a batch's registers pass through it, so that
+// nothing that uses them moves above.
+__device__ __forceinline__ void tc_wait_ld8(uint32_t *r) {
+  asm volatile("tcgen05.wait::ld.sync.aligned;"
+               : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]), "+r"(r[7])
+               :
+               : "memory");
+}
+
 __device__ __forceinline__ void tc_ld8(uint32_t taddr, float *v) {
   uint32_t r[8];
   asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
@@ -173,6 +195,40 @@ __device__ __forceinline__ void two_sum_acc(float &hi, float &lo, float p) {
   const float bp = s - hi;
   lo += (hi - (s - bp)) + (p - bp);
   hi = s;
+}
+
+// Pairs of FP32 values, one instruction for both.
+__device__ __forceinline__ uint64_t f2_add(uint64_t a, uint64_t b) {
+  uint64_t r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ uint64_t f2_sub(uint64_t a, uint64_t b) {
+  uint64_t r;
+  asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ uint64_t f2_pack(uint32_t a, uint32_t b) {
+  uint64_t r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "r"(a), "r"(b));
+  return r;
+}
+__device__ __forceinline__ void f2_unpack(uint64_t v, float &a, float &b) {
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v));
+}
+// two_sum_acc on both halves
+__device__ __forceinline__ void f2_two_sum_acc(uint64_t &hi, uint64_t &lo, uint64_t p) {
+  const uint64_t s = f2_add(hi, p), bp = f2_sub(s, hi);
+  lo = f2_add(lo, f2_add(f2_sub(hi, f2_sub(s, bp)), f2_sub(p, bp)));
+  hi = s;
+}
+// hi + lo of both halves in FP64
+__device__ __forceinline__ void f2_sum(uint64_t hi, uint64_t lo, double &a, double &b) {
+  float h0, h1, l0, l1;
+  f2_unpack(hi, h0, h1);
+  f2_unpack(lo, l0, l1);
+  a = (double)h0 + (double)l0;
+  b = (double)h1 + (double)l1;
 }
 
 typedef CUresult (*EncodeTiledFn)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *,
