@@ -869,10 +869,9 @@ __global__ void __launch_bounds__(CP_MAX_THREADS, 1)
   // Entry d of a column comes from where d leads back through the interchanges.
   const int nc = (k0 - p0) + (p1 - k0 - w);
   if (nc > 0) {
-    for (int k = tid; k < w * w; k += nt) {
-      const int r = k % w, c = k / w;
-      LU[r * ROW + c] = __ldcg(A2 + k0 + r + lda * (int64_t)(k0 + c));
-    }
+#pragma unroll 8
+    for (int c = wid; c < w; c += nwarps)
+      if (lane < w) LU[lane * ROW + c] = __ldcg(A2 + k0 + lane + lda * (int64_t)(k0 + c));
     __syncthreads();
     const int d1 = k0 + lane, d2 = lane < w ? s_piv[lane] : 0;
     const bool on1 = lane < w, on2 = lane < w && d2 >= k0 + w;
@@ -993,17 +992,31 @@ __global__ void __launch_bounds__(256) panel_update_kernel(int m, int n, int k, 
 // own triangle by substitution (a warp has NC / warps columns, lane = row), then
 // its product with the rows that remain.
 //
+// The block column's triangle and the rows under (over) it come by cp.async, all
+// of a thread's copies in flight at once; complex64 keeps two buffers, so the next
+// block's copies run under this one's work (complex128 would leave one CTA per SM
+// with two).  Loaded one after the other, with the row and column of each element
+// from a division, a launch took 57 us where it now takes 23 (complex64, w = 128), 34
+// and 45 where it takes 28 and 35 (complex128, w = 64, lower and upper): the 32
+// dependent steps of each block are what is left.
+//
 // Complex64 (NC = 32): the update is most of the work and runs from shared
-// memory at one load per 3.7 FMA; a warp that substituted all 128 rows of one
-// column by itself took 95 us at n = 7680 where this takes ~15.  Complex128
-// (NC = 4, a warp per scheduler): bound by the FP64 pipe, so the columns spread
-// over as many SMs as there are.
+// memory at one load per 3.7 FMA.  Complex128 (NC = 4, a warp per scheduler):
+// bound by the FP64 pipe, so the columns spread over as many SMs as there are.
 template <typename T>
 struct TriCfg;
 template <>
-struct TriCfg<float> { static constexpr int NC = 32, THREADS = 256; };
+struct TriCfg<float> { static constexpr int NC = 32, THREADS = 256, BUFS = 2; };
 template <>
-struct TriCfg<double> { static constexpr int NC = 4, THREADS = 128; };
+struct TriCfg<double> { static constexpr int NC = 4, THREADS = 128, BUFS = 1; };
+
+// One complex element to shared memory, or zero.
+template <typename T2>
+__device__ __forceinline__ void cp_async_elem(T2 *dst, const T2 *src, bool valid) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], %2, %3;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src),
+               "n"(sizeof(T2)), "r"(valid ? (int)sizeof(T2) : 0)
+               : "memory");
+}
 
 template <typename T, int W, bool UPPER>
 __global__ void __launch_bounds__(TriCfg<T>::THREADS) tri_block_kernel(const T *Ad, int64_t lda, int w, T *B, int64_t ldb,
@@ -1011,40 +1024,65 @@ __global__ void __launch_bounds__(TriCfg<T>::THREADS) tri_block_kernel(const T *
   typedef typename V2<T>::type T2;
   constexpr int NC = TriCfg<T>::NC, THREADS = TriCfg<T>::THREADS, WARPS = THREADS / 32, CPW = NC / WARPS;
   constexpr int RPP = THREADS / NC, PER = (W - 32) / RPP;  // rows per pass of the update, passes
+  constexpr int BUFS = TriCfg<T>::BUFS, XS = NC + 1;  // an odd row stride: a warp's lanes along the rows meet other banks
+  static_assert(THREADS % W == 0 && THREADS % 32 == 0, "a thread's copies keep one row");
   extern __shared__ __align__(16) unsigned char tri_raw[];
-  T2 *X = reinterpret_cast<T2 *>(tri_raw);  // [W][NC]
-  T2 *Ts = X + W * NC;                      // [W][33] the triangle's columns of one block
-  T2 *rd = Ts + W * 33;                     // [W] reciprocals of the diagonal (upper)
+  T2 *X = reinterpret_cast<T2 *>(tri_raw);  // [W][XS]
+  T2 *Tb = X + W * XS;                      // [BUFS][W][33] the triangle's columns of one block
+  T2 *rd = Tb + BUFS * W * 33;              // [W] reciprocals of the diagonal (upper)
   const T2 *A2 = reinterpret_cast<const T2 *>(Ad);
   T2 *B2 = reinterpret_cast<T2 *>(B);
   const T2 zero = V2<T>::make(0, 0);
   const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5, n0 = blockIdx.x * NC;
-  for (int k = tid; k < W * NC; k += THREADS) {
-    const int r = k % W, c = k / W;
-    X[r * NC + c] = r < w && n0 + c < ncols ? B2[r + ldb * (int64_t)(n0 + c)] : zero;
+  const int nblk = (w + 31) / 32;
+  const int row = tid % W;  // of this thread's copies
+  auto load_block = [&](int q) {
+    const int b = UPPER ? nblk - 1 - q : q, o = b * 32;
+    if (row >= (UPPER ? 0 : o) && row < (UPPER ? min(w, o + 32) : w)) {
+      const T2 *src = A2 + row + lda * (int64_t)o;
+      T2 *dst = Tb + (q % BUFS) * (W * 33) + row * 33;
+#pragma unroll
+      for (int c0 = 0; c0 < 32; c0 += THREADS / W) {
+        const int c = c0 + tid / W;
+        const bool in = o + c < w;
+        cp_async_elem(dst + c, in ? src + lda * (int64_t)c : src, in);
+      }
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+#pragma unroll
+  for (int c0 = 0; c0 < NC; c0 += THREADS / W) {
+    const int c = c0 + tid / W;
+    const bool in = row < w && n0 + c < ncols;
+    cp_async_elem(X + row * XS + c, in ? B2 + row + ldb * (int64_t)(n0 + c) : B2, in);
   }
+  load_block(0);
   if (UPPER)
     for (int r = tid; r < W; r += THREADS) {
       cx<T> d = {1, 0};
       if (r < w) d = crecip(cld(Ad, r + lda * (int64_t)r));
       rd[r] = V2<T>::make(d.r, d.i);
     }
-  const int nblk = (w + 31) / 32;
 #pragma unroll 1
   for (int q = 0; q < nblk; q++) {
     const int b = UPPER ? nblk - 1 - q : q, o = b * 32;
-    const int r0 = UPPER ? 0 : o, r1 = UPPER ? min(w, o + 32) : w;  // the block column's rows
-    __syncthreads();  // the previous block's readers are done
-    for (int k = tid; k < (r1 - r0) * 32; k += THREADS) {
-      const int r = r0 + k % (r1 - r0), c = k / (r1 - r0);
-      Ts[r * 33 + c] = o + c < w ? A2[r + lda * (int64_t)(o + c)] : zero;
+    const T2 *Ts = Tb + (q % BUFS) * (W * 33);
+    if (q > 0) {
+      __syncthreads();  // the previous block's readers are done
+      if (BUFS == 1) load_block(q);
+    }
+    if (BUFS == 2 && q + 1 < nblk) {
+      load_block(q + 1);
+      asm volatile("cp.async.wait_group 1;" ::: "memory");
+    } else {
+      asm volatile("cp.async.wait_group 0;" ::: "memory");
     }
     __syncthreads();
     {
       const int row = o + lane;
       T2 x[CPW];
 #pragma unroll
-      for (int e = 0; e < CPW; e++) x[e] = row < W ? X[row * NC + wid * CPW + e] : zero;
+      for (int e = 0; e < CPW; e++) x[e] = row < W ? X[row * XS + wid * CPW + e] : zero;
       const int m = min(32, w - o);
       for (int i0 = 0; i0 < m; i0++) {
         const int i = UPPER ? m - 1 - i0 : i0;
@@ -1063,7 +1101,7 @@ __global__ void __launch_bounds__(TriCfg<T>::THREADS) tri_block_kernel(const T *
       }
 #pragma unroll
       for (int e = 0; e < CPW; e++)
-        if (row < W) X[row * NC + wid * CPW + e] = x[e];
+        if (row < W) X[row * XS + wid * CPW + e] = x[e];
     }
     __syncthreads();
     // the remaining rows: [o + 32, w) below, or [0, o) above
@@ -1074,11 +1112,11 @@ __global__ void __launch_bounds__(TriCfg<T>::THREADS) tri_block_kernel(const T *
 #pragma unroll
       for (int e = 0; e < PER; e++) {
         const int r = u0 + ry + RPP * e;
-        acc[e] = r < u1 ? X[r * NC + c] : zero;
+        acc[e] = r < u1 ? X[r * XS + c] : zero;
       }
 #pragma unroll 4
       for (int k = 0; k < 32; k++) {
-        const T2 x = o + k < W ? X[(o + k) * NC + c] : zero;
+        const T2 x = o + k < W ? X[(o + k) * XS + c] : zero;
 #pragma unroll
         for (int e = 0; e < PER; e++) {
           const int r = u0 + ry + RPP * e;
@@ -1092,14 +1130,15 @@ __global__ void __launch_bounds__(TriCfg<T>::THREADS) tri_block_kernel(const T *
 #pragma unroll
       for (int e = 0; e < PER; e++) {
         const int r = u0 + ry + RPP * e;
-        if (r < u1) X[r * NC + c] = acc[e];
+        if (r < u1) X[r * XS + c] = acc[e];
       }
     }
   }
   __syncthreads();
-  for (int k = tid; k < W * NC; k += THREADS) {
-    const int r = k % W, c = k / W;
-    if (r < w && n0 + c < ncols) B2[r + ldb * (int64_t)(n0 + c)] = X[r * NC + c];
+#pragma unroll
+  for (int c0 = 0; c0 < NC; c0 += THREADS / W) {
+    const int c = c0 + tid / W;
+    if (row < w && n0 + c < ncols) B2[row + ldb * (int64_t)(n0 + c)] = X[row * XS + c];
   }
 }
 
@@ -1241,7 +1280,7 @@ struct GemmCfg<float> {
 };
 
 template <typename T, int W>
-constexpr int tri_smem_bytes() { return (W * TriCfg<T>::NC + W * 33 + W) * (int)sizeof(typename V2<T>::type); }
+constexpr int tri_smem_bytes() { return (W * (TriCfg<T>::NC + 1) + TriCfg<T>::BUFS * W * 33 + W) * (int)sizeof(typename V2<T>::type); }
 
 template <typename T>
 int set_tri_attrs(bemgpu_ctx_s *ctx) {
