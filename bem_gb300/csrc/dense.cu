@@ -1143,29 +1143,62 @@ __global__ void __launch_bounds__(TriCfg<T>::THREADS) tri_block_kernel(const T *
 }
 
 // ---------------- complex GEMM (FMA pipes) ----------------
-// C = alpha op(A) B + beta C, BM x BN complex tile per CTA, TM x TN per thread,
-// 256 threads.  FP64: 64x64 tiles; FP32: 128x64 tiles.
+// C = alpha op(A) B + beta C, BM x BN complex tile per CTA, TM x TN per thread.  The
+// next BK-deep K step is loaded into registers while one is multiplied from
+// shared memory (two buffers, one barrier a step).
 // COMP: the FP32 sums of each BK-deep K tile are added into a two-float
 // (hi + lo) running sum (TwoSum), so accumulation error does not grow with K;
 // TC is the output type (double to accumulate FP32 products into an FP64 C).
 template <typename T, int BM, int BN, int TM, int TN, int BK, bool CONJ_A, typename TC = T, bool COMP = false>
-__global__ void __launch_bounds__(256) cgemm_fma_kernel(int m, int n, int k, cx<T> alpha, const T *__restrict__ A,
-                                                        int64_t lda, const T *__restrict__ B, int64_t ldb, cx<TC> beta,
-                                                        TC *__restrict__ C, int64_t ldc, int64_t sA, int64_t sB,
-                                                        int64_t sC) {
+__global__ void __launch_bounds__((BM / TM) * (BN / TN))
+    cgemm_fma_kernel(int m, int n, int k, cx<T> alpha, const T *__restrict__ A, int64_t lda, const T *__restrict__ B,
+                     int64_t ldb, cx<TC> beta, TC *__restrict__ C, int64_t ldc, int64_t sA, int64_t sB, int64_t sC) {
   typedef typename V2<T>::type T2;
   // strided batch: problem blockIdx.z (strides in elements of T / TC)
   A += sA * blockIdx.z;
   B += sB * blockIdx.z;
   C += sC * blockIdx.z;
-  constexpr int TX = BN / TN, TY = BM / TM;
-  static_assert(TX * TY == 256, "256 threads");
-  __shared__ T2 As[BK][BM];
-  __shared__ T2 Bs[BK][BN];
+  constexpr int TX = BN / TN, TY = BM / TM, THREADS = TX * TY;
+  constexpr int PA = BM * BK / THREADS, PB = BN * BK / THREADS;  // elements a thread loads per K step
+  static_assert(PA * THREADS == BM * BK && PB * THREADS == BN * BK, "whole loads");
+  __shared__ T2 As[2][BK][BM];
+  __shared__ T2 Bs[2][BK][BN];
   const int tx = threadIdx.x % TX, ty = threadIdx.x / TX;
   const int m0 = blockIdx.x * BM, n0 = blockIdx.y * BN;
   const T2 *A2 = reinterpret_cast<const T2 *>(A);
   const T2 *B2 = reinterpret_cast<const T2 *>(B);
+  T2 va[PA], vb[PB];  // the next K step, on its way
+  auto load = [&](int kk0) {
+#pragma unroll
+    for (int e = 0; e < PA; e++) {
+      const int idx = threadIdx.x + THREADS * e;
+      const int r = CONJ_A ? idx / BK : idx % BM, kk = CONJ_A ? idx % BK : idx / BM;
+      const int gr = m0 + r, gk = kk0 + kk;
+      T2 v = V2<T>::make(0, 0);
+      if (gr < m && gk < k) v = CONJ_A ? A2[gk + lda * (int64_t)gr] : A2[gr + lda * (int64_t)gk];
+      if (CONJ_A) v.y = -v.y;
+      va[e] = v;
+    }
+#pragma unroll
+    for (int e = 0; e < PB; e++) {
+      const int idx = threadIdx.x + THREADS * e;
+      const int kk = idx % BK, c = idx / BK;
+      const int gk = kk0 + kk, gc = n0 + c;
+      vb[e] = gk < k && gc < n ? B2[gk + ldb * (int64_t)gc] : V2<T>::make(0, 0);
+    }
+  };
+  auto store = [&](int buf) {
+#pragma unroll
+    for (int e = 0; e < PA; e++) {
+      const int idx = threadIdx.x + THREADS * e;
+      As[buf][CONJ_A ? idx % BK : idx / BM][CONJ_A ? idx / BK : idx % BM] = va[e];
+    }
+#pragma unroll
+    for (int e = 0; e < PB; e++) {
+      const int idx = threadIdx.x + THREADS * e;
+      Bs[buf][idx % BK][idx / BK] = vb[e];
+    }
+  };
   cx<T> acc[TM][TN];
   cx<T> lo[COMP ? TM : 1][COMP ? TN : 1];
   cx<T> part[COMP ? TM : 1][COMP ? TN : 1];
@@ -1179,38 +1212,19 @@ __global__ void __launch_bounds__(256) cgemm_fma_kernel(int m, int n, int k, cx<
 #pragma unroll
       for (int b = 0; b < (COMP ? TN : 1); b++) { lo[a][b] = {0, 0}; part[a][b] = {0, 0}; }
   }
-  for (int kk0 = 0; kk0 < k; kk0 += BK) {
-#pragma unroll
-    for (int e = 0; e < (BM * BK) / 256; e++) {
-      const int idx = threadIdx.x + 256 * e;
-      int r, kk;
-      if (!CONJ_A) { r = idx % BM; kk = idx / BM; }
-      else { kk = idx % BK; r = idx / BK; }
-      const int gr = m0 + r, gk = kk0 + kk;
-      T2 v = V2<T>::make(0, 0);
-      if (gr < m && gk < k) {
-        if (!CONJ_A) v = A2[gr + lda * (int64_t)gk];
-        else { v = A2[gk + lda * (int64_t)gr]; v.y = -v.y; }
-      }
-      As[kk][r] = v;
-    }
-#pragma unroll
-    for (int e = 0; e < (BN * BK) / 256; e++) {
-      const int idx = threadIdx.x + 256 * e;
-      const int kk = idx % BK, c = idx / BK;
-      const int gk = kk0 + kk, gc = n0 + c;
-      T2 v = V2<T>::make(0, 0);
-      if (gk < k && gc < n) v = B2[gk + ldb * (int64_t)gc];
-      Bs[kk][c] = v;
-    }
-    __syncthreads();
+  load(0);
+  int buf = 0;
+  for (int kk0 = 0; kk0 < k; kk0 += BK, buf ^= 1) {
+    store(buf);
+    __syncthreads();  // and everyone is done with the other buffer
+    if (kk0 + BK < k) load(kk0 + BK);
 #pragma unroll
     for (int kk = 0; kk < BK; kk++) {
       T2 a[TM], b[TN];
 #pragma unroll
-      for (int q = 0; q < TM; q++) a[q] = As[kk][ty + TY * q];
+      for (int q = 0; q < TM; q++) a[q] = As[buf][kk][ty + TY * q];
 #pragma unroll
-      for (int q = 0; q < TN; q++) b[q] = Bs[kk][tx + TX * q];
+      for (int q = 0; q < TN; q++) b[q] = Bs[buf][kk][tx + TX * q];
 #pragma unroll
       for (int p = 0; p < TM; p++)
 #pragma unroll
@@ -1240,7 +1254,6 @@ __global__ void __launch_bounds__(256) cgemm_fma_kernel(int m, int n, int k, cx<
           x = {0, 0};
         }
     }
-    __syncthreads();
   }
   typedef typename V2<TC>::type C2t;
   C2t *C2 = reinterpret_cast<C2t *>(C);
@@ -1268,16 +1281,44 @@ __global__ void __launch_bounds__(256) cgemm_fma_kernel(int m, int n, int k, cx<
     }
 }
 
-template <typename T>
-struct GemmCfg;
-template <>
-struct GemmCfg<double> {
-  static constexpr int BM = 64, BN = 64, TM = 4, TN = 4, BK = 8;
-};
-template <>
-struct GemmCfg<float> {
-  static constexpr int BM = 128, BN = 64, TM = 8, TN = 4, BK = 8;
-};
+// One launch (nb > 1: a strided batch).
+//
+// FP64 runs at 2 FMA a cycle and SM, so any tile keeps its pipe busy (four warps are
+// enough, and 16 x 16 reads no more than the L2 gives) and what counts is how evenly
+// the tiles fill the SMs: the 53 products of a complex128 solve of n = 1152 took 20.7 ms in
+// 64 x 64 tiles, 13.8 in 32 x 32, 12.3 in 32 x 16 and 11.5 in 16 x 16.
+//
+// FP32: the tile whose waves take least.  128 x 64 runs at the FMA pipes' rate, 64 x 64 at
+// about 0.9 of it and 32 x 32, bound by its reads of shared memory, at half; but the
+// joins of a triangle's inverse are a few small products, which left most SMs
+// idle in 128 x 64 tiles (the 12 of an n = 1152 solve 551 -> 205 us).
+template <typename T, bool CONJ_A>
+void launch_gemm_fma(bemgpu_ctx_s *ctx, int m, int n, int k, cx<T> alpha, const T *A, int64_t lda, const T *B, int64_t ldb,
+                     cx<T> beta, T *C, int64_t ldc, cudaStream_t st, int nb = 1, int64_t sA = 0, int64_t sB = 0,
+                     int64_t sC = 0) {
+  auto grid = [&](int bm, int bn) { return dim3((m + bm - 1) / bm, (n + bn - 1) / bn, nb); };
+  if constexpr (sizeof(T) == 8) {
+    cgemm_fma_kernel<double, 16, 16, 1, 2, 16, CONJ_A>
+        <<<grid(16, 16), 128, 0, st>>>(m, n, k, alpha, A, lda, B, ldb, beta, C, ldc, sA, sB, sC);
+  } else {
+    auto cost = [&](int bm, int bn, double rate) {
+      const dim3 g = grid(bm, bn);
+      const int64_t tiles = (int64_t)g.x * g.y * g.z;
+      return (double)((tiles + ctx->num_sms - 1) / ctx->num_sms) * bm * bn / rate;
+    };
+    const double c0 = cost(128, 64, 1.0), c1 = cost(64, 64, 0.9), c2 = cost(32, 32, 0.55);
+    if (c2 < c1 && c2 < c0)
+      cgemm_fma_kernel<float, 32, 32, 2, 2, 16, CONJ_A>
+          <<<grid(32, 32), 256, 0, st>>>(m, n, k, alpha, A, lda, B, ldb, beta, C, ldc, sA, sB, sC);
+    else if (c1 < c0)
+      cgemm_fma_kernel<float, 64, 64, 4, 4, 8, CONJ_A>
+          <<<grid(64, 64), 256, 0, st>>>(m, n, k, alpha, A, lda, B, ldb, beta, C, ldc, sA, sB, sC);
+    else
+      cgemm_fma_kernel<float, 128, 64, 8, 4, 8, CONJ_A>
+          <<<grid(128, 64), 256, 0, st>>>(m, n, k, alpha, A, lda, B, ldb, beta, C, ldc, sA, sB, sC);
+  }
+  ctx->launches++;
+}
 
 template <typename T, int W>
 constexpr int tri_smem_bytes() { return (W * (TriCfg<T>::NC + 1) + TriCfg<T>::BUFS * W * 33 + W) * (int)sizeof(typename V2<T>::type); }
@@ -1323,19 +1364,13 @@ template <typename T>
 int gemm_fma(bemgpu_ctx_s *ctx, int kind, char opA, int m, int n, int k, const T alpha[2], const T *A, int64_t lda,
              const T *B, int64_t ldb, const T beta[2], T *C, int64_t ldc, cudaStream_t stream) {
   if (m <= 0 || n <= 0) return BEMGPU_OK;
-  typedef GemmCfg<T> G;
-  dim3 grd((m + G::BM - 1) / G::BM, (n + G::BN - 1) / G::BN);
   cx<T> al = {alpha[0], alpha[1]}, be = {beta[0], beta[1]};
   ProfScope ps(ctx, kind, stream, 8.0 * m * n * k,
                2.0 * sizeof(T) * ((double)m * k + (double)k * n + 2.0 * m * n));
-  if (opA == 'C') {
-    cgemm_fma_kernel<T, G::BM, G::BN, G::TM, G::TN, G::BK, true>
-        <<<grd, 256, 0, stream>>>(m, n, k, al, A, lda, B, ldb, be, C, ldc, 0, 0, 0);
-  } else {
-    cgemm_fma_kernel<T, G::BM, G::BN, G::TM, G::TN, G::BK, false>
-        <<<grd, 256, 0, stream>>>(m, n, k, al, A, lda, B, ldb, be, C, ldc, 0, 0, 0);
-  }
-  ctx->launches++;
+  if (opA == 'C')
+    launch_gemm_fma<T, true>(ctx, m, n, k, al, A, lda, B, ldb, be, C, ldc, stream);
+  else
+    launch_gemm_fma<T, false>(ctx, m, n, k, al, A, lda, B, ldb, be, C, ldc, stream);
   BEM_CUDA_TRY(ctx, cudaGetLastError());
   return BEMGPU_OK;
 }
@@ -1989,23 +2024,20 @@ int tri_inv_bottom_up(bemgpu_ctx_s *ctx, bool upper, float *X, int n, float *tmp
     const int b2_last = std::min(b, n - o_last - b);  // ragged pair at o_last, if any
     auto at = [&](int r, int c) { return X + 2 * ((int64_t)r + (int64_t)n * c); };
     if (b < 512 && full > 0) {
-      typedef GemmCfg<float> G;
-      const dim3 grd((b + G::BM - 1) / G::BM, (b + G::BN - 1) / G::BN, full);
       const int64_t sx = 2 * ((int64_t)2 * b + (int64_t)n * 2 * b), st_ = 2 * (int64_t)b * b;
       const cx<float> c1 = {1.f, 0.f}, cm1 = {-1.f, 0.f}, c0 = {0.f, 0.f};
       ProfScope ps(ctx, BEMGPU_K_TRSM, st, 16.0 * full * (double)b * b * b, 48.0 * full * (double)b * b);
       if (!upper) {
-        cgemm_fma_kernel<float, G::BM, G::BN, G::TM, G::TN, G::BK, false><<<grd, 256, 0, st>>>(
-            b, b, b, c1, at(b, 0), n, at(0, 0), n, c0, tmp, b, sx, sx, st_);
-        cgemm_fma_kernel<float, G::BM, G::BN, G::TM, G::TN, G::BK, false><<<grd, 256, 0, st>>>(
-            b, b, b, cm1, at(b, b), n, tmp, b, c0, at(b, 0), n, sx, st_, sx);
+        launch_gemm_fma<float, false>(ctx, b, b, b, c1, at(b, 0), n, at(0, 0), n, c0, tmp, b, st, full,
+                                      sx, sx, st_);
+        launch_gemm_fma<float, false>(ctx, b, b, b, cm1, at(b, b), n, tmp, b, c0, at(b, 0), n, st, full,
+                                      sx, st_, sx);
       } else {
-        cgemm_fma_kernel<float, G::BM, G::BN, G::TM, G::TN, G::BK, false><<<grd, 256, 0, st>>>(
-            b, b, b, c1, at(0, b), n, at(b, b), n, c0, tmp, b, sx, sx, st_);
-        cgemm_fma_kernel<float, G::BM, G::BN, G::TM, G::TN, G::BK, false><<<grd, 256, 0, st>>>(
-            b, b, b, cm1, at(0, 0), n, tmp, b, c0, at(0, b), n, sx, st_, sx);
+        launch_gemm_fma<float, false>(ctx, b, b, b, c1, at(0, b), n, at(b, b), n, c0, tmp, b, st, full,
+                                      sx, sx, st_);
+        launch_gemm_fma<float, false>(ctx, b, b, b, cm1, at(0, 0), n, tmp, b, c0, at(0, b), n, st, full,
+                                      sx, st_, sx);
       }
-      ctx->launches += 2;
       BEM_CUDA_TRY(ctx, cudaGetLastError());
     }
     for (int pi = (b < 512 ? full : 0); pi <= full && !rc; pi++) {
