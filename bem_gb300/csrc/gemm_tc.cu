@@ -10,11 +10,12 @@
 //     magnitude (x = s1 + s2 + s3 exactly); the six products with
 //     slice indices (0-based) summing to <= 2 are accumulated into one FP32 TMEM accumulator,
 //     which reproduces an FP32 product to ~2^-24.
-//   * one CTA computes a 128 x 128 tile of D': warp 0 streams the three A and
-//     three B slice tiles of each 64-deep K step with TMA (128-byte swizzle)
-//     into a 2-stage mbarrier pipeline, warp 1 issues tcgen05.mma (one elected
-//     thread, M=128 N=128 K=16, bf16 in, FP32 accumulate in TMEM), warps 2..5
-//     read the accumulator back with tcgen05.ld and write C.
+//   * a persistent CTA per SM computes 128 x 256, 128 x 128 or 128 x 64 tiles of D':
+//     warp 0 streams the three A and three B slice tiles of each K step with TMA
+//     into an mbarrier pipeline, warp 1 issues tcgen05.mma (one elected thread,
+//     M=128, N the tile's width, K=16, bf16 in, FP32 accumulate in TMEM), warps
+//     2..9 read a tile's accumulator back with tcgen05.ld and write C
+//     while the next tile's products run into the other one.
 //   * every wait is bounded; a wait that runs out sets an error flag, the CTA
 //     finishes, frees its TMEM and the host returns BEMGPU_ERR_TIMEOUT.
 #include "bemgpu_internal.h"
@@ -25,24 +26,32 @@
 
 namespace {
 
-constexpr int TC_BM = 128, TC_BN = 128, TC_BK = 64;   // tile of D'; K step (bf16 elements, 128 bytes)
-constexpr int TC_STAGES = 2;
+constexpr int TC_BM = 128, TC_BN = 128;               // operands are padded to whole 128-row tiles
+constexpr int TC_BK = 64;                             // and to 64 in K
 constexpr int TC_SLICES = 3;
-constexpr int TC_TILE_BYTES = TC_BM * TC_BK * 2;      // 16 KB per slice tile (A and B alike)
-constexpr int TC_STAGE_BYTES = 2 * TC_SLICES * TC_TILE_BYTES;  // 96 KB
-constexpr int TC_SMEM_BYTES = TC_STAGES * TC_STAGE_BYTES + 1024 + 256;
-constexpr int TC_THREADS = 192;
+constexpr int TC_TILE_BYTES = TC_BM * TC_BK * 2;      // 16 KB: 128 rows of a slice, 64 deep
+constexpr int TC_SMEM_MAX = 232448;                   // dynamic shared memory of one CTA (227 KB)
+constexpr int TC_EPI_WARPS = 8;
+constexpr int TC_THREADS = 64 + 32 * TC_EPI_WARPS;
+
+// The tile of tc_gemm_kernel: 128 x BN.  K steps of 64 (128-byte rows) where three or two
+// stages of them fit, else of 32 (64-byte rows), which take longer to land.
+template <int BN>
+struct TcCfg {
+  static constexpr int BK = BN == 256 ? 32 : 64;
+  static constexpr int A_TILE = TC_BM * BK * 2, B_TILE = BN * BK * 2, STAGE = TC_SLICES * (A_TILE + B_TILE);
+  static constexpr int STAGES = (TC_SMEM_MAX - 1280) / STAGE;
+  static constexpr int SMEM = STAGES * STAGE + 1024 + 256;
+  static constexpr int TMEM_COLS = 2 * BN;  // two accumulators
+  static_assert(STAGES >= 2, "shared memory");
+};
+inline int tc_bk(int bn) { return bn == 256 ? TcCfg<256>::BK : TcCfg<128>::BK; }
 
 // products (a, b) with a + b <= 2 (0-based slice indices), level-major:
 // (0,0) (0,1) (1,0) (0,2) (1,1) (2,0)
 __host__ __device__ constexpr int tc_level(int p) { return p < 1 ? 0 : p < 3 ? 1 : 2; }
 __host__ __device__ constexpr int tc_prod_a(int p) { return p - tc_level(p) * (tc_level(p) + 1) / 2; }
 __host__ __device__ constexpr int tc_prod_b(int p) { return tc_level(p) - tc_prod_a(p); }
-
-__device__ __forceinline__ void drain_copies(uint64_t *full, int issued, int *err) {
-  for (int kt = issued > TC_STAGES ? issued - TC_STAGES : 0; kt < issued; kt++)
-    if (!mbar_wait(&full[kt % TC_STAGES], (kt / TC_STAGES) & 1, err)) return;
-}
 
 struct TcMaps {
   CUtensorMap a[TC_SLICES];
@@ -53,36 +62,48 @@ struct TcMaps {
 
 namespace {
 
-// One 128 x 128 tile of D' = sum_{(a,b)} A'_a B'_b^T over ktiles 64-deep K steps.
-// C is written as TOUT at C[rho + ldcf * c] for rho < mvalid, c < nvalid
+// D' = sum_{(a,b)} A'_a B'_b^T over ktiles K steps, in 128 x BN tiles.
+// C is written at C[rho + ldcf * c] for rho < mvalid, c < nvalid
 // (accumulate: C += D'; otherwise C = D').
-template <typename TOUT>
+//
+// A step of a 128 x 128 tile is six products of 256 cycles (64 deep) for 96 KB of
+// slices: 64 bytes a cycle and SM, all that TMA delivers.  128 x 256 needs 48.  And C
+// of an LU update (K = 256) takes as long to read and write as its products, so a
+// tile's epilogue runs beside the next tile's products: the CTAs are persistent, the
+// accumulator is double-buffered, and a warp's next 32 columns of C are on their way
+// while it adds the last.  One tile per CTA, its epilogue after its products, took 697
+// us for 7680 x 7680 x 256 (accumulating) where this takes 443, and 6.25 ms for 7680 x 3840 x
+// 7680 where this takes 5.03 (2.16 PF/s of slice products).
+template <int BN>
 __global__ void __launch_bounds__(TC_THREADS, 1)
-    tc_gemm_kernel(const __grid_constant__ TcMaps maps, int ktiles, TOUT *__restrict__ C, int64_t ldcf, int mvalid,
-                   int nvalid, int accumulate, int tri, int raster, int *err) {
+    tc_gemm_kernel(const __grid_constant__ TcMaps maps, int ktiles, int nM, int nN, float *__restrict__ C, int64_t ldcf,
+                   int mvalid, int nvalid, int accumulate, int tri, int raster, int *err) {
+  typedef TcCfg<BN> CF;
+  constexpr int STAGE = CF::STAGE, NST = CF::STAGES, BK = CF::BK, A_TILE = CF::A_TILE, B_TILE = CF::B_TILE;
   extern __shared__ unsigned char tc_smem_raw[];
   unsigned char *smem = reinterpret_cast<unsigned char *>((reinterpret_cast<uintptr_t>(tc_smem_raw) + 1023) &
                                                           ~(uintptr_t)1023);
-  uint64_t *full = reinterpret_cast<uint64_t *>(smem + TC_STAGES * TC_STAGE_BYTES);
-  uint64_t *empty = full + TC_STAGES;
-  uint64_t *accum_bar = empty + TC_STAGES;
-  uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(accum_bar + 1);
+  uint64_t *full = reinterpret_cast<uint64_t *>(smem + NST * STAGE);
+  uint64_t *empty = full + NST;
+  uint64_t *accf = empty + NST;  // accumulator b written (MMA -> epilogue)
+  uint64_t *acce = accf + 2;     // accumulator b read back (epilogue -> MMA)
+  uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(acce + 2);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  int mt, nt;
-  grouped_tile(raster, mt, nt);
-  const int m0 = mt * TC_BM, n0 = nt * TC_BN;
 
   if (threadIdx.x == 0) {
-    for (int s = 0; s < TC_STAGES; s++) {
+    for (int s = 0; s < NST; s++) {
       mbar_init(&full[s], 1);
       mbar_init(&empty[s], 1);
     }
-    mbar_init(accum_bar, 1);
+    for (int b = 0; b < 2; b++) {
+      mbar_init(&accf[b], 1);
+      mbar_init(&acce[b], TC_EPI_WARPS);
+    }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 1) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)),
-                 "r"(TC_BN));
+                 "r"(CF::TMEM_COLS));
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
     asm volatile("tcgen05.fence::before_thread_sync;");
   }
@@ -90,80 +111,124 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
   asm volatile("tcgen05.fence::after_thread_sync;");
   const uint32_t tmem = *tmem_slot;
 
-  // K range: all of it, or for a triangular complex A only the K steps that
-  // meet nonzero entries of this tile's rows (lower: columns <= row, upper:
-  // columns >= row; realified row rho and column kappa belong to complex
-  // row rho / 2 and column kappa / 2).
-  const int kb = tri == 2 ? m0 / TC_BK : 0;
-  const int ke = tri == 1 ? min(ktiles, (m0 + TC_BM + TC_BK - 1) / TC_BK) : ktiles;
-  const int nk = max(0, ke - kb);
+  // Tile t of this CTA's round: its origin, and its K range: all of it, or for a
+  // triangular complex A only the K steps that meet nonzero entries of the tile's
+  // rows (lower: columns <= row, upper: columns >= row; realified row rho and
+  // column kappa belong to complex row rho / 2 and column kappa / 2).  The longest
+  // ones come first, so that the CTAs finish together.
+  struct Tile {
+    int m0, n0, kb, nk;
+  };
+  const int tiles = nM * nN;
+  auto tile_at = [&](int t) {
+    int mt, nt;
+    grouped_tile(raster, t, nM, nN, mt, nt);
+    if (tri == 1) mt = nM - 1 - mt;
+    Tile x;
+    x.m0 = mt * TC_BM;
+    x.n0 = nt * BN;
+    x.kb = tri == 2 ? x.m0 / BK : 0;
+    const int ke = tri == 1 ? min(ktiles, (x.m0 + TC_BM) / BK) : ktiles;
+    x.nk = max(0, ke - x.kb);
+    return x;
+  };
   if (warp == 0) {
     if (elect_one()) {
-      int issued = 0;
-      for (int j = 0; j < nk; j++) {
-        const int kt = kb + j, s = j % TC_STAGES, round = j / TC_STAGES;
-        if (j >= TC_STAGES && !mbar_wait(&empty[s], (round - 1) & 1, err)) break;
-        mbar_expect_tx(&full[s], TC_STAGE_BYTES);
-        unsigned char *st = smem + s * TC_STAGE_BYTES;
+      int it = 0;
+      bool ok = true;
+      for (int t = blockIdx.x; t < tiles && ok; t += gridDim.x) {
+        const Tile x = tile_at(t);
+        for (int j = 0; j < x.nk; j++, it++) {
+          const int kt = x.kb + j, s = it % NST, round = it / NST;
+          if (it >= NST && !mbar_wait(&empty[s], (round - 1) & 1, err)) {
+            ok = false;
+            break;
+          }
+          mbar_expect_tx(&full[s], STAGE);
+          unsigned char *st = smem + s * STAGE;
 #pragma unroll
-        for (int a = 0; a < TC_SLICES; a++) tma_load_2d(st + a * TC_TILE_BYTES, &maps.a[a], kt * TC_BK, m0, &full[s]);
+          for (int a = 0; a < TC_SLICES; a++) tma_load_2d(st + a * A_TILE, &maps.a[a], kt * BK, x.m0, &full[s]);
 #pragma unroll
-        for (int b = 0; b < TC_SLICES; b++)
-          tma_load_2d(st + (TC_SLICES + b) * TC_TILE_BYTES, &maps.b[b], kt * TC_BK, n0, &full[s]);
-        issued = j + 1;
+          for (int b = 0; b < TC_SLICES; b++)
+            tma_load_2d(st + TC_SLICES * A_TILE + b * B_TILE, &maps.b[b], kt * BK, x.n0, &full[s]);
+        }
       }
-      drain_copies(full, issued, err);
+      // copies still in flight after an early stop land before the CTA exits
+      for (int g = it > NST ? it - NST : 0; g < it; g++)
+        if (!mbar_wait(&full[g % NST], (g / NST) & 1, err)) break;
     }
   } else if (warp == 1) {
     if (elect_one()) {
-      constexpr uint32_t idesc = tc_idesc(TC_BM, TC_BN);
+      constexpr uint32_t idesc = tc_idesc(TC_BM, BN);
+      int it = 0, i = 0;
       bool ok = true;
-      for (int j = 0; j < nk && ok; j++) {
-        const int s = j % TC_STAGES, round = j / TC_STAGES;
-        ok = mbar_wait(&full[s], round & 1, err);
-        if (!ok) break;
+      for (int t = blockIdx.x; t < tiles && ok; t += gridDim.x, i++) {
+        const Tile x = tile_at(t);
+        const int b = i & 1;
+        if (i >= 2 && !mbar_wait(&acce[b], ((i >> 1) - 1) & 1, err)) break;
         asm volatile("tcgen05.fence::after_thread_sync;");
-        const uint64_t dbase = smem_desc_sw128(smem_u32(smem + s * TC_STAGE_BYTES));
+        const uint32_t acc = tmem + (uint32_t)(b * BN);
+        for (int j = 0; j < x.nk; j++, it++) {
+          const int s = it % NST, round = it / NST;
+          ok = mbar_wait(&full[s], round & 1, err);
+          if (!ok) break;
+          asm volatile("tcgen05.fence::after_thread_sync;");
+          const uint64_t dbase =
+              BK == 64 ? smem_desc_sw128(smem_u32(smem + s * STAGE)) : smem_desc_sw64(smem_u32(smem + s * STAGE));
 #pragma unroll
-        for (int ks = 0; ks < TC_BK / 16; ks++) {
+          for (int ks = 0; ks < BK / 16; ks++) {
 #pragma unroll
-          for (int p = 0; p < 6; p++) {
-            const uint64_t da = dbase + (uint64_t)((tc_prod_a(p) * TC_TILE_BYTES + ks * 32) >> 4);
-            const uint64_t db = dbase + (uint64_t)(((TC_SLICES + tc_prod_b(p)) * TC_TILE_BYTES + ks * 32) >> 4);
-            tc_mma(tmem, da, db, idesc, (j | ks | p) != 0 ? 1u : 0u);
+            for (int p = 0; p < 6; p++) {
+              const uint64_t da = dbase + (uint64_t)((tc_prod_a(p) * A_TILE + ks * 32) >> 4);
+              const uint64_t db = dbase + (uint64_t)((TC_SLICES * A_TILE + tc_prod_b(p) * B_TILE + ks * 32) >> 4);
+              tc_mma(acc, da, db, idesc, (j | ks | p) != 0 ? 1u : 0u);
+            }
           }
+          tc_commit(&empty[s]);
         }
-        tc_commit(&empty[s]);
+        tc_commit(&accf[b]);
       }
-      tc_commit(accum_bar);
     }
   } else {
-    // epilogue: warps 2..5; warp w reads TMEM lanes 32*(w % 4) .. +31
-    const int sub = warp & 3;
-    const bool ok = mbar_wait(accum_bar, 0, err);
-    __syncwarp();
-    asm volatile("tcgen05.fence::after_thread_sync;");
-    const int rho = m0 + sub * 32 + lane;
-#pragma unroll 1
-    for (int c0 = 0; c0 < TC_BN; c0 += 32) {
-      // the chunk's old C values first, all loads in flight together
-      TOUT old[32];
-#pragma unroll
-      for (int j = 0; j < 32; j++) {
-        const int c = n0 + c0 + j;
-        old[j] = (accumulate && ok && rho < mvalid && c < nvalid) ? C[rho + ldcf * (int64_t)c] : (TOUT)0;
-      }
-      float v[32];
-      tc_ld32(tmem + ((uint32_t)(sub * 32) << 16) + (uint32_t)c0, v);
-      if (nk == 0) {
-#pragma unroll
-        for (int j = 0; j < 32; j++) v[j] = 0.f;
-      }
-      if (ok && rho < mvalid) {
+    // warp w reads TMEM lanes 32 (w % 4) .. +31, half of the tile's columns
+    const int quarter = warp & 3, half = (warp - 2) >> 2;
+    int i = 0;
+    for (int t = blockIdx.x; t < tiles; t += gridDim.x, i++) {
+      const Tile x = tile_at(t);
+      const int b = i & 1, rho = x.m0 + quarter * 32 + lane, c0 = x.n0 + half * (BN / 2);
+      float old[32];
+      auto load_old = [&](int q) {  // 32 columns of C, all loads in flight together
 #pragma unroll
         for (int j = 0; j < 32; j++) {
-          const int c = n0 + c0 + j;
-          if (c < nvalid) C[rho + ldcf * (int64_t)c] = old[j] + (TOUT)v[j];
+          const int c = c0 + 32 * q + j;
+          old[j] = (accumulate && rho < mvalid && c < nvalid) ? C[rho + ldcf * (int64_t)c] : 0.f;
+        }
+      };
+      load_old(0);
+      int got = 1;
+      if (lane == 0) got = mbar_wait(&accf[b], (i >> 1) & 1, err) ? 1 : 0;
+      got = __shfl_sync(0xffffffffu, got, 0);
+      if (!got) break;
+      asm volatile("tcgen05.fence::after_thread_sync;");
+#pragma unroll 1
+      for (int q = 0; q < BN / 64; q++) {
+        float v[32];
+        tc_ld32(tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(b * BN + half * (BN / 2) + 32 * q), v);
+        if (q == BN / 64 - 1) {
+          asm volatile("tcgen05.fence::before_thread_sync;");
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&acce[b]);
+        }
+        float sum[32];
+#pragma unroll
+        for (int j = 0; j < 32; j++) sum[j] = old[j] + (x.nk > 0 ? v[j] : 0.f);
+        if (q + 1 < BN / 64) load_old(q + 1);
+        if (rho < mvalid) {
+#pragma unroll
+          for (int j = 0; j < 32; j++) {
+            const int c = c0 + 32 * q + j;
+            if (c < nvalid) C[rho + ldcf * (int64_t)c] = sum[j];
+          }
         }
       }
     }
@@ -172,10 +237,9 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
   __syncthreads();
   if (warp == 1) {
     asm volatile("tcgen05.fence::after_thread_sync;");
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(TC_BN));
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(CF::TMEM_COLS));
   }
 }
-
 
 constexpr int TCC_BN = 64;                     // tile of D': 128 x 64
 constexpr int TCC_STAGES = 3;
@@ -448,8 +512,9 @@ __global__ void tc_prep_b_kernel(const float *__restrict__ B, int64_t ldb, int k
   reinterpret_cast<__nv_bfloat162 *>(S + 2 * plane + idx)[0] = __halves2bfloat162(a3, b3);
 }
 
-bool make_map(CUtensorMap *map, const void *base, int64_t rows, int64_t kp, int box_rows = TC_BM) {
-  return make_map_bf16(map, base, rows, kp, TC_BK, box_rows, CU_TENSOR_MAP_SWIZZLE_128B);
+bool make_map(CUtensorMap *map, const void *base, int64_t rows, int64_t kp, int box_k, int box_rows) {
+  return make_map_bf16(map, base, rows, kp, box_k, box_rows,
+                       box_k == 64 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B);
 }
 
 }  // namespace
@@ -465,7 +530,7 @@ int bem_tc_error(bemgpu_ctx_s *ctx, bool reset) {
 }
 
 // C (+)= sign * A B on the tensor cores.  out: TC_OUT_F32 (complex64 C),
-// TC_OUT_F64 (complex128 C, FP32 accumulation), TC_OUT_F64_COMP (complex128
+// TC_OUT_F64_COMP (complex128
 // C, per-K-step FP32 sums accumulated as two-float sums).  Column-major, ldc.
 void bem_cgemm_tc_bytes(int m, int n, int k, size_t &a_bytes, size_t &b_bytes) {
   const int64_t Mp = ((2 * (int64_t)m + TC_BM - 1) / TC_BM) * TC_BM;
@@ -474,6 +539,33 @@ void bem_cgemm_tc_bytes(int m, int n, int k, size_t &a_bytes, size_t &b_bytes) {
   a_bytes = sizeof(__nv_bfloat16) * TC_SLICES * (size_t)(Mp * Kp);
   b_bytes = sizeof(__nv_bfloat16) * TC_SLICES * (size_t)(Np * Kp);
 }
+
+namespace {
+
+// Tile width: the persistent CTAs' rounds, a K element of a round taking 0.75 (128 x 64), 1
+// (128 x 128) or 1.65 (128 x 256: n x n x n products of several rounds), and the filling of
+// the pipeline and the last epilogue, which nothing hides, as long as 8 K elements a
+// column.  Measured in us (128 x 64, 128, 256): 576^3 20, 26, 49; 1152 x 1152 x 128 18, 20,
+// 25; 1152^3 84, 78, 83; 2048 x 2048 x 256 53, 46, 52; 4001 x 2003 x 4001 1194, 933, 870;
+// 7680 x 7680 x 256 611, 482, 443.
+int tc_tile_n(const bemgpu_ctx_s *ctx, int64_t nM, int n, int64_t Kp) {
+  auto cost = [&](int bn, double c) {
+    const int64_t tiles = nM * ((n + bn - 1) / bn);
+    return c * (double)(Kp * ((tiles + ctx->num_sms - 1) / ctx->num_sms)) + 8.0 * bn;
+  };
+  const double c64 = cost(64, 0.75), c128 = cost(128, 1.0), c256 = cost(256, 1.65);
+  return c256 < c128 && c256 < c64 ? 256 : c128 < c64 ? 128 : 64;
+}
+
+template <int BN>
+void tc_launch(bemgpu_ctx_s *ctx, const TcMaps &maps, int nM, int64_t Kp, float *C, int64_t ldc, int m, int n,
+               int accumulate, int tri, int *err, cudaStream_t st) {
+  const int nN = (n + BN - 1) / BN;
+  tc_gemm_kernel<BN><<<std::min(nM * nN, ctx->num_sms), TC_THREADS, TcCfg<BN>::SMEM, st>>>(
+      maps, (int)(Kp / TcCfg<BN>::BK), nM, nN, C, 2 * ldc, 2 * m, n, accumulate, tri, ctx->tune.raster, err);
+}
+
+}  // namespace
 
 int bem_cgemm_tc(bemgpu_ctx_s *ctx, int kind, int m, int n, int k, float sign, const float *A, int64_t lda,
                  const float *B, int64_t ldb, void *C, int64_t ldc, int out, int accumulate, cudaStream_t st,
@@ -486,10 +578,12 @@ int bem_cgemm_tc(bemgpu_ctx_s *ctx, int kind, int m, int n, int k, float sign, c
   const int64_t Kp = ((2 * (int64_t)k + TC_BK - 1) / TC_BK) * TC_BK;
   if (Mp / 2 > 65535 || Np > 65535) return bem_fail(ctx, BEMGPU_ERR_ARG, "cgemm_tc: %d x %d too large", m, n);
   if (!ctx->tc_ready) {
-    BEM_CUDA_TRY(ctx, cudaFuncSetAttribute(tc_gemm_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                           TC_SMEM_BYTES));
-    BEM_CUDA_TRY(ctx, cudaFuncSetAttribute(tc_gemm_kernel<double>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                           TC_SMEM_BYTES));
+    BEM_CUDA_TRY(ctx, cudaFuncSetAttribute(tc_gemm_kernel<64>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                           TcCfg<64>::SMEM));
+    BEM_CUDA_TRY(ctx, cudaFuncSetAttribute(tc_gemm_kernel<128>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                           TcCfg<128>::SMEM));
+    BEM_CUDA_TRY(ctx, cudaFuncSetAttribute(tc_gemm_kernel<256>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                           TcCfg<256>::SMEM));
     BEM_CUDA_TRY(ctx, cudaFuncSetAttribute(tc_gemm_comp_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                            TCC_SMEM_BYTES));
     ctx->tc_ready = true;
@@ -502,9 +596,12 @@ int bem_cgemm_tc(bemgpu_ctx_s *ctx, int kind, int m, int n, int k, float sign, c
     BEM_CUDA_TRY(ctx, cudaMemsetAsync(err, 0, sizeof(int), st));
     ctx->tc_err_ready = true;
   }
+  const bool comp = out == TC_OUT_F64_COMP;
+  const int tn = comp ? TCC_BN : tc_tile_n(ctx, Mp / TC_BM, n, Kp), box_k = comp ? TC_BK : tc_bk(tn);
   TcMaps maps;
   for (int i = 0; i < TC_SLICES; i++) {
-    if (!make_map(&maps.a[i], SA + i * Mp * Kp, Mp, Kp) || !make_map(&maps.b[i], SB + i * Np * Kp, Np, Kp, bn))
+    if (!make_map(&maps.a[i], SA + i * Mp * Kp, Mp, Kp, box_k, TC_BM) ||
+        !make_map(&maps.b[i], SB + i * Np * Kp, Np, Kp, box_k, tn))
       return bem_fail(ctx, BEMGPU_ERR_CUDA, "cgemm_tc: tensor map encoding failed");
   }
   {
@@ -524,12 +621,12 @@ int bem_cgemm_tc(bemgpu_ctx_s *ctx, int kind, int m, int n, int k, float sign, c
     // bounds of tc_gemm_kernel) count as work
     double run = 1.0;
     if (tri) {
-      const int64_t mtiles = Mp / TC_BM, ktiles = Kp / TC_BK;
+      const int64_t mtiles = Mp / TC_BM, bk = tc_bk(tn), ktiles = Kp / bk;
       int64_t steps = 0;
       for (int64_t mt = 0; mt < mtiles; mt++) {
         const int64_t m0 = mt * TC_BM;
-        const int64_t kb = tri == 2 ? m0 / TC_BK : 0;
-        const int64_t ke = tri == 1 ? std::min(ktiles, (m0 + TC_BM + TC_BK - 1) / TC_BK) : ktiles;
+        const int64_t kb = tri == 2 ? m0 / bk : 0;
+        const int64_t ke = tri == 1 ? std::min(ktiles, (m0 + TC_BM) / bk) : ktiles;
         steps += std::max<int64_t>(0, ke - kb);
       }
       run = (double)steps / ((double)mtiles * (double)ktiles);
@@ -537,17 +634,14 @@ int bem_cgemm_tc(bemgpu_ctx_s *ctx, int kind, int m, int n, int k, float sign, c
     ProfScope ps(ctx, kind, st, 8.0 * m * n * (double)k * run,
                  12.0 * ((double)Mp * Kp * run + (double)Np * Kp) + cbytes);
     ps.tensor = 6.0 * ps.flops;  // slice products (a, b) with a + b <= 2 of 3 slices
-    const dim3 grid((unsigned)(Mp / TC_BM), (unsigned)(Np / bn));
-    const int kt = (int)(Kp / TC_BK);
-    if (out == TC_OUT_F64_COMP)
-      tc_gemm_comp_kernel<<<grid, TCC_THREADS, TCC_SMEM_BYTES, st>>>(maps, kt, (double *)C, 2 * ldc, 2 * m, n,
-                                                                    accumulate, ctx->tune.raster, err);
-    else if (out == TC_OUT_F64)
-      tc_gemm_kernel<double><<<grid, TC_THREADS, TC_SMEM_BYTES, st>>>(maps, kt, (double *)C, 2 * ldc, 2 * m, n,
-                                                                      accumulate, tri, ctx->tune.raster, err);
-    else
-      tc_gemm_kernel<float><<<grid, TC_THREADS, TC_SMEM_BYTES, st>>>(maps, kt, (float *)C, 2 * ldc, 2 * m, n,
-                                                                     accumulate, tri, ctx->tune.raster, err);
+    const int nM = (int)(Mp / TC_BM);
+    if (comp) {
+      tc_gemm_comp_kernel<<<dim3(nM, (unsigned)(Np / bn)), TCC_THREADS, TCC_SMEM_BYTES, st>>>(
+          maps, (int)(Kp / TC_BK), (double *)C, 2 * ldc, 2 * m, n, accumulate, ctx->tune.raster, err);
+    } else {
+      (tn == 256 ? tc_launch<256> : tn == 128 ? tc_launch<128> : tc_launch<64>)(ctx, maps, nM, Kp, (float *)C, ldc, m, n,
+                                                                                accumulate, tri, err, st);
+    }
     ctx->launches++;
   }
   BEM_CUDA_TRY(ctx, cudaGetLastError());

@@ -173,20 +173,21 @@ __device__ __forceinline__ uint64_t smem_desc_sw64(uint32_t addr) {
   return d;
 }
 
-// Grouped rasterization of a (gridDim.x M-tiles) x (gridDim.y N-tiles) grid:
-// CTAs launched consecutively (linear id, x fastest) cover a band of `group`
-// M-tiles across the N-tiles, so the band's A tiles are re-read from L2, not
-// HBM, by every N-tile passing them.  `group` is the context's tuning
+// Grouped rasterization of a grid of nM x nN tiles: tiles of consecutive number L cover
+// a band of `group` M-tiles across the N-tiles, so the band's A tiles are re-read
+// from L2, not HBM, by every N-tile passing them.  `group` is the context's tuning
 // (BEMGPU_TUNE_RASTER, default 8).
-__device__ __forceinline__ void grouped_tile(int group, int &mt, int &nt) {
-  const int nM = gridDim.x, nN = gridDim.y;
-  const int L = blockIdx.y * nM + blockIdx.x;
+__device__ __forceinline__ void grouped_tile(int group, int L, int nM, int nN, int &mt, int &nt) {
   const int per = group * nN;
   const int g = L / per, first = g * group;
   const int gm = min(nM - first, group);
   const int local = L - g * per;
   mt = first + local % gm;
   nt = local / gm;
+}
+// The tile of a CTA of such a grid (linear id, x fastest).
+__device__ __forceinline__ void grouped_tile(int group, int &mt, int &nt) {
+  grouped_tile(group, blockIdx.y * gridDim.x + blockIdx.x, gridDim.x, gridDim.y, mt, nt);
 }
 
 // hi + lo += p (Knuth's TwoSum: the rounding error of hi + p goes to lo).
