@@ -1939,73 +1939,98 @@ namespace {
 
 // In-place inverses of the 64 x 64 diagonal blocks of X (n x n, ld ldx; the
 // last block may be smaller): unit lower (UPPER = false) or upper.  CTA b
-// inverts block b; thread j computes column j.
-constexpr int TRI_INV_SMEM = 2 * 64 * 65 * 8;
+// inverts block b; four threads of a warp hold a column, rows i % 4 each, and take it
+// column by column of the triangle (the row updates of a column do not depend on one
+// another; a dot product per entry by one thread a column took 58 us a launch for the
+// lower and 65 us for the upper triangle where this takes 32 for both).
+constexpr int TRI_INV_RS = 68;  // row stride of R: four columns of a half warp meet different banks
+constexpr int TRI_INV_SMEM = (64 * 65 + 64 * TRI_INV_RS + 64) * 8;
 
 template <bool UPPER>
-__global__ void __launch_bounds__(64) tri_inv_block_kernel(float *X0, int64_t ldx, int n) {
-  extern __shared__ float2 tri_smem[];
-  float2(*T)[65] = reinterpret_cast<float2(*)[65]>(tri_smem);            // T[col][row]
-  float2(*R)[65] = reinterpret_cast<float2(*)[65]>(tri_smem + 64 * 65);  // R[col][row]
-  const int o = blockIdx.x * 64, w = min(64, n - o);
-  float *X = X0 + 2 * ((int64_t)o + ldx * o);
-  const int j = threadIdx.x;
-  for (int c = 0; c < w; c++)
-    if (j < w) T[c][j] = reinterpret_cast<const float2 *>(X)[j + ldx * (int64_t)c];
+__device__ __forceinline__ void tri_inv_block(float *X0, int64_t ldx, int n, float2 *tri_smem) {
+  float2(*T)[65] = reinterpret_cast<float2(*)[65]>(tri_smem);                            // T[col][row]
+  float2(*R)[TRI_INV_RS] = reinterpret_cast<float2(*)[TRI_INV_RS]>(tri_smem + 64 * 65);  // R[col][row]
+  float2 *rd = tri_smem + 64 * 65 + 64 * TRI_INV_RS;                                     // reciprocal diagonal (upper)
+  const int o = blockIdx.x * 64, w = min(64, n - o), tid = threadIdx.x;
+  float2 *X = reinterpret_cast<float2 *>(X0) + o + ldx * o;
+#pragma unroll
+  for (int e = 0; e < 16; e++) {
+    const int r = tid & 63, c = (tid >> 6) + 4 * e;
+    if (r < w && c < w) T[c][r] = X[r + ldx * (int64_t)c];
+    R[c][r] = make_float2(r == c ? 1.f : 0.f, 0.f);
+  }
   __syncthreads();
-  if (j < w) {
-    if (!UPPER) {
-      for (int i = 0; i < w; i++) R[j][i] = make_float2(i == j ? 1.f : 0.f, 0.f);
-      for (int i = j + 1; i < w; i++) {  // x_i = -sum_{j <= k < i} L_ik x_k
-        float sr = 0.f, si = 0.f;
-        for (int k = j; k < i; k++) {
-          const float2 l = T[k][i], x = R[j][k];
-          sr += l.x * x.x - l.y * x.y;
-          si += l.x * x.y + l.y * x.x;
+  if (UPPER) {
+    if (tid < w) {
+      const float2 d = T[tid][tid];
+      const float dd = d.x * d.x + d.y * d.y;
+      rd[tid] = make_float2(d.x / dd, -d.y / dd);
+    }
+    __syncthreads();
+  }
+  const int j = tid >> 2, p = tid & 3, j0 = (tid & ~31) >> 2;  // column, share of its rows, the warp's first column
+  float2 *x = R[j];
+  if (!UPPER) {
+    for (int k = j0; k < w; k++) {
+      const float2 xk = x[k];
+      if (k >= j && j < w)
+#pragma unroll 4
+        for (int i = k + 1 + ((p - k - 1) & 3); i < w; i += 4) {
+          const float2 l = T[k][i];
+          float2 v = x[i];
+          v.x -= l.x * xk.x - l.y * xk.y;
+          v.y -= l.x * xk.y + l.y * xk.x;
+          x[i] = v;
         }
-        R[j][i] = make_float2(-sr, -si);
-      }
-    } else {
-      for (int i = 0; i < w; i++) R[j][i] = make_float2(0.f, 0.f);
-      {
-        const float2 d = T[j][j];
-        const float dd = d.x * d.x + d.y * d.y;
-        R[j][j] = make_float2(d.x / dd, -d.y / dd);
-      }
-      for (int i = j - 1; i >= 0; i--) {  // x_i = -(sum_{i < k <= j} U_ik x_k) / U_ii
-        float sr = 0.f, si = 0.f;
-        for (int k = i + 1; k <= j; k++) {
-          const float2 u = T[k][i], x = R[j][k];
-          sr += u.x * x.x - u.y * x.y;
-          si += u.x * x.y + u.y * x.x;
+      __syncwarp();
+    }
+  } else {
+    for (int k = min(w - 1, j0 + 7); k >= 0; k--) {
+      const float2 s = x[k], d = rd[k];
+      const float2 xk = make_float2(s.x * d.x - s.y * d.y, s.x * d.y + s.y * d.x);
+      __syncwarp();
+      if (k <= j && j < w) {
+        if (p == (k & 3)) x[k] = xk;
+#pragma unroll 4
+        for (int i = p; i < k; i += 4) {
+          const float2 u = T[k][i];
+          float2 v = x[i];
+          v.x -= u.x * xk.x - u.y * xk.y;
+          v.y -= u.x * xk.y + u.y * xk.x;
+          x[i] = v;
         }
-        const float2 d = T[i][i];
-        const float dd = d.x * d.x + d.y * d.y;
-        // -(s / d) = -(s conj(d)) / |d|^2
-        R[j][i] = make_float2(-(sr * d.x + si * d.y) / dd, -(si * d.x - sr * d.y) / dd);
       }
+      __syncwarp();
     }
   }
   __syncthreads();
-  for (int c = 0; c < w; c++)
-    if (j < w) reinterpret_cast<float2 *>(X)[j + ldx * (int64_t)c] = R[c][j];
+#pragma unroll
+  for (int e = 0; e < 16; e++) {
+    const int r = tid & 63, c = (tid >> 6) + 4 * e;
+    if (r < w && c < w) X[r + ldx * (int64_t)c] = R[c][r];
+  }
 }
 
-// Copies the unit-lower factor (UPPER = false: ones on the diagonal, zeros
-// above) or the upper factor (zeros below) of the packed LU into D.
-template <bool UPPER>
-__global__ void tri_extract_kernel(const float *__restrict__ LU, int64_t ld, int n, float *__restrict__ D) {
+// Both triangles: blockIdx.y 0 lower, 1 upper.
+__global__ void __launch_bounds__(256) tri_inv_block_kernel(float *L, float *U, int64_t ldx, int n) {
+  extern __shared__ float2 tri_smem[];
+  if (blockIdx.y == 0)
+    tri_inv_block<false>(L, ldx, n, tri_smem);
+  else
+    tri_inv_block<true>(U, ldx, n, tri_smem);
+}
+
+// The unit-lower factor (ones on the diagonal, zeros above) and the upper factor
+// (zeros below) of the packed LU.
+__global__ void tri_extract_kernel(const float *__restrict__ LU, int64_t ld, int n, float *__restrict__ L,
+                                   float *__restrict__ U) {
   const int r = blockIdx.x * blockDim.x + threadIdx.x;
   const int c = blockIdx.y;
   if (r >= n) return;
-  float2 v = reinterpret_cast<const float2 *>(LU)[r + ld * (int64_t)c];
-  if (!UPPER) {
-    if (r < c) v = make_float2(0.f, 0.f);
-    if (r == c) v = make_float2(1.f, 0.f);
-  } else if (r > c) {
-    v = make_float2(0.f, 0.f);
-  }
-  reinterpret_cast<float2 *>(D)[r + (int64_t)n * c] = v;
+  const float2 v = reinterpret_cast<const float2 *>(LU)[r + ld * (int64_t)c], zero = make_float2(0.f, 0.f);
+  const int64_t i = r + (int64_t)n * c;
+  reinterpret_cast<float2 *>(L)[i] = r > c ? v : r == c ? make_float2(1.f, 0.f) : zero;
+  reinterpret_cast<float2 *>(U)[i] = r > c ? zero : v;
 }
 
 // In-place inversion of a triangle X (n x n, ld n) whose 64 x 64 diagonal
@@ -2065,26 +2090,22 @@ int bem_ctri_inverses(bemgpu_ctx_s *ctx, const float *LU, int64_t ld, int n, flo
   float *tmp = (float *)bem_workspace(ctx, "tri_tmp", 8 * (size_t)(n / 2 + NB) * (size_t)(n / 2 + NB));
   if (!tmp) return bem_fail(ctx, BEMGPU_ERR_OOM, "tri_inverses: workspace");
   {
-    ProfScope ps(ctx, BEMGPU_K_TRSM, st, 0.0, 32.0 * (double)n * n);
+    ProfScope ps(ctx, BEMGPU_K_TRSM, st, 0.0, 24.0 * (double)n * n);
     const dim3 g((n + 255) / 256, n);
-    tri_extract_kernel<false><<<g, 256, 0, st>>>(LU, ld, n, Linv);
-    tri_extract_kernel<true><<<g, 256, 0, st>>>(LU, ld, n, Uinv);
-    ctx->launches += 2;
+    tri_extract_kernel<<<g, 256, 0, st>>>(LU, ld, n, Linv, Uinv);
+    ctx->launches++;
   }
   {
     static bool attr[64] = {false};
     if (!attr[ctx->device]) {
-      BEM_CUDA_TRY(ctx, cudaFuncSetAttribute(tri_inv_block_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             TRI_INV_SMEM));
-      BEM_CUDA_TRY(ctx, cudaFuncSetAttribute(tri_inv_block_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+      BEM_CUDA_TRY(ctx, cudaFuncSetAttribute(tri_inv_block_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                              TRI_INV_SMEM));
       attr[ctx->device] = true;
     }
     const int nb = (n + NB - 1) / NB;
     ProfScope ps(ctx, BEMGPU_K_TRSM, st, 2.0 * nb * 4.0 * NB * NB * NB / 3.0, 2.0 * 16.0 * NB * (double)n);
-    tri_inv_block_kernel<false><<<nb, 64, TRI_INV_SMEM, st>>>(Linv, n, n);
-    tri_inv_block_kernel<true><<<nb, 64, TRI_INV_SMEM, st>>>(Uinv, n, n);
-    ctx->launches += 2;
+    tri_inv_block_kernel<<<dim3(nb, 2), 256, TRI_INV_SMEM, st>>>(Linv, Uinv, n, n);
+    ctx->launches++;
   }
   int rc = tri_inv_bottom_up(ctx, false, Linv, n, tmp, st);
   if (!rc) rc = tri_inv_bottom_up(ctx, true, Uinv, n, tmp, st);
