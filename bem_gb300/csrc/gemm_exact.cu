@@ -116,6 +116,28 @@ struct ExMaps {
   CUtensorMap b[5];
 };
 
+// Eight columns of a row of C from column c: scale (hi + lo + z3 + z4), [+ C].  The old
+// values are loaded together: one after the other, each behind the store before it,
+// the 32 loads of a tile's row took half of a small product's time (m = k = 288, n =
+// 144, 3 x 3, accumulating: 27.0 -> 23.2 us).
+__device__ __forceinline__ void ex_store8(double *C, int64_t ldcf, int c, int nvalid, int accumulate, double scale,
+                                          const uint64_t *hi, const uint64_t *lo, const float *z3, const float *z4) {
+  double old[8];
+#pragma unroll
+  for (int j = 0; j < 8; j++) old[j] = accumulate && c + j < nvalid ? C[ldcf * (int64_t)(c + j)] : 0.0;
+#pragma unroll
+  for (int j = 0; j < 8; j += 2) {
+    double v[2];
+    f2_sum(hi[j / 2], lo[j / 2], v[0], v[1]);
+#pragma unroll
+    for (int e = 0; e < 2; e++)
+      if (c + j + e < nvalid) {
+        const double w = scale * (v[e] + ((double)z3[j + e] + (double)z4[j + e]));
+        C[ldcf * (int64_t)(c + j + e)] = accumulate ? old[j + e] + w : w;
+      }
+  }
+}
+
 template <int SA, int SB>
 __global__ void __launch_bounds__(EX_THREADS, 1)
     ex_gemm_kernel(const __grid_constant__ ExMaps maps, int ktiles, double *__restrict__ C, int64_t ldcf, int mvalid,
@@ -274,22 +296,8 @@ __global__ void __launch_bounds__(EX_THREADS, 1)
         tc_ld8(lane_base + (uint32_t)(6 * EX_BN) + 8 * q, z3);
         if (SA > 4) tc_ld8(lane_base + (uint32_t)(7 * EX_BN) + 8 * q, z4);
       }
-      if (ok && rho < mvalid) {
-#pragma unroll
-        for (int j = 0; j < 8; j += 2) {
-          double v[2];
-          f2_sum(hi[4 * q + j / 2], lo[4 * q + j / 2], v[0], v[1]);
-#pragma unroll
-          for (int e = 0; e < 2; e++) {
-            const int c = n0 + group * 32 + 8 * q + j + e;
-            if (c < nvalid) {
-              double *p = C + rho + ldcf * (int64_t)c;
-              const double w = scale * (v[e] + ((double)z3[j + e] + (double)z4[j + e]));
-              *p = accumulate ? *p + w : w;
-            }
-          }
-        }
-      }
+      if (ok && rho < mvalid)
+        ex_store8(C + rho, ldcf, n0 + group * 32 + 8 * q, nvalid, accumulate, scale, hi + 4 * q, lo + 4 * q, z3, z4);
     }
   }
   asm volatile("tcgen05.fence::before_thread_sync;");
