@@ -114,10 +114,10 @@ struct bemgpu_ctx_s {
     int near_minb = 3;   // CTAs per SM of the double-float near-pair kernel's register budget (2, 3, 4)
     int far_rows = 4;    // warps per CTA of the far-pair kernel (1, 2, 4, 8)
     int raster = 8;      // M-tiles per rasterization band of the tensor-core products (1..64)
-    int panel_ctas = 0;  // CTAs of a cooperative LU panel at most (0: one per SM)
-    int near_sync = 1;   // double-float near-pair CTAs barrier after each pair couple (0, 1)
+    int panel_ctas = 0;  // CTAs of an LU panel at most (0: 16 of a cluster, one per SM in a cooperative panel)
+    int near_sync = 1;   // double-float near-pair CTAs barrier after each pair (0, 1)
     int near_grid = 16;  // CTAs per SM in the near-pair launch's grid at most (1..64)
-    int ex_wide = 1;     // exact products with level-3/4 work on 128 x 128 tiles: 0 never, 1 large grids, 2 always
+    int ex_wide = 1;     // exact products of 4 and 5 slices on wide tiles: 0 never, 1 by the grid, 2 always
     int lu_super = 1;    // complex64 LU panels in pairs, trailing updates of K = 256 (0, 1)
   } tune;
   double escalate_tol = 1e-6;  // complex64 refinement error estimate above which the solve escalates

@@ -196,8 +196,8 @@ void bem_build_near_pairs(const bemgpu_tree_s *t, const bemgpu_tree_s *s, std::v
   }
   // Self pairs (no neighbour-edge correction, a shorter finish) first, then
   // coplanar pairs (every outer node takes the in-plane branch of the
-  // close-pair contraction), then the rest, so that the near-pair kernels'
-  // CTAs, which barrier after each pair couple, take couples of one kind.
+  // close-pair contraction), then the rest, so that the warps of a near-pair
+  // CTA, which barrier after each pair, take pairs of one kind.
   // Each pair writes its own half-pair slots: the order changes no result.
   auto kind = [&](const NearPair &p) {
     if (p.same) return 0;

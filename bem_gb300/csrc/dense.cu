@@ -5,12 +5,12 @@
 // All matrices are column-major with interleaved (re, im) values, as the
 // reference's ComplexDenseMatrix stores them (src/util/DenseMatrix.h:195-198).
 //
-// LU: right-looking, panel width NB.  The panel is factored one column per
-// launch (scale + rank-1 update of the panel + pivot search across CTAs, the
-// last CTA to finish reduces the pivot and swaps the rows inside the panel),
-// then the row interchanges are applied outside the panel, the U12 block is
-// solved with the unit-lower L11 (warp per right-hand side, L11 in shared
-// memory) and the trailing matrix is updated by the complex GEMM.
+// LU: right-looking, panel width 64 (complex128) or 128 (complex64, in pairs).  A
+// panel is factored by one thread-block cluster with its rows in registers
+// (panel_cluster_kernel; a cooperative grid beyond 16384 rows), then the row
+// interchanges are applied outside the panel, the U12 block is solved with the
+// unit-lower L11 (tri_block_kernel) and the trailing matrix is updated by the
+// complex GEMM.
 // Pivot choice is LAPACK's: the first row of largest |re|+|im| (izamax).
 #include "bemgpu_internal.h"
 
@@ -1296,6 +1296,9 @@ template <typename T, bool CONJ_A>
 void launch_gemm_fma(bemgpu_ctx_s *ctx, int m, int n, int k, cx<T> alpha, const T *A, int64_t lda, const T *B, int64_t ldb,
                      cx<T> beta, T *C, int64_t ldc, cudaStream_t st, int nb = 1, int64_t sA = 0, int64_t sB = 0,
                      int64_t sC = 0) {
+  constexpr int MAX_COLS = 65535 * 16;  // what a grid of the narrowest tiles covers
+  for (; n > MAX_COLS; n -= MAX_COLS, B += 2 * ldb * (int64_t)MAX_COLS, C += 2 * ldc * (int64_t)MAX_COLS)
+    launch_gemm_fma<T, CONJ_A>(ctx, m, MAX_COLS, k, alpha, A, lda, B, ldb, beta, C, ldc, st, nb, sA, sB, sC);
   auto grid = [&](int bm, int bn) { return dim3((m + bm - 1) / bm, (n + bn - 1) / bn, nb); };
   if constexpr (sizeof(T) == 8) {
     cgemm_fma_kernel<double, 16, 16, 1, 2, 16, CONJ_A>

@@ -135,22 +135,24 @@ int bemgpu_ctx_set_fp64_fallback_tol(bemgpu_ctx_t ctx, double tol);
  *   BEMGPU_TUNE_FAR_ROWS   warps per CTA of the far-pair kernel: 1, 2, 4 (default), 8;
  *   BEMGPU_TUNE_RASTER     M-tiles per rasterization band of the tensor-core
  *                          products: 1..64 (default 8);
- *   BEMGPU_TUNE_PANEL_CTAS CTAs of a cooperative LU panel at most (fewer,
- *                          fuller CTAs leave SMs to other lanes' work while a
- *                          latency-bound panel runs): 0 (one per SM, default)
- *                          or a cap, raised where shared memory requires;
+ *   BEMGPU_TUNE_PANEL_CTAS CTAs of an LU panel at most (fewer, fuller CTAs
+ *                          leave SMs to other lanes' work while a
+ *                          latency-bound panel runs): 0 (default: up to 16 of a
+ *                          cluster, one per SM in a cooperative panel) or a
+ *                          cap, raised where registers or shared memory require;
  *   BEMGPU_TUNE_NEAR_SYNC  1 (default): the double-float near-pair kernel's
- *                          CTAs barrier after each pair couple, keeping their
- *                          warps in the same code region; 0: no barrier;
+ *                          CTAs barrier after each pair, keeping their warps in
+ *                          the same code region; 0: no barrier;
  *   BEMGPU_TUNE_NEAR_GRID  CTAs per SM of the near-pair launch's grid at most:
  *                          1..64 (default 16);
- *   BEMGPU_TUNE_EX_WIDE    1 (default): the exact products with level-3/4
- *                          slice products (5 x 2, 5 x 3, 4 x 4) on 128 x 128
- *                          tiles when that grid has at least 4 waves; 2:
- *                          on 128 x 128 tiles at any size; 0: all on
- *                          128 x 64 tiles.  The two differ in the last bits
- *                          of an FP32 sum (levels 3 and 4 in one buffer or
- *                          two), well inside the products' 2^-40 accuracy;
+ *   BEMGPU_TUNE_EX_WIDE    1 (default): the exact products of 5 x 2, 5 x 3 and
+ *                          4 x 4 slices on 128 x 128 tiles when that grid
+ *                          has at least 4 waves, those of 5 x 5 slices on
+ *                          128 x 96 tiles where their waves take less; 2: on
+ *                          those tiles at any size; 0: all on 128 x 64 tiles.
+ *                          On 128 x 128 tiles the levels from 3 (4 x 4: from
+ *                          2) up share one FP32 sum, which changes the last
+ *                          bits; the others are the same;
  *   BEMGPU_TUNE_LU_SUPER   1 (default): the complex64 LU factors its 128-wide
  *                          panels in pairs and updates the trailing matrix
  *                          once per pair (K = 256); 0: after every panel.

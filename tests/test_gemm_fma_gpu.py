@@ -10,9 +10,10 @@ pytestmark = pytest.mark.gpu
 
 
 # 32 x 32, 64 x 64 and 128 x 64 tiles (by their waves on the GPU's SMs), each with edges
-# inside a tile, and K of one, less than one and several steps
+# inside a tile, and K of one, less than one and several steps; more columns than one
+# launch covers
 @pytest.mark.parametrize("m,n,k", [(1, 1, 1), (31, 33, 15), (33, 32, 17), (129, 65, 16), (700, 500, 33), (769, 641, 7),
-                                   (2049, 1025, 24), (2500, 1300, 9)])
+                                   (2049, 1025, 24), (2500, 1300, 9), (2, 1048600, 3)])
 @pytest.mark.parametrize("accumulate", [0, 1])
 def test_cgemm_fma_tiles(m, n, k, accumulate):
     """A sum of k complex products in FP32 is off by at most (2 k + 2) roundings of the sum of
