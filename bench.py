@@ -242,18 +242,18 @@ def peaks():
 FP64_NOMINAL_TFLOPS = 1.25
 # FP32 lanes of the GPU (152 SMs x 128): the issue rate of the double-float fill.
 FP32_LANES = 152 * 128
-# FP32-pipe thread instructions per algorithmic FP64-class flop of the
-# double-float fill kernels, from ncu's smsp__inst_executed on the ico2
-# workload (one launch each over the three fills of a solve): near pairs 7.76
-# (6.24e9 warp instructions, 16400 pairs x 1.57 Mflop), far pairs 7.2 (1.01e9
-# warp instructions for 598000 pairs, 5 % more per pair than the 6.85 counted
-# on the exterior fill alone with the rules' frozen flop counts).
-DF_INSTR_PER_FLOP = {"fill_near": 7.76, "fill_far": 7.2}
+# Thread instructions per algorithmic FP64-class flop of the double-float fill
+# kernels (the frozen counts of the rules), from ncu's smsp__inst_executed on one
+# solve of this workload (N = 7680): near pairs 1.12 (3.63e9 warp instructions, 66320
+# pairs x 1.57 Mflop; both Green's functions of a pair in one pass, by series), far
+# pairs 2.0 (4.58e9 for 7.33e10 flops; each unordered pair once).  Requests whose
+# interior |k| R leaves the series take more near-pair instructions: 3.8 a flop on
+# an ico2 request half of whose passes are direct.
+DF_INSTR_PER_FLOP = {"fill_near": 1.12, "fill_far": 2.0}
 # DRAM bytes of the fill (far and near launch together) per matrix entry of the
-# three Zts outputs, from ncu on the ico2 workload: 246.7 MB (far 118.2 MB +
-# near 128.5 MB) for 5.53 M entries; the half-pair blocks the fill writes are
-# 32 B per entry (177 MB), so the measured traffic is 1.39x the algorithmic.
-FILL_DRAM_BYTES_PER_ENTRY = 44.6
+# three Zts outputs, from ncu on the ico2 workload: 186.4 MB for 5.53 M entries; the
+# half-pair blocks the fill writes are 32 B per entry (177 MB).
+FILL_DRAM_BYTES_PER_ENTRY = 33.7
 # The exact product's DRAM bytes against the library's operand-traffic model
 # (its ProfScope bytes: A re-read once per band of N-tiles, B once, C written):
 # ncu 313.7 MB against 327 MB modelled for ex_gemm_kernel<5, 3> at ico2.
@@ -649,7 +649,7 @@ def group_roofline(dom, stats, precision, pk, pk_kind, fp64class=False, sm_mhz=N
                     note="the fill is FP64-class arithmetic in double-float on the FP32 pipes: its algorithmic "
                          "FP64-class flops (frozen count, live) per CUDA-event second times the FP32-pipe "
                          "thread instructions per algorithmic flop that ncu counted on each fill kernel "
-                         "(smsp__inst_executed, ico2)")
+                         "(smsp__inst_executed, one solve of N = 7680)")
     if bound == "tensor":
         if dom == "ex_gemm":
             base["traffic"] = EX_TRAFFIC_PER_MODEL_BYTE * by / max(1, n)
@@ -937,10 +937,9 @@ def main():
                     help="launch shapes from the autotuner's cache (tuned first when missing), re-tuned, or the "
                          "library defaults")
     ap.add_argument("--ex-wide", type=int, default=None, choices=[0, 1, 2],
-                    help="exact products' 128 x 128 tiles: 0 never, 1 grids of 4 waves or more (the library's "
-                         "default), 2 always")
+                    help="exact products' wide tiles: 0 never, 1 by the grid (the library's default), 2 always")
     ap.add_argument("--panel-ctas", type=int, default=0,
-                    help="CTAs of a cooperative LU panel at most (0: one per SM)")
+                    help="CTAs of an LU panel at most (0: the library's choice)")
     ap.add_argument("--lite", action="store_true",
                     help="skip the end-to-end and per-kernel segments (sub-workload runs)")
     args = ap.parse_args()
