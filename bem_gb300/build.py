@@ -17,7 +17,8 @@ LIB = os.path.join(HERE, "libbemgpu.so")
 
 SOURCES = ["context.cu", "fill.cu", "dense.cu", "gemm_tc.cu", "gemm_exact.cu", "mixed.cu", "heat_transfer.cu", "farm.cu",
            "mesh_device.cu"]
-HEADERS = ["bemgpu_internal.h", "quadrature_tables.h", "tc_common.cuh", "df64.cuh", "fill_num.cuh", "even_rules.h", "df_constants.h", os.path.join("..", "..", "include", "bemgpu.h")]
+HEADERS = ["bemgpu_internal.h", "quadrature_tables.h", "tc_common.cuh", "df64.cuh", "fill_num.cuh", "even_rules.h", "df_constants.h",
+           "panel_slots.h", os.path.join("..", "..", "include", "bemgpu.h")]
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_103a,code=sm_103a",

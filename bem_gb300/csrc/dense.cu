@@ -13,6 +13,7 @@
 // complex GEMM.
 // Pivot choice is LAPACK's: the first row of largest |re|+|im| (izamax).
 #include "bemgpu_internal.h"
+#include "panel_slots.h"
 
 #include <algorithm>
 #include <mutex>
@@ -671,7 +672,8 @@ __global__ void __launch_bounds__(CP_MAX_THREADS, 1)
   T2 *LU = reinterpret_cast<T2 *>(msg + (2 * CP_MAX_CLUSTER + 1) * MSG);   // [SW][ROW] the factored diagonal block
   T2 *P = LU + SW * ROW;                                                   // [chunk][ROW] the CTA's rows, final values
   __shared__ __align__(8) unsigned long long bars[2];
-  __shared__ unsigned s_hi[CP_MAX_THREADS / 32], s_lo[CP_MAX_THREADS / 32], s_pos[CP_MAX_THREADS / 32];
+  constexpr int WARPS = CP_MAX_THREADS / 32;  // the warps' candidates, by panel_slot_set()
+  __shared__ unsigned s_hi[PANEL_SLOT_SETS][WARPS], s_lo[PANEL_SLOT_SETS][WARPS], s_pos[PANEL_SLOT_SETS][WARPS];
   __shared__ int s_piv[SW];
   __shared__ volatile int s_abort;
   const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5, nt = blockDim.x, nwarps = nt >> 5;
@@ -726,15 +728,16 @@ __global__ void __launch_bounds__(CP_MAX_THREADS, 1)
       cp = better ? q : cp;
     }
     cp_reduce<T>(hi, lo, cp);
+    const int set = panel_slot_set(j);
     if (lane == 0) {
-      s_hi[wid] = hi;
-      s_lo[wid] = lo;
-      s_pos[wid] = cp;
+      s_hi[set][wid] = hi;
+      s_lo[set][wid] = lo;
+      s_pos[set][wid] = cp;
     }
     __syncthreads();
-    hi = lane < nwarps ? s_hi[lane] : 0u;
-    lo = lane < nwarps ? s_lo[lane] : 0u;
-    cp = lane < nwarps ? s_pos[lane] : 0xffffffffu;
+    hi = lane < nwarps ? s_hi[set][lane] : 0u;
+    lo = lane < nwarps ? s_lo[set][lane] : 0u;
+    cp = lane < nwarps ? s_pos[set][lane] : 0xffffffffu;
     cp_reduce<T>(hi, lo, cp);
     // 2. its warp sends the row (warp 0 an empty message when there is none)
     int own = -1;
