@@ -599,10 +599,11 @@ __device__ __forceinline__ void cp_send16(uint32_t dst, uint32_t bar, uint4 v) {
                "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w), "r"(bar)
                : "memory");
 }
+// The messages come from other CTAs: acquired at the cluster's scope, as the stores' completion releases them.
 __device__ __forceinline__ bool cp_try_wait(uint32_t bar, unsigned parity) {
   unsigned ok;
   asm volatile(
-      "{\n .reg .pred p;\n mbarrier.try_wait.parity.acquire.cta.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}\n"
+      "{\n .reg .pred p;\n mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}\n"
       : "=r"(ok)
       : "r"(bar), "r"(parity)
       : "memory");
