@@ -814,7 +814,9 @@ __global__ void __launch_bounds__(CP_MAX_THREADS, 1)
     const int wc = win ? __ffs(win) - 1 : 0;
     const CpHeader<T> *hd = reinterpret_cast<const CpHeader<T> *>(in + wc * MSG);
     const T2 *u = reinterpret_cast<const T2 *>(in + wc * MSG + sizeof(CpHeader<T>));  // columns j, j + 1, ...
-    const unsigned pv = none ? dr : hd->pos;
+    // (clamped: after a wait that ran out the message may be of any content, and a
+    // position addresses rows)
+    const unsigned pv = none ? dr : min(hd->pos, (unsigned)n - 1u);
     if (tid == 0) {
       s_piv[j] = s_abort ? (int)dr : (int)pv;
       if (g == 0) {
