@@ -583,29 +583,43 @@ namespace {
 
 // Largest FP64 exponent field of max(|re|, |im|) over a complex128 matrix
 // (m x k, column-major) -> *out (atomicMax).  Bound by the read of the matrix: a CTA
-// takes chunks of a column, eight loads a thread in flight and a division a chunk
-// instead of one an element (7680 x 7680: 422 -> 151 us).
-constexpr int EX_CHUNK = 2048;
-__global__ void __launch_bounds__(256) ex_absmax_kernel(const double *__restrict__ A, int64_t lda, int m, int k,
-                                                        unsigned *out) {
+// takes chunks of 2048 elements, eight loads a thread in flight and a division a
+// chunk instead of one an element (7680 x 7680: 422 -> 151 us).  A chunk is as
+// many rows as the columns have, up to 2048, rounded up to a power of two (2^lw
+// threads along a column, 2^ly of the eight loads) and columns for the rest.  With
+// one column a chunk, short ones left most threads idle and each CTA many
+// dependent rounds; all of an operand pair's slicing then and now: 1 x 60000 by 60000 x 2 161
+// and 63 us, 300 x 30 by 30 x 20000 81 and 41, 64 x 7680 by 7680 x 64 46 and 38.
+constexpr int EX_LOADS = 3;  // log2 of a thread's loads per chunk
+__global__ void __launch_bounds__(256) ex_absmax_kernel(const double *__restrict__ A, int64_t lda, int m, int k, int lw,
+                                                        int ly, unsigned *out) {
   unsigned mx = 0;
-  const int per_col = (m + EX_CHUNK - 1) / EX_CHUNK;
-  const int64_t chunks = (int64_t)per_col * k;
-  for (int64_t i = blockIdx.x; i < chunks; i += gridDim.x) {
-    const int64_t c = i / per_col;
-    const int r0 = (int)(i - c * per_col) * EX_CHUNK + threadIdx.x;
-    const uint4 *col = reinterpret_cast<const uint4 *>(A) + lda * c;
+  const int rows = 1 << (lw + ly), cols = 1 << (8 - lw + EX_LOADS - ly);  // of a chunk
+  const int per_col = (m + rows - 1) / rows;
+  const int chunks = per_col * ((k + cols - 1) / cols);
+  const int tr = threadIdx.x & ((1 << lw) - 1), tc = threadIdx.x >> lw;
+  for (int i = blockIdx.x; i < chunks; i += gridDim.x) {
+    const int q = i / per_col;
+    const int r0 = (i - q * per_col) * rows + tr, c0 = q * cols + tc;
 #pragma unroll
-    for (int e = 0; e < EX_CHUNK / 256; e++) {
-      const int r = r0 + 256 * e;
-      if (r < m) {
-        const uint4 v = col[r];  // the high words hold the exponents
+    for (int e = 0; e < 1 << EX_LOADS; e++) {
+      const int r = r0 + ((e & ((1 << ly) - 1)) << lw), c = c0 + ((e >> ly) << (8 - lw));
+      if (r < m && c < k) {
+        const uint4 v = reinterpret_cast<const uint4 *>(A)[r + lda * c];  // the high words hold the exponents
         mx = max(mx, max((v.y >> 20) & 0x7ff, (v.w >> 20) & 0x7ff));
       }
     }
   }
   mx = __reduce_max_sync(0xffffffffu, mx);
   if ((threadIdx.x & 31) == 0 && mx > 0) atomicMax(out, mx);
+}
+
+void launch_absmax(bemgpu_ctx_s *ctx, const double *A, int64_t lda, int m, int k, unsigned *out, cudaStream_t st) {
+  int lw = 0, ly = 0;
+  while (lw < 8 && (1 << lw) < m) lw++;
+  while (ly < EX_LOADS && (1 << (lw + ly)) < m) ly++;
+  ex_absmax_kernel<<<2 * 152, 256, 0, st>>>(A, lda, m, k, lw, ly, out);
+  ctx->launches++;
 }
 
 // Scaling exponent g of the matrix whose largest exponent field is *amax:
@@ -822,8 +836,7 @@ int bem_exact_prep(bemgpu_ctx_s *ctx, const char *name, bool is_a, const double 
   {
     ProfScope ps(ctx, BEMGPU_K_SLICE, st, 0.0, 16.0 * (double)rows * k * 2 + 4.0 * slices * (double)rp * kp);
     BEM_CUDA_TRY(ctx, cudaMemsetAsync(amax, 0, sizeof(unsigned), st));
-    ex_absmax_kernel<<<2 * 152, 256, 0, st>>>(M, ld, is_a ? rows : k, is_a ? k : rows, amax);
-    ctx->launches++;
+    launch_absmax(ctx, M, ld, is_a ? rows : k, is_a ? k : rows, amax, st);
     const dim3 grid((unsigned)((kp / 2 + 127) / 128), (unsigned)(is_a ? rp / 2 / EX_PREP_ROWS : rp));
     __nv_bfloat16 *S = (__nv_bfloat16 *)op.S;
     if (is_a) {
