@@ -1149,14 +1149,18 @@ __global__ void __launch_bounds__(TriCfg<T>::THREADS) tri_block_kernel(const T *
 }
 
 // ---------------- complex GEMM (FMA pipes) ----------------
-// C = alpha op(A) B + beta C, BM x BN complex tile per CTA, TM x TN per thread.  The
-// next BK-deep K step is loaded into registers while one is multiplied from
-// shared memory (two buffers, one barrier a step).
+// C = alpha op(A) B + beta C, BM x BN complex tile per CTA, TM x TN per thread, MINB
+// CTAs per SM (0: as many registers as it takes).  AHEAD: the next BK-deep K step is loaded into registers while one is
+// multiplied from shared memory (two buffers, one barrier a step).  Not in 128 x 64
+// FP32 tiles, whose 64 sums a thread leave no registers for it: with 139 of them one CTA was
+// resident where two hide each other's loads better (2500^3 3.66 ms against 2.98; the
+// accumulating 4096 x 4096 x 512 1.94 against 1.51).
 // COMP: the FP32 sums of each BK-deep K tile are added into a two-float
 // (hi + lo) running sum (TwoSum), so accumulation error does not grow with K;
 // TC is the output type (double to accumulate FP32 products into an FP64 C).
-template <typename T, int BM, int BN, int TM, int TN, int BK, bool CONJ_A, typename TC = T, bool COMP = false>
-__global__ void __launch_bounds__((BM / TM) * (BN / TN))
+template <typename T, int BM, int BN, int TM, int TN, int BK, bool CONJ_A, int MINB, bool AHEAD, typename TC = T,
+          bool COMP = false>
+__global__ void __launch_bounds__((BM / TM) * (BN / TN), MINB)
     cgemm_fma_kernel(int m, int n, int k, cx<T> alpha, const T *__restrict__ A, int64_t lda, const T *__restrict__ B,
                      int64_t ldb, cx<TC> beta, TC *__restrict__ C, int64_t ldc, int64_t sA, int64_t sB, int64_t sC) {
   typedef typename V2<T>::type T2;
@@ -1167,8 +1171,9 @@ __global__ void __launch_bounds__((BM / TM) * (BN / TN))
   constexpr int TX = BN / TN, TY = BM / TM, THREADS = TX * TY;
   constexpr int PA = BM * BK / THREADS, PB = BN * BK / THREADS;  // elements a thread loads per K step
   static_assert(PA * THREADS == BM * BK && PB * THREADS == BN * BK, "whole loads");
-  __shared__ T2 As[2][BK][BM];
-  __shared__ T2 Bs[2][BK][BN];
+  constexpr int BUFS = AHEAD ? 2 : 1;
+  __shared__ T2 As[BUFS][BK][BM];
+  __shared__ T2 Bs[BUFS][BK][BN];
   const int tx = threadIdx.x % TX, ty = threadIdx.x / TX;
   const int m0 = blockIdx.x * BM, n0 = blockIdx.y * BN;
   const T2 *A2 = reinterpret_cast<const T2 *>(A);
@@ -1218,12 +1223,16 @@ __global__ void __launch_bounds__((BM / TM) * (BN / TN))
 #pragma unroll
       for (int b = 0; b < (COMP ? TN : 1); b++) { lo[a][b] = {0, 0}; part[a][b] = {0, 0}; }
   }
-  load(0);
+  if (AHEAD) load(0);
   int buf = 0;
-  for (int kk0 = 0; kk0 < k; kk0 += BK, buf ^= 1) {
+  for (int kk0 = 0; kk0 < k; kk0 += BK, buf ^= AHEAD) {
+    if (!AHEAD) {
+      if (kk0 > 0) __syncthreads();
+      load(kk0);
+    }
     store(buf);
-    __syncthreads();  // and everyone is done with the other buffer
-    if (kk0 + BK < k) load(kk0 + BK);
+    __syncthreads();  // and, with two buffers, everyone is done with the other one
+    if (AHEAD && kk0 + BK < k) load(kk0 + BK);
 #pragma unroll
     for (int kk = 0; kk < BK; kk++) {
       T2 a[TM], b[TN];
@@ -1294,10 +1303,11 @@ __global__ void __launch_bounds__((BM / TM) * (BN / TN))
 // the tiles fill the SMs: the 53 products of a complex128 solve of n = 1152 took 20.7 ms in
 // 64 x 64 tiles, 13.8 in 32 x 32, 12.3 in 32 x 16 and 11.5 in 16 x 16.
 //
-// FP32: the tile whose waves take least.  128 x 64 runs at the FMA pipes' rate, 64 x 64 at
-// about 0.9 of it and 32 x 32, bound by its reads of shared memory, at half; but the
-// joins of a triangle's inverse are a few small products, which left most SMs
-// idle in 128 x 64 tiles (the 12 of an n = 1152 solve 551 -> 205 us).
+// FP32: the tile whose waves take least.  64 x 64 runs at 0.86 of 128 x 64's rate (2500^3 3.20 and
+// 2.98 ms) and 32 x 32, bound by its reads of shared memory, at half; but 5000 x 300 x 300 takes 119 us in
+// 64 x 64 tiles, three to an SM, against 132, and the joins of a triangle's inverse
+// are a few small products, which left most SMs idle in 128 x 64 tiles
+// (the 12 of an n = 1152 solve 551 -> 205 us).
 template <typename T, bool CONJ_A>
 void launch_gemm_fma(bemgpu_ctx_s *ctx, int m, int n, int k, cx<T> alpha, const T *A, int64_t lda, const T *B, int64_t ldb,
                      cx<T> beta, T *C, int64_t ldc, cudaStream_t st, int nb = 1, int64_t sA = 0, int64_t sB = 0,
@@ -1307,7 +1317,7 @@ void launch_gemm_fma(bemgpu_ctx_s *ctx, int m, int n, int k, cx<T> alpha, const 
     launch_gemm_fma<T, CONJ_A>(ctx, m, MAX_COLS, k, alpha, A, lda, B, ldb, beta, C, ldc, st, nb, sA, sB, sC);
   auto grid = [&](int bm, int bn) { return dim3((m + bm - 1) / bm, (n + bn - 1) / bn, nb); };
   if constexpr (sizeof(T) == 8) {
-    cgemm_fma_kernel<double, 16, 16, 1, 2, 16, CONJ_A>
+    cgemm_fma_kernel<double, 16, 16, 1, 2, 16, CONJ_A, 0, true>
         <<<grid(16, 16), 128, 0, st>>>(m, n, k, alpha, A, lda, B, ldb, beta, C, ldc, sA, sB, sC);
   } else {
     auto cost = [&](int bm, int bn, double rate) {
@@ -1315,15 +1325,15 @@ void launch_gemm_fma(bemgpu_ctx_s *ctx, int m, int n, int k, cx<T> alpha, const 
       const int64_t tiles = (int64_t)g.x * g.y * g.z;
       return (double)((tiles + ctx->num_sms - 1) / ctx->num_sms) * bm * bn / rate;
     };
-    const double c0 = cost(128, 64, 1.0), c1 = cost(64, 64, 0.9), c2 = cost(32, 32, 0.55);
+    const double c0 = cost(128, 64, 1.0), c1 = cost(64, 64, 0.86), c2 = cost(32, 32, 0.55);
     if (c2 < c1 && c2 < c0)
-      cgemm_fma_kernel<float, 32, 32, 2, 2, 16, CONJ_A>
+      cgemm_fma_kernel<float, 32, 32, 2, 2, 16, CONJ_A, 0, true>
           <<<grid(32, 32), 256, 0, st>>>(m, n, k, alpha, A, lda, B, ldb, beta, C, ldc, sA, sB, sC);
     else if (c1 < c0)
-      cgemm_fma_kernel<float, 64, 64, 4, 4, 8, CONJ_A>
+      cgemm_fma_kernel<float, 64, 64, 4, 4, 8, CONJ_A, 3, true>
           <<<grid(64, 64), 256, 0, st>>>(m, n, k, alpha, A, lda, B, ldb, beta, C, ldc, sA, sB, sC);
     else
-      cgemm_fma_kernel<float, 128, 64, 8, 4, 8, CONJ_A>
+      cgemm_fma_kernel<float, 128, 64, 8, 4, 8, CONJ_A, 2, false>
           <<<grid(128, 64), 256, 0, st>>>(m, n, k, alpha, A, lda, B, ldb, beta, C, ldc, sA, sB, sC);
   }
   ctx->launches++;
@@ -1405,7 +1415,7 @@ int bem_cgemm_comp64_fma(bemgpu_ctx_s *ctx, int kind, int m, int n, int k, const
   cx<float> al = {alpha[0], alpha[1]};
   cx<double> be = {beta[0], beta[1]};
   ProfScope ps(ctx, kind, stream, 8.0 * m * n * k, 8.0 * ((double)m * k + (double)k * n) + 32.0 * m * n);
-  cgemm_fma_kernel<float, 64, 64, 4, 4, 8, false, double, true>
+  cgemm_fma_kernel<float, 64, 64, 4, 4, 8, false, 1, true, double, true>
       <<<grd, 256, 0, stream>>>(m, n, k, al, A, lda, B, ldb, be, C, ldc, 0, 0, 0);
   ctx->launches++;
   BEM_CUDA_TRY(ctx, cudaGetLastError());
