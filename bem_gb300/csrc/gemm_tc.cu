@@ -71,9 +71,11 @@ namespace {
 // of an LU update (K = 256) takes as long to read and write as its products, so a
 // tile's epilogue runs beside the next tile's products: the CTAs are persistent, the
 // accumulator is double-buffered, and a warp's next 32 columns of C are on their way
-// while it adds the last.  One tile per CTA, its epilogue after its products, took 697
-// us for 7680 x 7680 x 256 (accumulating) where this takes 443, and 6.25 ms for 7680 x 3840 x
-// 7680 where this takes 5.03 (2.16 PF/s of slice products).
+// while it adds the last (the pointers into C run along a row: with a product for each
+// element's address 261 x 2632 x 407, a single round, took 21.0 us instead of 19.2).  One tile per
+// CTA, its epilogue after its products, took 701 us for 7680 x 7680 x 256 (accumulating)
+// where this takes 404, and 6.2 ms for 7680 x 3840 x 7680 where this takes 5.03 (2.16 PF/s
+// of slice products).
 template <int BN>
 __global__ void __launch_bounds__(TC_THREADS, 1)
     tc_gemm_kernel(const __grid_constant__ TcMaps maps, int ktiles, int nM, int nN, float *__restrict__ C, int64_t ldcf,
@@ -196,15 +198,20 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
     for (int t = blockIdx.x; t < tiles; t += gridDim.x, i++) {
       const Tile x = tile_at(t);
       const int b = i & 1, rho = x.m0 + quarter * 32 + lane, c0 = x.n0 + half * (BN / 2);
+      const int cols = rho < mvalid ? nvalid - c0 : 0;  // of this thread's row
+      float *const row = C + rho + ldcf * (int64_t)c0;
       float old[32];
       auto load_old = [&](int q) {  // 32 columns of C, all loads in flight together
+        const float *p = row + ldcf * (int64_t)(32 * q);
 #pragma unroll
-        for (int j = 0; j < 32; j++) {
-          const int c = c0 + 32 * q + j;
-          old[j] = (accumulate && rho < mvalid && c < nvalid) ? C[rho + ldcf * (int64_t)c] : 0.f;
-        }
+        for (int j = 0; j < 32; j++, p += ldcf) old[j] = 32 * q + j < cols ? *p : 0.f;
       };
-      load_old(0);
+      if (accumulate) {
+        load_old(0);
+      } else {
+#pragma unroll
+        for (int j = 0; j < 32; j++) old[j] = 0.f;
+      }
       int got = 1;
       if (lane == 0) got = mbar_wait(&accf[b], (i >> 1) & 1, err) ? 1 : 0;
       got = __shfl_sync(0xffffffffu, got, 0);
@@ -219,17 +226,13 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
           __syncwarp();
           if (lane == 0) mbar_arrive(&acce[b]);
         }
-        float sum[32];
 #pragma unroll
-        for (int j = 0; j < 32; j++) sum[j] = old[j] + (x.nk > 0 ? v[j] : 0.f);
-        if (q + 1 < BN / 64) load_old(q + 1);
-        if (rho < mvalid) {
+        for (int j = 0; j < 32; j++) v[j] = old[j] + (x.nk > 0 ? v[j] : 0.f);
+        if (accumulate && q + 1 < BN / 64) load_old(q + 1);
+        float *p = row + ldcf * (int64_t)(32 * q);
 #pragma unroll
-          for (int j = 0; j < 32; j++) {
-            const int c = c0 + 32 * q + j;
-            if (c < nvalid) C[rho + ldcf * (int64_t)c] = sum[j];
-          }
-        }
+        for (int j = 0; j < 32; j++, p += ldcf)
+          if (32 * q + j < cols) *p = v[j];
       }
     }
   }
@@ -548,18 +551,20 @@ void bem_cgemm_tc_bytes(int m, int n, int k, size_t &a_bytes, size_t &b_bytes) {
 
 namespace {
 
-// Tile width: the persistent CTAs' rounds, a K element of a round taking 0.75 (128 x 64), 1
-// (128 x 128) or 1.65 (128 x 256: n x n x n products of several rounds), and the filling of
-// the pipeline and the last epilogue, which nothing hides, as long as 8 K elements a
-// column.  Measured in us (128 x 64, 128, 256): 576^3 20, 26, 49; 1152 x 1152 x 128 18, 20,
-// 25; 1152^3 84, 78, 83; 2048 x 2048 x 256 53, 46, 52; 4001 x 2003 x 4001 1194, 933, 870;
-// 7680 x 7680 x 256 611, 482, 443.
+// Tile width: the one whose rounds of the persistent CTAs take least.  A round takes its K
+// elements times 0.67 (128 x 64), 1 (128 x 128) or 1.63 (128 x 256), and as long as 50, 65 or
+// 210 more for what nothing hides of the pipeline's filling and the epilogue: fitted to 60
+// shapes from 64^3 to 7680 x 3840 x 7680, the choice is within 1.2 % of the best of the three
+// on each.  (With one such time for all rounds together, products of few K elements took two
+// rounds of 64 columns where one of 128 is faster: 1500 x 700 x 300 19.4 us for 16.2.)
+// Measured in us (128 x 64, 128, 256): 576^3 17, 23, 36; 1152 x 1152 x 128 15, 15, 14; 1152^3 79, 73,
+// 66; 1219 x 3826 x 99 32, 26, 26; 4001 x 2003 x 4001 1193, 932, 858; 7680 x 7680 x 256 585, 443, 390.
 int tc_tile_n(const bemgpu_ctx_s *ctx, int64_t nM, int n, int64_t Kp) {
-  auto cost = [&](int bn, double c) {
+  auto cost = [&](int bn, double c, double e) {
     const int64_t tiles = nM * ((n + bn - 1) / bn);
-    return c * (double)(Kp * ((tiles + ctx->num_sms - 1) / ctx->num_sms)) + 8.0 * bn;
+    return (double)((tiles + ctx->num_sms - 1) / ctx->num_sms) * (c * (double)Kp + e);
   };
-  const double c64 = cost(64, 0.75), c128 = cost(128, 1.0), c256 = cost(256, 1.65);
+  const double c64 = cost(64, 0.67, 50.0), c128 = cost(128, 1.0, 65.0), c256 = cost(256, 1.63, 210.0);
   return c256 < c128 && c256 < c64 ? 256 : c128 < c64 ? 128 : 64;
 }
 
