@@ -127,6 +127,7 @@ __device__ __forceinline__ void ex_store8(double *C, int64_t ldcf, int c, int nv
   for (int j = 0; j < 8; j++) old[j] = accumulate && c + j < nvalid ? C[ldcf * (int64_t)(c + j)] : 0.0;
 #pragma unroll
   for (int j = 0; j < 8; j += 2) {
+    if (c + j >= nvalid) break;  // the FP64 pipe bounds this: nothing for columns that are not there
     double v[2];
     f2_sum(hi[j / 2], lo[j / 2], v[0], v[1]);
 #pragma unroll
@@ -544,16 +545,18 @@ __global__ void __launch_bounds__(EXW_THREADS, 1)
     if (ok) asm volatile("tcgen05.fence::after_thread_sync;");
 #pragma unroll
     for (int c = 0; c < CW / 8; c++) {
+      constexpr bool TWO = SUMS > ZLEV + 1;  // levels ZLEV and ZLEV + 1 in a sum each
       float z[8], z4[8];
 #pragma unroll
       for (int j = 0; j < 8; j++) z[j] = z4[j] = 0.f;
       if (ok) {
         tc_ld8(lane_base + (uint32_t)(ZLEV * BN + 8 * c), z);
-        if (SUMS > ZLEV + 1) tc_ld8(lane_base + (uint32_t)((ZLEV + 1) * BN + 8 * c), z4);
+        if (TWO) tc_ld8(lane_base + (uint32_t)((ZLEV + 1) * BN + 8 * c), z4);
       }
       if (ok && rho < mvalid) {
 #pragma unroll
         for (int j = 0; j < 8; j += 2) {
+          if (n0 + group * CW + 8 * c + j >= nvalid) break;
           double v[2];
           f2_sum(hi[4 * c + j / 2], lo[4 * c + j / 2], v[0], v[1]);
 #pragma unroll
@@ -561,7 +564,9 @@ __global__ void __launch_bounds__(EXW_THREADS, 1)
             const int col = n0 + group * CW + 8 * c + j + e;
             if (col < nvalid) {
               double *p = C + rho + ldcf * (int64_t)col;
-              const double w = scale * (v[e] + ((double)z[j + e] + (double)z4[j + e]));
+              // (an addition of zero would stay: the FP64 pipe bounds products of one block)
+              const double zz = TWO ? (double)z[j + e] + (double)z4[j + e] : (double)z[j + e];
+              const double w = scale * (v[e] + zz);
               *p = accumulate ? *p + w : w;
             }
           }
