@@ -201,10 +201,9 @@ __device__ __forceinline__ void wave_at(const GreenT<T> &g, T R, T &er, T &ei, T
     return;
   }
   const T a = g.ikr * R;
-  if (N::head(a) < -85) {  // below FP32's range: e^-85 of the neighbouring nodes' size
-    const T z = N::of(0.0);
-    er = ei = ur = ui = z;
-    em = N::LESS ? -th : z;
+  if (N::LESS && N::head(a) < -85) {  // double-float, below FP32's range: e^-85 of the neighbouring nodes' size
+    er = ei = ur = ui = N::of(0.0);
+    em = -th;
     return;
   }
   T m1;
