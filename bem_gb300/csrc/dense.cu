@@ -640,15 +640,13 @@ __device__ __forceinline__ void cp_reduce(unsigned &hi, unsigned &lo, unsigned &
   pos = __reduce_min_sync(0xffffffffu, in ? pos : 0xffffffffu);
 }
 
-// 1/a by one division; the plain form where |a|^2 leaves the range in which its
-// reciprocal is a normal number.
+// crecip(a) by a whole warp: one division for both parts, the even lanes' and the odd
+// lanes'.
 template <typename T>
-__device__ __forceinline__ cx<T> cp_recip(cx<T> a) {
+__device__ __forceinline__ cx<T> cp_recip(cx<T> a, int lane) {
   const T d = a.r * a.r + a.i * a.i;
-  const T small = sizeof(T) == 8 ? T(1e-290) : T(1e-30);
-  if (!(d > small && d < T(1) / small)) return crecip(a);
-  const T q = T(1) / d;
-  return {a.r * q, -a.i * q};
+  const T q = (lane & 1 ? -a.i : a.r) / d;
+  return {__shfl_sync(0xffffffffu, q, 0), __shfl_sync(0xffffffffu, q, 1)};
 }
 
 template <typename T, int SW, int RPT>
@@ -762,7 +760,7 @@ __global__ void __launch_bounds__(CP_MAX_THREADS, 1)
       if (sizeof(T) == 8) reinterpret_cast<unsigned *>(&h)[0] = lo;
       h.key = who ? hi : 0u;
       h.pos = cp;
-      const cx<T> rp = who && (hi | lo) ? cp_recip(cx<T>{pv.x, pv.y}) : cx<T>{0, 0};
+      const cx<T> rp = who && (hi | lo) ? cp_recip(cx<T>{pv.x, pv.y}, lane) : cx<T>{0, 0};  // (warp-uniform)
       h.rr = rp.r;
       h.ri = rp.i;
       __syncwarp();

@@ -98,3 +98,20 @@ def test_first_of_equals(how, power):
     assert np.array_equal(ipiv, np.arange(n))
     want = r[:, None] * (Lf - np.eye(n)) / r[None, :] + r[:, None] * U
     assert torch.equal(got, _dense(sp.coo_matrix(want), got.dtype))
+
+
+@pytest.mark.parametrize("how", ["c", "z", "zexact"])
+def test_pivot_reciprocals_are_rounded_twice(how):
+    """2 x 2 blocks [[p, 0], [1, 1]] with p real or imaginary: the multiplier is 1/p as p / |p|^2
+    gives it, the square rounded once and the division once."""
+    n, real = 512, np.float32 if how == "c" else np.float64
+    rng = np.random.default_rng(11)
+    p = np.exp(rng.uniform(0.1, 9.0, n // 2)).astype(real)
+    turn = UNITS[rng.integers(0, 4, n // 2)]
+    i = np.arange(0, n, 2)
+    A = sp.coo_matrix((np.concatenate([p * turn, np.ones(n)]),
+                       (np.concatenate([i, i + 1, i + 1]), np.concatenate([i, i, i + 1]))), shape=(n, n))
+    got, ipiv, info = _factor(how, A)
+    assert info == 0 and np.array_equal(ipiv, np.arange(n))
+    want = (p / (p * p)).astype(np.float64) * turn.conj()
+    assert np.array_equal(got.cpu().numpy().T[i + 1, i], want)
