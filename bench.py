@@ -649,7 +649,8 @@ def group_roofline(dom, stats, precision, pk, pk_kind, fp64class=False, sm_mhz=N
                     note="the fill is FP64-class arithmetic in double-float on the FP32 pipes: its algorithmic "
                          "FP64-class flops (frozen count, live) per CUDA-event second times the FP32-pipe "
                          "thread instructions per algorithmic flop that ncu counted on each fill kernel "
-                         "(smsp__inst_executed, one solve of N = 7680)")
+                         "(smsp__inst_executed, one solve of N = 7680 whose near pairs all run as series; direct "
+                         "ones take more, so there the fraction is a lower bound)")
     if bound == "tensor":
         if dom == "ex_gemm":
             base["traffic"] = EX_TRAFFIC_PER_MODEL_BYTE * by / max(1, n)
@@ -885,10 +886,57 @@ SUB_KEYS = ("value", "unit", "ms_per_step", "steps", "config", "err_est", "facto
             "fp64_path", "accuracy", "mixed_over_fp64", "clocks", "gpu_launches", "fill_gentries_per_s", "tiles")
 
 
+def compact(out):
+    """The line without what a log's tail has no room for (--full keeps it): lists of one
+    entry per solve as their largest, notes, and all but the figures of the sub-workloads
+    and of the kernel groups."""
+    def short(v):
+        if isinstance(v, float):
+            return float(f"{v:.4g}")
+        if isinstance(v, dict):
+            return {k: short(x) for k, x in v.items() if "note" not in k and k != "traffic_source"}
+        return v
+
+    def largest(d):
+        return {(k + "_max" if isinstance(v, list) and k != "reasons" else k):
+                (max(v, default=None) if isinstance(v, list) and k != "reasons" else v) for k, v in d.items()}
+
+    line = largest({k: v for k, v in out.items() if "note" not in k and k not in
+                    ("P_sample", "rooflines", "subs", "cpu_baseline", "fill_write_gbs", "gather_gbs")})
+    if line.get("serving"):
+        line["serving"] = {k: line["serving"][k] for k in ("requests", "p50_ms", "p99_ms", "solves_per_s")}
+    if "fp64_path" in out:
+        line["fp64_path"] = {k: out["fp64_path"][k] for k in ("value", "steps")}
+    if "kernel_ms_per_step" in out:
+        line["kernel_ms_per_step"] = {k: v for k, v in out["kernel_ms_per_step"].items() if v}
+    if "accuracy" in out:
+        line["accuracy"] = {k: out["accuracy"][k] for k in ("err_vs_fp64_max", "solves_checked")}
+    if "rooflines" in out:
+        line["rooflines"] = {g: {k: r[k] for k in (("executed_frac" if "executed_frac" in r else "frac"), "ms_share")}
+                             for g, r in out["rooflines"].items()}
+    if "roofline" in out:
+        line["roofline"] = {k: v for k, v in out["roofline"].items()
+                            if k not in ("kinds", "traffic_algorithmic", "slice_products_per_mac")}
+    if "cpu_baseline" in out:
+        line["cpu_baseline"] = {k: out["cpu_baseline"][k] for k in ("value", "cores", "kind")}
+    if "subs" in out:
+        line["subs"] = {}
+        for nm, d in out["subs"].items():
+            sub = {k: d[k] for k in ("failed", "value", "mixed_over_fp64") if k in d}
+            if "config" in d:
+                sub["N"] = d["config"]["N"]
+                sub["factorizations"] = list(d["factorization"].values())
+            if "accuracy" in d:
+                sub["err_vs_fp64_max"] = d["accuracy"]["err_vs_fp64_max"]
+            line["subs"][nm] = sub
+    exact = {k: out[k] for k in ("value", "ms_per_step", "clocks", "e2e") if k in out}
+    return {**{k: short(v) for k, v in line.items()}, **exact}
+
+
 def run_subs(names):
     out = {}
     for nm in names:
-        cmd = [sys.executable, os.path.abspath(__file__), *SUBS[nm], "--no-cpu-baseline", "--subs", "none"]
+        cmd = [sys.executable, os.path.abspath(__file__), *SUBS[nm], "--no-cpu-baseline", "--subs", "none", "--full"]
         t0 = time.perf_counter()
         r = subprocess.run(cmd, capture_output=True, text=True)
         wall = time.perf_counter() - t0
@@ -942,6 +990,9 @@ def main():
                     help="CTAs of an LU panel at most (0: the library's choice)")
     ap.add_argument("--lite", action="store_true",
                     help="skip the end-to-end and per-kernel segments (sub-workload runs)")
+    ap.add_argument("--full", action="store_true",
+                    help="every field in the line (each solve's error estimate, notes, all of the sub-workloads' "
+                         "figures); without it the line keeps to a few kilobytes")
     args = ap.parse_args()
     rank, world, local = env_rank()
     if world > 1 and args.impl == "ours":
@@ -961,7 +1012,7 @@ def main():
             r = cpu_baseline_run(args.workload, CPU_BASELINE_STEPS)
             out["cpu_baseline"] = {"value": r["value"], "unit": "solves/s", "cores": r["cores"], "kind": "port",
                                    "sample": r["sample"], "spread": r["spread"]}
-        print(json.dumps(out))
+        print(json.dumps(out if args.full else compact(out)))
     if world > 1:
         import torch.distributed as dist
         dist.destroy_process_group()
