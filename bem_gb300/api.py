@@ -305,9 +305,8 @@ def CalcHeatTransfer(a: float, eV: float, T1: float, T2: float, top: RWGTree, s:
 def CalcHeatTransferBatch(jobs, options: Options | None = None, precision: int = _lib.PREC_FP64,
                           infos: list | None = None, strict: bool = True) -> list:
     """CalcHeatTransfer for several (a, eV, T1, T2, top, s, t) at once
-    (bemgpu_heat_transfer_batch): one fill launch pair for all of them and,
-    for requests of equal size, one cooperative LU panel launch per block
-    column.  The results equal CalcHeatTransfer's one by one, bit for bit."""
+    (bemgpu_heat_transfer_batch): grouped fill launches for all of them and,
+    for requests of equal size, their LU panels in the same launches.  The results equal CalcHeatTransfer's one by one, bit for bit."""
     options = options or Options()
     jobs = list(jobs)
     n = len(jobs)

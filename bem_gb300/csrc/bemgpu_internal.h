@@ -104,7 +104,7 @@ struct bemgpu_ctx_s {
   bool ex_ready = false;      // gemm_exact.cu kernels: shared-memory attribute set
   bool perm_ready = false;    // dense.cu perm_from_ipiv_kernel: shared-memory attribute set
   bool tc_err_ready = false;  // tensor-core pipeline error flag zeroed
-  bool coop_panel = true;  // LU panels in one cooperative launch (else one launch per column)
+  bool coop_panel = true;  // LU panels by clusters or cooperative grids (else one launch per column)
   int gemm_engine = 0;   // complex64 LU/solve GEMMs: 0 tensor cores where possible, 2 FMA pipes only
   int acc_engine = 0;    // residual/trace GEMMs with FP64 output: same choices
   int solver = 0;        // mixed path: 0 complex64 with FP64-class escalation, 1 complex64, 2 FP64-class
@@ -244,7 +244,7 @@ int bem_zgetrs_exact(bemgpu_ctx_s *ctx, const double *A, int64_t lda, int n, con
 // complex64 versions (mixed path).
 int bem_cgetrf(bemgpu_ctx_s *ctx, float *A, int64_t lda, int n, int *d_ipiv, int *d_info, cudaStream_t stream);
 // The same for nb matrices A + i strideA (pivots d_ipiv + i n, info d_info + i),
-// their panels factored together in one cooperative launch.
+// their panels factored together in the same launches.
 int bem_cgetrf_batch(bemgpu_ctx_s *ctx, float *A, int64_t strideA, int nb, int64_t lda, int n, int *d_ipiv,
                      int *d_info, cudaStream_t stream);
 int bem_cgetrs(bemgpu_ctx_s *ctx, const float *A, int64_t lda, int n, const int *d_ipiv, float *B, int64_t ldb,

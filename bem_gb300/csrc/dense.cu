@@ -1639,9 +1639,9 @@ bool panel_cluster(bemgpu_ctx_s *ctx, T *A, int64_t lda, int n, int k0, int w, i
 }
 
 // LU with partial pivoting of nb equal-size matrices A + i strideA (pivots
-// d_ipiv + i n, info d_info + i): every panel of the batch in one cooperative
-// launch (each matrix with its own CTAs and barrier), the interchanges,
-// triangular blocks and trailing updates per matrix.  Each matrix gets the
+// d_ipiv + i n, info d_info + i): every panel of the batch in the same launches (a
+// cluster, or its own CTAs and barrier in a cooperative grid, for each matrix), the
+// interchanges, triangular blocks and trailing updates per matrix.  Each matrix gets the
 // arithmetic of a batch of one.
 template <typename T>
 int getrf_impl(bemgpu_ctx_s *ctx, T *A0, int64_t lda, int n, int *d_ipiv0, int *d_info0, cudaStream_t stream,
@@ -1831,7 +1831,7 @@ int exact_mul(bemgpu_ctx_s *ctx, int kind, const double *Ablk, int64_t lda, int 
 }  // namespace
 
 // FP64-class LU on the tensor cores, blocked twice: 512-column super-panels
-// are factored by 64-column cooperative panels whose updates stay inside the
+// are factored by 64-column panels whose updates stay inside the
 // super-panel; then the super-panel's pivots are applied to the other
 // columns, U12 = L11^{-1} A12 with the inverse of the 512 x 512 unit-lower
 // diagonal block, and A22 -= A21 U12 as one K = 512 exact product.  The

@@ -878,7 +878,6 @@ int bem_exact_gemm(bemgpu_ctx_s *ctx, int kind, const ExactOperand &a, const Exa
   const int m = a.rows, n = b.rows, SB = b.slices, SA = b.exact ? a.slices : b.slices;
   if (!((SA == SB && SA >= 3 && SA <= 5) || (SA == 5 && (SB == 3 || SB == 2))))
     return bem_fail(ctx, BEMGPU_ERR_ARG, "exact gemm: slices (%d, %d) not built", SA, SB);
-  const int SL = SB;
   // Wide tiles.  Plain 5 x 5 (128 x 96, the same sums as 128 x 64): where they take less
   // time by their waves, a wide tile taking 1.2 times a narrow one (n = 7680: 33.8 ms
   // against 41.5; n = 1440, 3 waves against 4: 379 us against 410).  The others
@@ -934,7 +933,6 @@ int bem_exact_gemm(bemgpu_ctx_s *ctx, int kind, const ExactOperand &a, const Exa
   ProfScope ps(ctx, kind, st, 8.0 * m * (double)n * a.k,
                2.0 * SA * ((double)a.rows_p * a.kp * ((b.rows + bn - 1) / bn) / 8.0) +
                    2.0 * SB * (double)b.rows_p * b.kp + 16.0 * m * (double)n * (accumulate ? 2 : 1));
-  (void)SL;
   {
     // slice products (a, b) with a < SA, b < SB, a + b < SA
     int products = 0;

@@ -18,9 +18,9 @@ def two(val):
     return hi, float(sp.N(val - sp.Rational(hi), 50))
 
 
-def four(val, bits=(16, 16, 16, 24)):
-    """FP32 Cody-Waite parts: the first three carry 16 significant bits, so that
-    n * part is exact for integers |n| < 2^8; the fourth carries 24."""
+def three(val, bits=(16, 16, 16)):
+    """FP32 Cody-Waite parts of 16 significant bits, so that n * part is exact for
+    integers |n| < 2^8."""
     rem, out = sp.N(val, 80), []
     for b in bits:
         x = float(rem)
@@ -33,7 +33,6 @@ def four(val, bits=(16, 16, 16, 24)):
 
 
 pio2 = two(sp.pi / 2)
-ln2 = two(sp.log(2))
 lines = ["// Generated by gen_df_constants.py (exact values from sympy); do not edit.", "#pragma once", "",
          f"#define DF_NFACT {N}",
          "// 1/n! = DF_FACT_HI[n] + DF_FACT_LO[n] (FP32 parts)",
@@ -41,10 +40,8 @@ lines = ["// Generated by gen_df_constants.py (exact values from sympy); do not 
          "static __constant__ const float DF_FACT_LO[DF_NFACT] = {" + ", ".join(f"{x!r}f" for x in L) + "};",
          f"#define DF_PIO2_HI {pio2[0]!r}", f"#define DF_PIO2_LO {pio2[1]!r}",
          f"#define DF_TWO_OVER_PI {float(sp.N(2 / sp.pi, 50))!r}",
-         f"#define DF_LN2_HI {ln2[0]!r}", f"#define DF_LN2_LO {ln2[1]!r}",
-         f"#define DF_LOG2E {float(sp.N(1 / sp.log(2), 50))!r}",
-         "// FP32 Cody-Waite parts of pi/2 and ln 2 (n * part exact for |n| < 2^8 in the first three)"]
-for nm, parts in (("DF_PIO2_F", four(sp.pi / 2)), ("DF_LN2_F", four(sp.log(2)))):
+         "// FP32 Cody-Waite parts of pi/2 and ln 2 (n * part exact for |n| < 2^8)"]
+for nm, parts in (("DF_PIO2_F", three(sp.pi / 2)), ("DF_LN2_F", three(sp.log(2)))):
     for i, x in enumerate(parts):
         lines.append(f"#define {nm}{i} {x!r}f")
 lines += [f"#define DF_TWO_OVER_PI_F {float(np.float32(float(sp.N(2 / sp.pi, 30))))!r}f",

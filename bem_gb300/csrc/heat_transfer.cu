@@ -446,7 +446,7 @@ extern "C" int bemgpu_heat_transfer_batch(bemgpu_ctx_t ctx, int nreq, const bemg
     release_fill_if_short(ctx, need, fill, {"bH"});
   }
   // the complex64 LU of equal-size requests together: their panels in one
-  // cooperative launch per block column
+  // sequence of panel launches
   std::vector<MixedLU> pre;
   if (precision != BEMGPU_PREC_FP64 && ctx->solver != 2 && same && nreq > 1) {
     const int n = r[0].n;

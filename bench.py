@@ -671,7 +671,7 @@ def group_roofline(dom, stats, precision, pk, pk_kind, fp64class=False, sm_mhz=N
     out = dict(base, bound="hbm", achieved=ach, peak=pk["hbm_gbs"], unit="GB/s", frac=ach / pk["hbm_gbs"],
                peak_source=pk_kind)
     if bound == "latency":
-        out["note"] = "latency-bound: one grid barrier per matrix column (cooperative panel); bytes are the panel's"
+        out["note"] = "latency-bound: one exchange of a cluster's CTAs per matrix column; bytes are the panel's"
     return out
 
 

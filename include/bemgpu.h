@@ -329,9 +329,10 @@ int bemgpu_heat_transfer(bemgpu_ctx_t ctx, bemgpu_tree_t top, bemgpu_tree_t s, b
 /* Several CalcHeatTransfer requests solved together (no counterpart in the
  * reference, whose task farm solves one per process): request i is
  * (tops[i], ss[i], ts[i], reqs[i]).  The three fills of every request run in
- * one far-pair and one near-pair launch; the complex64 LU panels of requests
- * of equal size (a frequency sweep of one geometry) run in one cooperative
- * launch per block column; the rest is per request.  P_out[i] and infos[i]
+ * one far-pair launch and at most three near-pair launches (one for each way
+ * that |k| R selects); the complex64 LU panels of requests of equal size (a
+ * frequency sweep of one geometry) run in the same launches, a thread-block
+ * cluster each (a cooperative grid beyond 16384 rows); the rest is per request.  P_out[i] and infos[i]
  * (infos may be NULL; its ms_fill is the batch's fill time / nreq) equal
  * bemgpu_heat_transfer's for the same request bit for bit, and status[i] is
  * its status.  Returns the first non-zero status (BEMGPU_OK when all
